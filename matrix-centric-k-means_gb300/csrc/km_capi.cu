@@ -458,7 +458,7 @@ km_status km_update(const float* X_dev, const uint32_t* labels_dev, uint64_t n, 
   KM_TRY(e.enqueue_sort(labels_dev));
   KM_TRY(e.check_device_error());   // labels >= k are rejected before the sums run
   KM_TRY(launch_update_sums(X_dev, e.perm, e.cstart, d, k, nullptr, C_dev, nullptr, nullptr, e.st,
-                            e.stream));
+                            e.stream, k <= 1024u ? e.order : nullptr));
   if (counts_dev) KM_CUDA_TRY(cudaMemcpyAsync(counts_dev, e.counts, sizeof(uint32_t) * k, cudaMemcpyDeviceToDevice, e.stream));
   if (perm_dev) KM_CUDA_TRY(cudaMemcpyAsync(perm_dev, e.perm, sizeof(uint32_t) * n, cudaMemcpyDeviceToDevice, e.stream));
   if (offsets_dev) KM_CUDA_TRY(cudaMemcpyAsync(offsets_dev, e.cstart, sizeof(uint32_t) * (k + 1), cudaMemcpyDeviceToDevice, e.stream));

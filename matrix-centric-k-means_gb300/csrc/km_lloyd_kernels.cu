@@ -1169,187 +1169,84 @@ __global__ void seg_scatter_kernel(const uint32_t* __restrict__ labels, uint64_t
 }
 
 // ---------------------------------------------------------------------------
-// (c) Exact centroid update V.X.  One warp per (cluster, 32*VEC-column chunk),
-// each lane on VEC adjacent columns: the cluster's rows are visited in
-// ascending index order (the label-sorted permutation) and summed in float
-// exactly as the reference's CPU loop (kmeans.cpp:133-137).  Row segments are
-// gathered with cp.async (16 bytes per lane for VEC = 4, 4 bytes for VEC = 1,
-// zero-filled past d) into a per-warp ring of UPD_STAGES batches of UPD_ROWS
-// rows, so that three batches are in flight while the ordered additions consume
-// the fourth; the permutation indices of a batch come in with one coalesced
-// load and are broadcast by shuffles.  Also: squared move per element for the
-// shift test and the FP64 objective of this iteration's assignment against the
-// centroids that produced it (FP32 partials per batch, FP64 above).
+// (c) Exact centroid update V.X: the cluster's rows are visited in ascending
+// index order (the label-sorted permutation) and every column is summed in
+// float exactly as the reference's CPU loop (kmeans.cpp:133-137).  Also: the
+// squared move per element for the shift test and the objective of this
+// iteration's assignment against the centroids that produced it.
+//
+// One CTA per (cluster, 32-column block), so a cluster's d/32 column chains run
+// on as many SMs.  Producer warp p of blk_producers(VEC) fills batches
+// p, p + PROD, ... with VEC-column cp.async per lane into a BLK_STAGES-deep ring;
+// arrival on the stage's mbarrier fires when its copies land
+// (cp.async.mbarrier.arrive.noinc).  VEC is the widest copy that the row starts
+// allow (4, 2 or 1 columns: 16, 8 or 4 bytes); the ring and the consumers are the
+// same.  Two consumer warps: one holds the ordered chain alone, one the
+// objective.
+//
+// Bounds: the chain of the largest cluster, then HBM.  A dependent FP32 addition
+// takes 4.1 cycles and 4.6 with a shared-memory load beside it (5.6 when the loads
+// stand in front of the additions), so the chain warp does nothing else; the
+// objective warp takes 16-byte loads and packed FP32 pairs, a third of the
+// instructions of one load and two operations a row.  Measured: a cluster alone
+// 177 -> 322 rows/us (39 -> 263 / 173 for 8- / 4-byte rows, which one warp per 32
+// columns gathered and summed before), n = 1M d = 128 k = 256 with 20,473 rows in
+// the largest cluster 135 -> 105 us = 5.16 TB/s, n = 300,007 d = 50 k = 37
+// 447 -> 72 us.  TMA row gathers (tile::gather4) were slower: 119 rows/us.
+//
+// Every wait is bounded; on timeout the CTA flags KM_DEVERR_TIMEOUT and drains
+// its copies before exiting.  Permutation indices are prefetched P batches ahead
+// in registers consumed in place.  A batch is BLK_ROWS = 128 rows (four groups of
+// 32): every batch costs a consumer one wait and one release of fixed latency.
+// BLK_STAGES is a multiple of the producers, so a stage is always refilled by the
+// same producer, which waits on its phases in order (a parity wait can never alias
+// a later phase).
 // ---------------------------------------------------------------------------
 namespace {
-constexpr int UPD_ROWS = 32, UPD_STAGES = 8;
+constexpr int BLK_ROWS = 128, BLK_GRP = 32, BLK_STAGES = 6, BLK_COLS = 32;
+// Producer warps by copy width: narrower copies take two or four times the
+// instructions, so six warps issue them.  Measured, one cluster of 100,000 rows:
+// 16 bytes 322 rows/us with two, three or six producers (the chain's rate), 8
+// bytes 212 with three and 263 with six, 4 bytes 113 and 173.
+constexpr int blk_producers(int vec) { return vec == 4 ? 3 : 6; }
+static_assert(BLK_ROWS == 4 * BLK_GRP, "the chain warp alternates two register groups over four groups a batch");
+constexpr uint64_t BLK_WAIT_NS = 2000000000ull;
+constexpr uint32_t BLK_SUSPEND_NS = 2000;       // try_wait suspend hint
+constexpr size_t BLK_SMEM = (size_t)BLK_STAGES * BLK_ROWS * BLK_COLS * sizeof(float);
+constexpr int blk_threads(int vec) { return 32 * (blk_producers(vec) + 2); }
 
-__device__ __forceinline__ void cp_async_16(void* smem, const void* gmem, uint32_t src_bytes) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_u32(smem)), "l"(gmem),
-               "r"(src_bytes)
-               : "memory");
+// An ordered shared-memory load (kept beside the arithmetic that follows it).
+__device__ __forceinline__ float ld_shared_f32(uint32_t addr) {
+  float v;
+  asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(addr));
+  return v;
 }
-__device__ __forceinline__ void cp_async_4(void* smem, const void* gmem, uint32_t src_bytes) {
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(smem_u32(smem)), "l"(gmem),
-               "r"(src_bytes)
-               : "memory");
+
+// VEC columns (4 * VEC bytes, aligned to their size), zero-filled when !ok.
+template <int VEC>
+__device__ __forceinline__ void cp_async_cols(void* smem, const float* gmem, bool ok) {
+  const uint32_t bytes = ok ? 4u * VEC : 0u;
+  if constexpr (VEC == 4) {
+    cp_async16_zfill(smem, gmem, bytes);
+  } else if constexpr (VEC == 2) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(smem_u32(smem)), "l"(gmem), "r"(bytes)
+                 : "memory");
+  } else {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(smem_u32(smem)), "l"(gmem), "r"(bytes)
+                 : "memory");
+  }
 }
 }  // namespace
 
 template <int VEC>
-__global__ void __launch_bounds__(32)
-update_sums_kernel(const float* __restrict__ X, const uint32_t* __restrict__ perm,
-                   const uint32_t* __restrict__ cstart, uint32_t d, uint32_t k,
-                   const float* __restrict__ C, float* __restrict__ Cn,
-                   float* __restrict__ dsq, double* __restrict__ objpart, DevState* st) {
-  griddep_wait();
-  if (st && st->done) return;
-  extern __shared__ __align__(128) float ring[];   // [UPD_STAGES][UPD_ROWS][32 * VEC]
-  constexpr uint32_t W = 32u * VEC;
-  const uint32_t nchunk = (d + W - 1) / W;
-  const uint64_t gw = blockIdx.x;
-  if (gw >= (uint64_t)k * nchunk) return;
-  const int lane = threadIdx.x & 31;
-  const uint32_t c = (uint32_t)(gw / nchunk);
-  const uint32_t j0 = (uint32_t)(gw % nchunk) * W + (uint32_t)lane * VEC;
-  const uint32_t s0 = cstart[c], s1 = cstart[c + 1];
-  const uint32_t nb = (s1 - s0 + UPD_ROWS - 1) / UPD_ROWS;
-  float cold[VEC], sum[VEC];
-  double e64[VEC];
-#pragma unroll
-  for (int q = 0; q < VEC; ++q) {
-    cold[q] = (C && j0 + q < d) ? C[(uint64_t)c * d + j0 + q] : 0.0f;
-    sum[q] = 0.0f;
-    e64[q] = 0.0;
-  }
-  // Permutation index of this lane's row in batch b (loaded one batch ahead of
-  // its use so that the gather issue never waits on it).
-  auto load_perm = [&](uint32_t b) -> uint32_t {
-    const uint32_t i = s0 + b * UPD_ROWS + (uint32_t)lane;
-    return (b < nb && i < s1) ? perm[i] : 0u;
-  };
-  auto issue = [&](uint32_t b, uint32_t rl) {
-    if (b < nb) {
-      const uint32_t base = s0 + b * UPD_ROWS;
-      const uint32_t m = min((uint32_t)UPD_ROWS, s1 - base);
-      float* dst = ring + (size_t)(b % UPD_STAGES) * UPD_ROWS * W + (uint32_t)lane * VEC;
-#pragma unroll 8
-      for (int u = 0; u < UPD_ROWS; ++u) {
-        const uint32_t r = __shfl_sync(0xffffffffu, rl, u);
-        const bool ok = (uint32_t)u < m && j0 < d;
-        const float* src = ok ? X + (uint64_t)r * d + j0 : X;
-        if constexpr (VEC == 4) cp_async_16(dst + (size_t)u * W, src, ok ? 16u : 0u);
-        else cp_async_4(dst + (size_t)u * W, src, ok ? 4u : 0u);
-      }
-    }
-    cp_async_commit();
-  };
-  {
-    uint32_t p0[UPD_STAGES - 1];
-#pragma unroll
-    for (int b = 0; b < UPD_STAGES - 1; ++b) p0[b] = load_perm((uint32_t)b);
-#pragma unroll
-    for (int b = 0; b < UPD_STAGES - 1; ++b) issue((uint32_t)b, p0[b]);
-  }
-  // pq[i] holds the permutation indices of batch b + UPD_STAGES - 1 + i: the
-  // load of a batch's indices is issued UPD_PREFETCH iterations before use.
-  // The loop is unrolled by UPD_PREFETCH so that pq[i] is consumed in place,
-  // UPD_PREFETCH batches after its load was issued.
-  constexpr int UPD_PREFETCH = 8;
-  uint32_t pq[UPD_PREFETCH];
-#pragma unroll
-  for (int i = 0; i < UPD_PREFETCH; ++i) pq[i] = load_perm((uint32_t)(UPD_STAGES - 1 + i));
-  for (uint32_t b0 = 0; b0 < nb; b0 += UPD_PREFETCH)
-#pragma unroll
-  for (int i = 0; i < UPD_PREFETCH; ++i) {
-    const uint32_t b = b0 + (uint32_t)i;
-    if (b >= nb) break;
-    issue(b + UPD_STAGES - 1, pq[i]);
-    pq[i] = load_perm(b + UPD_STAGES - 1 + UPD_PREFETCH);
-    cp_async_wait<UPD_STAGES - 1>();
-    __syncwarp();
-    const uint32_t m = min((uint32_t)UPD_ROWS, s1 - (s0 + b * UPD_ROWS));
-    const float* src = ring + (size_t)(b % UPD_STAGES) * UPD_ROWS * W + (uint32_t)lane * VEC;
-    float e32[VEC];
-#pragma unroll
-    for (int q = 0; q < VEC; ++q) e32[q] = 0.0f;
-#pragma unroll 8
-    for (int u = 0; u < UPD_ROWS; ++u) {
-      if ((uint32_t)u < m) {
-        float v[VEC];
-        if constexpr (VEC == 4) {
-          const float4 f = *reinterpret_cast<const float4*>(src + (size_t)u * W);
-          v[0] = f.x; v[1] = f.y; v[2] = f.z; v[3] = f.w;
-        } else {
-          v[0] = src[(size_t)u * W];
-        }
-#pragma unroll
-        for (int q = 0; q < VEC; ++q) {
-          sum[q] = __fadd_rn(sum[q], v[q]);
-          const float t = v[q] - cold[q];
-          e32[q] = fmaf(t, t, e32[q]);
-        }
-      }
-    }
-#pragma unroll
-    for (int q = 0; q < VEC; ++q) e64[q] += e32[q];
-    __syncwarp();
-  }
-  cp_async_wait<0>();
-  const uint32_t cnt = s1 - s0;
-  const float scale = __double2float_rn(1.0 / (double)(cnt > 1 ? cnt : 1));
-#pragma unroll
-  for (int q = 0; q < VEC; ++q) {
-    if (j0 + q >= d) break;
-    const uint64_t p = (uint64_t)c * d + j0 + q;
-    const float cn = __fmul_rn(sum[q], scale);
-    Cn[p] = cn;
-    if (dsq) {
-      const float t = __fsub_rn(cn, cold[q]);
-      dsq[p] = __fmul_rn(t, t);
-    }
-    if (objpart) objpart[p] = e64[q];
-  }
-}
-
-// Pipelined variant (d % 4 == 0, 16-byte aligned X): one CTA per (cluster,
-// 32-column block), so a cluster's d/32 column chains run on as many SMs.
-// Warps 0..BLK_PROD-1 produce: producer p fills batches p, p + BLK_PROD, ...
-// with 16-byte cp.async per lane (one instruction copies BLK_RPI row segments)
-// into a BLK_STAGES-deep ring; arrival on the stage's mbarrier fires when its
-// copies land (cp.async.mbarrier.arrive.noinc).  A single producer warp caps a
-// CTA at about half the row rate of three.  Warp BLK_PROD consumes, lane =
-// column: a full batch is loaded into registers first, then summed in row
-// order exactly as the reference (kmeans.cpp:133-137).  The objective term is
-// summed per batch in FP32 and across batches as an unevaluated FP32 pair
-// (TwoSum), which keeps FP64-level accuracy without a loop-carried FP64 add
-// (a long-latency operation on this GPU).  Every wait is bounded; on timeout
-// the CTA flags KM_DEVERR_TIMEOUT and drains its copies before exiting.
-// Permutation indices are prefetched P batches ahead in registers consumed in
-// place.  A batch is BLK_ROWS = 128 rows (four groups of 32): every batch costs
-// the consumer one wait and one release of fixed latency, which at 32 rows per
-// batch capped a CTA at about 140 rows/us (measured); at 128 rows the largest
-// clusters' chains run at about 280 rows/us.  BLK_STAGES is a multiple of
-// BLK_PROD, so a stage is always refilled by the same producer, which waits on
-// its phases in order (a parity wait can never alias a later phase).
-namespace {
-constexpr int BLK_ROWS = 128, BLK_GRP = 32, BLK_STAGES = 6, BLK_COLS = 32, BLK_PROD = 3;
-static_assert(BLK_STAGES % BLK_PROD == 0, "a stage must always belong to the same producer");
-static_assert(BLK_ROWS % BLK_GRP == 0, "batches are whole groups of 32 rows");
-constexpr uint64_t BLK_WAIT_NS = 2000000000ull;
-constexpr uint32_t BLK_SUSPEND_NS = 2000;       // try_wait suspend hint
-constexpr size_t BLK_SMEM = (size_t)BLK_STAGES * BLK_ROWS * BLK_COLS * sizeof(float);
-constexpr int BLK_LPR = BLK_COLS / 4;           // lanes per row (16 bytes each)
-constexpr int BLK_RPI = 32 / BLK_LPR;           // rows per copy instruction
-constexpr int BLK_THREADS = 32 * (BLK_PROD + (BLK_COLS + 31) / 32);
-}  // namespace
-
-__global__ void __launch_bounds__(BLK_THREADS)
+__global__ void __launch_bounds__(blk_threads(VEC))
 update_sums_bulk_kernel(const float* __restrict__ X, const uint32_t* __restrict__ perm,
                         const uint32_t* __restrict__ cstart, uint32_t d, uint32_t k,
                         const float* __restrict__ C, float* __restrict__ Cn,
                         float* __restrict__ dsq, double* __restrict__ objpart, DevState* st,
                         const uint32_t* __restrict__ order) {
+  constexpr int PROD = blk_producers(VEC);
+  static_assert(BLK_STAGES % PROD == 0, "a stage must always belong to the same producer");
   griddep_wait();
   if (st && st->done) return;
   extern __shared__ __align__(128) float ring[];        // [BLK_STAGES][BLK_ROWS][BLK_COLS]
@@ -1360,13 +1257,12 @@ update_sums_bulk_kernel(const float* __restrict__ X, const uint32_t* __restrict_
   // index order), so that the longest ordered sums start first
   const uint32_t c = order ? order[blockIdx.x / nblk] : blockIdx.x / nblk;
   const uint32_t j0 = (blockIdx.x % nblk) * BLK_COLS;
-  const uint32_t w = min((uint32_t)BLK_COLS, d - j0);   // columns of this block (multiple of 4)
-  const uint32_t nc = (w + 31) / 32;                    // consumer warps doing work
+  const uint32_t w = min((uint32_t)BLK_COLS, d - j0);   // columns of this block
   const uint32_t s0 = cstart[c], s1 = cstart[c + 1];
   const uint32_t nb = (s1 - s0 + BLK_ROWS - 1) / BLK_ROWS;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (threadIdx.x == 0) {
-    for (int s = 0; s < BLK_STAGES; ++s) { mbar_init(&full[s], 32); mbar_init(&empty[s], nc); }
+    for (int s = 0; s < BLK_STAGES; ++s) { mbar_init(&full[s], 32); mbar_init(&empty[s], objpart ? 2 : 1); }
     abort_flag = 0;
     mbar_fence_init();
   }
@@ -1377,159 +1273,195 @@ update_sums_bulk_kernel(const float* __restrict__ X, const uint32_t* __restrict_
     if (st) atomicOr(&st->err, KM_DEVERR_TIMEOUT);
   };
 
-  if (warp < BLK_PROD) {
+  if (warp < PROD) {
     constexpr int P = 2;                       // batches of indices prefetched per producer
     constexpr int G = BLK_ROWS / BLK_GRP;
     const uint32_t p0 = (uint32_t)warp;
     uint32_t pq[P][G];
-#pragma unroll
-    for (int i = 0; i < P; ++i) {
-      const uint32_t b = p0 + (uint32_t)i * BLK_PROD;
+    auto load_idx = [&](uint32_t (&q)[G], uint32_t b) {     // group g of batch b: rows 32 g + lane
 #pragma unroll
       for (int g = 0; g < G; ++g) {
         const uint32_t idx = s0 + b * BLK_ROWS + (uint32_t)(g * BLK_GRP) + (uint32_t)lane;
-        pq[i][g] = (b < nb && idx < s1) ? perm[idx] : 0u;
+        q[g] = (b < nb && idx < s1) ? perm[idx] : 0u;
       }
-    }
+    };
+#pragma unroll
+    for (int i = 0; i < P; ++i) load_idx(pq[i], p0 + (uint32_t)i * PROD);
     // Unrolled by P so that pq[i] is consumed in place, P batches after its
     // load was issued (moving a register whose load is in flight would wait).
     bool ok = true;
-    for (uint32_t lb0 = 0; p0 + lb0 * BLK_PROD < nb && ok; lb0 += P) {
+    for (uint32_t lb0 = 0; p0 + lb0 * PROD < nb && ok; lb0 += P) {
 #pragma unroll
       for (int i = 0; i < P; ++i) {
-        const uint32_t b = p0 + (lb0 + (uint32_t)i) * BLK_PROD;
+        const uint32_t b = p0 + (lb0 + (uint32_t)i) * PROD;
         if (b >= nb || !ok) break;
         const uint32_t s = b % BLK_STAGES, ph = (b / BLK_STAGES) & 1u;
         const bool okw = mbar_wait_bounded(&empty[s], ph ^ 1u, ab, BLK_WAIT_NS, BLK_SUSPEND_NS);
         if (!__all_sync(0xffffffffu, okw)) { if (lane == 0) fail(); ok = false; break; }
+        constexpr int LPR = BLK_COLS / VEC;    // lanes per row
+        constexpr int RPI = 32 / LPR;          // rows per copy instruction
         const uint32_t m = min((uint32_t)BLK_ROWS, s1 - (s0 + b * BLK_ROWS));
-        // One instruction copies BLK_RPI rows: BLK_LPR lanes of 16 bytes per
-        // row; columns past w and rows past m zero-fill.
-        const uint32_t sub = (uint32_t)lane / BLK_LPR, c4 = ((uint32_t)lane % BLK_LPR) * 4u;
-        const bool lane_has_cols = c4 < w;
-        const float* xl = X + j0 + c4;
+        // columns past w and rows past m zero-fill
+        const uint32_t sub = (uint32_t)lane / LPR, cv = ((uint32_t)lane % LPR) * (uint32_t)VEC;
+        const bool lane_has_cols = cv < w;
+        const float* xl = X + j0 + cv;
 #pragma unroll
         for (int g = 0; g < G; ++g) {
-          float* dst = ring + ((size_t)s * BLK_ROWS + (size_t)(g * BLK_GRP) + sub) * BLK_COLS + c4;
+          float* dst = ring + ((size_t)s * BLK_ROWS + (size_t)(g * BLK_GRP) + sub) * BLK_COLS + cv;
           // All row indices of the group first: each cp.async is an ordered asm
           // statement, so a shuffle placed between two of them would put its
           // latency on every row.
-          uint32_t rr[BLK_GRP / BLK_RPI];
+          uint32_t rr[BLK_GRP / RPI];
 #pragma unroll
-          for (int ii = 0; ii < BLK_GRP / BLK_RPI; ++ii)
-            rr[ii] = __shfl_sync(0xffffffffu, pq[i][g], ii * BLK_RPI + (int)sub);
+          for (int ii = 0; ii < BLK_GRP / RPI; ++ii)
+            rr[ii] = __shfl_sync(0xffffffffu, pq[i][g], ii * RPI + (int)sub);
 #pragma unroll
-          for (int ii = 0; ii < BLK_GRP / BLK_RPI; ++ii) {
-            const uint32_t u = (uint32_t)(g * BLK_GRP + ii * BLK_RPI) + sub;
+          for (int ii = 0; ii < BLK_GRP / RPI; ++ii) {
+            const uint32_t u = (uint32_t)(g * BLK_GRP + ii * RPI) + sub;
             const bool okr = u < m && lane_has_cols;
             const float* src = okr ? xl + (uint64_t)rr[ii] * d : X;
-            cp_async16_zfill(dst + (size_t)ii * BLK_RPI * BLK_COLS, src, okr ? 16u : 0u);
+            cp_async_cols<VEC>(dst + (size_t)ii * RPI * BLK_COLS, src, okr);
           }
         }
         cp_async_mbar_arrive_noinc(&full[s]);
-        const uint32_t nbb = b + (uint32_t)P * BLK_PROD;
-#pragma unroll
-        for (int g = 0; g < G; ++g) {
-          const uint32_t idx = s0 + nbb * BLK_ROWS + (uint32_t)(g * BLK_GRP) + (uint32_t)lane;
-          pq[i][g] = (nbb < nb && idx < s1) ? perm[idx] : 0u;
-        }
+        load_idx(pq[i], b + (uint32_t)P * PROD);
       }
     }
     // Drain: this warp's copies must land before the CTA exits.
     asm volatile("cp.async.wait_all;" ::: "memory");
-  } else if ((uint32_t)(warp - BLK_PROD) < nc) {
-    const uint32_t col = (uint32_t)(warp - BLK_PROD) * 32u + (uint32_t)lane;   // column within the block
-    const bool vj = col < w;
-    const uint64_t p = (uint64_t)c * d + j0 + col;
-    const float cold = (C && vj) ? C[p] : 0.0f;
+    return;
+  }
+
+  if (warp == PROD) {
+    // The ordered chain, lane = column within the block.  A group of 32 rows is
+    // added while the next one is loaded, one load beside each addition (32
+    // loads in a block would hold the warp's issue until the shared-memory queue
+    // took them all); the next batch's barrier is tested a group ahead of its
+    // use.  Rows past the cluster's end are zero-filled: adding +0 leaves the sum
+    // as it is (a sum that starts at +0 is never -0).
+    constexpr uint32_t RB = BLK_COLS * 4u, GB = BLK_GRP * RB, SB = BLK_ROWS * RB;   // bytes of a row, group, stage
+    float va[BLK_GRP], vb[BLK_GRP];
     float sum = 0.0f;
-    float eh = 0.0f, el = 0.0f;          // objective: FP32 pair hi + lo
-    for (uint32_t b = 0; b < nb; ++b) {
-      const uint32_t s = b % BLK_STAGES, ph = (b / BLK_STAGES) & 1u;
-      const bool ok = mbar_wait_bounded(&full[s], ph, ab, BLK_WAIT_NS, BLK_SUSPEND_NS);
-      if (!__all_sync(0xffffffffu, ok)) { if (lane == 0) fail(); break; }
-      const uint32_t m = min((uint32_t)BLK_ROWS, s1 - (s0 + b * BLK_ROWS));
-      // Groups of 32 rows in order; the group's objective partial joins the
-      // FP32 pair, as one batch of 32 rows did.
-      for (uint32_t g0 = 0; g0 < m; g0 += BLK_GRP) {
-        const uint32_t mg = min((uint32_t)BLK_GRP, m - g0);
-        const float* src = ring + ((size_t)s * BLK_ROWS + g0) * BLK_COLS + col;
-        float e32 = 0.0f, e32b = 0.0f;
-        if (mg == (uint32_t)BLK_GRP) {
-          // Full group: all loads first, then the ordered chain (no branch or
-          // load latency on the dependent additions).
-          float v[BLK_GRP];
+    auto step = [&](const float (&v)[BLK_GRP], float (&x)[BLK_GRP], uint32_t src) {
 #pragma unroll
-          for (int u = 0; u < BLK_GRP; ++u) v[u] = vj ? src[(size_t)u * BLK_COLS] : 0.0f;
-#pragma unroll
-          for (int u = 0; u < BLK_GRP; ++u) {
-            sum = __fadd_rn(sum, v[u]);
-            const float t = v[u] - cold;
-            if (u & 1) e32b = fmaf(t, t, e32b); else e32 = fmaf(t, t, e32);
-          }
-        } else {
-          for (uint32_t u = 0; u < mg; ++u) {
-            const float v = vj ? src[(size_t)u * BLK_COLS] : 0.0f;
-            sum = __fadd_rn(sum, v);
-            const float t = v - cold;
-            e32 = fmaf(t, t, e32);
-          }
-        }
-        e32 = __fadd_rn(e32, e32b);
-        // TwoSum: eh + e32 = s_ + err exactly; err accumulates into el
-        const float s_ = __fadd_rn(eh, e32), bb = __fsub_rn(s_, eh);
-        el = __fadd_rn(el, __fadd_rn(__fsub_rn(eh, __fsub_rn(s_, bb)), __fsub_rn(e32, bb)));
-        eh = s_;
+      for (int u = 0; u < BLK_GRP; ++u) {
+        x[u] = ld_shared_f32(src + (uint32_t)u * RB);
+        asm volatile("add.rn.f32 %0, %0, %1;" : "+f"(sum) : "f"(v[u]));
       }
+    };
+    const uint32_t base = smem_u32(ring) + (uint32_t)lane * 4u;
+    uint32_t s = 0, ph = 0;
+    bool ok = nb == 0u || mbar_wait_bounded(&full[0], 0, ab, BLK_WAIT_NS, BLK_SUSPEND_NS);
+    if (!__all_sync(0xffffffffu, ok)) { if (lane == 0) fail(); return; }
+    if (nb) {
+#pragma unroll
+      for (int u = 0; u < BLK_GRP; ++u) va[u] = ld_shared_f32(base + (uint32_t)u * RB);
+    }
+    for (uint32_t left = nb; left; --left) {
+      const uint32_t src = base + s * SB;
+      const uint32_t sn = s + 1u == (uint32_t)BLK_STAGES ? 0u : s + 1u, phn = sn ? ph : ph ^ 1u;
+      step(va, vb, src + GB);
+      step(vb, va, src + 2 * GB);
+      ok = left == 1u || mbar_test_wait(&full[sn], phn);
+      step(va, vb, src + 3 * GB);
+      if (!__all_sync(0xffffffffu, ok)) {
+        ok = mbar_wait_bounded(&full[sn], phn, ab, BLK_WAIT_NS, BLK_SUSPEND_NS);
+        if (!__all_sync(0xffffffffu, ok)) { if (lane == 0) fail(); return; }
+      }
+      // (after the last batch the next stage holds old rows or none: unused)
+      step(vb, va, base + sn * SB);
       __syncwarp();
       if (lane == 0) mbar_arrive(&empty[s]);
+      s = sn;
+      ph = phn;
     }
-    if (vj) {
+    if ((uint32_t)lane < w) {
+      const uint64_t p = (uint64_t)c * d + j0 + (uint32_t)lane;
       const uint32_t cnt = s1 - s0;
       const float scale = __double2float_rn(1.0 / (double)(cnt > 1 ? cnt : 1));
       const float cn = __fmul_rn(sum, scale);
       Cn[p] = cn;
       if (dsq) {
-        const float t = __fsub_rn(cn, cold);
+        const float t = __fsub_rn(cn, C ? C[p] : 0.0f);
         dsq[p] = __fmul_rn(t, t);
       }
-      if (objpart) objpart[p] = (double)eh + (double)el;
+    }
+  } else if (objpart) {
+    // The objective: lane l on columns 4 (l % 8) .. + 3 of every fourth row
+    // (rows l / 8, + 4, ...), 16 bytes a load.  Per batch a lane sums its 32
+    // rows in FP32, across batches as an unevaluated FP32 pair (TwoSum).
+    const uint32_t c4 = ((uint32_t)lane & 7u) * 4u, r0 = (uint32_t)lane >> 3;
+    const uint64_t p = (uint64_t)c * d + j0 + c4;
+    float cold[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) cold[q] = (C && c4 + q < w) ? C[p + q] : 0.0f;
+    const float2 ma = make_float2(-cold[0], -cold[1]), mb = make_float2(-cold[2], -cold[3]);
+    float2 ha = make_float2(0.0f, 0.0f), la = ha, hb = ha, lb = ha;   // pairs hi + lo of columns 0,1 and 2,3
+    auto neg = [](float2 v) { return make_float2(-v.x, -v.y); };
+    // TwoSum: h + g = s + err exactly; err accumulates into l
+    auto two_sum = [&](float2& h, float2& l, float2 g) {
+      const float2 s_ = __fadd2_rn(h, g), bb = __fadd2_rn(s_, neg(h));
+      l = __fadd2_rn(l, __fadd2_rn(__fadd2_rn(h, neg(__fadd2_rn(s_, neg(bb)))), __fadd2_rn(g, neg(bb))));
+      h = s_;
+    };
+    for (uint32_t b = 0; b < nb; ++b) {
+      const uint32_t s = b % BLK_STAGES, ph = (b / BLK_STAGES) & 1u;
+      const bool ok = mbar_wait_bounded(&full[s], ph, ab, BLK_WAIT_NS, BLK_SUSPEND_NS);
+      if (!__all_sync(0xffffffffu, ok)) { if (lane == 0) fail(); return; }
+      const uint32_t m = min((uint32_t)BLK_ROWS, s1 - (s0 + b * BLK_ROWS));
+      const float4* src = reinterpret_cast<const float4*>(ring + ((size_t)s * BLK_ROWS + r0) * BLK_COLS + c4);
+      float2 ea = make_float2(0.0f, 0.0f), eb = ea;
+      auto add = [&](const float4 v) {
+        const float2 ta = __fadd2_rn(make_float2(v.x, v.y), ma), tb = __fadd2_rn(make_float2(v.z, v.w), mb);
+        ea = __ffma2_rn(ta, ta, ea);
+        eb = __ffma2_rn(tb, tb, eb);
+      };
+      if (m == (uint32_t)BLK_ROWS) {
+#pragma unroll
+        for (int u0 = 0; u0 < BLK_ROWS / 4; u0 += 8) {
+          float4 v[8];
+#pragma unroll
+          for (int u = 0; u < 8; ++u) v[u] = src[(u0 + u) * BLK_COLS];
+#pragma unroll
+          for (int u = 0; u < 8; ++u) add(v[u]);
+        }
+      } else {
+        for (uint32_t u = 0; r0 + 4u * u < m; ++u) add(src[u * BLK_COLS]);
+      }
+      two_sum(ha, la, ea);
+      two_sum(hb, lb, eb);
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&empty[s]);
+    }
+    double o[4] = {(double)ha.x + (double)la.x, (double)ha.y + (double)la.y, (double)hb.x + (double)lb.x,
+                   (double)hb.y + (double)lb.y};
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      o[q] += __shfl_xor_sync(0xffffffffu, o[q], 8);
+      o[q] += __shfl_xor_sync(0xffffffffu, o[q], 16);
+      if (r0 == 0u && c4 + q < w) objpart[p + q] = o[q];
     }
   }
 }
 
-// Opt-in shared memory for the VEC = 4 ring; called before any capture.
+// Opt-in shared memory for the ring; called before any capture.
 km_status update_sums_prepare() {
-  KM_CUDA_TRY(cudaFuncSetAttribute(update_sums_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   UPD_STAGES * UPD_ROWS * 128 * (int)sizeof(float)));
-  KM_CUDA_TRY(cudaFuncSetAttribute(update_sums_bulk_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   (int)BLK_SMEM));
+  for (auto kern : {update_sums_bulk_kernel<4>, update_sums_bulk_kernel<2>, update_sums_bulk_kernel<1>})
+    KM_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)BLK_SMEM));
   return KM_OK;
 }
 
-// One lane per column (32 columns per warp) exposes the most independent
-// (cluster, column) chains: the largest cluster is spread over d/32 warps, each
-// with UPD_STAGES*UPD_ROWS rows in flight.  The 4-column variant is used only
-// when the chains already outnumber the GPU many times over.
+// Rows are copied in the widest pieces whose alignment every row start has
+// (row stride d floats from X): 16 bytes, else 8, else 4.
 km_status launch_update_sums(const float* X, const uint32_t* perm, const uint32_t* cstart, uint32_t d,
                              uint32_t k, const float* C, float* Cn, float* dsq, double* objpart,
                              DevState* st, cudaStream_t s, const uint32_t* order) {
-  if (d % 4 == 0 && reinterpret_cast<uintptr_t>(X) % 16 == 0) {
-    const uint64_t ctas = (uint64_t)k * ((d + BLK_COLS - 1) / BLK_COLS);
-    KM_CUDA_TRY(launch_pdl(update_sums_bulk_kernel, (unsigned)ctas, BLK_THREADS, BLK_SMEM, s, X, perm, cstart, d,
-                           k, C, Cn, dsq, objpart, st, order));
-    KM_CUDA_TRY(cudaGetLastError());
-    return KM_OK;
-  }
-  const bool v4 = false;
-  const uint32_t W = v4 ? 128u : 32u;
-  const uint64_t warps = (uint64_t)k * ((d + W - 1) / W);
-  const size_t smem = (size_t)UPD_STAGES * UPD_ROWS * W * sizeof(float);
-  if (v4) {
-    update_sums_kernel<4><<<(unsigned)warps, 32, smem, s>>>(X, perm, cstart, d, k, C, Cn, dsq, objpart, st);
-  } else {
-    update_sums_kernel<1><<<(unsigned)warps, 32, smem, s>>>(X, perm, cstart, d, k, C, Cn, dsq, objpart, st);
-  }
+  const uintptr_t xa = reinterpret_cast<uintptr_t>(X);
+  const int vec = (d % 4 == 0 && xa % 16 == 0) ? 4 : (d % 2 == 0 && xa % 8 == 0) ? 2 : 1;
+  auto kern = vec == 4 ? update_sums_bulk_kernel<4> : vec == 2 ? update_sums_bulk_kernel<2> : update_sums_bulk_kernel<1>;
+  const uint64_t ctas = (uint64_t)k * ((d + BLK_COLS - 1) / BLK_COLS);
+  KM_CUDA_TRY(launch_pdl(kern, (unsigned)ctas, blk_threads(vec), BLK_SMEM, s, X, perm, cstart, d, k, C, Cn, dsq,
+                         objpart, st, order));
   KM_CUDA_TRY(cudaGetLastError());
   return KM_OK;
 }
