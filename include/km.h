@@ -330,13 +330,13 @@ typedef struct km_batch km_batch;
 /* No counterpart in the reference (its -r repeats one problem sequentially,
  * src/main.cu:95-120): every restart of every problem runs the reference CPU
  * algorithm (seeded sample picks, kmeans.cpp:49-200) with labels and
- * centroids identical to a single run, all in one persistent kernel launch. */
+ * centroids identical to a single run, all instances advanced together. */
 km_status km_batch_create(const km_batch_params* p, const km_batch_problem* problems, km_batch** out);
 /* X: all problems' points, packed, host memory. */
 km_status km_batch_set_data(km_batch* h, const float* X);
-/* Times the kernel's tile variants on a sample of the instances and keeps the
- * fastest (km_batch_fit does this on first use). variant_out / ms (6 doubles)
- * may be NULL. */
+/* Times the assignment's tile variants on a sample of the instances and keeps
+ * the fastest (without this call km_batch_fit uses the default variant; the
+ * results are the same). variant_out / ms (6 doubles) may be NULL. */
 km_status km_batch_tune(km_batch* h, int32_t* variant_out, double* ms_per_variant);
 /* results: problems*restarts entries (problem-major).  best_labels: the labels
  * of each problem's lowest-objective restart, packed (n per problem);

@@ -1,29 +1,28 @@
 // Batched Lloyd k-means: many independent problems of uneven n, d, k, each
-// with several seeded restarts, in ONE persistent kernel launch.
+// with several seeded restarts, advanced together.
 //
-// Every restart of every problem is an "instance".  A CTA takes the next
-// instance from a work counter (instances are ordered largest first, so the
-// long ones start early) and runs the reference CPU algorithm on it to the
-// end, iterations included, without leaving the kernel:
-//   assign   each thread owns rows; distances by the CPU formula
-//            sum_j fl((x_j - c_j)^2) in column order (exact, no bound or
-//            refinement needed), strict '<' over centroids in ascending order
-//            (comparisons/CPU_Kmeans/src/kmeans.cpp:86-129);
-//   sort     counts in shared memory and a stable counting sort of the rows by
-//            label (chunks of blockDim rows, warp match + per-warp counts);
-//   update   one thread per (cluster, column): sum of the cluster's rows in row
-//            order, then scale by float(1/(double)max(count,1)) (kmeans.cpp:131-155);
-//   stop     from the second iteration, every centroid moved <= tol (float
-//            sqrt of the column-ordered sum of squares, kmeans.cpp:170-200).
-// The centroids live in shared memory (transposed, d x kpad) for the whole
-// instance; X, the labels and the per-CTA scratch (permutation, next
-// centroids) are in global memory.  Initial centroids are the reference's
-// seeded sample picks, drawn on the host (std::mt19937 as the reference does).
-//
-// Tile shape: each thread computes CG centroids at a time for its row (CG in
-// {8, 16, 32}) with NT threads per CTA (128 or 256); the pair is chosen by
-// timing the candidates on a sample of the instances (km_batch_fit).
+// Every restart of every problem is an "instance" and runs the reference CPU
+// algorithm to its own end; all instances still running take an iteration in the
+// same few launches, whose work items are cut from the instances so that one
+// large instance spreads over the whole GPU (one CTA per instance instead left
+// the GPU waiting for the largest ones: 64 problems x 4 restarts, n 1024..65536,
+// 767 ms, now 88 ms):
+//   assign   a tile of rows against all centroids of its instance; distances by
+//            the CPU formula sum_j fl((x_j - c_j)^2) in column order (exact, no
+//            bound or refinement needed), strict '<' over centroids in ascending
+//            order (comparisons/CPU_Kmeans/src/kmeans.cpp:86-129);
+//   sort     a CTA per instance: stable counting sort of the rows by label;
+//   update   a task per (instance, cluster, 32 columns): sum of the cluster's rows
+//            in row order, then scale by float(1/(double)max(count,1))
+//            (kmeans.cpp:131-155);
+//   stop     a CTA per instance: from the second iteration, every centroid moved
+//            <= tol (float sqrt of the column-ordered sum of squares,
+//            kmeans.cpp:170-200); the CTA that finishes last lists the instances
+//            that go on and cuts their work into items.
+// Initial centroids are the reference's seeded sample picks, drawn on the host
+// (std::mt19937 as the reference does).
 #include "km_lloyd.cuh"
+#include "km_sums.cuh"
 
 #include <algorithm>
 #include <chrono>
@@ -36,9 +35,10 @@ namespace km {
 
 struct BatchInst {
   uint64_t xoff;      // floats: first coordinate of the problem's points
-  uint64_t loff;      // uint32: first label of this instance
+  uint64_t loff;      // uint32: first label (and sorted row) of this instance
   uint64_t coff;      // floats: first centroid value of this instance (k*d)
-  uint32_t n, d, k, kpad;
+  uint64_t toff;      // doubles: first tile objective of this instance
+  uint32_t n, d, k;
   uint32_t prob, restart;
 };
 
@@ -48,177 +48,628 @@ struct BatchOut {
   double objective;   // FP64 sum of the final assignment's (FP32 CPU-formula) distances
 };
 
-constexpr uint32_t BATCH_MAX_SMEM_C = 160u * 1024u;
+// One ordered sum: 32 columns (w of them in use) of one cluster of one instance.
+struct BatchTask {
+  const float* x;             // first column of the problem's first row
+  const uint32_t* perm;       // the cluster's rows, ascending
+  float* out;                 // next centroid, same columns
+  uint32_t cnt, d, w, vec;    // rows, row stride, columns, columns per copy (4, 2 or 1)
+};
+
+// Loop state on the device: the instances still running (act, in descending
+// work), the first assign tile of each, the update tasks of this iteration, and
+// the counters that hand tiles and tasks out.
+struct BatchCtl {
+  unsigned long long iter;    // iterations done
+  uint32_t nact;
+  uint32_t nlong, nshort;     // update tasks of at least BATCH_RING_ROWS rows / of fewer
+  uint32_t tile_end[3], next_tile[3];   // assign tiles by group of shapes (batch_group)
+  uint32_t next_short, ticket;
+  uint32_t err;               // KM_DEVERR_*
+};
+
+constexpr uint32_t BATCH_MAX_SMEM_C = 160u * 1024u;   // accepted shapes: d * round_up(k, 32) * 4 bytes at most
 
 namespace {
 
 __device__ __forceinline__ float f_inf_b() { return __int_as_float(0x7f800000); }
 
-template <int NT, int CG>
-__global__ void __launch_bounds__(NT)
-batch_lloyd_kernel(const float* __restrict__ X, const BatchInst* __restrict__ insts, uint32_t ninst,
-                   const float* __restrict__ C0, float* __restrict__ Cout,
-                   uint32_t* __restrict__ labels_all, uint32_t* __restrict__ perm_scratch,
-                   float* __restrict__ cnew_scratch, uint64_t perm_stride, uint64_t cnew_stride,
-                   uint32_t* __restrict__ next, float tol, uint64_t maxiter, BatchOut* __restrict__ out) {
-  constexpr int NW = NT / 32;
-  extern __shared__ float Cs[];                          // d x kpad, transposed centroids
-  __shared__ uint32_t cnt[256], cstart[257], running[256];
-  __shared__ uint32_t wcnt[NW][256];
-  __shared__ uint32_t s_inst;
-  __shared__ int s_moved;
-  __shared__ double s_obj[NW];
+// Assign tiles: BA_NT threads as (BA_NT / TX) x TX, each RT rows and CT centroids,
+// so TX * CT centroids side by side.  The shapes are 16, 24, 32, 48, 64, 96 and
+// 128 centroids wide, so that at most a third of a tile is padding for k > 16
+// (k > 128: chunks of 128, or of 96 for k <= 192).
+constexpr int BA_NT = 128;
+__host__ __device__ constexpr uint32_t batch_cols(uint32_t k) {
+  return k <= 16u ? 16u : k <= 24u ? 24u : k <= 32u ? 32u : k <= 48u ? 48u : k <= 64u ? 64u
+         : (k <= 96u || (k > 128u && k <= 192u)) ? 96u : 128u;
+}
+// Shapes are compiled into one kernel per group (two or three shapes each: with
+// four the kernel spills), the widest group first.
+__host__ __device__ constexpr uint32_t batch_group(uint32_t k) {
+  return batch_cols(k) > 64u ? 0u : batch_cols(k) > 32u ? 1u : 2u;
+}
+__host__ __device__ constexpr uint32_t batch_tile_rows(uint32_t k, uint32_t rt) {
+  const uint32_t c = batch_cols(k);
+  return rt * (BA_NT / (c <= 32u ? 4u : c <= 64u ? 8u : 16u));
+}
+__host__ __device__ constexpr uint32_t batch_tiles(uint32_t n, uint32_t k, uint32_t rt) {
+  return (n + batch_tile_rows(k, rt) - 1u) / batch_tile_rows(k, rt);
+}
+// Clusters of at least this many rows are summed by a CTA's ring, smaller ones by
+// a warp alone.
+constexpr uint32_t BATCH_RING_ROWS = 256;
 
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  uint32_t* perm = perm_scratch + (uint64_t)blockIdx.x * perm_stride;
-  float* Cn = cnew_scratch + (uint64_t)blockIdx.x * cnew_stride;
+template <int RT, int TX, int CT>
+struct BatchTile {
+  static constexpr int ROWS = RT * (BA_NT / TX), COLS = CT * TX;
+  static constexpr int KC = TX == 4 && CT == 8 ? 8 : 16;    // coordinates per shared-memory stage
+  static constexpr int LDA = ROWS + 4;
+  static constexpr int A_FLOATS = KC * LDA, B_FLOATS = KC * COLS * 2, FLOATS = A_FLOATS + B_FLOATS;
+  static constexpr int NA = ROWS * KC / (4 * BA_NT);       // float4 loads per thread and stage
+  static constexpr int NB = (COLS * KC + 4 * BA_NT - 1) / (4 * BA_NT);
+};
+template <int RT>
+constexpr size_t batch_assign_smem() {
+  constexpr int a = BatchTile<RT, 16, 8>::FLOATS, b = BatchTile<RT, 8, 8>::FLOATS, c = BatchTile<RT, 4, 6>::FLOATS;
+  static_assert(BatchTile<RT, 4, 8>::FLOATS <= c && BatchTile<RT, 4, 4>::FLOATS <= c, "the widest of its group");
+  return 2 * sizeof(float) * (size_t)(a > b ? (a > c ? a : c) : (b > c ? b : c));
+}
 
-  for (;;) {
-    if (tid == 0) s_inst = atomicAdd(next, 1u);
-    __syncthreads();
-    const uint32_t ii = s_inst;
-    __syncthreads();
-    if (ii >= ninst) break;
-    const BatchInst I = insts[ii];
-    const uint32_t n = I.n, d = I.d, k = I.k, kpad = I.kpad;
-    const float* Xp = X + I.xoff;
-    uint32_t* lab = labels_all + I.loff;
-    // initial centroids, transposed
-    for (uint32_t q = tid; q < d * kpad; q += NT) {
-      const uint32_t j = q / kpad, c = q % kpad;
-      Cs[q] = (c < k) ? C0[I.coff + (uint64_t)c * d + j] : 0.0f;
-    }
-    for (uint32_t q = tid; q < NW * 256u; q += NT) (&wcnt[0][0])[q] = 0u;
-    __syncthreads();
-    uint64_t converged = maxiter, iter = 0;
-    double obj = 0.0;
-    while (iter++ < maxiter) {
-      // ---- assign (reference CPU distance and argmin) ----
-      double myobj = 0.0;
-      for (uint32_t row = tid; row < n; row += NT) {
-        const float* x = Xp + (uint64_t)row * d;
-        float best = f_inf_b();
-        uint32_t bi = 0;
-        for (uint32_t g = 0; g < kpad; g += CG) {
-          float acc[CG];
+// One tile.  Bound by the FP32 pipes: three roundings an element (x - c, square,
+// add) as the CPU formula has them.  They are done two rows at a time in packed
+// FP32 pairs, which take half the issue slots of scalar operations (n = 65536
+// d = 128 k = 64: 31.1 T operations/s against 29.5 T scalar, of 33.6 T measured
+// for the three in registers alone).  The square is an FMA with -0 (nz, which the
+// caller passes so that the compiler cannot see its value): it rounds as the
+// product alone, whereas a packed product followed by a packed sum is fused into
+// one FMA by the assembler.  The points are staged transposed (pairs of rows
+// adjacent), the centroids negated and duplicated (x + (-c) rounds as x - c), both
+// a stage ahead in registers.
+extern __shared__ __align__(16) float batch_smem[];
+template <int RT, int TX, int CT>
+__device__ __forceinline__ void batch_tile(const float* __restrict__ Xp, const float* __restrict__ C, uint32_t n,
+                                           uint32_t d, uint32_t k, bool v4, uint32_t m0, uint32_t* __restrict__ lab,
+                                           double* __restrict__ objtile, float2 nz) {
+  __shared__ double s_obj[BA_NT / 32];
+  float* const smem = batch_smem;
+  using T = BatchTile<RT, TX, CT>;
+  const int tid = threadIdx.x, tx = tid % TX, ty = tid / TX;
+  float bv[RT];
+  uint32_t bi[RT];
 #pragma unroll
-          for (int c = 0; c < CG; ++c) acc[c] = 0.0f;
-          for (uint32_t j = 0; j < d; ++j) {
-            const float xj = __ldg(x + j);
-            const float4* cs4 = reinterpret_cast<const float4*>(Cs + (uint64_t)j * kpad + g);
+  for (int i = 0; i < RT; ++i) { bv[i] = f_inf_b(); bi[i] = 0u; }
+  const uint32_t nk = (d + T::KC - 1) / T::KC;
+  for (uint32_t c0 = 0; c0 < k; c0 += T::COLS) {
+    float2 acc[RT / 2][CT];
 #pragma unroll
-            for (int c4 = 0; c4 < CG / 4; ++c4) {
-              const float4 cc = cs4[c4];
-              float t;
-              t = __fsub_rn(xj, cc.x); acc[4 * c4 + 0] = __fadd_rn(acc[4 * c4 + 0], __fmul_rn(t, t));
-              t = __fsub_rn(xj, cc.y); acc[4 * c4 + 1] = __fadd_rn(acc[4 * c4 + 1], __fmul_rn(t, t));
-              t = __fsub_rn(xj, cc.z); acc[4 * c4 + 2] = __fadd_rn(acc[4 * c4 + 2], __fmul_rn(t, t));
-              t = __fsub_rn(xj, cc.w); acc[4 * c4 + 3] = __fadd_rn(acc[4 * c4 + 3], __fmul_rn(t, t));
+    for (int i = 0; i < RT / 2; ++i)
+#pragma unroll
+      for (int j = 0; j < CT; ++j) acc[i][j] = make_float2(0.0f, 0.0f);
+    float4 ra[T::NA], rb[T::NB];
+    // Four coordinates of a row (of X, or of C): zeros past n / k and past d.
+    auto load4 = [&](const float* base, uint32_t row, uint32_t rows, uint32_t col) {
+      float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (row < rows) {
+        const float* p = base + (uint64_t)row * d + col;
+        if (v4) {
+          if (col < d) v = __ldg(reinterpret_cast<const float4*>(p));
+        } else {
+          if (col + 0 < d) v.x = __ldg(p);
+          if (col + 1 < d) v.y = __ldg(p + 1);
+          if (col + 2 < d) v.z = __ldg(p + 2);
+          if (col + 3 < d) v.w = __ldg(p + 3);
+        }
+      }
+      return v;
+    };
+    constexpr int QR = T::KC / 4;                          // float4 per row and stage
+    auto gload = [&](uint32_t kc) {
+#pragma unroll
+      for (int e = 0; e < T::NA; ++e) {
+        const uint32_t idx = (uint32_t)(e * BA_NT + tid);
+        ra[e] = load4(Xp, m0 + idx / QR, n, kc + 4u * (idx % QR));
+      }
+#pragma unroll
+      for (int e = 0; e < T::NB; ++e) {
+        const uint32_t idx = (uint32_t)(e * BA_NT + tid);
+        if (idx < (uint32_t)(T::COLS * QR)) rb[e] = load4(C, c0 + idx / QR, k, kc + 4u * (idx % QR));
+      }
+    };
+    auto sstore = [&](int buf) {
+      float* A = smem + buf * T::FLOATS;
+      float2* B = reinterpret_cast<float2*>(A + T::A_FLOATS);
+#pragma unroll
+      for (int e = 0; e < T::NA; ++e) {
+        const int idx = e * BA_NT + tid, r = idx / QR, j = 4 * (idx % QR);
+        A[(j + 0) * T::LDA + r] = ra[e].x;
+        A[(j + 1) * T::LDA + r] = ra[e].y;
+        A[(j + 2) * T::LDA + r] = ra[e].z;
+        A[(j + 3) * T::LDA + r] = ra[e].w;
+      }
+#pragma unroll
+      for (int e = 0; e < T::NB; ++e) {
+        const int idx = e * BA_NT + tid, c = idx / QR, j = 4 * (idx % QR);
+        if (idx < T::COLS * QR) {
+          B[(j + 0) * T::COLS + c] = make_float2(-rb[e].x, -rb[e].x);
+          B[(j + 1) * T::COLS + c] = make_float2(-rb[e].y, -rb[e].y);
+          B[(j + 2) * T::COLS + c] = make_float2(-rb[e].z, -rb[e].z);
+          B[(j + 3) * T::COLS + c] = make_float2(-rb[e].w, -rb[e].w);
+        }
+      }
+    };
+    gload(0);
+    sstore(0);
+    __syncthreads();
+    for (uint32_t kt = 0; kt < nk; ++kt) {
+      const float* A = smem + (kt & 1u) * T::FLOATS + ty * RT;
+      const float* B = smem + (kt & 1u) * T::FLOATS + T::A_FLOATS + 4 * tx;
+      if (kt + 1 < nk) gload((kt + 1) * T::KC);
+      const uint32_t left = d - kt * T::KC;                // coordinates of this stage (zeros up to a multiple of 4)
+#pragma unroll 1
+      for (uint32_t kk = 0; kk < (uint32_t)T::KC && kk < left; kk += 4) {
+#pragma unroll 2                    // 4 would spill
+        for (int q = 0; q < 4; ++q) {
+          const float* a_ = A + (kk + q) * T::LDA;
+          const float* b_ = B + (kk + q) * (2 * T::COLS);
+          float2 a[RT / 2], b[CT];
+#pragma unroll
+          for (int i = 0; i < RT / 4; ++i) {
+            const float4 v = *reinterpret_cast<const float4*>(a_ + 4 * i);
+            a[2 * i] = make_float2(v.x, v.y);
+            a[2 * i + 1] = make_float2(v.z, v.w);
+          }
+#pragma unroll
+          for (int j = 0; j < CT / 2; ++j) {
+            const float4 v = *reinterpret_cast<const float4*>(b_ + 4 * TX * j);
+            b[2 * j] = make_float2(v.x, v.y);
+            b[2 * j + 1] = make_float2(v.z, v.w);
+          }
+#pragma unroll
+          for (int i = 0; i < RT / 2; ++i)
+#pragma unroll
+            for (int j = 0; j < CT; ++j) {
+              const float2 t = __fadd2_rn(a[i], b[j]);
+              acc[i][j] = __fadd2_rn(acc[i][j], __ffma2_rn(t, t, nz));
             }
-          }
+        }
+      }
+      if (kt + 1 < nk) sstore((int)((kt + 1) & 1u));
+      __syncthreads();
+    }
+    // this thread's columns in ascending order: 2 (j/2 TX + tx) + j % 2
 #pragma unroll
-          for (int c = 0; c < CG; ++c)
-            if (g + c < k && acc[c] < best) { best = acc[c]; bi = g + c; }
-        }
-        lab[row] = bi;
-        myobj += (double)best;
-      }
-      for (int o = 16; o > 0; o >>= 1) myobj += __shfl_xor_sync(0xffffffffu, myobj, o);
-      if (lane == 0) s_obj[warp] = myobj;
-      for (uint32_t c = tid; c < k; c += NT) { cnt[c] = 0; running[c] = 0; }
-      __syncthreads();
-      if (tid == 0) {
-        double t = 0.0;
-        for (int w = 0; w < NW; ++w) t += s_obj[w];
-        obj = t;
-      }
-      // ---- counts and exclusive scan ----
-      for (uint32_t row = tid; row < n; row += NT) atomicAdd(&cnt[lab[row]], 1u);
-      __syncthreads();
-      if (tid == 0) {
-        uint32_t s = 0;
-        for (uint32_t c = 0; c < k; ++c) { cstart[c] = s; s += cnt[c]; }
-        cstart[k] = s;
-      }
-      __syncthreads();
-      // ---- stable scatter: chunks of NT rows in order ----
-      for (uint32_t base = 0; base < n; base += NT) {
-        const uint32_t row = base + tid;
-        const bool valid = row < n;
-        const uint32_t L = valid ? lab[row] : 0xffffffffu;
-        const unsigned same = __match_any_sync(0xffffffffu, L);
-        const uint32_t rank = (uint32_t)__popc(same & ((1u << lane) - 1u));
-        if (valid && rank == 0) wcnt[warp][L] = (uint32_t)__popc(same);
-        __syncthreads();
-        if (valid) {
-          uint32_t before = 0;
-          for (int w = 0; w < warp; ++w) {
-            // a warp that had no row with label L left wcnt[w][L] at zero
-            before += wcnt[w][L];
-          }
-          perm[cstart[L] + running[L] + before + rank] = row;
-        }
-        __syncthreads();
-        for (uint32_t c = tid; c < k; c += NT) {
-          uint32_t t = 0;
-          for (int w = 0; w < NW; ++w) { t += wcnt[w][c]; wcnt[w][c] = 0; }
-          running[c] += t;
-        }
-        __syncthreads();
-      }
-      // ---- update: ordered sums per (cluster, column) ----
-      for (uint32_t q = tid; q < k * d; q += NT) {
-        const uint32_t c = q / d, j = q % d;
-        const uint32_t p0 = cstart[c], p1 = cstart[c + 1];
-        float s = 0.0f;
-        uint32_t p = p0;
-        for (; p + 4 <= p1; p += 4) {
-          const float v0 = __ldg(Xp + (uint64_t)perm[p] * d + j);
-          const float v1 = __ldg(Xp + (uint64_t)perm[p + 1] * d + j);
-          const float v2 = __ldg(Xp + (uint64_t)perm[p + 2] * d + j);
-          const float v3 = __ldg(Xp + (uint64_t)perm[p + 3] * d + j);
-          s = __fadd_rn(s, v0); s = __fadd_rn(s, v1); s = __fadd_rn(s, v2); s = __fadd_rn(s, v3);
-        }
-        for (; p < p1; ++p) s = __fadd_rn(s, __ldg(Xp + (uint64_t)perm[p] * d + j));
-        const uint32_t count = (p1 - p0) > 1u ? (p1 - p0) : 1u;
-        const float scale = (float)(1.0 / (double)count);
-        Cn[q] = __fmul_rn(s, scale);
-      }
-      if (tid == 0) s_moved = 0;
-      __syncthreads();
-      // ---- stop rule (from the second iteration) and centroid swap ----
-      if (iter > 1) {
-        for (uint32_t c = tid; c < k; c += NT) {
-          float s = 0.0f;
-          for (uint32_t j = 0; j < d; ++j) {
-            const float t = __fsub_rn(Cn[(uint64_t)c * d + j], Cs[(uint64_t)j * kpad + c]);
-            s = __fadd_rn(s, __fmul_rn(t, t));
-          }
-          if (sqrtf(s) > tol) s_moved = 1;
+    for (int j = 0; j < CT; ++j) {
+      const uint32_t c = c0 + 2u * (uint32_t)((j >> 1) * TX + tx) + (uint32_t)(j & 1);
+      if (c < k) {
+#pragma unroll
+        for (int i = 0; i < RT / 2; ++i) {
+          if (acc[i][j].x < bv[2 * i]) { bv[2 * i] = acc[i][j].x; bi[2 * i] = c; }
+          if (acc[i][j].y < bv[2 * i + 1]) { bv[2 * i + 1] = acc[i][j].y; bi[2 * i + 1] = c; }
         }
       }
-      __syncthreads();
-      const bool stop = iter > 1 && s_moved == 0;
-      for (uint32_t q = tid; q < k * d; q += NT) {
-        const uint32_t c = q / d, j = q % d;
-        Cs[(uint64_t)j * kpad + c] = Cn[q];
-      }
-      __syncthreads();
-      if (stop) { converged = iter; break; }
     }
-    if (iter > maxiter) iter = maxiter;
-    // results
-    for (uint32_t q = tid; q < k * d; q += NT) {
-      const uint32_t c = q / d, j = q % d;
-      Cout[I.coff + q] = Cs[(uint64_t)j * kpad + c];
+  }
+  // The rows' TX lists: smallest distance, lowest index on ties (a thread whose
+  // distances are all +inf holds index 0, as the reference's argmin starts with).
+  // Each step also halves the rows that a thread goes on with.
+  int row0 = ty * RT;
+#pragma unroll
+  for (int o = 1, live = RT; o < TX; o <<= 1) {
+    const bool up = (tx & o) != 0;
+    const int h = live > 1 ? live / 2 : 0;
+#pragma unroll
+    for (int i = 0; i < (h ? h : 1); ++i) {
+      const float sv = h ? (up ? bv[i] : bv[i + h]) : bv[i];
+      const uint32_t sx = h ? (up ? bi[i] : bi[i + h]) : bi[i];
+      float v = h && up ? bv[i + h] : bv[i];
+      uint32_t x = h && up ? bi[i + h] : bi[i];
+      const float ov = __shfl_xor_sync(0xffffffffu, sv, o);
+      const uint32_t ox = __shfl_xor_sync(0xffffffffu, sx, o);
+      if (ov < v || (ov == v && ox < x)) { v = ov; x = ox; }
+      bv[i] = v;
+      bi[i] = x;
     }
-    if (tid == 0) {
-      out[ii].converged_iter = converged;
-      out[ii].iterations = iter;
-      out[ii].objective = obj;
+    if (h) { row0 += up ? h : 0; live = h; }
+  }
+  constexpr int LEFT = RT > TX ? RT / TX : 1;              // rows a thread ends with
+  double obj = 0.0;
+#pragma unroll
+  for (int i = 0; i < LEFT; ++i) {
+    const uint32_t row = m0 + (uint32_t)(row0 + i);
+    if ((tx < RT || RT > TX) && row < n) {                 // TX > RT: the lanes above hold copies
+      lab[row] = bi[i];
+      obj += (double)bv[i];
+    }
+  }
+  for (int o = 16; o > 0; o >>= 1) obj += __shfl_xor_sync(0xffffffffu, obj, o);
+  if ((tid & 31) == 0) s_obj[tid >> 5] = obj;
+  __syncthreads();
+  if (tid == 0) {
+    double t = 0.0;
+    for (int w = 0; w < BA_NT / 32; ++w) t += s_obj[w];
+    *objtile = t;
+  }
+}
+
+// Index of the running instance that owns item t: the last a with first[a] <= t.
+__device__ __forceinline__ uint32_t batch_owner(const uint32_t* __restrict__ first, uint32_t nact, uint32_t t) {
+  uint32_t lo = 0, hi = nact;
+  while (hi - lo > 1u) {
+    const uint32_t mid = (lo + hi) / 2u;
+    if (__ldg(first + mid) <= t) lo = mid; else hi = mid;
+  }
+  return lo;
+}
+
+// The tiles of one group.  The groups' kernels follow one another in the stream
+// and may overlap: the first waits for the iteration before (so the later ones,
+// which start only when all its blocks have passed that wait, need not), and each
+// later one waits for its predecessor before it ends.
+template <int RT, int GROUP>
+__global__ void __launch_bounds__(BA_NT, RT == 8 ? 3 : 4)
+batch_assign_kernel(const float* __restrict__ X, const BatchInst* __restrict__ insts, BatchCtl* ctl,
+                    const uint32_t* __restrict__ act, const uint32_t* __restrict__ tile0,
+                    const float* __restrict__ Call, uint32_t* __restrict__ labels, double* __restrict__ objtile,
+                    int first, float neg0) {
+  if (first) griddep_wait();
+  griddep_launch();
+  __shared__ uint32_t s_tile;
+  const uint32_t nact = ctl->nact, begin = GROUP ? ctl->tile_end[GROUP ? GROUP - 1 : 0] : 0u,
+                 end = ctl->tile_end[GROUP];
+  for (;;) {
+    __syncthreads();                       // the tile before is done with s_tile and the stages
+    if (threadIdx.x == 0) s_tile = end > begin ? begin + atomicAdd(&ctl->next_tile[GROUP], 1u) : end;
+    __syncthreads();
+    const uint32_t t = s_tile;
+    if (t >= end) break;
+    const uint32_t a = batch_owner(tile0, nact, t);
+    const BatchInst I = insts[act[a]];
+    const uint32_t ti = t - tile0[a], m0 = ti * batch_tile_rows(I.k, RT);
+    const float* Xp = X + I.xoff;
+    const float* C = Call + I.coff;
+    const bool v4 = (I.d % 4u) == 0u && (I.xoff % 4u) == 0u;
+    uint32_t* lab = labels + I.loff;
+    double* ob = objtile + I.toff + ti;
+#define KM_BATCH_TILE(TX_, CT_) batch_tile<RT, TX_, CT_>(Xp, C, I.n, I.d, I.k, v4, m0, lab, ob, make_float2(neg0, neg0))
+    if constexpr (GROUP == 0) {
+      if (batch_cols(I.k) == 96u) KM_BATCH_TILE(16, 6); else KM_BATCH_TILE(16, 8);
+    } else if constexpr (GROUP == 1) {
+      if (batch_cols(I.k) == 48u) KM_BATCH_TILE(8, 6); else KM_BATCH_TILE(8, 8);
+    } else {
+      switch (batch_cols(I.k)) {
+        case 16: KM_BATCH_TILE(4, 4); break;
+        case 24: KM_BATCH_TILE(4, 6); break;
+        default: KM_BATCH_TILE(4, 8); break;
+      }
+    }
+#undef KM_BATCH_TILE
+  }
+  if (!first) griddep_wait();
+}
+
+// Stable counting sort of an instance's rows by label: each warp counts and then
+// scatters a contiguous run of rows.  Also lists the instance's update tasks.
+constexpr int BS_WARPS = 16;
+__global__ void __launch_bounds__(32 * BS_WARPS)
+batch_sort_kernel(const float* __restrict__ X, const BatchInst* __restrict__ insts, BatchCtl* ctl,
+                  const uint32_t* __restrict__ act, const uint32_t* __restrict__ labels,
+                  uint32_t* __restrict__ perm_all, float* __restrict__ Cn, BatchTask* __restrict__ longs,
+                  BatchTask* __restrict__ shorts) {
+  griddep_wait();
+  __shared__ uint32_t pos[BS_WARPS][256];
+  __shared__ uint32_t part[8];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const uint32_t nact = ctl->nact;
+  for (uint32_t a = blockIdx.x; a < nact; a += gridDim.x) {
+    const BatchInst& I = insts[act[a]];
+    const uint32_t n = I.n, k = I.k, d = I.d;
+    const uint32_t* lab = labels + I.loff;
+    uint32_t* perm = perm_all + I.loff;
+    for (uint32_t q = tid; q < BS_WARPS * 256u; q += 32 * BS_WARPS) (&pos[0][0])[q] = 0u;
+    __syncthreads();
+    const uint32_t per = ((n + BS_WARPS - 1) / BS_WARPS + 31u) & ~31u;
+    const uint32_t r0 = min(n, (uint32_t)warp * per), r1 = min(n, r0 + per);
+    constexpr int U = 8;                                   // labels in flight per lane
+    for (uint32_t g = r0; g < r1; g += 32u * U) {
+      uint32_t lv[U];
+#pragma unroll
+      for (int q = 0; q < U; ++q) {
+        const uint32_t r = g + 32u * q + lane;
+        lv[q] = r < r1 ? lab[r] : 0xffffffffu;
+      }
+#pragma unroll
+      for (int q = 0; q < U; ++q)
+        if (lv[q] != 0xffffffffu) atomicAdd(&pos[warp][lv[q]], 1u);
+    }
+    __syncthreads();
+    // thread c: the cluster's count over the warps, then an exclusive scan over
+    // the clusters (k <= 256) and over each cluster's warps
+    uint32_t cnt = 0;
+    if (tid < 256)
+      for (int w = 0; w < BS_WARPS; ++w) cnt += pos[w][tid];
+    uint32_t inc = cnt;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t y = __shfl_up_sync(0xffffffffu, inc, o);
+      if (lane >= o) inc += y;
+    }
+    if (tid < 256 && lane == 31) part[warp] = inc;
+    __syncthreads();
+    if (tid < 256) {
+      uint32_t base = inc - cnt;
+      for (int w = 0; w < warp; ++w) base += part[w];
+      // this warp's clusters to the two task lists (their order is free)
+      const bool in = (uint32_t)tid < k, ring = in && cnt >= BATCH_RING_ROWS;
+      const uint32_t nblk = (d + 31u) / 32u;
+      const unsigned ml = __ballot_sync(0xffffffffu, ring), ms = __ballot_sync(0xffffffffu, in && !ring);
+      uint32_t bl = 0, bs = 0;
+      if (lane == 0) {
+        if (ml) bl = atomicAdd(&ctl->nlong, (uint32_t)__popc(ml) * nblk);
+        if (ms) bs = atomicAdd(&ctl->nshort, (uint32_t)__popc(ms) * nblk);
+      }
+      bl = __shfl_sync(0xffffffffu, bl, 0);
+      bs = __shfl_sync(0xffffffffu, bs, 0);
+      if (in) {
+        const uint32_t at = (uint32_t)__popc((ring ? ml : ms) & ((1u << lane) - 1u)) * nblk + (ring ? bl : bs);
+        const uint32_t vec = (d % 4u == 0u && I.xoff % 4u == 0u) ? 4u : (d % 2u == 0u && I.xoff % 2u == 0u) ? 2u : 1u;
+        BatchTask* out = (ring ? longs : shorts) + at;
+        for (uint32_t b = 0; b < nblk; ++b)
+          out[b] = BatchTask{X + I.xoff + 32u * b, perm + base, Cn + I.coff + (uint64_t)tid * d + 32u * b, cnt, d,
+                             min(32u, d - 32u * b), vec};
+      }
+      for (int w = 0; w < BS_WARPS; ++w) {
+        const uint32_t v = pos[w][tid];
+        pos[w][tid] = base;
+        base += v;
+      }
+    }
+    __syncthreads();
+    for (uint32_t g = r0; g < r1; g += 32u * U) {
+      uint32_t lv[U];
+#pragma unroll
+      for (int q = 0; q < U; ++q) {
+        const uint32_t r = g + 32u * q + lane;
+        lv[q] = r < r1 ? lab[r] : 0xffffffffu;
+      }
+#pragma unroll
+      for (int q = 0; q < U; ++q) {
+        if (g + 32u * q >= r1) break;
+        const uint32_t l = lv[q];
+        const unsigned m = __match_any_sync(0xffffffffu, l);
+        const uint32_t rank = (uint32_t)__popc(m & ((1u << lane) - 1u));
+        const bool ok = l != 0xffffffffu;
+        const uint32_t base = ok ? pos[warp][l] : 0u;
+        __syncwarp();
+        if (ok) {
+          perm[base + rank] = g + 32u * q + lane;
+          if (rank == 0) pos[warp][l] = base + (uint32_t)__popc(m);
+        }
+        __syncwarp();
+      }
     }
     __syncthreads();
   }
+}
+
+// A predicated load (0 when !ok) that stays where it is written: plain loads
+// were moved down to the additions that use them, one latency each.
+__device__ __forceinline__ float ld_global_pinned(const float* p, bool ok) {
+  float v;
+  asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %2, 0;\n\tmov.f32 %0, 0f00000000;\n\t"
+               "@q ld.global.nc.f32 %0, [%1];\n\t}"
+               : "=f"(v)
+               : "l"(p), "r"((uint32_t)ok));
+  return v;
+}
+
+// Ordered sums.  Warps 0..3 of a CTA walk the long tasks (every gridDim-th) as
+// the producers and the chain of a shared-memory ring that runs on from task to
+// task (km_sums.cuh); the other warps, and these four once their long tasks are
+// done, take short tasks, a warp each, lane = column: 32 rows' loads at a time.
+// Rows past the cluster's end add +0, which leaves the sum as it is (it starts at
+// +0).  First iteration of the problems above: 0.57 ms for 10 M row segments of up
+// to 32 columns, against 4.1 ms with a warp for every task, whose longest chain
+// set the time.
+constexpr int BU_PROD = 3, BU_WARPS = 8;
+__global__ void __launch_bounds__(32 * BU_WARPS, 2)
+batch_update_kernel(BatchCtl* ctl, const BatchTask* __restrict__ longs, const BatchTask* __restrict__ shorts) {
+  griddep_wait();
+  extern __shared__ __align__(128) float ring[];
+  __shared__ __align__(8) uint64_t full[BLK_STAGES], empty[BLK_STAGES];
+  __shared__ int abort_flag;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const uint32_t nlong = ctl->nlong, nshort = ctl->nshort;
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < BLK_STAGES; ++s) { mbar_init(&full[s], 32); mbar_init(&empty[s], 1); }
+    abort_flag = 0;
+    mbar_fence_init();
+  }
+  __syncthreads();
+  auto write = [&](const BatchTask& t, float sum) {
+    if ((uint32_t)lane < t.w) {
+      const float scale = (float)(1.0 / (double)(t.cnt > 1u ? t.cnt : 1u));
+      t.out[lane] = __fmul_rn(sum, scale);
+    }
+  };
+  if (warp <= BU_PROD) {
+    const SumsRing R{ring, full, empty, &abort_flag};
+    uint32_t first = 0;
+    bool ok = true;
+    BatchTask next{};
+    if (blockIdx.x < nlong) next = longs[blockIdx.x];
+    for (uint32_t e = blockIdx.x; e < nlong && ok; e += gridDim.x) {
+      const BatchTask t = next;
+      if (e + gridDim.x < nlong) next = longs[e + gridDim.x];
+      if (warp < BU_PROD) {
+        const uint32_t p = (uint32_t)warp;
+        ok = t.vec == 4u   ? sums_produce<4, BU_PROD>(R, t.x, t.perm, t.cnt, t.d, t.w, first, p)
+             : t.vec == 2u ? sums_produce<2, BU_PROD>(R, t.x, t.perm, t.cnt, t.d, t.w, first, p)
+                           : sums_produce<1, BU_PROD>(R, t.x, t.perm, t.cnt, t.d, t.w, first, p);
+      } else {
+        float sum;
+        ok = sums_chain(R, t.cnt, first, sum);
+        if (ok) write(t, sum);
+      }
+      first += (t.cnt + BLK_ROWS - 1) / BLK_ROWS;
+    }
+    if (!ok && lane == 0) {
+      *(volatile int*)&abort_flag = 1;
+      atomicOr(&ctl->err, KM_DEVERR_TIMEOUT);
+    }
+    asm volatile("cp.async.wait_all;" ::: "memory");   // this warp's copies land before the CTA exits
+  }
+  for (;;) {
+    uint32_t e = 0;
+    if (lane == 0) e = nshort ? atomicAdd(&ctl->next_short, 1u) : 0u;
+    e = __shfl_sync(0xffffffffu, e, 0);
+    if (e >= nshort) break;
+    const BatchTask t = shorts[e];
+    const float* xc = t.x + lane;
+    float sum = 0.0f;
+    uint32_t idx = (uint32_t)lane < t.cnt ? __ldg(t.perm + lane) : 0u;
+    for (uint32_t g = 0; g < t.cnt; g += 32u) {
+      float v[32];
+#pragma unroll
+      for (int u = 0; u < 32; ++u) {
+        const uint32_t r = __shfl_sync(0xffffffffu, idx, u);
+        v[u] = ld_global_pinned(xc + (uint64_t)r * t.d, (uint32_t)lane < t.w && g + (uint32_t)u < t.cnt);
+      }
+      const uint32_t q = g + 32u + (uint32_t)lane;
+      idx = q < t.cnt ? __ldg(t.perm + q) : 0u;
+#pragma unroll
+      for (int u = 0; u < 32; ++u) sum = __fadd_rn(sum, v[u]);
+    }
+    write(t, sum);
+  }
+}
+
+// Lists the instances of act[0 .. nact) that are not done (all of them when
+// done is null), in order, with the first tile of each; resets the counters.
+// One block.
+__device__ void batch_list(const BatchInst* __restrict__ insts, BatchCtl* ctl, uint32_t* act, uint32_t* tile0,
+                           const uint32_t* done, uint32_t nact, uint32_t rt, uint32_t* sh) {
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nw = (int)blockDim.x >> 5;
+  uint32_t b0 = 0, b1 = 0;                                 // running totals: instances, tiles
+  if (tid < 3) sh[64 + tid] = 0u;                          // last tile of each group + 1
+  for (uint32_t g = 0; g < nact; g += blockDim.x) {
+    const uint32_t q = g + (uint32_t)tid;
+    uint32_t id = 0, f0 = 0, f1 = 0;
+    if (q < nact) {
+      id = done ? __ldcg(act + q) : q;
+      if (!done || __ldcg(done + id) == 0u) {
+        const BatchInst& I = insts[id];
+        f0 = 1u;
+        f1 = batch_tiles(I.n, I.k, rt);
+      }
+    }
+    uint32_t x0 = f0, x1 = f1;                             // inclusive scans over the warp
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t y0 = __shfl_up_sync(0xffffffffu, x0, o), y1 = __shfl_up_sync(0xffffffffu, x1, o);
+      if (lane >= o) { x0 += y0; x1 += y1; }
+    }
+    if (lane == 31) { sh[warp] = x0; sh[32 + warp] = x1; }
+    __syncthreads();                                       // every read of this chunk of act is done, too
+    uint32_t t0 = 0, t1 = 0, e0 = 0, e1 = 0;
+    for (int w = 0; w < nw; ++w) {
+      if (w == warp) { e0 = t0; e1 = t1; }
+      t0 += sh[w]; t1 += sh[32 + w];
+    }
+    if (f0) {
+      const uint32_t at = b0 + e0 + x0 - 1u;
+      act[at] = id;
+      tile0[at] = b1 + e1 + x1 - f1;
+      atomicMax(&sh[64 + batch_group(insts[id].k)], b1 + e1 + x1);
+    }
+    b0 += t0; b1 += t1;
+    __syncthreads();
+  }
+  if (tid == 0) {
+    ctl->nact = b0;
+    for (uint32_t q = 0, e = 0; q < 3u; ++q) {             // an empty group ends where the one before it does
+      e = max(e, sh[64 + q]);
+      ctl->tile_end[q] = e;
+      ctl->next_tile[q] = 0u;
+    }
+    ctl->nlong = ctl->nshort = ctl->next_short = ctl->ticket = 0u;
+  }
+}
+
+__global__ void __launch_bounds__(1024)
+batch_begin_kernel(const BatchInst* __restrict__ insts, BatchCtl* ctl, uint32_t* act, uint32_t* tile0,
+                   uint32_t* done, uint32_t ninst, uint32_t rt) {
+  __shared__ uint32_t sh[67];
+  for (uint32_t i = threadIdx.x; i < ninst; i += blockDim.x) done[i] = 0u;
+  batch_list(insts, ctl, act, tile0, nullptr, ninst, rt, sh);
+  if (threadIdx.x == 0) { ctl->iter = 0; ctl->err = 0u; }
+}
+
+__global__ void __launch_bounds__(256)
+batch_stop_kernel(const BatchInst* __restrict__ insts, BatchCtl* ctl, uint32_t* act, uint32_t* tile0, uint32_t* done,
+                  float* __restrict__ Call, const float* __restrict__ Cn_all,
+                  const double* __restrict__ objtile, float tol, uint64_t maxiter, uint32_t rt,
+                  BatchOut* __restrict__ out) {
+  griddep_wait();
+  __shared__ int s_moved;
+  __shared__ int is_last;
+  __shared__ uint32_t sh[67];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const uint32_t nact = ctl->nact;
+  if (nact == 0u) return;
+  const uint64_t iter = ctl->iter + 1;
+  for (uint32_t a = blockIdx.x; a < nact; a += gridDim.x) {
+    const uint32_t id = act[a];
+    const BatchInst& I = insts[id];
+    const uint32_t d = I.d, k = I.k;
+    float* C = Call + I.coff;
+    const float* Cn = Cn_all + I.coff;
+    if (tid == 0) s_moved = 0;
+    __syncthreads();
+    if (iter > 1) {
+      // a warp per cluster, until one is found that moved
+      for (uint32_t c = (uint32_t)warp; c < k && *(volatile int*)&s_moved == 0; c += 8u) {
+        float s = 0.0f;                                    // column order
+        for (uint32_t j0 = 0; j0 < d; j0 += 32u) {
+          const uint32_t j = j0 + (uint32_t)lane;
+          float q = 0.0f;
+          if (j < d) {
+            const float t = __fsub_rn(Cn[(uint64_t)c * d + j], C[(uint64_t)c * d + j]);
+            q = __fmul_rn(t, t);
+          }
+#pragma unroll
+          for (int l = 0; l < 32; ++l) s = __fadd_rn(s, __shfl_sync(0xffffffffu, q, l));   // past d: + 0
+        }
+        if (lane == 0 && sqrtf(s) > tol) s_moved = 1;
+        __syncwarp();
+      }
+    }
+    __syncthreads();
+    const bool stop = iter > 1 && s_moved == 0;
+    for (uint32_t q = tid; q < k * d; q += 256u) C[q] = Cn[q];
+    if (stop || iter >= maxiter) {
+      if (warp == 0) {
+        const uint32_t nt = batch_tiles(I.n, I.k, rt);
+        double o = 0.0;
+        for (uint32_t t = (uint32_t)lane; t < nt; t += 32u) o += objtile[I.toff + t];
+        for (int w = 16; w > 0; w >>= 1) o += __shfl_xor_sync(0xffffffffu, o, w);
+        if (lane == 0) {
+          out[id].converged_iter = stop ? iter : maxiter;
+          out[id].iterations = iter;
+          out[id].objective = o;
+          done[id] = 1u;
+        }
+      }
+    }
+    __syncthreads();
+  }
+  __threadfence();
+  __syncthreads();
+  if (tid == 0) is_last = (atomicAdd(&ctl->ticket, 1u) == gridDim.x - 1u) ? 1 : 0;
+  __syncthreads();
+  if (!is_last) return;
+  __threadfence();
+  batch_list(insts, ctl, act, tile0, done, nact, rt, sh);
+  if (tid == 0) ctl->iter = iter;
 }
 
 // Reference sample picks (kmeans.cpp:22-29, :49-84) on the host copy of X.
@@ -242,19 +693,12 @@ bool host_sample_picks(const float* X, uint64_t n, uint32_t d, uint32_t k, int s
   return true;
 }
 
-using BatchKernel = void (*)(const float*, const BatchInst*, uint32_t, const float*, float*, uint32_t*,
-                             uint32_t*, float*, uint64_t, uint64_t, uint32_t*, float, uint64_t, BatchOut*);
-
+// Tile variants of the assign step: rows per thread and CTAs per SM.
 struct BatchVariant {
-  BatchKernel fn;
-  int nt, cg;
+  int rt, ctas;
 };
-
-const BatchVariant kVariants[] = {
-    {batch_lloyd_kernel<128, 8>, 128, 8},   {batch_lloyd_kernel<128, 16>, 128, 16},
-    {batch_lloyd_kernel<128, 32>, 128, 32}, {batch_lloyd_kernel<256, 8>, 256, 8},
-    {batch_lloyd_kernel<256, 16>, 256, 16}, {batch_lloyd_kernel<256, 32>, 256, 32},
-};
+const BatchVariant kVariants[] = {{8, 3}, {8, 2}, {8, 1}, {4, 4}, {4, 3}, {4, 2}};
+constexpr int kDefaultVariant = 0;
 
 }  // namespace
 }  // namespace km
@@ -268,25 +712,30 @@ struct km_batch {
   int device = 0, num_sms = 0;
   cudaStream_t stream = nullptr;
   bool own_stream = false;
-  uint64_t x_floats = 0, lab_total = 0, c_total = 0, max_n = 0, max_kd = 0;
-  size_t smem = 0;
+  uint32_t groups = 0;                  // groups of assign shapes in use (bit mask)
+  uint64_t x_floats = 0, lab_total = 0, c_total = 0, task_total = 0, t_total = 0;
   float* X = nullptr;
   float* C0 = nullptr;
-  float* Cout = nullptr;
+  float* C = nullptr;                   // current centroids, the result at the end
+  float* Cn = nullptr;                  // next centroids
   uint32_t* labels = nullptr;
   uint32_t* perm = nullptr;
-  float* cnew = nullptr;
+  BatchTask* tasks = nullptr;           // long, then short: task_total each
+  double* objtile = nullptr;
   BatchInst* dinst = nullptr;
   BatchOut* dout = nullptr;
-  uint32_t* next = nullptr;
-  int variant = -1;
+  BatchCtl* ctl = nullptr;
+  uint32_t* lists = nullptr;            // act, tile0, done: one entry per instance each
+  BatchCtl* h_ctl = nullptr;            // pinned
+  int variant = kDefaultVariant;
   double tune_ms[6] = {0, 0, 0, 0, 0, 0};
   bool ready = false;
   ~km_batch() {
     if (device >= 0) cudaSetDevice(device);
-    for (void* q : {(void*)X, (void*)C0, (void*)Cout, (void*)labels, (void*)perm, (void*)cnew, (void*)dinst,
-                    (void*)dout, (void*)next})
+    for (void* q : {(void*)X, (void*)C0, (void*)C, (void*)Cn, (void*)labels, (void*)perm, (void*)tasks,
+                    (void*)objtile, (void*)dinst, (void*)dout, (void*)ctl, (void*)lists})
       if (q) cudaFree(q);
+    if (h_ctl) cudaFreeHost(h_ctl);
     if (own_stream && stream) cudaStreamDestroy(stream);
   }
 };
@@ -302,29 +751,73 @@ km_status balloc(T** p, size_t count) {
   return KM_OK;
 }
 
-// One launch of the persistent kernel over instances [0, ninst) of dinst.
+// The launches of one iteration of the running instances.
+template <int RT>
+km_status enqueue_batch_iteration(km_batch* h, int ctas, const BatchInst* dinst, uint32_t ninst, uint64_t maxiter) {
+  uint32_t *act = h->lists, *tile0 = act + h->inst.size(), *done = tile0 + h->inst.size();
+  BatchTask *longs = h->tasks, *shorts = h->tasks + h->task_total;
+  const unsigned per_inst = (unsigned)std::min<uint32_t>(ninst, (uint32_t)h->num_sms * 2u);
+  int first = 1;
+  auto assign = [&](auto kern, int group) -> km_status {
+    if (!(h->groups & (1u << group))) return KM_OK;
+    KM_CUDA_TRY(launch_pdl(kern, h->num_sms * ctas, BA_NT, batch_assign_smem<RT>(), h->stream, h->X, dinst, h->ctl, act,
+                           tile0, h->C, h->labels, h->objtile, first, -0.0f));
+    first = 0;
+    return KM_OK;
+  };
+  KM_TRY(assign(batch_assign_kernel<RT, 0>, 0));
+  KM_TRY(assign(batch_assign_kernel<RT, 1>, 1));
+  KM_TRY(assign(batch_assign_kernel<RT, 2>, 2));
+  KM_CUDA_TRY(launch_pdl(batch_sort_kernel, per_inst, 32 * BS_WARPS, 0, h->stream, h->X, dinst, h->ctl, act, h->labels,
+                         h->perm, h->Cn, longs, shorts));
+  KM_CUDA_TRY(launch_pdl(batch_update_kernel, h->num_sms * 2, 32 * BU_WARPS, BLK_SMEM, h->stream, h->ctl, longs,
+                         shorts));
+  KM_CUDA_TRY(launch_pdl(batch_stop_kernel, per_inst, 256, 0, h->stream, dinst, h->ctl, act, tile0, done, h->C, h->Cn,
+                         h->objtile, h->p.tol, maxiter, (uint32_t)RT, h->dout));
+  return KM_OK;
+}
+
+// All iterations of instances [0, ninst) of dinst.
 km_status run_batch(km_batch* h, int v, const BatchInst* dinst, uint32_t ninst, uint64_t maxiter,
                     float* ms_out) {
   const BatchVariant& V = kVariants[v];
-  const uint64_t perm_stride = (h->max_n + 31) / 32 * 32, cnew_stride = (h->max_kd + 31) / 32 * 32;
-  KM_CUDA_TRY(cudaMemsetAsync(h->next, 0, sizeof(uint32_t), h->stream));
+  const size_t total = h->inst.size();
   cudaEvent_t e0, e1;
   KM_CUDA_TRY(cudaEventCreate(&e0));
-  KM_CUDA_TRY(cudaEventCreate(&e1));
-  KM_CUDA_TRY(cudaEventRecord(e0, h->stream));
-  V.fn<<<h->num_sms, V.nt, h->smem, h->stream>>>(h->X, dinst, ninst, h->C0, h->Cout, h->labels, h->perm,
-                                                  h->cnew, perm_stride, cnew_stride, h->next, h->p.tol,
-                                                  maxiter, h->dout);
-  cudaError_t le = cudaGetLastError();
-  KM_CUDA_TRY(cudaEventRecord(e1, h->stream));
-  KM_CUDA_TRY(cudaEventSynchronize(e1));
-  float ms = 0.f;
-  cudaEventElapsedTime(&ms, e0, e1);
+  if (cudaEventCreate(&e1) != cudaSuccess) { cudaEventDestroy(e0); return KM_ERR_CUDA; }
+  auto body = [&]() -> km_status {
+    KM_CUDA_TRY(cudaEventRecord(e0, h->stream));
+    KM_CUDA_TRY(cudaMemcpyAsync(h->C, h->C0, sizeof(float) * h->c_total, cudaMemcpyDeviceToDevice, h->stream));
+    batch_begin_kernel<<<1, 1024, 0, h->stream>>>(dinst, h->ctl, h->lists, h->lists + total, h->lists + 2 * total,
+                                                  ninst, (uint32_t)V.rt);
+    KM_CUDA_TRY(cudaGetLastError());
+    // A few iterations are queued between looks at the device's count of
+    // running instances (launches past the end find none and return).
+    uint64_t done = 0, step = 2;
+    while (done < maxiter) {
+      const uint64_t target = std::min<uint64_t>(maxiter, done + step);
+      for (; done < target; ++done)
+        KM_TRY(V.rt == 8 ? enqueue_batch_iteration<8>(h, V.ctas, dinst, ninst, maxiter)
+                         : enqueue_batch_iteration<4>(h, V.ctas, dinst, ninst, maxiter));
+      if (done >= maxiter) break;
+      KM_CUDA_TRY(cudaMemcpyAsync(h->h_ctl, h->ctl, sizeof(BatchCtl), cudaMemcpyDeviceToHost, h->stream));
+      KM_CUDA_TRY(cudaStreamSynchronize(h->stream));
+      if (h->h_ctl->nact == 0u || h->h_ctl->err) break;
+      step = 4;
+    }
+    KM_CUDA_TRY(cudaEventRecord(e1, h->stream));
+    KM_CUDA_TRY(cudaMemcpyAsync(h->h_ctl, h->ctl, sizeof(BatchCtl), cudaMemcpyDeviceToHost, h->stream));
+    KM_CUDA_TRY(cudaStreamSynchronize(h->stream));
+    KM_TRY(status_of_device_error(h->h_ctl->err));
+    float ms = 0.f;
+    KM_CUDA_TRY(cudaEventElapsedTime(&ms, e0, e1));
+    if (ms_out) *ms_out = ms;
+    return KM_OK;
+  };
+  const km_status s = body();
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
-  KM_CUDA_TRY(le);
-  if (ms_out) *ms_out = ms;
-  return KM_OK;
+  return s;
 }
 
 }  // namespace
@@ -347,32 +840,40 @@ km_status km_batch_create(const km_batch_params* p, const km_batch_problem* prob
     if (q.n == 0 || q.d == 0 || q.k == 0 || q.k > q.n || q.k > 256 || q.n >= (1ull << 31)) { delete h; return KM_ERR_ARG; }
     const uint32_t kpad = (q.k + 31) / 32 * 32;
     if ((uint64_t)q.d * kpad * 4 > BATCH_MAX_SMEM_C) { delete h; return KM_ERR_UNSUPPORTED; }
-    h->max_n = std::max<uint64_t>(h->max_n, q.n);
-    h->max_kd = std::max<uint64_t>(h->max_kd, (uint64_t)q.k * q.d);
-    h->smem = std::max<size_t>(h->smem, (size_t)q.d * kpad * 4);
     xoff += q.n * q.d;
   }
   h->x_floats = xoff;
-  // instances in LPT order (n*k*d descending, then problem, restart)
+  // instances by group of assign shapes, then in LPT order (n*k*d descending,
+  // then problem, restart)
   uint64_t px = 0;
   std::vector<BatchInst> inst;
   for (uint32_t pi = 0; pi < p->problems; ++pi) {
     const km_batch_problem& q = h->probs[pi];
     for (uint32_t r = 0; r < p->restarts; ++r) {
       BatchInst I{};
-      I.xoff = px; I.n = (uint32_t)q.n; I.d = q.d; I.k = q.k; I.kpad = (q.k + 31) / 32 * 32;
+      I.xoff = px; I.n = (uint32_t)q.n; I.d = q.d; I.k = q.k;
       I.prob = pi; I.restart = r;
       inst.push_back(I);
     }
     px += q.n * q.d;
   }
   std::stable_sort(inst.begin(), inst.end(), [](const BatchInst& a, const BatchInst& b) {
-    return (uint64_t)a.n * a.k * a.d > (uint64_t)b.n * b.k * b.d;
+    const uint32_t ga = batch_group(a.k), gb = batch_group(b.k);
+    return ga != gb ? ga < gb : (uint64_t)a.n * a.k * a.d > (uint64_t)b.n * b.k * b.d;
   });
-  uint64_t loff = 0, coff = 0;
-  for (BatchInst& I : inst) { I.loff = loff; I.coff = coff; loff += I.n; coff += (uint64_t)I.k * I.d; }
+  for (const BatchInst& I : inst) h->groups |= 1u << batch_group(I.k);
+  uint64_t loff = 0, coff = 0, tasks = 0, toff = 0;
+  for (BatchInst& I : inst) {
+    I.loff = loff; I.coff = coff; I.toff = toff;
+    loff += I.n;
+    coff += ((uint64_t)I.k * I.d + 3) / 4 * 4;              // 16-byte aligned centroids
+    tasks += (uint64_t)I.k * ((I.d + 31) / 32);
+    toff += batch_tiles(I.n, I.k, 4);                       // the smallest tiles of the variants
+  }
   h->lab_total = loff;
   h->c_total = coff;
+  h->task_total = tasks;
+  h->t_total = toff;
   h->inst = inst;
   km_status s = KM_OK;
   if (cudaSetDevice(h->device) != cudaSuccess) { (void)cudaGetLastError(); delete h; return KM_ERR_CUDA; }
@@ -382,20 +883,29 @@ km_status km_batch_create(const km_batch_params* p, const km_batch_problem* prob
   else { (void)cudaGetLastError(); delete h; return KM_ERR_CUDA; }
   if (s == KM_OK) s = balloc(&h->X, h->x_floats);
   if (s == KM_OK) s = balloc(&h->C0, h->c_total);
-  if (s == KM_OK) s = balloc(&h->Cout, h->c_total);
+  if (s == KM_OK) s = balloc(&h->C, h->c_total);
+  if (s == KM_OK) s = balloc(&h->Cn, h->c_total);
   if (s == KM_OK) s = balloc(&h->labels, h->lab_total);
-  if (s == KM_OK) s = balloc(&h->perm, (size_t)h->num_sms * ((h->max_n + 31) / 32 * 32));
-  if (s == KM_OK) s = balloc(&h->cnew, (size_t)h->num_sms * ((h->max_kd + 31) / 32 * 32));
+  if (s == KM_OK) s = balloc(&h->perm, h->lab_total);
+  if (s == KM_OK) s = balloc(&h->tasks, 2 * h->task_total);
+  if (s == KM_OK) s = balloc(&h->objtile, h->t_total);
   if (s == KM_OK) s = balloc(&h->dinst, inst.size());
   if (s == KM_OK) s = balloc(&h->dout, inst.size());
-  if (s == KM_OK) s = balloc(&h->next, 1);
+  if (s == KM_OK) s = balloc(&h->ctl, 1);
+  if (s == KM_OK) s = balloc(&h->lists, 3 * inst.size());
+  if (s == KM_OK && cudaMallocHost(reinterpret_cast<void**>(&h->h_ctl), sizeof(BatchCtl)) != cudaSuccess)
+    s = KM_ERR_ALLOC;
   if (s == KM_OK && cudaMemcpyAsync(h->dinst, inst.data(), sizeof(BatchInst) * inst.size(), cudaMemcpyHostToDevice,
                                     h->stream) != cudaSuccess) s = KM_ERR_CUDA;
   if (s == KM_OK) {
-    for (const BatchVariant& V : kVariants)
-      if (h->smem > 48 * 1024 &&
-          cudaFuncSetAttribute(V.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)h->smem) != cudaSuccess)
-        s = KM_ERR_CUDA;
+    cudaError_t e = cudaFuncSetAttribute(batch_update_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)BLK_SMEM);
+    for (auto kern : {batch_assign_kernel<8, 0>, batch_assign_kernel<8, 1>, batch_assign_kernel<8, 2>})
+      if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)batch_assign_smem<8>());
+    for (auto kern : {batch_assign_kernel<4, 0>, batch_assign_kernel<4, 1>, batch_assign_kernel<4, 2>})
+      if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)batch_assign_smem<4>());
+    if (e != cudaSuccess) s = KM_ERR_CUDA;
   }
   if (s != KM_OK) { (void)cudaGetLastError(); delete h; return s; }
   *out = h;
@@ -464,7 +974,6 @@ km_status km_batch_fit(km_batch* h, km_batch_result* results, uint32_t* best_lab
   if (!h) return KM_ERR_ARG;
   if (!h->ready) return KM_ERR_STATE;
   KM_CUDA_TRY(cudaSetDevice(h->device));
-  if (h->variant < 0) KM_TRY(km_batch_tune(h, nullptr, nullptr));
   float ms = 0.f;
   KM_TRY(run_batch(h, h->variant, h->dinst, (uint32_t)h->inst.size(), h->p.maxiter, &ms));
   if (fit_ms) *fit_ms = ms;
@@ -492,7 +1001,7 @@ km_status km_batch_fit(km_batch* h, km_batch_result* results, uint32_t* best_lab
     if (best_labels)
       KM_CUDA_TRY(cudaMemcpy(best_labels + lo, h->labels + I.loff, sizeof(uint32_t) * I.n, cudaMemcpyDeviceToHost));
     if (best_centroids)
-      KM_CUDA_TRY(cudaMemcpy(best_centroids + co, h->Cout + I.coff, sizeof(float) * I.k * I.d,
+      KM_CUDA_TRY(cudaMemcpy(best_centroids + co, h->C + I.coff, sizeof(float) * I.k * I.d,
                              cudaMemcpyDeviceToHost));
     lo += I.n;
     co += (uint64_t)I.k * I.d;
@@ -509,7 +1018,7 @@ km_status km_batch_instance_labels(km_batch* h, uint32_t problem, uint32_t resta
     if (labels_out)
       KM_CUDA_TRY(cudaMemcpy(labels_out, h->labels + I.loff, sizeof(uint32_t) * I.n, cudaMemcpyDeviceToHost));
     if (centroids_out)
-      KM_CUDA_TRY(cudaMemcpy(centroids_out, h->Cout + I.coff, sizeof(float) * I.k * I.d, cudaMemcpyDeviceToHost));
+      KM_CUDA_TRY(cudaMemcpy(centroids_out, h->C + I.coff, sizeof(float) * I.k * I.d, cudaMemcpyDeviceToHost));
     return KM_OK;
   }
   return KM_ERR_ARG;

@@ -69,6 +69,10 @@ enum : uint32_t {
 // visible).  In a kernel launched without the attribute the wait is a no-op.
 __device__ __forceinline__ void griddep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
+// Lets the next kernel of the stream (launched with launch_pdl) start as this
+// one's blocks make room, instead of after its end.
+__device__ __forceinline__ void griddep_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 template <typename... KArgs, typename... Args>
 inline cudaError_t launch_pdl(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t s,
                               Args... args) {

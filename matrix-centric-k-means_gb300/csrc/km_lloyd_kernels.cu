@@ -13,6 +13,7 @@
 //   convergence           comparisons/CPU_Kmeans/src/kmeans.cpp:170-200;
 //                         src/kmeans.cu:1054-1073 (score rule)
 #include "km_lloyd.cuh"
+#include "km_sums.cuh"
 
 #include <cmath>
 #include <cfloat>
@@ -1195,47 +1196,16 @@ __global__ void seg_scatter_kernel(const uint32_t* __restrict__ labels, uint64_t
 // 447 -> 72 us.  TMA row gathers (tile::gather4) were slower: 119 rows/us.
 //
 // Every wait is bounded; on timeout the CTA flags KM_DEVERR_TIMEOUT and drains
-// its copies before exiting.  Permutation indices are prefetched P batches ahead
-// in registers consumed in place.  A batch is BLK_ROWS = 128 rows (four groups of
-// 32): every batch costs a consumer one wait and one release of fixed latency.
-// BLK_STAGES is a multiple of the producers, so a stage is always refilled by the
-// same producer, which waits on its phases in order (a parity wait can never alias
-// a later phase).
+// its copies before exiting.  A batch is BLK_ROWS = 128 rows (four groups of 32):
+// every batch costs a consumer one wait and one release of fixed latency.
 // ---------------------------------------------------------------------------
 namespace {
-constexpr int BLK_ROWS = 128, BLK_GRP = 32, BLK_STAGES = 6, BLK_COLS = 32;
 // Producer warps by copy width: narrower copies take two or four times the
 // instructions, so six warps issue them.  Measured, one cluster of 100,000 rows:
 // 16 bytes 322 rows/us with two, three or six producers (the chain's rate), 8
 // bytes 212 with three and 263 with six, 4 bytes 113 and 173.
 constexpr int blk_producers(int vec) { return vec == 4 ? 3 : 6; }
-static_assert(BLK_ROWS == 4 * BLK_GRP, "the chain warp alternates two register groups over four groups a batch");
-constexpr uint64_t BLK_WAIT_NS = 2000000000ull;
-constexpr uint32_t BLK_SUSPEND_NS = 2000;       // try_wait suspend hint
-constexpr size_t BLK_SMEM = (size_t)BLK_STAGES * BLK_ROWS * BLK_COLS * sizeof(float);
 constexpr int blk_threads(int vec) { return 32 * (blk_producers(vec) + 2); }
-
-// An ordered shared-memory load (kept beside the arithmetic that follows it).
-__device__ __forceinline__ float ld_shared_f32(uint32_t addr) {
-  float v;
-  asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(addr));
-  return v;
-}
-
-// VEC columns (4 * VEC bytes, aligned to their size), zero-filled when !ok.
-template <int VEC>
-__device__ __forceinline__ void cp_async_cols(void* smem, const float* gmem, bool ok) {
-  const uint32_t bytes = ok ? 4u * VEC : 0u;
-  if constexpr (VEC == 4) {
-    cp_async16_zfill(smem, gmem, bytes);
-  } else if constexpr (VEC == 2) {
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(smem_u32(smem)), "l"(gmem), "r"(bytes)
-                 : "memory");
-  } else {
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(smem_u32(smem)), "l"(gmem), "r"(bytes)
-                 : "memory");
-  }
-}
 }  // namespace
 
 template <int VEC>
@@ -1246,7 +1216,6 @@ update_sums_bulk_kernel(const float* __restrict__ X, const uint32_t* __restrict_
                         float* __restrict__ dsq, double* __restrict__ objpart, DevState* st,
                         const uint32_t* __restrict__ order) {
   constexpr int PROD = blk_producers(VEC);
-  static_assert(BLK_STAGES % PROD == 0, "a stage must always belong to the same producer");
   griddep_wait();
   if (st && st->done) return;
   extern __shared__ __align__(128) float ring[];        // [BLK_STAGES][BLK_ROWS][BLK_COLS]
@@ -1273,108 +1242,17 @@ update_sums_bulk_kernel(const float* __restrict__ X, const uint32_t* __restrict_
     if (st) atomicOr(&st->err, KM_DEVERR_TIMEOUT);
   };
 
+  const SumsRing R{ring, full, empty, ab};
   if (warp < PROD) {
-    constexpr int P = 2;                       // batches of indices prefetched per producer
-    constexpr int G = BLK_ROWS / BLK_GRP;
-    const uint32_t p0 = (uint32_t)warp;
-    uint32_t pq[P][G];
-    auto load_idx = [&](uint32_t (&q)[G], uint32_t b) {     // group g of batch b: rows 32 g + lane
-#pragma unroll
-      for (int g = 0; g < G; ++g) {
-        const uint32_t idx = s0 + b * BLK_ROWS + (uint32_t)(g * BLK_GRP) + (uint32_t)lane;
-        q[g] = (b < nb && idx < s1) ? perm[idx] : 0u;
-      }
-    };
-#pragma unroll
-    for (int i = 0; i < P; ++i) load_idx(pq[i], p0 + (uint32_t)i * PROD);
-    // Unrolled by P so that pq[i] is consumed in place, P batches after its
-    // load was issued (moving a register whose load is in flight would wait).
-    bool ok = true;
-    for (uint32_t lb0 = 0; p0 + lb0 * PROD < nb && ok; lb0 += P) {
-#pragma unroll
-      for (int i = 0; i < P; ++i) {
-        const uint32_t b = p0 + (lb0 + (uint32_t)i) * PROD;
-        if (b >= nb || !ok) break;
-        const uint32_t s = b % BLK_STAGES, ph = (b / BLK_STAGES) & 1u;
-        const bool okw = mbar_wait_bounded(&empty[s], ph ^ 1u, ab, BLK_WAIT_NS, BLK_SUSPEND_NS);
-        if (!__all_sync(0xffffffffu, okw)) { if (lane == 0) fail(); ok = false; break; }
-        constexpr int LPR = BLK_COLS / VEC;    // lanes per row
-        constexpr int RPI = 32 / LPR;          // rows per copy instruction
-        const uint32_t m = min((uint32_t)BLK_ROWS, s1 - (s0 + b * BLK_ROWS));
-        // columns past w and rows past m zero-fill
-        const uint32_t sub = (uint32_t)lane / LPR, cv = ((uint32_t)lane % LPR) * (uint32_t)VEC;
-        const bool lane_has_cols = cv < w;
-        const float* xl = X + j0 + cv;
-#pragma unroll
-        for (int g = 0; g < G; ++g) {
-          float* dst = ring + ((size_t)s * BLK_ROWS + (size_t)(g * BLK_GRP) + sub) * BLK_COLS + cv;
-          // All row indices of the group first: each cp.async is an ordered asm
-          // statement, so a shuffle placed between two of them would put its
-          // latency on every row.
-          uint32_t rr[BLK_GRP / RPI];
-#pragma unroll
-          for (int ii = 0; ii < BLK_GRP / RPI; ++ii)
-            rr[ii] = __shfl_sync(0xffffffffu, pq[i][g], ii * RPI + (int)sub);
-#pragma unroll
-          for (int ii = 0; ii < BLK_GRP / RPI; ++ii) {
-            const uint32_t u = (uint32_t)(g * BLK_GRP + ii * RPI) + sub;
-            const bool okr = u < m && lane_has_cols;
-            const float* src = okr ? xl + (uint64_t)rr[ii] * d : X;
-            cp_async_cols<VEC>(dst + (size_t)ii * RPI * BLK_COLS, src, okr);
-          }
-        }
-        cp_async_mbar_arrive_noinc(&full[s]);
-        load_idx(pq[i], b + (uint32_t)P * PROD);
-      }
-    }
+    if (!sums_produce<VEC, PROD>(R, X + j0, perm + s0, s1 - s0, d, w, 0u, (uint32_t)warp) && lane == 0) fail();
     // Drain: this warp's copies must land before the CTA exits.
     asm volatile("cp.async.wait_all;" ::: "memory");
     return;
   }
 
   if (warp == PROD) {
-    // The ordered chain, lane = column within the block.  A group of 32 rows is
-    // added while the next one is loaded, one load beside each addition (32
-    // loads in a block would hold the warp's issue until the shared-memory queue
-    // took them all); the next batch's barrier is tested a group ahead of its
-    // use.  Rows past the cluster's end are zero-filled: adding +0 leaves the sum
-    // as it is (a sum that starts at +0 is never -0).
-    constexpr uint32_t RB = BLK_COLS * 4u, GB = BLK_GRP * RB, SB = BLK_ROWS * RB;   // bytes of a row, group, stage
-    float va[BLK_GRP], vb[BLK_GRP];
-    float sum = 0.0f;
-    auto step = [&](const float (&v)[BLK_GRP], float (&x)[BLK_GRP], uint32_t src) {
-#pragma unroll
-      for (int u = 0; u < BLK_GRP; ++u) {
-        x[u] = ld_shared_f32(src + (uint32_t)u * RB);
-        asm volatile("add.rn.f32 %0, %0, %1;" : "+f"(sum) : "f"(v[u]));
-      }
-    };
-    const uint32_t base = smem_u32(ring) + (uint32_t)lane * 4u;
-    uint32_t s = 0, ph = 0;
-    bool ok = nb == 0u || mbar_wait_bounded(&full[0], 0, ab, BLK_WAIT_NS, BLK_SUSPEND_NS);
-    if (!__all_sync(0xffffffffu, ok)) { if (lane == 0) fail(); return; }
-    if (nb) {
-#pragma unroll
-      for (int u = 0; u < BLK_GRP; ++u) va[u] = ld_shared_f32(base + (uint32_t)u * RB);
-    }
-    for (uint32_t left = nb; left; --left) {
-      const uint32_t src = base + s * SB;
-      const uint32_t sn = s + 1u == (uint32_t)BLK_STAGES ? 0u : s + 1u, phn = sn ? ph : ph ^ 1u;
-      step(va, vb, src + GB);
-      step(vb, va, src + 2 * GB);
-      ok = left == 1u || mbar_test_wait(&full[sn], phn);
-      step(va, vb, src + 3 * GB);
-      if (!__all_sync(0xffffffffu, ok)) {
-        ok = mbar_wait_bounded(&full[sn], phn, ab, BLK_WAIT_NS, BLK_SUSPEND_NS);
-        if (!__all_sync(0xffffffffu, ok)) { if (lane == 0) fail(); return; }
-      }
-      // (after the last batch the next stage holds old rows or none: unused)
-      step(vb, va, base + sn * SB);
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&empty[s]);
-      s = sn;
-      ph = phn;
-    }
+    float sum;
+    if (!sums_chain(R, s1 - s0, 0u, sum)) { if (lane == 0) fail(); return; }
     if ((uint32_t)lane < w) {
       const uint64_t p = (uint64_t)c * d + j0 + (uint32_t)lane;
       const uint32_t cnt = s1 - s0;

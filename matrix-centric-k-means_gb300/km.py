@@ -337,7 +337,7 @@ def update(X, labels, k):
 
 class Batch:
     """Handle over km_batch_*: many independent Lloyd problems (list of (n, d, k)),
-    `restarts` seeded restarts each, in one persistent launch."""
+    `restarts` seeded restarts each, advanced together."""
 
     def __init__(self, shapes, restarts=8, seed=0, tol=1e-4, maxiter=300, device=0, stream=0):
         self.shapes = [(int(n), int(d), int(k)) for n, d, k in shapes]
