@@ -11,12 +11,16 @@
 // (std::mt19937_64), so the result is reproducible, and every sum has a fixed
 // order, so the same seed gives the same centroids on every run.
 //
-// Rows are processed in chunks of PP_CHUNK; bsum[b] is the FP64 sum of d2
-// over chunk b, which the sampler walks to find the chunk holding a draw and
-// then scans inside the chunk.  Distances are FP32, ||x - c||^2 with the
-// differences squared and summed in column order.
+// Two launches a round: distances and costs of the candidates, whose last block
+// chooses; the update of d2 and of its chunk sums, whose last block draws the next
+// round's candidates.  bsum[b] is the FP64 sum of d2 over the PP_CHUNK rows of
+// chunk b, which the sampler walks to find the chunk holding a draw and then scans
+// inside the chunk.  Distances are FP32, ||x - c||^2 with partial sums over the
+// columns l, l + 32, ... (l = 0..31) added in a fixed tree: bit 4 of l, then bits 3
+// to 0, as a 32-lane exchange would add them.
 #include "km_lloyd.cuh"
 
+#include <algorithm>
 #include <cmath>
 #include <random>
 #include <vector>
@@ -25,14 +29,140 @@ namespace km {
 
 constexpr uint32_t PP_CHUNK = 1024;
 constexpr uint32_t PP_MAX_S = 16;
+constexpr uint32_t PP_TILE_MAX_D = 256;    // widest rows of the tiled cost kernel
 
 __device__ __forceinline__ uint64_t umin64(uint64_t a, uint64_t b) { return a < b ? a : b; }
 
-// d2_i = ||x_i - x_first||^2; bsum per chunk.
+// The device state of one seeding.
+struct PpState {
+  uint32_t ticket;      // blocks done in this launch (the last one resets it)
+  int32_t best;         // chosen candidate of the round
+};
+
+// True in the block that finishes last; the other blocks' results are then
+// visible to reads past L1 (__ldcg).
+__device__ __forceinline__ bool pp_last_block(PpState* st, int* flag) {
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) *flag = (atomicAdd(&st->ticket, 1u) == gridDim.x - 1u) ? 1 : 0;
+  __syncthreads();
+  if (!*flag) return false;
+  __threadfence();
+  if (threadIdx.x == 0) st->ticket = 0u;
+  return true;
+}
+
+// Inclusive FP64 scan over the lanes.
+__device__ __forceinline__ double pp_scan(double v) {
+  const int lane = threadIdx.x & 31;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const double t = __shfl_up_sync(0xffffffffu, v, o);
+    if (lane >= o) v += t;
+  }
+  return v;
+}
+
+// One warp draws a row ~ d2 / sum(d2) for the uniform u: the chunk holding
+// u * sum, then the row inside it, each found by the lanes' runs of consecutive
+// values (one scan) and then the values of one run (another).  Rounding at a top
+// end takes the last positive value.  Bound by the latency of four loads and four
+// scans: the update launch with the draws of 7 candidates at n = 262,144 takes 14
+// us (24 us with a scan of every 32 values in turn; 27 us for the draws alone as a
+// launch of their own, with the loads between the scans).
+__device__ int32_t pp_draw(const float* d2, uint64_t n, const double* bsum, uint32_t nblk, double u) {
+  const int lane = threadIdx.x & 31;
+  const uint32_t R = (nblk + 31u) / 32u;                       // chunks per lane
+  const uint32_t b0 = min(nblk, (uint32_t)lane * R), b1 = min(nblk, b0 + R);
+  double own = 0.0;
+  for (uint32_t b = b0; b < b1; b += 8) {
+    double v[8];
+#pragma unroll
+    for (int g = 0; g < 8; ++g) v[g] = b + g < b1 ? __ldcg(bsum + b + g) : 0.0;
+    own += ((v[0] + v[1]) + (v[2] + v[3])) + ((v[4] + v[5]) + (v[6] + v[7]));
+  }
+  double inc = pp_scan(own);
+  const double tot = __shfl_sync(0xffffffffu, inc, 31);
+  // every point coincides with a chosen one: uniform draw
+  if (!(tot > 0.0)) return (int32_t)umin64(n - 1, (uint64_t)(u * (double)n));
+  double target = u * tot;
+  bool top = false;                                            // rounding at the top end
+  unsigned hit = __ballot_sync(0xffffffffu, own > 0.0 && inc > target);
+  if (!hit) { hit = 0x80000000u >> __clz(__ballot_sync(0xffffffffu, own > 0.0)); top = true; }
+  int L = __ffs(hit) - 1;
+  target -= __shfl_sync(0xffffffffu, inc - own, L);
+  const uint32_t run0 = (uint32_t)L * R, run1 = min(nblk, run0 + R);
+  uint32_t blk = run0;
+  double base = 0.0;
+  bool found = false;
+  for (uint32_t g = run0; g < run1 && !found; g += 32u) {
+    const uint32_t b = g + (uint32_t)lane;
+    const double v = b < run1 ? __ldcg(bsum + b) : 0.0;
+    inc = pp_scan(v);
+    const unsigned h = __ballot_sync(0xffffffffu, !top && v > 0.0 && base + inc > target);
+    const unsigned pos = __ballot_sync(0xffffffffu, v > 0.0);
+    if (h) {
+      L = __ffs(h) - 1;
+      blk = g + (uint32_t)L;
+      target -= __shfl_sync(0xffffffffu, base + inc - v, L);
+      found = true;
+    } else {
+      if (pos) blk = g + 31u - (uint32_t)__clz(pos);
+      base += __shfl_sync(0xffffffffu, inc, 31);
+    }
+  }
+  top = !found;
+  // row inside the chunk: 32 consecutive rows per lane (float4: a chunk starts
+  // 16-byte aligned)
+  const uint64_t r0 = (uint64_t)blk * PP_CHUNK, r1 = umin64(n, r0 + PP_CHUNK), l0 = r0 + 32u * (uint32_t)lane;
+  double s4[4] = {0.0, 0.0, 0.0, 0.0};
+  if (l0 + 32u <= r1) {
+    float4 w[8];
+#pragma unroll
+    for (int g = 0; g < 8; ++g) w[g] = __ldcg(reinterpret_cast<const float4*>(d2 + l0) + g);
+#pragma unroll
+    for (int g = 0; g < 8; ++g) {
+      s4[0] += (double)w[g].x; s4[1] += (double)w[g].y; s4[2] += (double)w[g].z; s4[3] += (double)w[g].w;
+    }
+  } else {
+    for (uint64_t i = l0; i < r1; ++i) s4[0] += (double)__ldcg(d2 + i);
+  }
+  own = (s4[0] + s4[1]) + (s4[2] + s4[3]);
+  inc = pp_scan(own);
+  hit = __ballot_sync(0xffffffffu, !top && own > 0.0 && inc > target);
+  if (!hit) {
+    const unsigned pos = __ballot_sync(0xffffffffu, own > 0.0);
+    hit = pos ? 0x80000000u >> __clz(pos) : 1u;
+    top = true;
+  }
+  L = __ffs(hit) - 1;
+  target -= __shfl_sync(0xffffffffu, inc - own, L);
+  const uint64_t i = r0 + 32u * (uint32_t)L + (uint32_t)lane;
+  const double v = i < r1 ? (double)__ldcg(d2 + i) : 0.0;
+  inc = pp_scan(v);
+  const unsigned h = __ballot_sync(0xffffffffu, !top && v > 0.0 && inc > target);
+  const unsigned pos = __ballot_sync(0xffffffffu, v > 0.0);
+  const int at = h ? __ffs(h) - 1 : pos ? 31 - __clz(pos) : 0;
+  return (int32_t)(r0 + 32u * (uint32_t)L + (uint32_t)at);
+}
+
+// The last block's warps draw the s candidates of a round.
+__device__ __forceinline__ void pp_draw_all(const float* d2, uint64_t n, const double* bsum, uint32_t nblk,
+                                            const double* u, uint32_t s, int32_t* cand) {
+  const uint32_t warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  for (uint32_t j = warp; j < s; j += nw) {
+    const int32_t pick = pp_draw(d2, n, bsum, nblk, u[j]);
+    if ((threadIdx.x & 31) == 0) cand[j] = pick;
+  }
+}
+
+// d2_i = ||x_i - x_first||^2; bsum per chunk; draws the first candidates (u
+// non-null).
 __global__ void __launch_bounds__(256)
 pp_first_kernel(const float* __restrict__ X, uint64_t n, uint32_t d, uint64_t first,
-                float* __restrict__ d2, double* __restrict__ bsum) {
+                float* d2, double* bsum, PpState* st, const double* __restrict__ u, uint32_t s, int32_t* cand) {
   __shared__ double red[8];
+  __shared__ int flag;
   const uint64_t r0 = (uint64_t)blockIdx.x * PP_CHUNK;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const float* c = X + first * d;
@@ -56,77 +186,170 @@ pp_first_kernel(const float* __restrict__ X, uint64_t n, uint32_t d, uint64_t fi
     for (int w = 0; w < 8; ++w) t += red[w];
     bsum[blockIdx.x] = t;
   }
+  if (pp_last_block(st, &flag) && u) pp_draw_all(d2, n, bsum, gridDim.x, u, s, cand);
 }
 
-// One warp per candidate: draw index ~ d2 / sum(d2) for the uniform u[j].
-__global__ void pp_sample_kernel(const float* __restrict__ d2, uint64_t n, const double* __restrict__ bsum,
-                                 uint32_t nblk, const double* __restrict__ u, uint32_t s,
-                                 int32_t* __restrict__ cand) {
-  const uint32_t j = blockIdx.x;
-  const int lane = threadIdx.x;
-  if (j >= s) return;
-  double tot = 0.0;
-  for (uint32_t b = lane; b < nblk; b += 32) tot += bsum[b];
-  for (int o = 16; o > 0; o >>= 1) tot += __shfl_xor_sync(0xffffffffu, tot, o);
-  if (!(tot > 0.0)) {   // every point coincides with a chosen one: uniform draw
-    if (lane == 0) cand[j] = (int32_t)umin64(n - 1, (uint64_t)(u[j] * (double)n));
-    return;
-  }
-  double target = u[j] * tot;
-  // chunk holding the draw
-  uint32_t blk = 0xffffffffu, last_pos = 0;
-  double base = 0.0;
-  for (uint32_t b0 = 0; b0 < nblk && blk == 0xffffffffu; b0 += 32) {
-    const uint32_t b = b0 + lane;
-    const double v = (b < nblk) ? bsum[b] : 0.0;
-    double inc = v;
-    for (int o = 1; o < 32; o <<= 1) {
-      const double t = __shfl_up_sync(0xffffffffu, inc, o);
-      if (lane >= o) inc += t;
+// The last block of a cost launch: total cost per candidate over the blocks'
+// partial sums, the cheapest (lowest index on ties) becomes centroid number r.
+__device__ void pp_choose(const double* cpart, uint32_t nblk, uint32_t s, const int32_t* cand, uint32_t r,
+                          int32_t* chosen, PpState* st, double* sh) {
+  const uint32_t warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  const int lane = threadIdx.x & 31;
+  for (uint32_t j = warp; j < s; j += nw) {
+    double t = 0.0;
+    for (uint32_t b0 = 0; b0 < nblk; b0 += 32 * 8) {
+      double v[8];
+#pragma unroll
+      for (int g = 0; g < 8; ++g) {
+        const uint32_t b = b0 + 32u * g + lane;
+        v[g] = b < nblk ? __ldcg(cpart + (uint64_t)j * nblk + b) : 0.0;
+      }
+#pragma unroll
+      for (int g = 0; g < 8; ++g) t += v[g];
     }
-    const unsigned hit = __ballot_sync(0xffffffffu, b < nblk && v > 0.0 && base + inc > target);
-    const unsigned pos = __ballot_sync(0xffffffffu, b < nblk && v > 0.0);
-    if (pos) last_pos = b0 + 31 - __clz(pos);
-    if (hit) {
-      const int l = __ffs(hit) - 1;
-      blk = b0 + l;
-      const double excl = __shfl_sync(0xffffffffu, base + inc - v, l);
-      target -= excl;
-    } else {
-      base += __shfl_sync(0xffffffffu, inc, 31);
-    }
+    for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+    if (lane == 0) sh[j] = t;
   }
-  if (blk == 0xffffffffu) { blk = last_pos; target = -1.0; }   // rounding at the top end
-  // row inside the chunk
-  const uint64_t r0 = (uint64_t)blk * PP_CHUNK;
-  const uint64_t r1 = umin64(n, r0 + PP_CHUNK);
-  uint64_t pick = 0xffffffffffffffffull, last_row = r0;
-  base = 0.0;
-  for (uint64_t i0 = r0; i0 < r1 && pick == 0xffffffffffffffffull; i0 += 32) {
-    const uint64_t i = i0 + lane;
-    const double v = (i < r1) ? (double)d2[i] : 0.0;
-    double inc = v;
-    for (int o = 1; o < 32; o <<= 1) {
-      const double t = __shfl_up_sync(0xffffffffu, inc, o);
-      if (lane >= o) inc += t;
-    }
-    const unsigned hit = __ballot_sync(0xffffffffu, i < r1 && v > 0.0 && target >= 0.0 && base + inc > target);
-    const unsigned pos = __ballot_sync(0xffffffffu, i < r1 && v > 0.0);
-    if (pos) last_row = i0 + 31 - __clz(pos);
-    if (hit) pick = i0 + (__ffs(hit) - 1);
-    else base += __shfl_sync(0xffffffffu, inc, 31);
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    uint32_t bj = 0;
+    for (uint32_t j = 1; j < s; ++j)
+      if (sh[j] < sh[bj]) bj = j;
+    chosen[r] = cand[bj];
+    st->best = (int32_t)bj;
   }
-  if (pick == 0xffffffffffffffffull) pick = last_row;
-  if (lane == 0) cand[j] = (int32_t)pick;
 }
 
-// D[i, j] = ||x_i - x_cand_j||^2 and per-chunk FP64 costs sum_i min(d2_i, D[i, j]).
+// The tree over the partial sums of columns l = V mod 2^K: S distances of one row
+// in packed pairs, the row in xs (columns LD floats apart), the candidates negated
+// in cs[column][S].
+template <int S, int K, int V>
+__device__ __forceinline__ void pp_tree(const float* xs, int LD, const float* cs, uint32_t d, float2 (&out)[S / 2]) {
+  if constexpr (K == 5) {
+#pragma unroll
+    for (int c = 0; c < S / 2; ++c) out[c] = make_float2(0.0f, 0.0f);
+#pragma unroll 1
+    for (uint32_t j = V; j < d; j += 32) {
+      const float2 x = make_float2(xs[j * LD], xs[j * LD]);
+#pragma unroll
+      for (int q = 0; q < S / 4; ++q) {
+        const float4 c4 = *reinterpret_cast<const float4*>(cs + j * S + 4 * q);
+        const float2 u = __fadd2_rn(x, make_float2(c4.x, c4.y)), w = __fadd2_rn(x, make_float2(c4.z, c4.w));
+        out[2 * q] = __ffma2_rn(u, u, out[2 * q]);
+        out[2 * q + 1] = __ffma2_rn(w, w, out[2 * q + 1]);
+      }
+    }
+  } else {
+    pp_tree<S, K + 1, V>(xs, LD, cs, d, out);
+    float2 t[S / 2];
+    pp_tree<S, K + 1, V + (1 << K)>(xs, LD, cs, d, t);
+#pragma unroll
+    for (int c = 0; c < S / 2; ++c) out[c] = __fadd2_rn(out[c], t[c]);
+  }
+}
+
+// h + l <- h + l + a + al, an unevaluated FP32 pair (TwoSum): FP64 additions are
+// slow on this GPU.
+__device__ __forceinline__ void pp_pair_add(float& h, float& l, float a, float al) {
+  const float t = __fadd_rn(h, a), bp = __fsub_rn(t, h);
+  const float err = __fadd_rn(__fsub_rn(h, __fsub_rn(t, bp)), __fsub_rn(a, bp));
+  h = t;
+  l = __fadd_rn(l, __fadd_rn(al, err));
+}
+
+// D[j][i] = ||x_i - x_cand_j||^2 and the block's costs sum_i min(d2_i, D[j][i]) (FP32
+// pairs, stored as FP64), d <= PP_TILE_MAX_D: a thread per row for all candidates, the rows staged
+// transposed in shared memory.  Bound by the FP32 pipes (two operations an element
+// and candidate, 31 a row and candidate for the tree) and by reading X.  A warp per
+// row instead spends most of its instructions exchanging partial sums: n = 262,144
+// d = 32, 7 candidates 336 us, now 22 us (46 us with FP64 cost sums in every warp).
+template <int S>
 __global__ void __launch_bounds__(256)
-pp_cost_kernel(const float* __restrict__ X, uint64_t n, uint32_t d, const int32_t* __restrict__ cand,
-               uint32_t s, const float* __restrict__ d2, float* __restrict__ D,
-               double* __restrict__ cpart) {
+pp_cost_kernel(const float* __restrict__ X, uint64_t n, uint32_t d, bool v4, const int32_t* cand, uint32_t s,
+               const float* __restrict__ d2, float* __restrict__ D, double* cpart, PpState* st, uint32_t r,
+               int32_t* chosen) {
+  griddep_wait();
+  extern __shared__ __align__(16) float pp_smem[];
+  __shared__ double tot[S];
+  __shared__ int flag;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const uint32_t rows = blockDim.x, LD = rows + 1u;
+  float* cs = pp_smem;                             // [d][S], zeros past s
+  float* xs = pp_smem + (size_t)d * S;             // [d][LD]
+  for (uint32_t t = tid; t < S * d; t += rows) {
+    const uint32_t c = t / d, j = t % d;
+    cs[j * S + c] = c < s ? -X[(uint64_t)cand[c] * d + j] : 0.0f;
+  }
+  const uint64_t r0 = (uint64_t)blockIdx.x * rows;
+  const uint32_t nr = (uint32_t)umin64(rows, n - r0);
+  const float* xb = X + r0 * d;
+  if (v4) {                                        // 16-byte loads: d % 4 == 0 and X 16-byte aligned
+    const uint32_t d4 = d / 4u;
+    uint32_t rr = (uint32_t)tid / d4, cc = (uint32_t)tid % d4;
+    const uint32_t dr = rows / d4, dc = rows % d4;
+#pragma unroll 4
+    for (uint32_t t = tid; t < nr * d4; t += rows) {
+      const float4 v = __ldg(reinterpret_cast<const float4*>(xb) + t);
+      float* x = xs + 4u * cc * LD + rr;
+      x[0] = v.x; x[LD] = v.y; x[2 * LD] = v.z; x[3 * LD] = v.w;
+      rr += dr;
+      cc += dc;
+      if (cc >= d4) { cc -= d4; ++rr; }
+    }
+  } else {
+    uint32_t rr = (uint32_t)tid / d, cc = (uint32_t)tid % d;
+    const uint32_t dr = rows / d, dc = rows % d;
+#pragma unroll 8
+    for (uint32_t t = tid; t < nr * d; t += rows) {
+      xs[cc * LD + rr] = __ldg(xb + t);
+      rr += dr;
+      cc += dc;
+      if (cc >= d) { cc -= d; ++rr; }
+    }
+  }
+  __syncthreads();
+  const bool valid = (uint32_t)tid < nr;
+  float2 v[S / 2];
+  pp_tree<S, 0, 0>(xs + (valid ? tid : 0), (int)LD, cs, d, v);
+  const float old = valid ? d2[r0 + tid] : 0.0f;
+  __syncthreads();                                 // the staged rows are done with
+  float* const mins = xs;                          // [s][rows]
+#pragma unroll
+  for (int c = 0; c < S; ++c) {
+    if ((uint32_t)c >= s) break;
+    const float vc = (c & 1) ? v[c / 2].y : v[c / 2].x;
+    if (valid) D[(uint64_t)c * n + r0 + tid] = vc;
+    mins[c * rows + tid] = valid ? fminf(vc, old) : 0.0f;
+  }
+  __syncthreads();
+  // a warp per candidate: each lane every 32nd row, then the lanes
+  for (uint32_t c = (uint32_t)warp; c < s; c += rows / 32u) {
+    float h = 0.0f, l = 0.0f;
+    for (uint32_t t = (uint32_t)lane; t < rows; t += 32u) pp_pair_add(h, l, mins[c * rows + t], 0.0f);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1)
+      pp_pair_add(h, l, __shfl_xor_sync(0xffffffffu, h, o), __shfl_xor_sync(0xffffffffu, l, o));
+    double t = (double)h + (double)l;
+    if (__any_sync(0xffffffffu, !isfinite(h))) {     // past the FP32 range: the sum in FP64
+      t = 0.0;
+      for (uint32_t q = (uint32_t)lane; q < rows; q += 32u) t += (double)mins[c * rows + q];
+      for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+    }
+    if (lane == 0) cpart[(uint64_t)c * gridDim.x + blockIdx.x] = t;
+  }
+  if (pp_last_block(st, &flag)) pp_choose(cpart, gridDim.x, s, cand, r, chosen, st, tot);
+}
+
+// The same for wider rows: a warp per row, lanes over the columns.
+__global__ void __launch_bounds__(256)
+pp_cost_wide_kernel(const float* __restrict__ X, uint64_t n, uint32_t d, const int32_t* cand,
+                    uint32_t s, const float* __restrict__ d2, float* __restrict__ D,
+                    double* cpart, PpState* st, uint32_t r, int32_t* chosen) {
+  griddep_wait();
   extern __shared__ float cs[];                    // s x d candidate rows
   __shared__ double red[8][PP_MAX_S];
+  __shared__ double tot[PP_MAX_S];
+  __shared__ int flag;
   for (uint32_t t = threadIdx.x; t < s * d; t += blockDim.x) {
     const uint32_t j = t / d, c = t % d;
     cs[t] = X[(uint64_t)cand[j] * d + c];
@@ -160,7 +383,7 @@ pp_cost_kernel(const float* __restrict__ X, uint64_t n, uint32_t d, const int32_
         float v = p[j];
         for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
         if (lane == 0) {
-          D[i * s + j] = v;
+          D[(uint64_t)j * n + i] = v;
           acc[j] += (double)fminf(v, d2[i]);
         }
       }
@@ -174,45 +397,36 @@ pp_cost_kernel(const float* __restrict__ X, uint64_t n, uint32_t d, const int32_
   if (threadIdx.x < s) {
     double t = 0.0;
     for (int w = 0; w < 8; ++w) t += red[w][threadIdx.x];
-    cpart[(uint64_t)blockIdx.x * s + threadIdx.x] = t;
+    cpart[(uint64_t)threadIdx.x * gridDim.x + blockIdx.x] = t;
   }
+  if (pp_last_block(st, &flag)) pp_choose(cpart, gridDim.x, s, cand, r, chosen, st, tot);
 }
 
-// Single warp: total cost per candidate, the cheapest (lowest index on ties)
-// becomes centroid number r.
-__global__ void pp_choose_kernel(const double* __restrict__ cpart, uint32_t nblk, uint32_t s,
-                                 const int32_t* __restrict__ cand, uint32_t r,
-                                 int32_t* __restrict__ chosen, int32_t* __restrict__ best) {
-  const int lane = threadIdx.x;
-  double bestv = 0.0;
-  int bj = -1;
-  for (uint32_t j = 0; j < s; ++j) {
-    double t = 0.0;
-    for (uint32_t b = lane; b < nblk; b += 32) t += cpart[(uint64_t)b * s + j];
-    for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
-    if (bj < 0 || t < bestv) { bestv = t; bj = (int)j; }
-  }
-  if (lane == 0) {
-    chosen[r] = cand[bj];
-    *best = bj;
-  }
-}
-
-// d2_i = min(d2_i, D[i, best]); bsum per chunk.
+// d2_i = min(d2_i, D[best][i]); bsum per chunk; draws the next round's candidates
+// (u non-null).
 __global__ void __launch_bounds__(256)
-pp_update_kernel(const float* __restrict__ D, uint64_t n, uint32_t s, const int32_t* __restrict__ best,
-                 float* __restrict__ d2, double* __restrict__ bsum) {
+pp_update_kernel(const float* __restrict__ D, uint64_t n, PpState* st, float* d2, double* bsum,
+                 const double* __restrict__ u, uint32_t s, int32_t* cand) {
+  griddep_wait();
   __shared__ double red[8];
+  __shared__ int flag;
   const uint64_t r0 = (uint64_t)blockIdx.x * PP_CHUNK;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int bj = *best;
+  const float* Db = D + (uint64_t)st->best * n;
   double acc = 0.0;
-  for (uint32_t t = threadIdx.x; t < PP_CHUNK; t += blockDim.x) {
-    const uint64_t i = r0 + t;
-    if (i >= n) break;
-    const float v = fminf(d2[i], D[i * s + bj]);
-    d2[i] = v;
-    acc += (double)v;
+  float v[PP_CHUNK / 256];
+#pragma unroll
+  for (int q = 0; q < (int)PP_CHUNK / 256; ++q) {
+    const uint64_t i = r0 + threadIdx.x + 256u * q;
+    v[q] = i < n ? fminf(d2[i], Db[i]) : 0.0f;
+  }
+#pragma unroll
+  for (int q = 0; q < (int)PP_CHUNK / 256; ++q) {
+    const uint64_t i = r0 + threadIdx.x + 256u * q;
+    if (i < n) {
+      d2[i] = v[q];
+      acc += (double)v[q];
+    }
   }
   for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
   if (lane == 0) red[warp] = acc;
@@ -222,6 +436,7 @@ pp_update_kernel(const float* __restrict__ D, uint64_t n, uint32_t s, const int3
     for (int w = 0; w < 8; ++w) t += red[w];
     bsum[blockIdx.x] = t;
   }
+  if (pp_last_block(st, &flag) && u) pp_draw_all(d2, n, bsum, gridDim.x, u, s, cand);
 }
 
 __global__ void pp_gather_kernel(const float* __restrict__ X, uint32_t d, const int32_t* __restrict__ idx,
@@ -256,25 +471,46 @@ km_status plusplus_init(LloydEngine& e, int seed) {
   for (auto& v : hu) v = uni(gen);
   std::vector<int32_t> hchosen(1, (int32_t)first);
 
+  // Cost tiles: a thread per row, 256 rows a block, 128 where 256 rows of d
+  // columns would take most of an SM's shared memory (one block an SM).
+  const bool tiled = d <= PP_TILE_MAX_D;
+  const uint32_t S = s <= 4u ? 4u : s <= 8u ? 8u : 16u, rows = d <= 128u ? 256u : 128u;
+  const uint32_t ncost = tiled ? (uint32_t)((n + rows - 1) / rows) : nblk;
+  // the rows' minima ([s][rows]) follow the staged rows in the same space
+  const size_t cost_smem = tiled ? sizeof(float) * ((size_t)d * S + std::max<size_t>((size_t)d * (rows + 1u), (size_t)s * rows))
+                                 : smem;
+  const bool v4 = d % 4 == 0 && reinterpret_cast<uintptr_t>(e.X) % 16 == 0;
+  auto tile = S == 4u ? pp_cost_kernel<4> : S == 8u ? pp_cost_kernel<8> : pp_cost_kernel<16>;
   DevBuf<float> d2, D;
   DevBuf<double> bsum, cpart, u;
-  DevBuf<int32_t> cand, chosen, best;
-  if (d2.alloc(n) || D.alloc(n * s) || bsum.alloc(nblk) || cpart.alloc((size_t)nblk * s) ||
-      u.alloc(hu.size()) || cand.alloc(s) || chosen.alloc(k) || best.alloc(1)) {
+  DevBuf<int32_t> cand, chosen;
+  DevBuf<PpState> state;
+  if (d2.alloc(n) || D.alloc(n * s) || bsum.alloc(nblk) || cpart.alloc((size_t)ncost * s) ||
+      u.alloc(hu.size()) || cand.alloc(s) || chosen.alloc(k) || state.alloc(1)) {
     (void)cudaGetLastError();
     return KM_ERR_ALLOC;
   }
-  if (smem > 48 * 1024)
-    KM_CUDA_TRY(cudaFuncSetAttribute(pp_cost_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  if (cost_smem > 48 * 1024) {
+    if (tiled)
+      KM_CUDA_TRY(cudaFuncSetAttribute(tile, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cost_smem));
+    else
+      KM_CUDA_TRY(cudaFuncSetAttribute(pp_cost_wide_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cost_smem));
+  }
   cudaStream_t st = e.stream;
+  KM_CUDA_TRY(cudaMemsetAsync(state.p, 0, sizeof(PpState), st));
   KM_CUDA_TRY(cudaMemcpyAsync(u.p, hu.data(), sizeof(double) * hu.size(), cudaMemcpyHostToDevice, st));
   KM_CUDA_TRY(cudaMemcpyAsync(chosen.p, hchosen.data(), sizeof(int32_t), cudaMemcpyHostToDevice, st));
-  pp_first_kernel<<<nblk, 256, 0, st>>>(e.X, n, d, first, d2.p, bsum.p);
+  pp_first_kernel<<<nblk, 256, 0, st>>>(e.X, n, d, first, d2.p, bsum.p, state.p, k > 1 ? u.p : nullptr, s, cand.p);
+  KM_CUDA_TRY(cudaGetLastError());
   for (uint32_t r = 1; r < k; ++r) {
-    pp_sample_kernel<<<s, 32, 0, st>>>(d2.p, n, bsum.p, nblk, u.p + (size_t)(r - 1) * s, s, cand.p);
-    pp_cost_kernel<<<nblk, 256, smem, st>>>(e.X, n, d, cand.p, s, d2.p, D.p, cpart.p);
-    pp_choose_kernel<<<1, 32, 0, st>>>(cpart.p, nblk, s, cand.p, r, chosen.p, best.p);
-    pp_update_kernel<<<nblk, 256, 0, st>>>(D.p, n, s, best.p, d2.p, bsum.p);
+    if (tiled)
+      KM_CUDA_TRY(launch_pdl(tile, ncost, rows, cost_smem, st, e.X, n, d, v4, cand.p, s, d2.p, D.p, cpart.p, state.p,
+                             r, chosen.p));
+    else
+      KM_CUDA_TRY(launch_pdl(pp_cost_wide_kernel, ncost, 256, cost_smem, st, e.X, n, d, cand.p, s, d2.p, D.p, cpart.p,
+                             state.p, r, chosen.p));
+    KM_CUDA_TRY(launch_pdl(pp_update_kernel, nblk, 256, 0, st, D.p, n, state.p, d2.p, bsum.p,
+                           r + 1 < k ? u.p + (size_t)r * s : (const double*)nullptr, s, cand.p));
   }
   pp_gather_kernel<<<(unsigned)(((uint64_t)k * d + 255) / 256), 256, 0, st>>>(e.X, d, chosen.p, k, e.C);
   KM_CUDA_TRY(cudaGetLastError());
