@@ -80,12 +80,14 @@ km_status sample_init(LloydEngine& e, int seed) {
   int32_t* d_idx = nullptr;
   float* d_rows = nullptr;
   const uint32_t cap = std::max<uint32_t>(64, 2 * e.k + 16);
-  if (cudaMalloc(&d_idx, sizeof(int32_t) * cap) != cudaSuccess ||
-      cudaMalloc(&d_rows, sizeof(float) * (size_t)cap * e.d) != cudaSuccess) {
-    (void)cudaGetLastError();
-    if (d_idx) cudaFree(d_idx);
-    return KM_ERR_ALLOC;
+  void *q_idx = nullptr, *q_rows = nullptr;
+  KM_TRY(scratch_alloc(&q_idx, sizeof(int32_t) * cap, e.device, e.stream));
+  if (km_status s = scratch_alloc(&q_rows, sizeof(float) * (size_t)cap * e.d, e.device, e.stream)) {
+    scratch_free(q_idx, e.device, e.stream);
+    return s;
   }
+  d_idx = static_cast<int32_t*>(q_idx);
+  d_rows = static_cast<float*>(q_rows);
   std::vector<int32_t> cand;
   std::vector<float> rows;
   km_status rc = KM_OK;
@@ -117,8 +119,8 @@ km_status sample_init(LloydEngine& e, int seed) {
         cudaStreamSynchronize(e.stream) != cudaSuccess)
       rc = KM_ERR_CUDA;
   }
-  cudaFree(d_idx);
-  cudaFree(d_rows);
+  scratch_free(d_idx, e.device, e.stream);
+  scratch_free(d_rows, e.device, e.stream);
   return rc;
 }
 
@@ -204,7 +206,7 @@ km_status km_lloyd_create(const km_lloyd_params* p, km_lloyd** out) {
   km_lloyd* h = new (std::nothrow) km_lloyd();
   if (!h) return KM_ERR_ALLOC;
   h->p = *p;
-  km_status s = h->eng.init(p->n, p->d, p->k, p->precision, p->device, p->stream, true);
+  km_status s = h->eng.init(p->n, p->d, p->k, p->precision, p->device, p->stream, EngineUse::FIT);
   if (s == KM_OK && cudaMallocHost(reinterpret_cast<void**>(&h->h_done), sizeof(int32_t)) != cudaSuccess) s = KM_ERR_ALLOC;
   if (s == KM_OK && (cudaEventCreate(&h->ev0) != cudaSuccess || cudaEventCreate(&h->ev1) != cudaSuccess)) s = KM_ERR_CUDA;
   if (s != KM_OK) { km_lloyd_destroy(h); return s; }
@@ -421,13 +423,12 @@ km_status km_assign(const float* X_dev, const float* C_dev, uint64_t n, uint32_t
   int dev;
   KM_TRY(current_device(&dev));
   LloydEngine e;
-  KM_TRY(e.init(n, d, k, precision, dev, stream, false));
+  KM_TRY(e.init(n, d, k, precision, dev, stream, EngineUse::ASSIGN));
   KM_TRY(e.set_points(X_dev, true, false));
   KM_TRY(e.set_centroids_dev(C_dev));
+  e.labels = labels_dev;
+  e.mindist = mindist_dev;
   KM_TRY(e.enqueue_assign(nullptr));
-  KM_CUDA_TRY(cudaMemcpyAsync(labels_dev, e.labels, sizeof(uint32_t) * n, cudaMemcpyDeviceToDevice, e.stream));
-  if (mindist_dev)
-    KM_CUDA_TRY(cudaMemcpyAsync(mindist_dev, e.mindist, sizeof(float) * n, cudaMemcpyDeviceToDevice, e.stream));
   KM_TRY(e.check_device_error());
   if (refined_rows) *refined_rows = e.h_st->refined_total;
   return KM_OK;
@@ -439,9 +440,10 @@ km_status km_distances(const float* X_dev, const float* C_dev, uint64_t n, uint3
   int dev;
   KM_TRY(current_device(&dev));
   LloydEngine e;
-  KM_TRY(e.init(n, d, k, precision, dev, stream, false));
+  KM_TRY(e.init(n, d, k, precision, dev, stream, EngineUse::ASSIGN));
   KM_TRY(e.set_points(X_dev, true, false));
   KM_TRY(e.set_centroids_dev(C_dev));
+  KM_TRY(e.take(&e.labels, n));
   KM_TRY(e.enqueue_assign(D_dev));
   return e.check_device_error();
 }
@@ -453,7 +455,7 @@ km_status km_update(const float* X_dev, const uint32_t* labels_dev, uint64_t n, 
   int dev;
   KM_TRY(current_device(&dev));
   LloydEngine e;
-  KM_TRY(e.init(n, d, k, KM_PREC_FP32, dev, stream, true));
+  KM_TRY(e.init(n, d, k, KM_PREC_FP32, dev, stream, EngineUse::UPDATE));
   e.X = X_dev;
   KM_TRY(e.enqueue_sort(labels_dev));
   KM_TRY(e.check_device_error());   // labels >= k are rejected before the sums run

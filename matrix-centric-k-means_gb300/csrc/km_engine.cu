@@ -13,23 +13,31 @@ namespace km {
 namespace {
 thread_local std::string g_last_error;
 
-template <class T>
-km_status dalloc(T** p, size_t count) {
-  *p = nullptr;
-  if (count == 0) count = 1;
-  cudaError_t e = cudaMalloc(reinterpret_cast<void**>(p), count * sizeof(T));
-  if (e != cudaSuccess) {
-    set_last_error(e, "cudaMalloc", __FILE__, __LINE__);
-    (void)cudaGetLastError();
-    return KM_ERR_ALLOC;
-  }
-  return KM_OK;
-}
+constexpr int MAX_DEVICES = 64;
+std::mutex g_pool_mu;
+cudaMemPool_t g_pool[MAX_DEVICES] = {};
+bool g_pool_tried[MAX_DEVICES] = {};
 
-template <class T>
-void dfree(T*& p) {
-  if (p) cudaFree(p);
-  p = nullptr;
+// The device's pool (null: none), made on the first use.
+cudaMemPool_t device_pool(int device) {
+  if (device < 0 || device >= MAX_DEVICES) return nullptr;
+  std::lock_guard<std::mutex> lk(g_pool_mu);
+  if (!g_pool_tried[device]) {
+    g_pool_tried[device] = true;
+    int ok = 0;
+    cudaMemPoolProps props = {};
+    props.allocType = cudaMemAllocationTypePinned;
+    props.location.type = cudaMemLocationTypeDevice;
+    props.location.id = device;
+    uint64_t keep = SCRATCH_KEEP;
+    cudaMemPool_t pool = nullptr;
+    if (cudaDeviceGetAttribute(&ok, cudaDevAttrMemoryPoolsSupported, device) == cudaSuccess && ok &&
+        cudaMemPoolCreate(&pool, &props) == cudaSuccess &&
+        cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep) == cudaSuccess)
+      g_pool[device] = pool;
+    (void)cudaGetLastError();
+  }
+  return g_pool[device];
 }
 
 uint32_t round_up(uint32_t v, uint32_t m) { return (v + m - 1) / m * m; }
@@ -42,6 +50,56 @@ void set_last_error(cudaError_t e, const char* what, const char* file, int line)
 }
 
 const char* last_error_text() { return g_last_error.c_str(); }
+
+km_status scratch_alloc(void** p, size_t bytes, int device, cudaStream_t s) {
+  *p = nullptr;
+  cudaMemPool_t pool = device_pool(device);
+  for (int attempt = 0; attempt < 2; ++attempt) {
+    const cudaError_t e = pool ? cudaMallocFromPoolAsync(p, bytes, pool, s) : cudaMalloc(p, bytes);
+    if (e == cudaSuccess) return KM_OK;
+    set_last_error(e, "scratch allocation", __FILE__, __LINE__);
+    (void)cudaGetLastError();
+    *p = nullptr;
+    if (e != cudaErrorMemoryAllocation) return KM_ERR_CUDA;
+    scratch_trim(device);
+  }
+  return KM_ERR_ALLOC;
+}
+
+void scratch_free(void* p, int device, cudaStream_t s) {
+  if (!p) return;
+  if (device_pool(device)) cudaFreeAsync(p, s);
+  else cudaFree(p);
+}
+
+void scratch_trim(int device) {
+  if (cudaMemPool_t pool = device_pool(device)) {
+    cudaMemPoolTrimTo(pool, 0);
+    (void)cudaGetLastError();
+  }
+}
+
+km_status LloydEngine::take_bytes(void** p, size_t bytes) {
+  *p = nullptr;
+  if (use != EngineUse::FIT) {
+    KM_TRY(scratch_alloc(p, bytes, device, stream));
+  } else {
+    cudaError_t e = cudaMalloc(p, bytes);
+    if (e == cudaErrorMemoryAllocation) {
+      (void)cudaGetLastError();
+      scratch_trim(device);
+      e = cudaMalloc(p, bytes);
+    }
+    if (e != cudaSuccess) {
+      set_last_error(e, "cudaMalloc", __FILE__, __LINE__);
+      (void)cudaGetLastError();
+      *p = nullptr;
+      return KM_ERR_ALLOC;
+    }
+  }
+  owned.push_back(*p);
+  return KM_OK;
+}
 
 // Relative error coefficients of the fast distance path (see TieBound).
 TieBound make_tie_bound(int precision, uint32_t d, bool a_exact) {
@@ -73,15 +131,11 @@ TieBound make_tie_bound(int precision, uint32_t d, bool a_exact) {
 
 LloydEngine::~LloydEngine() {
   if (device >= 0) cudaSetDevice(device);
-  dfree(X_owned); dfree(xn2); dfree(xn2d); dfree(Xb); dfree(Xlo);
-  dfree(C); dfree(Cn); dfree(cn2); dfree(dsq); dfree(objpart); dfree(shift_c); dfree(obj_c);
-  dfree(Cb); dfree(Clo); dfree(labels); dfree(mindist); dfree(queue); dfree(qfull); dfree(Ct);
-  dfree(qcnt); dfree(qfcnt); dfree(qwide); dfree(qwcnt); dfree(wlc); dfree(wl);
-  dfree(q2); dfree(q2full); dfree(q2cnt); dfree(q2fcnt); dfree(fidx); dfree(nfull);
-  dfree(seghist); dfree(counts); dfree(cstart); dfree(order); dfree(perm); dfree(red_part); dfree(st);
-  if (h_st) cudaFreeHost(h_st);
-  for (auto& l : kmat_lists)
-    if (l.dev) cudaFree(l.dev);
+  for (void* p : owned) {
+    if (use != EngineUse::FIT) scratch_free(p, device, stream);
+    else cudaFree(p);
+  }
+  if (h_st && h_st != &h_one) cudaFreeHost(h_st);
   if (aux) cudaStreamDestroy(aux);
   if (ev_fork) cudaEventDestroy(ev_fork);
   if (ev_join) cudaEventDestroy(ev_join);
@@ -89,20 +143,21 @@ LloydEngine::~LloydEngine() {
 }
 
 km_status LloydEngine::init(uint64_t n_, uint32_t d_, uint32_t k_, int precision_, int device_,
-                            void* stream_, bool need_update) {
+                            void* stream_, EngineUse use_) {
   if (n_ == 0 || d_ == 0 || k_ == 0 || k_ > n_) return KM_ERR_ARG;
   if (n_ >= (1ull << 32) - 256) return KM_ERR_ARG;           // labels / perm are 32-bit
   if ((uint64_t)d_ * n_ / d_ != n_) return KM_ERR_ARG;
   if (precision_ < KM_PREC_FP32 || precision_ > KM_PREC_BF16X3) return KM_ERR_ARG;
-  n = n_; d = d_; k = k_; precision = precision_; device = device_;
+  n = n_; d = d_; k = k_; precision = precision_; device = device_; use = use_;
   int ndev = 0;
   if (cudaGetDeviceCount(&ndev) != cudaSuccess || ndev == 0) { (void)cudaGetLastError(); return KM_ERR_NO_DEVICE; }
   if (device < 0 || device >= ndev) return KM_ERR_ARG;
   KM_CUDA_TRY(cudaSetDevice(device));
-  cudaDeviceProp prop;
-  KM_CUDA_TRY(cudaGetDeviceProperties(&prop, device));
-  if (prop.major != 10 || prop.minor != 3) return KM_ERR_NO_DEVICE;  // code is built for sm_103a only
-  num_sms = prop.multiProcessorCount;
+  int major = 0, minor = 0;
+  KM_CUDA_TRY(cudaDeviceGetAttribute(&major, cudaDevAttrComputeCapabilityMajor, device));
+  KM_CUDA_TRY(cudaDeviceGetAttribute(&minor, cudaDevAttrComputeCapabilityMinor, device));
+  if (major != 10 || minor != 3) return KM_ERR_NO_DEVICE;  // code is built for sm_103a only
+  KM_CUDA_TRY(cudaDeviceGetAttribute(&num_sms, cudaDevAttrMultiProcessorCount, device));
   if (stream_) {
     stream = static_cast<cudaStream_t>(stream_);
   } else {
@@ -128,53 +183,64 @@ km_status LloydEngine::init(uint64_t n_, uint32_t d_, uint32_t k_, int precision
   }
   tb = make_tie_bound(precision, d, false);
 
-  KM_TRY(dalloc(&xn2, n));
-  KM_TRY(dalloc(&xn2d, n));
-  if (precision != KM_PREC_FP32) {
-    KM_TRY(dalloc(&Xb, (size_t)n * dp));
-    KM_TRY(dalloc(&Cb, (size_t)kp * dp));
-    if (precision == KM_PREC_BF16X3) {
-      KM_TRY(dalloc(&Xlo, (size_t)n * dp));
-      KM_TRY(dalloc(&Clo, (size_t)kp * dp));
+  const bool points = use != EngineUse::UPDATE, assigns = use == EngineUse::FIT || use == EngineUse::ASSIGN,
+             updates = use == EngineUse::FIT || use == EngineUse::UPDATE;
+  if (points) {
+    KM_TRY(take(&xn2, n));
+    if (use == EngineUse::FIT) {               // sum ||x||^2 (the score) belongs to a fit
+      KM_TRY(take(&xn2d, n));
+      KM_TRY(take(&red_part, 256));
+    }
+    if (precision != KM_PREC_FP32) {
+      KM_TRY(take(&Xb, (size_t)n * dp));
+      if (precision == KM_PREC_BF16X3) KM_TRY(take(&Xlo, (size_t)n * dp));
     }
   }
-  KM_TRY(dalloc(&C, (size_t)k * d));
-  KM_TRY(dalloc(&cn2, (kp + 63) & ~63u));        // padded: +inf up to a multiple of 64
-  KM_TRY(dalloc(&labels, n));
-  KM_TRY(dalloc(&mindist, n));
-  {
+  if (assigns) {
+    if (precision != KM_PREC_FP32) {
+      KM_TRY(take(&Cb, (size_t)kp * dp));
+      if (precision == KM_PREC_BF16X3) KM_TRY(take(&Clo, (size_t)kp * dp));
+    }
+    KM_TRY(take(&C, (size_t)k * d));
+    KM_TRY(take(&Ct, (size_t)k * d));
+    KM_TRY(take(&cn2, (kp + 63) & ~63u));        // padded: +inf up to a multiple of 64
+    if (use == EngineUse::FIT) {               // one call writes the caller's arrays
+      KM_TRY(take(&labels, n));
+      KM_TRY(take(&mindist, n));
+    }
     const uint64_t rows = (n + 127) / 128 * 128;     // whole 128-row tiles
-    KM_TRY(dalloc(&queue, rows));
-    KM_TRY(dalloc(&qfull, rows));
-    KM_TRY(dalloc(&qcnt, rows / 32));
-    KM_TRY(dalloc(&qfcnt, rows / 32));
+    KM_TRY(take(&queue, rows));
+    KM_TRY(take(&qfull, rows));
+    KM_TRY(take(&qcnt, rows / 32));
+    KM_TRY(take(&qfcnt, rows / 32));
     rq = RefineQueues{queue, qfull, qcnt, qfcnt, rows / 32};
     if (precision != KM_PREC_FP32 && tc.chunked) {
       // candidate lists of the chunked distance kernel: up to 256 per row,
       // fewer when the lists would pass 16 GiB
       uint32_t L = 256;
       while (L > 32 && (uint64_t)rows * L * sizeof(uint2) > (16ull << 30)) L -= 32;
-      KM_TRY(dalloc(&qwide, rows));
-      KM_TRY(dalloc(&qwcnt, rows / 32));
-      KM_TRY(dalloc(&wlc, rows));
-      KM_TRY(dalloc(&wl, (size_t)rows * L));
+      KM_TRY(take(&qwide, rows));
+      KM_TRY(take(&qwcnt, rows / 32));
+      KM_TRY(take(&wlc, rows));
+      KM_TRY(take(&wl, (size_t)rows * L));
       rq.wide = qwide; rq.wcnt = qwcnt; rq.wl = wl; rq.wlc = wlc; rq.L = L;
-      KM_TRY(dalloc(&q2, rows));
-      KM_TRY(dalloc(&q2full, rows));
-      KM_TRY(dalloc(&q2cnt, rows / 32));
-      KM_TRY(dalloc(&q2fcnt, rows / 32));
-      KM_TRY(dalloc(&fidx, rows));
-      KM_TRY(dalloc(&nfull, 1));
+      KM_TRY(take(&q2, rows));
+      KM_TRY(take(&q2full, rows));
+      KM_TRY(take(&q2cnt, rows / 32));
+      KM_TRY(take(&q2fcnt, rows / 32));
+      KM_TRY(take(&fidx, rows));
+      KM_TRY(take(&nfull, 1));
       rq2 = RefineQueues{q2, q2full, q2cnt, q2fcnt, rows / 32};
       tb32 = make_tie_bound(KM_PREC_FP32, d, false);
     }
+    KM_TRY(refine_prepare());
   }
-  KM_TRY(dalloc(&Ct, (size_t)k * d));
-  KM_TRY(dalloc(&red_part, 256));
-  KM_TRY(dalloc(&st, 1));
-  KM_CUDA_TRY(cudaMallocHost(reinterpret_cast<void**>(&h_st), sizeof(DevState)));
+  KM_TRY(take(&st, 1));
+  if (use == EngineUse::FIT) KM_CUDA_TRY(cudaMallocHost(reinterpret_cast<void**>(&h_st), sizeof(DevState)));
+  else h_st = &h_one;
   std::memset(h_st, 0, sizeof(DevState));
   KM_CUDA_TRY(cudaMemsetAsync(st, 0, sizeof(DevState), stream));
+  if (!updates) return KM_OK;
 
   // Stable-sort geometry: segments of `seg` rows, k x nseg counts.
   seg = 1024;
@@ -189,23 +255,22 @@ km_status LloydEngine::init(uint64_t n_, uint32_t d_, uint32_t k_, int precision
   sort_smem = per_warp * sort_wpb;
   if (sort_smem > 227 * 1024) return KM_ERR_UNSUPPORTED;
   if (sort_smem > 48 * 1024) {
-    KM_CUDA_TRY(cudaFuncSetAttribute(seg_hist_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sort_smem));
-    KM_CUDA_TRY(cudaFuncSetAttribute(seg_scatter_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sort_smem));
+    KM_CUDA_TRY(cudaFuncSetAttribute(seg_hist_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, DYN_SMEM_MAX));
+    KM_CUDA_TRY(cudaFuncSetAttribute(seg_scatter_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, DYN_SMEM_MAX));
   }
-  KM_TRY(refine_prepare());
-  if (need_update) {
-    KM_TRY(update_sums_prepare());
-    KM_TRY(dalloc(&Cn, (size_t)k * d));
-    KM_TRY(dalloc(&dsq, (size_t)k * d));
-    KM_TRY(dalloc(&objpart, (size_t)k * d));
-    KM_TRY(dalloc(&shift_c, k));
-    KM_TRY(dalloc(&obj_c, k));
-    KM_TRY(dalloc(&seghist, (size_t)k * nseg));
-    KM_TRY(dalloc(&counts, k));
-    KM_TRY(dalloc(&cstart, (size_t)k + 1));
-    KM_TRY(dalloc(&order, k));
-    KM_TRY(dalloc(&perm, n));
+  KM_TRY(update_sums_prepare());
+  if (use == EngineUse::FIT) {
+    KM_TRY(take(&Cn, (size_t)k * d));
+    KM_TRY(take(&dsq, (size_t)k * d));
+    KM_TRY(take(&objpart, (size_t)k * d));
+    KM_TRY(take(&shift_c, k));
+    KM_TRY(take(&obj_c, k));
   }
+  KM_TRY(take(&seghist, (size_t)k * nseg));
+  KM_TRY(take(&counts, k));
+  KM_TRY(take(&cstart, (size_t)k + 1));
+  KM_TRY(take(&order, k));
+  KM_TRY(take(&perm, n));
   return KM_OK;
 }
 
@@ -218,7 +283,7 @@ km_status LloydEngine::set_points(const float* Xsrc, bool on_device, bool copy) 
   // the copies of the chunks after it.
   const bool chunked = !on_device && bytes >= (64ull << 20);
   if (copy || !on_device) {
-    if (!X_owned) KM_TRY(dalloc(&X_owned, (size_t)n * d));
+    if (!X_owned) KM_TRY(take(&X_owned, (size_t)n * d));
     X = X_owned;
   } else {
     X = Xsrc;
@@ -242,7 +307,7 @@ km_status LloydEngine::set_points(const float* Xsrc, bool on_device, bool copy) 
       KM_CUDA_TRY(cudaMemcpyAsync(X_owned + r0 * d, Xsrc + r0 * d, sizeof(float) * (r1 - r0) * d,
                                   cudaMemcpyHostToDevice, sc));
       const int blocks = (int)std::min<uint64_t>((r1 - r0 + 7) / 8, (uint64_t)num_sms * 8);
-      prep_points_kernel<<<blocks, 256, 0, sc>>>(X + r0 * d, r1 - r0, d, dp, xn2 + r0, xn2d + r0,
+      prep_points_kernel<<<blocks, 256, 0, sc>>>(X + r0 * d, r1 - r0, d, dp, xn2 + r0, xn2d ? xn2d + r0 : nullptr,
                                                  Xb ? Xb + r0 * dp : nullptr, Xlo ? Xlo + r0 * dp : nullptr, st);
     }
     KM_CUDA_TRY(cudaEventRecord(ev_join, aux));
@@ -255,10 +320,12 @@ km_status LloydEngine::set_points(const float* Xsrc, bool on_device, bool copy) 
     prep_points_kernel<<<blocks, 256, 0, stream>>>(X, n, d, dp, xn2, xn2d, Xb, Xlo, st);
   }
   KM_CUDA_TRY(cudaGetLastError());
-  reduce_f64_partial_kernel<<<256, 256, 0, stream>>>(xn2d, n, red_part);
-  reduce_f64_final_kernel<<<1, 32, 0, stream>>>(red_part, 256, &st->sum_x2);
-  KM_CUDA_TRY(cudaGetLastError());
-  if (precision != KM_PREC_FP32) {
+  if (xn2d) {
+    reduce_f64_partial_kernel<<<256, 256, 0, stream>>>(xn2d, n, red_part);
+    reduce_f64_final_kernel<<<1, 256, 0, stream>>>(red_part, 256, &st->sum_x2);
+    KM_CUDA_TRY(cudaGetLastError());
+  }
+  if (precision != KM_PREC_FP32 && Cb) {
     KM_TRY(encode_tmap_bf16(&tmA, Xb, dp, n, 64, 128));
     const uint32_t bbox = tc.chunked ? tc.NC : kp;    // rows of one B load
     KM_TRY(encode_tmap_bf16(&tmB, Cb, dp, kp, 64, bbox));
@@ -289,13 +356,15 @@ __global__ void bf16_decode_kernel(const uint16_t* __restrict__ src, uint64_t co
 
 km_status LloydEngine::set_points_bf16(const uint16_t* Xsrc, bool on_device) {
   KM_CUDA_TRY(cudaSetDevice(device));
-  if (!X_owned) KM_TRY(dalloc(&X_owned, (size_t)n * d));
+  if (!X_owned) KM_TRY(take(&X_owned, (size_t)n * d));
   const uint64_t count = n * (uint64_t)d;
   const uint16_t* src = Xsrc;
   uint16_t* tmp = nullptr;
   if (!on_device) {
     // host BF16 bits go to a staging buffer (half the bytes of the FP32 copy)
-    KM_TRY(dalloc(&tmp, count));
+    void* q = nullptr;
+    KM_TRY(scratch_alloc(&q, sizeof(uint16_t) * count, device, stream));
+    tmp = static_cast<uint16_t*>(q);
     KM_CUDA_TRY(cudaMemcpyAsync(tmp, Xsrc, sizeof(uint16_t) * count, cudaMemcpyHostToDevice, stream));
     src = tmp;
   }
@@ -304,7 +373,7 @@ km_status LloydEngine::set_points_bf16(const uint16_t* Xsrc, bool on_device) {
   cudaError_t le = cudaGetLastError();
   if (tmp) {
     cudaError_t se = cudaStreamSynchronize(stream);
-    cudaFree(tmp);
+    scratch_free(tmp, device, stream);
     KM_CUDA_TRY(le);
     KM_CUDA_TRY(se);
   }

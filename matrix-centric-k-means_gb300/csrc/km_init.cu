@@ -450,9 +450,16 @@ __global__ void pp_gather_kernel(const float* __restrict__ X, uint32_t d, const 
 namespace {
 template <typename T>
 struct DevBuf {
+  LloydEngine& e;
   T* p = nullptr;
-  ~DevBuf() { if (p) cudaFree(p); }
-  cudaError_t alloc(size_t count) { return cudaMalloc(reinterpret_cast<void**>(&p), sizeof(T) * count); }
+  explicit DevBuf(LloydEngine& eng) : e(eng) {}
+  ~DevBuf() { scratch_free(p, e.device, e.stream); }
+  km_status alloc(size_t count) {
+    void* q = nullptr;
+    KM_TRY(scratch_alloc(&q, sizeof(T) * count, e.device, e.stream));
+    p = static_cast<T*>(q);
+    return KM_OK;
+  }
 };
 }  // namespace
 
@@ -481,20 +488,23 @@ km_status plusplus_init(LloydEngine& e, int seed) {
                                  : smem;
   const bool v4 = d % 4 == 0 && reinterpret_cast<uintptr_t>(e.X) % 16 == 0;
   auto tile = S == 4u ? pp_cost_kernel<4> : S == 8u ? pp_cost_kernel<8> : pp_cost_kernel<16>;
-  DevBuf<float> d2, D;
-  DevBuf<double> bsum, cpart, u;
-  DevBuf<int32_t> cand, chosen;
-  DevBuf<PpState> state;
-  if (d2.alloc(n) || D.alloc(n * s) || bsum.alloc(nblk) || cpart.alloc((size_t)ncost * s) ||
-      u.alloc(hu.size()) || cand.alloc(s) || chosen.alloc(k) || state.alloc(1)) {
-    (void)cudaGetLastError();
-    return KM_ERR_ALLOC;
-  }
+  DevBuf<float> d2(e), D(e);
+  DevBuf<double> bsum(e), cpart(e), u(e);
+  DevBuf<int32_t> cand(e), chosen(e);
+  DevBuf<PpState> state(e);
+  KM_TRY(d2.alloc(n));
+  KM_TRY(D.alloc(n * s));
+  KM_TRY(bsum.alloc(nblk));
+  KM_TRY(cpart.alloc((size_t)ncost * s));
+  KM_TRY(u.alloc(hu.size()));
+  KM_TRY(cand.alloc(s));
+  KM_TRY(chosen.alloc(k));
+  KM_TRY(state.alloc(1));
   if (cost_smem > 48 * 1024) {
     if (tiled)
-      KM_CUDA_TRY(cudaFuncSetAttribute(tile, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cost_smem));
+      KM_CUDA_TRY(cudaFuncSetAttribute(tile, cudaFuncAttributeMaxDynamicSharedMemorySize, DYN_SMEM_MAX - 4096));
     else
-      KM_CUDA_TRY(cudaFuncSetAttribute(pp_cost_wide_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cost_smem));
+      KM_CUDA_TRY(cudaFuncSetAttribute(pp_cost_wide_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, DYN_SMEM_MAX - 4096));
   }
   cudaStream_t st = e.stream;
   KM_CUDA_TRY(cudaMemsetAsync(state.p, 0, sizeof(PpState), st));
@@ -514,7 +524,7 @@ km_status plusplus_init(LloydEngine& e, int seed) {
   }
   pp_gather_kernel<<<(unsigned)(((uint64_t)k * d + 255) / 256), 256, 0, st>>>(e.X, d, chosen.p, k, e.C);
   KM_CUDA_TRY(cudaGetLastError());
-  // the scratch buffers are freed on return: wait for the kernels using them
+  // the host arrays copied from go on return
   KM_CUDA_TRY(cudaStreamSynchronize(st));
   return KM_OK;
 }

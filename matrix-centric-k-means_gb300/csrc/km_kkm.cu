@@ -962,12 +962,10 @@ km_status kmat_tiles_dev(LloydEngine& e, uint64_t n, uint64_t row0, uint64_t row
   l.row0 = row0;
   l.row_end = row_end;
   l.count = t.size() / 2;
-  if (cudaMalloc(&l.dev, sizeof(uint32_t) * std::max<size_t>(2, t.size())) != cudaSuccess) {
-    (void)cudaGetLastError();
-    return KM_ERR_ALLOC;
-  }
+  KM_TRY(e.take(&l.dev, std::max<size_t>(2, t.size())));
   e.kmat_lists.push_back(l);
-  KM_CUDA_TRY(cudaMemcpy(l.dev, t.data(), sizeof(uint32_t) * t.size(), cudaMemcpyHostToDevice));
+  // (a copy from pageable memory has left the vector when the call returns)
+  KM_CUDA_TRY(cudaMemcpyAsync(l.dev, t.data(), sizeof(uint32_t) * t.size(), cudaMemcpyHostToDevice, e.stream));
   *dev = l.dev;
   *count = l.count;
   return KM_OK;
@@ -1190,7 +1188,7 @@ km_status km_kernel_matrix(const float* X_dev, uint64_t n, uint32_t d, int32_t k
   int dev;
   if (cudaGetDevice(&dev) != cudaSuccess) { (void)cudaGetLastError(); return KM_ERR_NO_DEVICE; }
   LloydEngine e;
-  KM_TRY(e.init(n, d, 1, precision, dev, stream, false));
+  KM_TRY(e.init(n, d, 1, precision, dev, stream, EngineUse::KMAT));
   KM_TRY(e.set_points(X_dev, true, false));
   km_kkm_params p{};
   p.kernel_fn = kernel_fn; p.gamma = gamma; p.coef = coef; p.degree = degree; p.sigma = sigma;
@@ -1226,7 +1224,7 @@ km_status km_kkm_create(const km_kkm_params* p, km_kkm** out) {
   h->vk_smem = vk_smem;
   h->vk_warps = vk_warps;
   h->glab = glab;
-  km_status s = h->eng.init(p->n, p->d, p->k, p->precision, p->device, p->stream, true);
+  km_status s = h->eng.init(p->n, p->d, p->k, p->precision, p->device, p->stream, EngineUse::FIT);
   auto fail = [&](km_status st) { km_kkm_destroy(h); return st; };
   if (s != KM_OK) return fail(s);
   if (cudaMalloc(&h->diag, sizeof(float) * p->n) != cudaSuccess ||
@@ -1275,14 +1273,14 @@ km_status km_kkm_create(const km_kkm_params* p, km_kkm** out) {
   bool attr_ok = true;
   if (glab) {
     attr_ok = cudaFuncSetAttribute(kkm_vk_kernel<true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   (int)vk_smem) == cudaSuccess &&
+                                   DYN_SMEM_MAX) == cudaSuccess &&
               cudaFuncSetAttribute(kkm_vk_kernel<false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   (int)vk_smem) == cudaSuccess;
+                                   DYN_SMEM_MAX) == cudaSuccess;
   } else {
     attr_ok = cudaFuncSetAttribute(kkm_vk_kernel<true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   (int)vk_smem) == cudaSuccess &&
+                                   DYN_SMEM_MAX) == cudaSuccess &&
               cudaFuncSetAttribute(kkm_vk_kernel<false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   (int)vk_smem) == cudaSuccess;
+                                   DYN_SMEM_MAX) == cudaSuccess;
   }
   if (!attr_ok || cudaEventCreate(&h->ev0) != cudaSuccess || cudaEventCreate(&h->ev1) != cudaSuccess ||
       cudaMallocHost(reinterpret_cast<void**>(&h->h_done), sizeof(int32_t)) != cudaSuccess) {

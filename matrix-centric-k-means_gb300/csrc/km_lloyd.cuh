@@ -97,7 +97,13 @@ struct KmatTileList {
   uint32_t* dev = nullptr;
 };
 
+// What an engine is for: a handle that lives for many fits (its buffers come from
+// cudaMalloc), or one call (only the buffers of that call, from the scratch pool).
+enum class EngineUse { FIT, ASSIGN, UPDATE, KMAT };
+
 struct LloydEngine {
+  EngineUse use = EngineUse::FIT;
+  std::vector<void*> owned;   // every device buffer below
   int device = 0;
   cudaStream_t stream = nullptr;
   bool own_stream = false;
@@ -138,7 +144,8 @@ struct LloydEngine {
   uint32_t* perm = nullptr;
   double* red_part = nullptr;
   DevState* st = nullptr;
-  DevState* h_st = nullptr;   // pinned mirror
+  DevState* h_st = nullptr;   // host mirror (pinned for a handle)
+  DevState h_one{};           // the mirror of one call
   uint32_t seg = 1024, nseg = 0;
   int sort_wpb = 8;
   size_t sort_smem = 0;
@@ -160,8 +167,16 @@ struct LloydEngine {
   std::vector<KmatTileList> kmat_lists;   // symmetric kernel-matrix builds (km_kkm.cu)
 
   ~LloydEngine();
-  km_status init(uint64_t n, uint32_t d, uint32_t k, int precision, int device, void* stream,
-                 bool need_update);
+  km_status init(uint64_t n, uint32_t d, uint32_t k, int precision, int device, void* stream, EngineUse use);
+  // A device buffer of `count` elements, freed with the engine.
+  template <class T>
+  km_status take(T** p, size_t count) {
+    void* q = nullptr;
+    KM_TRY(take_bytes(&q, (count ? count : 1) * sizeof(T)));
+    *p = static_cast<T*>(q);
+    return KM_OK;
+  }
+  km_status take_bytes(void** p, size_t bytes);
   km_status set_points(const float* Xsrc, bool on_device, bool copy);
   // Points stored as BF16 (raw bit patterns, n*d): decoded once to the FP32
   // copy, which is then exactly representable in BF16 (Xb = the input).

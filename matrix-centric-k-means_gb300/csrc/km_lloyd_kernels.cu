@@ -96,10 +96,14 @@ __global__ void reduce_f64_partial_kernel(const double* __restrict__ v, uint64_t
   if (threadIdx.x == 0) part[blockIdx.x] = sh[0];
 }
 
+// One block of at least np threads: the loads together, then the sum in order.
 __global__ void reduce_f64_final_kernel(const double* __restrict__ part, int np, double* out) {
-  if (threadIdx.x == 0 && blockIdx.x == 0) {
+  __shared__ double sh[256];
+  if ((int)threadIdx.x < np) sh[threadIdx.x] = part[threadIdx.x];
+  __syncthreads();
+  if (threadIdx.x == 0) {
     double s = 0.0;
-    for (int i = 0; i < np; ++i) s += part[i];
+    for (int i = 0; i < np; ++i) s += sh[i];
     *out = s;
   }
 }

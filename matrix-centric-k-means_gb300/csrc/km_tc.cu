@@ -821,12 +821,12 @@ namespace {
 template <int MODE>
 km_status set_attr_mode(const TcPlan& pl) {
   if (pl.chunked)
-    KM_CUDA_TRY(cudaFuncSetAttribute(assign_tc_chunked_kernel<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pl.smem));
+    KM_CUDA_TRY(cudaFuncSetAttribute(assign_tc_chunked_kernel<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, DYN_SMEM_MAX));
   else {
     KM_CUDA_TRY(cudaFuncSetAttribute(assign_tc_kernel<MODE, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)pl.smem));
+                                     DYN_SMEM_MAX));
     KM_CUDA_TRY(cudaFuncSetAttribute(assign_tc_kernel<MODE, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)pl.smem));
+                                     DYN_SMEM_MAX));
   }
   return KM_OK;
 }
