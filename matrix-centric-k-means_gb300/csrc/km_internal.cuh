@@ -134,13 +134,13 @@ struct LoopConsts {
 // A = 2*eps_dot + 2u covers the dot-product error and the final rounding and
 // B = 2u covers the rounding of ||c||^2 and of the subtraction.  The
 // reference's CPU distance sum_j fl(fl(x_j - c_j)^2), summed in float, has
-// relative error at most g = gamma_{d+2}.  If, with T an upper bound of
-// ||x||^2, v1 <= v2 <= v3 the three smallest fast values and c1 the argmin,
-//   (v2 - v1) > Emax + E1 + g * (2T + v1 + v2 + E1 - Emax)
-// then the reference's argmin is c1 (class 0).  The same test with v3 in place
-// of v2 proves it is one of the two best fast candidates (class 1); otherwise
-// the row is re-scored against all k centroids (class 2).  Both refinements use
-// the reference's exact formula, so the final labels equal the reference's.
+// relative error at most g = gamma_{d+2}.  With T an upper bound of ||x||^2, v1 the
+// smallest fast value and Em the largest E(c), a centroid whose fast value is above
+//   tau(v1) = (v1 + 2 Em + g * max(0, 2T + v1 + 2 Em)) / (1 - g)
+// has a reference distance above the reference's best, so the reference's argmin
+// lies in {c : v(c) <= tau(v1)} (tie_tau).  Rows with several candidates are
+// re-scored with the reference's exact formula, so the final labels equal the
+// reference's.
 // ---------------------------------------------------------------------------
 struct TieBound {
   float A;      // coefficient of ||x||*||c||
@@ -152,81 +152,6 @@ struct TieBound {
 // a_exact: every point coordinate is exactly a BF16 value, so only the
 // centroid operand carries a rounding error.
 TieBound make_tie_bound(int precision, uint32_t d, bool a_exact);
-
-__device__ __forceinline__ int tie_class(float X2, float v1, float v2, float v3, float cn1,
-                                         float cmax, const TieBound& tb) {
-  const float nx = sqrtf(X2) * 1.0000005f;
-  const float T = X2 * 1.0000003f;
-  const float E1 = tb.A * nx * cn1 + tb.B * cn1 * cn1;
-  const float Em = tb.A * nx * cmax + tb.B * cmax * cmax;
-  const float base = Em + E1;
-  const float s = fmaxf(0.0f, 2.0f * T + v1 + E1 - Em);
-  const float rhs2 = tb.safety * (base + tb.g * (s + v2)) + 1e-30f;
-  const float rhs3 = tb.safety * (base + tb.g * (s + v3)) + 1e-30f;
-  // NaN or Inf anywhere makes the comparisons false: such rows take the full path.
-  const bool fin = isfinite(T + v1 + E1 + Em);
-  if (fin && (v2 - v1) > rhs2) return 0;
-  if (fin && (v3 - v1) > rhs3) return 1;
-  return 2;
-}
-
-// Top-3 of (value, index) under the order (v, i) < (w, j) iff v < w or
-// (v == w and i < j).  Only the two best keep their index; the third value can
-// never move into the top two when two such lists are merged.
-struct Top3 {
-  float v1, v2, v3;
-  uint32_t i1, i2;
-  __device__ __forceinline__ void init() {
-    v1 = v2 = v3 = __int_as_float(0x7f800000);
-    i1 = i2 = 0xffffffffu;
-  }
-  __device__ __forceinline__ void insert(float v, uint32_t i) {
-    if (v < v1 || (v == v1 && i < i1)) {
-      v3 = v2; v2 = v1; i2 = i1; v1 = v; i1 = i;
-    } else if (v < v2 || (v == v2 && i < i2)) {
-      v3 = v2; v2 = v; i2 = i;
-    } else if (v < v3) {
-      v3 = v;
-    }
-  }
-  // Branch-free insertion under the (v, i) order (selects only, so that lanes
-  // of a warp never diverge).
-  __device__ __forceinline__ void insert_nb(float v, uint32_t i) {
-    const bool c1 = v < v1 || (v == v1 && i < i1);
-    const bool c2 = v < v2 || (v == v2 && i < i2);
-    const bool c3 = v < v3;
-    v3 = c2 ? v2 : (c3 ? v : v3);
-    v2 = c1 ? v1 : (c2 ? v : v2);
-    i2 = c1 ? i1 : (c2 ? i : i2);
-    v1 = c1 ? v : v1;
-    i1 = c1 ? i : i1;
-  }
-  // Insertion when every index already held is below i (columns visited in
-  // ascending order): a tie keeps the earlier entry, so strict '<' gives the
-  // (v, i) order for finite values.
-  __device__ __forceinline__ void insert_asc(float v, uint32_t i) {
-    const bool c1 = v < v1, c2 = v < v2, c3 = v < v3;
-    v3 = c2 ? v2 : (c3 ? v : v3);
-    v2 = c1 ? v1 : (c2 ? v : v2);
-    i2 = c1 ? i1 : (c2 ? i : i2);
-    v1 = c1 ? v : v1;
-    i1 = c1 ? i : i1;
-  }
-  __device__ __forceinline__ void merge(const Top3& o) {
-    insert_nb(o.v1, o.i1);
-    insert_nb(o.v2, o.i2);
-    v3 = fminf(v3, o.v3);
-  }
-  __device__ __forceinline__ void shfl_merge_xor(int mask, unsigned members = 0xffffffffu) {
-    Top3 o;
-    o.v1 = __shfl_xor_sync(members, v1, mask);
-    o.v2 = __shfl_xor_sync(members, v2, mask);
-    o.v3 = __shfl_xor_sync(members, v3, mask);
-    o.i1 = __shfl_xor_sync(members, i1, mask);
-    o.i2 = __shfl_xor_sync(members, i2, mask);
-    merge(o);
-  }
-};
 
 // Refinement queue entry: a row whose reference argmin is proven to be one of
 // `cnt` (2..4) candidate centroids.  Rows with more candidates go to the

@@ -13,10 +13,12 @@
 //   convergence           comparisons/CPU_Kmeans/src/kmeans.cpp:170-200;
 //                         src/kmeans.cu:1054-1073 (score rule)
 #include "km_lloyd.cuh"
+#include "km_simt.cuh"
 #include "km_sums.cuh"
 
 #include <cmath>
 #include <cfloat>
+#include <type_traits>
 
 namespace km {
 
@@ -143,225 +145,216 @@ __global__ void prep_centroids_kernel(const float* __restrict__ C, uint32_t k, u
 }
 
 // ---------------------------------------------------------------------------
-// (a)+(b) SIMT FP32 distance GEMM with fused top-3 argmin.
-// Tile 128 rows x 128 centroids, 256 threads, 8x8 register micro-tiles,
-// K chunks of 16 staged through shared memory with register double buffering
-// (16-byte global loads when d % 4 == 0 and the rows are 16-byte aligned).
-// Every CTA walks all centroid tiles for its rows, so the row tile is read from
-// HBM once and re-read from L2.
+// (a)+(b) SIMT FP32 distances with the argmin fused (km_simt.cuh has the product).
+// A CTA takes ROWS rows and walks all centroids, COLS at a time.  After each
+// column tile a row's minimum over its TX threads (exchanged by shuffles) joins
+// the row's running minimum m, and every centroid with v(c) <= tau(m) (tie_tau)
+// goes to the row's list of up to F32_LIST (value, index) pairs in shared memory,
+// which drops the entries above the current tau between tiles.  tau only falls with
+// m, so the entries with v(c) <= tau(m_final) are the whole candidate set: one is the proven argmin, 2..4 go to the short re-score queue,
+// more (or a full list, or values that are not finite) to the full re-score.
+//
+// Bound by the FP32 pipes.  The tile is as wide as k asks (32, 48, 64, 96 or 128
+// centroids), so that k = 64 pays for 64.  Measured, distance kernel: n = 200,000
+// d = 100 k = 64 161 -> 75 us, k = 20 159 -> 55 us, k = 90 162 -> 109 us; n = 1M d =
+// 128 k = 256 1571 -> 1568 us = 22 T FMA/s (16 columns a thread instead, or 16 rows,
+// left eight warps an SM, 44 % of the issue slots used and 21 T).
 // ---------------------------------------------------------------------------
-namespace {
-constexpr int SM_ = 128, SN_ = 128, SK_ = 16, SPAD = 4;
-// Dynamic shared memory of assign_f32_kernel: each thread's running top-3 of
-// its eight rows, five arrays (v1, v2, v3, i1, i2) of [128 rows][F32_TOP_LD]
-// words, lane tx of a row at column tx.  The stride 18 keeps the epilogue's
-// accesses (two rows 8 apart per warp) conflict-free and the final per-row
-// merge two-way at most.
-constexpr int F32_TOP_LD = 18;
-constexpr size_t F32_TOP_SMEM = 5 * 128 * F32_TOP_LD * sizeof(float);
+constexpr int F32_NT = 128, F32_RT = 8, F32_LIST = 8;
+template <int TX, int CT>
+using F32Tile = SimtTile<F32_NT, F32_RT, TX, CT, TX == 16 && CT == 8 ? 16 : 8>;
+// Shared memory after the product's stages: per row m, tau's row terms, the
+// squared norm, the list and its length; per column the centroid's squared norm.
+struct F32Row {
+  float m, x2;
+  TauRow tr;
+  uint32_t cnt;
+  uint32_t row;                 // row of X
+};
+template <class T>
+constexpr size_t f32_smem() {
+  return T::SMEM + T::ROWS * (sizeof(F32Row) + F32_LIST * sizeof(uint2)) + T::COLS * sizeof(float);
 }
 
-// Thread (tx, ty) of the 16 x 16 grid owns rows ty*8 .. ty*8+7 and the two
-// column quads tx*4 .. tx*4+3 and 64 + tx*4 .. +3 of the 128 x 128 tile: the
-// quarter-warps' 16-byte centroid loads from shared memory then cover 128
-// contiguous bytes (no bank conflicts), and two CTAs fit an SM.
-// DOUT (distance-matrix output): one CTA per SM, so that its stores do not spill.
-template <bool V4, bool DOUT>
-__global__ void __launch_bounds__(256, DOUT ? 1 : 2)
-assign_f32_kernel(const float* __restrict__ X, const float* __restrict__ C,
+// Gather mode (ridx != null): logical row li of the tiles is row ridx[li] of X,
+// for li < *nidx; queue segments are taken over the logical rows.
+template <int TX, int CT, bool DOUT>
+__global__ void __launch_bounds__(F32_NT, CT == 8 ? 3 : 4)
+assign_f32_kernel(const float* __restrict__ X, const float* __restrict__ C, bool v4,
                   const float* __restrict__ cn2, const float* __restrict__ xn2, uint64_t n,
                   uint32_t d, uint32_t k, TieBound tb, DevState* st,
                   uint32_t* __restrict__ labels, float* __restrict__ mindist,
                   RefineQueues rq, float* __restrict__ Dout, const uint32_t* __restrict__ ridx,
                   const uint32_t* __restrict__ nidx) {
+  using T = F32Tile<TX, CT>;
   griddep_wait();
   if (st->done) return;
-  // Gather mode (ridx != null): logical row li of the tiles is row ridx[li] of X,
-  // for li < *nidx; queue segments are taken over the logical rows.
   const uint64_t n_log = ridx ? (uint64_t)*nidx : n;
-  if ((uint64_t)blockIdx.x * SM_ >= n_log) return;
-  __shared__ uint32_t rmap[SM_];
-  __shared__ __align__(16) float As[2][SK_][SM_ + SPAD];
-  __shared__ __align__(16) float Bs[2][SK_][SN_ + SPAD];
-  __shared__ float cns[SN_];
-  // Each thread's running top-3 of its eight rows over the column tiles so far.
-  // A thread visits its columns in ascending order (tx*4 + j, then 64 + tx*4 +
-  // j, tile by tile), so strict-order insertion keeps the lowest index on
-  // ties; after the last tile one thread per row merges the row's 16 lists
-  // under the (v, i) order.
-  extern __shared__ float f32_top[];
-  constexpr int TA = SM_ * F32_TOP_LD;
-  float* const tv1 = f32_top;
-  float* const tv2 = f32_top + TA;
-  float* const tv3 = f32_top + 2 * TA;
-  uint32_t* const ti1 = reinterpret_cast<uint32_t*>(f32_top + 3 * TA);
-  uint32_t* const ti2 = reinterpret_cast<uint32_t*>(f32_top + 4 * TA);
-
-  const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
-#pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    const int o = (ty * 8 + i) * F32_TOP_LD + tx;
-    tv1[o] = tv2[o] = tv3[o] = f_inf();
-    ti1[o] = ti2[o] = 0xffffffffu;
-  }
-  const uint64_t m0 = (uint64_t)blockIdx.x * SM_;
-  if (tid < SM_) {
-    const uint64_t li = m0 + tid;
-    rmap[tid] = ridx ? (li < n_log ? ridx[li] : 0u) : (uint32_t)li;
+  const uint64_t m0 = (uint64_t)blockIdx.x * T::ROWS;
+  // (Without a gather the grid covers every segment of the queues, whose counts
+  // all have to be written; a gather's start at zero.)
+  if (ridx && m0 >= n_log) return;
+  extern __shared__ __align__(16) float f32_smem_raw[];
+  uint2* const list = reinterpret_cast<uint2*>(f32_smem_raw + T::SMEM / sizeof(float));   // [ROWS][F32_LIST]
+  F32Row* const rs = reinterpret_cast<F32Row*>(list + T::ROWS * F32_LIST);
+  float* const cns = reinterpret_cast<float*>(rs + T::ROWS);
+  const int tid = threadIdx.x, tx = tid % TX, ty = tid / TX;
+  const float cmax = st->cmax;
+  for (int r = tid; r < T::ROWS; r += F32_NT) {
+    const uint64_t li = m0 + (uint64_t)r;
+    F32Row w{};
+    if (li < n_log) {
+      w.row = ridx ? ridx[li] : (uint32_t)li;
+      w.x2 = xn2[w.row];
+    }
+    w.m = f_inf();
+    w.tr = tie_tau_row(w.x2, cmax, tb);
+    rs[r] = w;
   }
   __syncthreads();
-  const uint32_t ntiles = (k + SN_ - 1) / SN_;
-  const uint32_t nk = (d + SK_ - 1) / SK_;
-
-  for (uint32_t nt = 0; nt < ntiles; ++nt) {
-    const uint32_t c0 = nt * SN_;
-    __syncthreads();
-    if (tid < SN_) cns[tid] = (c0 + tid < k) ? cn2[c0 + tid] : f_inf();
-
-    float acc[8][8];
+  for (uint32_t c0 = 0; c0 < k; c0 += T::COLS) {
+    for (int c = tid; c < T::COLS; c += F32_NT) cns[c] = c0 + (uint32_t)c < k ? cn2[c0 + c] : f_inf();
+    float2 acc[F32_RT / 2][CT];
+    simt_product<T>(
+        f32_smem_raw, d, v4,
+        [&](int r) { return m0 + (uint64_t)r < n_log ? X + (uint64_t)rs[r].row * d : (const float*)nullptr; },
+        [&](int c) { return c0 + (uint32_t)c < k ? C + (uint64_t)(c0 + c) * d : (const float*)nullptr; }, acc);
+    // v = ||c||^2 - 2 x.c in place; columns at or past k hold +inf (or NaN)
+    float cn[CT];
 #pragma unroll
-    for (int i = 0; i < 8; ++i)
+    for (int j = 0; j < CT; ++j) cn[j] = cns[T::col(tx, j)];
+    float mine[F32_RT];
 #pragma unroll
-      for (int j = 0; j < 8; ++j) acc[i][j] = 0.0f;
-
-    float ra[8], rb[8];
-    auto gload = [&](uint32_t kc) {
-      if constexpr (V4) {
+    for (int i = 0; i < F32_RT / 2; ++i) {
+      mine[2 * i] = mine[2 * i + 1] = f_inf();
 #pragma unroll
-        for (int e = 0; e < 2; ++e) {
-          const int idx = e * 256 + tid;
-          const int r = idx >> 2, c4 = idx & 3;
-          const uint32_t col = kc + 4u * (uint32_t)c4;
-          const bool rv = m0 + r < n_log;
-          const uint64_t row = rmap[r];
-          const uint32_t cc = c0 + r;
-          float4 a = make_float4(0.f, 0.f, 0.f, 0.f), b = a;
-          if (rv && col < d) a = __ldg(reinterpret_cast<const float4*>(X + row * d + col));
-          if (cc < k && col < d) b = __ldg(reinterpret_cast<const float4*>(C + (uint64_t)cc * d + col));
-          ra[4 * e + 0] = a.x; ra[4 * e + 1] = a.y; ra[4 * e + 2] = a.z; ra[4 * e + 3] = a.w;
-          rb[4 * e + 0] = b.x; rb[4 * e + 1] = b.y; rb[4 * e + 2] = b.z; rb[4 * e + 3] = b.w;
-        }
-      } else {
+      for (int j = 0; j < CT; ++j) {
+        acc[i][j] = __ffma2_rn(make_float2(-2.0f, -2.0f), acc[i][j], make_float2(cn[j], cn[j]));
+        mine[2 * i] = fminf(mine[2 * i], acc[i][j].x);
+        mine[2 * i + 1] = fminf(mine[2 * i + 1], acc[i][j].y);
+      }
+    }
 #pragma unroll
-        for (int e = 0; e < 8; ++e) {
-          const int idx = e * 256 + tid;
-          const int r = idx >> 4, kk = idx & 15;
-          const uint32_t col = kc + kk;
-          const uint64_t row = rmap[r];
-          ra[e] = (m0 + r < n_log && col < d) ? X[row * d + col] : 0.0f;
-          const uint32_t cc = c0 + r;
-          rb[e] = (cc < k && col < d) ? C[(uint64_t)cc * d + col] : 0.0f;
+    for (int i = 0; i < F32_RT; ++i) {
+      const int r = ty * F32_RT + i;
+      float m = mine[i];
+#pragma unroll
+      for (int o = 1; o < TX; o <<= 1) m = fminf(m, __shfl_xor_sync(0xffffffffu, m, o));
+      m = fminf(m, rs[r].m);
+      const float tau = tie_tau_at(rs[r].tr, m, tb);
+      auto val = [&](int j) { return (i & 1) ? acc[i / 2][j].y : acc[i / 2][j].x; };
+      if (DOUT && m0 + (uint64_t)r < n_log) {
+#pragma unroll
+        for (int j = 0; j < CT; ++j) {
+          const uint32_t c = c0 + (uint32_t)T::col(tx, j);
+          if (c < k) Dout[(uint64_t)rs[r].row * k + c] = val(j) + rs[r].x2;
         }
       }
-    };
-    auto sstore = [&](int buf) {
-      if constexpr (V4) {
+      // this thread holds candidates of the row (whose list has not overflowed)
+      if (mine[i] <= tau && *(volatile uint32_t*)&rs[r].cnt <= (uint32_t)F32_LIST) {
+        uint32_t mask = 0;
 #pragma unroll
-        for (int e = 0; e < 2; ++e) {
-          const int idx = e * 256 + tid;
-          const int r = idx >> 2, c4 = idx & 3;
+        for (int j = 0; j < CT; ++j) mask |= (val(j) <= tau ? 1u : 0u) << j;
+        while (mask) {
+          const int b = __ffs(mask) - 1;
+          mask &= mask - 1u;
+          float v = val(0);
 #pragma unroll
-          for (int q = 0; q < 4; ++q) {
-            As[buf][4 * c4 + q][r] = ra[4 * e + q];
-            Bs[buf][4 * c4 + q][r] = rb[4 * e + q];
+          for (int j = 1; j < CT; ++j) v = j == b ? val(j) : v;
+          const uint32_t c = c0 + (uint32_t)T::col(tx, b);
+          if (c < k) {
+            const uint32_t at = atomicAdd(&rs[r].cnt, 1u);
+            if (at < (uint32_t)F32_LIST) list[r * F32_LIST + at] = make_uint2(__float_as_uint(v), c);
           }
         }
-      } else {
-#pragma unroll
-        for (int e = 0; e < 8; ++e) {
-          const int idx = e * 256 + tid;
-          const int r = idx >> 4, kk = idx & 15;
-          As[buf][kk][r] = ra[e];
-          Bs[buf][kk][r] = rb[e];
-        }
       }
-    };
-    gload(0);
-    sstore(0);
-    __syncthreads();
-    for (uint32_t kt = 0; kt < nk; ++kt) {
-      const int buf = kt & 1;
-      if (kt + 1 < nk) gload((kt + 1) * SK_);
-#pragma unroll
-      for (int kk = 0; kk < SK_; ++kk) {
-        const float4 a0 = *reinterpret_cast<const float4*>(&As[buf][kk][ty * 8]);
-        const float4 a1 = *reinterpret_cast<const float4*>(&As[buf][kk][ty * 8 + 4]);
-        const float4 b0 = *reinterpret_cast<const float4*>(&Bs[buf][kk][tx * 4]);
-        const float4 b1 = *reinterpret_cast<const float4*>(&Bs[buf][kk][64 + tx * 4]);
-        const float a[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
-        const float b[8] = {b0.x, b0.y, b0.z, b0.w, b1.x, b1.y, b1.z, b1.w};
-#pragma unroll
-        for (int i = 0; i < 8; ++i)
-#pragma unroll
-          for (int j = 0; j < 8; ++j) acc[i][j] = fmaf(a[i], b[j], acc[i][j]);
-      }
-      if (kt + 1 < nk) sstore(buf ^ 1);
-      __syncthreads();
+      __syncwarp();                                        // the row's threads have read its m
+      if (tx == 0) rs[r].m = m;
     }
-
-    // Epilogue: v = ||c||^2 - 2 x.c into the thread's running top-3 per row.
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      const int r = ty * 8 + i;
-      const uint64_t row = m0 + r;                      // Dout is written in direct mode only
-      const int o = r * F32_TOP_LD + tx;
-      Top3 t;
-      t.v1 = tv1[o]; t.v2 = tv2[o]; t.v3 = tv3[o]; t.i1 = ti1[o]; t.i2 = ti2[o];
-#pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        const uint32_t cl = (j < 4) ? (uint32_t)(tx * 4 + j) : (uint32_t)(64 + tx * 4 + j - 4);
-        const uint32_t col = c0 + cl;
-        const float v = fmaf(-2.0f, acc[i][j], cns[cl]);
-        if (DOUT && row < n && col < k) Dout[row * k + col] = v + xn2[row];
-        // columns at or past k hold ||c||^2 = +inf, so v is +inf (or NaN)
-        // there and the strict insertion never takes them
-        t.insert_asc(v, col);
+    __syncthreads();
+    // Half-full lists drop the entries that m has left behind (the product's
+    // barriers come before the next entries).
+    if (c0 + T::COLS < k) {
+      for (int r = tid; r < T::ROWS; r += F32_NT) {
+        const uint32_t cnt = rs[r].cnt;
+        if (cnt <= (uint32_t)F32_LIST / 2 || cnt > (uint32_t)F32_LIST) continue;
+        const float tau = tie_tau_at(rs[r].tr, rs[r].m, tb);
+        uint32_t kept = 0;
+        for (uint32_t q = 0; q < cnt; ++q) {
+          const uint2 en = list[r * F32_LIST + q];
+          if (__uint_as_float(en.x) <= tau) list[r * F32_LIST + kept++] = en;
+        }
+        rs[r].cnt = kept;
       }
-      tv1[o] = t.v1; tv2[o] = t.v2; tv3[o] = t.v3; ti1[o] = t.i1; ti2[o] = t.i2;
     }
   }
-  __syncthreads();
 
-  // One thread per row: merge the row's 16 lists, classify, queue near ties.
-  if (tid < SM_) {
-    Top3 b;
-    b.init();
-#pragma unroll 4
-    for (int l = 0; l < 16; ++l) {
-      const int o = tid * F32_TOP_LD + l;
-      Top3 u;
-      u.v1 = tv1[o]; u.v2 = tv2[o]; u.v3 = tv3[o]; u.i1 = ti1[o]; u.i2 = ti2[o];
-      b.merge(u);
-    }
-    const uint64_t li = m0 + tid;
+  // One thread per row: the candidates in index order, classify, queue near ties.
+  for (int r = tid; r < T::ROWS; r += F32_NT) {
+    const F32Row w = rs[r];
+    const uint64_t li = m0 + (uint64_t)r, seg = li >> 5;
+    if (seg >= rq.nseg) break;                             // whole segments past the queues' end
     const bool valid = li < n_log;
-    const uint64_t row = rmap[tid];
-    int cls = 0;
-    uint32_t i1 = b.i1 == 0xffffffffu ? 0u : b.i1;
-    if (valid) {
-      const float cn1 = sqrtf(fmaxf(cn2[i1], 0.0f));
-      cls = tie_class(xn2[row], b.v1, b.v2, b.v3, cn1, st->cmax, tb);
-      labels[row] = i1;
-      if (mindist) mindist[row] = b.v1 + xn2[row];
+    const float tau = tie_tau_at(w.tr, w.m, tb);
+    uint32_t got = 0, e[4] = {0xffffffffu, 0xffffffffu, 0xffffffffu, 0xffffffffu};
+    const uint32_t nl = min(w.cnt, (uint32_t)F32_LIST);
+    for (uint32_t q = 0; q < nl; ++q) {
+      const uint2 en = list[r * F32_LIST + q];
+      if (!(__uint_as_float(en.x) <= tau)) continue;
+      ++got;
+      uint32_t c = en.y;                                   // insert, smallest index first
+#pragma unroll
+      for (int a = 0; a < 4; ++a) {
+        const uint32_t lo = min(c, e[a]);
+        c = max(c, e[a]);
+        e[a] = lo;
+      }
     }
-    RefineEntry e{(uint32_t)row, 2u, {i1, b.i2, 0u, 0u}};
-    const uint64_t seg = li >> 5;
-    seg_push(rq.cand, rq.ccnt, seg, valid && cls == 1, e);
-    seg_push(rq.full, rq.fcnt, seg, valid && cls == 2, (uint32_t)row);
+    // values that are not finite prove nothing: such rows take the full path
+    const bool fin = isfinite(w.tr.T + w.m + w.tr.Em);
+    const bool full = !fin || w.cnt > (uint32_t)F32_LIST || got == 0u || got > 4u;
+    if (valid) {
+      labels[w.row] = got ? e[0] : 0u;
+      if (mindist) mindist[w.row] = w.m + w.x2;
+    }
+    RefineEntry en{w.row, got, {e[0], e[1], e[2], e[3]}};
+    seg_push(rq.cand, rq.ccnt, seg, valid && !full && got >= 2u, en);
+    seg_push(rq.full, rq.fcnt, seg, valid && full, w.row);
   }
 }
+
+namespace {
+// The narrowest tile that holds k (chunks of 128 above, of 96 where two of them
+// hold k): the product's time goes with the tile's width.
+template <class F>
+void f32_shape(uint32_t k, F f) {
+  if (k <= 32u) f(std::integral_constant<int, 8>{}, std::integral_constant<int, 4>{});
+  else if (k <= 48u) f(std::integral_constant<int, 8>{}, std::integral_constant<int, 6>{});
+  else if (k <= 64u) f(std::integral_constant<int, 8>{}, std::integral_constant<int, 8>{});
+  else if (k <= 96u || (k > 128u && k <= 192u)) f(std::integral_constant<int, 16>{}, std::integral_constant<int, 6>{});
+  else f(std::integral_constant<int, 16>{}, std::integral_constant<int, 8>{});
+}
+void launch_f32(const float* X, const float* C, const float* cn2, const float* xn2, uint64_t n, uint32_t d, uint32_t k,
+                TieBound tb, DevState* st, uint32_t* labels, float* mindist, const RefineQueues& rq, float* Dout,
+                const uint32_t* ridx, const uint32_t* nidx, cudaStream_t s) {
+  const bool v4 = (d % 4 == 0) && (reinterpret_cast<uintptr_t>(X) % 16 == 0) &&
+                  (reinterpret_cast<uintptr_t>(C) % 16 == 0);
+  f32_shape(k, [&](auto tx, auto ct) {
+    using T = F32Tile<tx(), ct()>;
+    const uint64_t rows = rq.nseg * 32;                    // whole segments of the queues
+    const unsigned blocks = (unsigned)((rows + T::ROWS - 1) / T::ROWS);
+    auto kern = Dout ? assign_f32_kernel<tx(), ct(), true> : assign_f32_kernel<tx(), ct(), false>;
+    kern<<<blocks, F32_NT, f32_smem<T>(), s>>>(X, C, v4, cn2, xn2, n, d, k, tb, st, labels, mindist, rq, Dout, ridx,
+                                               nidx);
+  });
+}
+}  // namespace
 
 km_status launch_assign_f32(const float* X, const float* C, const float* cn2, const float* xn2,
                             uint64_t n, uint32_t d, uint32_t k, TieBound tb, DevState* st,
                             uint32_t* labels, float* mindist, const RefineQueues& rq,
                             float* Dout, cudaStream_t s) {
-  const unsigned blocks = (unsigned)((n + SM_ - 1) / SM_);
-  const bool v4 = (d % 4 == 0) && (reinterpret_cast<uintptr_t>(X) % 16 == 0) &&
-                  (reinterpret_cast<uintptr_t>(C) % 16 == 0);
-  auto kern = v4 ? (Dout ? assign_f32_kernel<true, true> : assign_f32_kernel<true, false>)
-                 : (Dout ? assign_f32_kernel<false, true> : assign_f32_kernel<false, false>);
-  kern<<<blocks, 256, F32_TOP_SMEM, s>>>(X, C, cn2, xn2, n, d, k, tb, st, labels, mindist, rq, Dout, nullptr,
-                                         nullptr);
+  launch_f32(X, C, cn2, xn2, n, d, k, tb, st, labels, mindist, rq, Dout, nullptr, nullptr, s);
   KM_CUDA_TRY(cudaGetLastError());
   return KM_OK;
 }
@@ -370,7 +363,7 @@ km_status launch_assign_f32(const float* X, const float* C, const float* cn2, co
 // aligned or d % 4 != 0 (refine_staged_kernel below is the vector path): four
 // lanes per row, one candidate per lane, the reference's CPU distance (float,
 // j ascending); smallest distance wins, lowest index on ties.  The candidate
-// set provably holds the reference argmin over all k (tie_tau / tie_class).
+// set provably holds the reference argmin over all k (tie_tau).
 // One warp per RC_SEGS consecutive queue segments, their entries flattened so
 // that every pass keeps eight rows in flight; the grid covers all segments at
 // once (no loop over segments, so a warp pays one count load and its rows).
@@ -612,7 +605,7 @@ refine_full_kernel(const float* __restrict__ X, const float* __restrict__ Ct, ui
 // instruction, and the L1 wavefronts, not DRAM, then set the time.  The
 // entry's lane picks the smallest distance over its candidates in ascending
 // index order with a strict '<' (lowest index on ties).  The candidate set
-// provably holds the reference argmin over all k (tie_tau / tie_class).
+// provably holds the reference argmin over all k (tie_tau).
 // FULL: the grid's warps then re-score the full queue against all k
 // (full_rescore_group), so that one launch covers the whole refinement.
 constexpr int RS_WARPS = 5;
@@ -907,10 +900,15 @@ refine_wide_kernel(const float* __restrict__ X, const float* __restrict__ C, uin
 }
 
 km_status refine_prepare() {
-  // assign_f32_kernel: 37 KB static + F32_TOP_SMEM dynamic is above the default 48 KB
-  for (auto kern : {assign_f32_kernel<true, true>, assign_f32_kernel<true, false>, assign_f32_kernel<false, true>,
-                    assign_f32_kernel<false, false>})
-    KM_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)F32_TOP_SMEM));
+  cudaError_t err = cudaSuccess;
+  for (uint32_t k : {32u, 48u, 64u, 96u, 128u})            // every shape of the FP32 distance kernel
+    f32_shape(k, [&](auto tx, auto ct) {
+      for (auto kern : {assign_f32_kernel<tx(), ct(), true>, assign_f32_kernel<tx(), ct(), false>})
+        if (err == cudaSuccess)
+          err = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     (int)f32_smem<F32Tile<tx(), ct()>>());
+    });
+  KM_CUDA_TRY(err);
   KM_CUDA_TRY(cudaFuncSetAttribute(refine_staged_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                    (int)RS_SMEM_MAX));
   KM_CUDA_TRY(cudaFuncSetAttribute(refine_staged_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -959,14 +957,7 @@ km_status launch_refine_gemm(bool v4, int num_sms, const float* X, const float* 
   KM_CUDA_TRY(cudaMemsetAsync(rq2.ccnt, 0, sizeof(uint32_t) * rq2.nseg, s));
   KM_CUDA_TRY(cudaMemsetAsync(rq2.fcnt, 0, sizeof(uint32_t) * rq2.nseg, s));
   full_compact_kernel<<<num_sms * 4, 256, 0, s>>>(st, rq, fidx, nfull);
-  const unsigned blocks = (unsigned)((n + SM_ - 1) / SM_);
-  const bool gv4 = v4 && (reinterpret_cast<uintptr_t>(C) % 16 == 0);
-  if (gv4)
-    assign_f32_kernel<true, false><<<blocks, 256, F32_TOP_SMEM, s>>>(X, C, cn2, xn2, n, d, k, tb32, st, labels, mindist,
-                                                   rq2, nullptr, fidx, nfull);
-  else
-    assign_f32_kernel<false, false><<<blocks, 256, F32_TOP_SMEM, s>>>(X, C, cn2, xn2, n, d, k, tb32, st, labels, mindist,
-                                                    rq2, nullptr, fidx, nfull);
+  launch_f32(X, C, cn2, xn2, n, d, k, tb32, st, labels, mindist, rq2, nullptr, fidx, nfull, s);
   launch_refine_cands(v4, num_sms, X, C, d, st, rq2, labels, mindist, false, s);
   refine_full_kernel<<<num_sms * 4, 256, 0, s>>>(X, Ct, d, k, st, rq2, labels, mindist, false);
   KM_CUDA_TRY(cudaGetLastError());
