@@ -230,7 +230,8 @@ km_status LloydEngine::init(uint64_t n_, uint32_t d_, uint32_t k_, int precision
       KM_TRY(take(&q2fcnt, rows / 32));
       KM_TRY(take(&fidx, rows));
       KM_TRY(take(&nfull, 1));
-      rq2 = RefineQueues{q2, q2full, q2cnt, q2fcnt, rows / 32};
+      // the FP32 pass's queues; its wide queue and lists take over the first ones'
+      rq2 = RefineQueues{q2, q2full, q2cnt, q2fcnt, rows / 32, qwide, qwcnt, wl, wlc, L};
       tb32 = make_tie_bound(KM_PREC_FP32, d, false);
     }
     KM_TRY(refine_prepare());

@@ -149,7 +149,7 @@ __global__ void prep_centroids_kernel(const float* __restrict__ C, uint32_t k, u
 // A CTA takes ROWS rows and walks all centroids, COLS at a time.  After each
 // column tile a row's minimum over its TX threads (exchanged by shuffles) joins
 // the row's running minimum m, and every centroid with v(c) <= tau(m) (tie_tau)
-// goes to the row's list of up to F32_LIST (value, index) pairs in shared memory,
+// goes to the row's list of up to F32_LIST (index, value) pairs in shared memory,
 // which drops the entries above the current tau between tiles.  tau only falls with
 // m, so the entries with v(c) <= tau(m_final) are the whole candidate set: one is the proven argmin, 2..4 go to the short re-score queue,
 // more (or a full list, or values that are not finite) to the full re-score.
@@ -176,9 +176,13 @@ constexpr size_t f32_smem() {
   return T::SMEM + T::ROWS * (sizeof(F32Row) + F32_LIST * sizeof(uint2)) + T::COLS * sizeof(float);
 }
 
-// Gather mode (ridx != null): logical row li of the tiles is row ridx[li] of X,
-// for li < *nidx; queue segments are taken over the logical rows.
-template <int TX, int CT, bool DOUT>
+// GATHER: logical row li of the tiles is row ridx[li] of X, for li < *nidx; queue
+// segments are taken over the logical rows.  These rows have many near ties (the
+// chunked tensor-core kernel found more than its lists hold), so their lists are the
+// global ones (rq.wl, L entries a row), filtered by a warp a row, and rows with
+// 5..L candidates go to the wide queue instead of the full re-score: n = 4M d = 256
+// k = 4096 (BF16 points, Zipf sizes) @GL@.
+template <int TX, int CT, bool DOUT, bool GATHER>
 __global__ void __launch_bounds__(F32_NT, CT == 8 ? 3 : 4)
 assign_f32_kernel(const float* __restrict__ X, const float* __restrict__ C, bool v4,
                   const float* __restrict__ cn2, const float* __restrict__ xn2, uint64_t n,
@@ -189,22 +193,39 @@ assign_f32_kernel(const float* __restrict__ X, const float* __restrict__ C, bool
   using T = F32Tile<TX, CT>;
   griddep_wait();
   if (st->done) return;
-  const uint64_t n_log = ridx ? (uint64_t)*nidx : n;
+  const uint64_t n_log = GATHER ? (uint64_t)*nidx : n;
   const uint64_t m0 = (uint64_t)blockIdx.x * T::ROWS;
   // (Without a gather the grid covers every segment of the queues, whose counts
   // all have to be written; a gather's start at zero.)
-  if (ridx && m0 >= n_log) return;
+  if (GATHER && m0 >= n_log) return;
   extern __shared__ __align__(16) float f32_smem_raw[];
   uint2* const list = reinterpret_cast<uint2*>(f32_smem_raw + T::SMEM / sizeof(float));   // [ROWS][F32_LIST]
   F32Row* const rs = reinterpret_cast<F32Row*>(list + T::ROWS * F32_LIST);
   float* const cns = reinterpret_cast<float*>(rs + T::ROWS);
   const int tid = threadIdx.x, tx = tid % TX, ty = tid / TX;
   const float cmax = st->cmax;
+  const uint32_t cap = GATHER ? rq.L : (uint32_t)F32_LIST;   // entries a list holds
+  auto list_of = [&](int r) -> uint2* { return GATHER ? rq.wl + (uint64_t)rs[r].row * rq.L : list + r * F32_LIST; };
+  // Drops a row's entries above tau (by the warp): the entries kept.
+  auto filter = [&](uint2* l, uint32_t cnt, float tau) -> uint32_t {
+    const int lane = tid & 31;
+    uint32_t kept = 0;
+    for (uint32_t q0 = 0; q0 < cnt; q0 += 32u) {
+      const uint32_t q = q0 + (uint32_t)lane;
+      const uint2 en = q < cnt ? l[q] : make_uint2(0u, 0u);
+      const bool keep = q < cnt && __uint_as_float(en.y) <= tau;
+      const unsigned b = __ballot_sync(0xffffffffu, keep);
+      if (keep) l[kept + (uint32_t)__popc(b & ((1u << lane) - 1u))] = en;    // at or before q: read already
+      kept += (uint32_t)__popc(b);
+      __syncwarp();
+    }
+    return kept;
+  };
   for (int r = tid; r < T::ROWS; r += F32_NT) {
     const uint64_t li = m0 + (uint64_t)r;
     F32Row w{};
     if (li < n_log) {
-      w.row = ridx ? ridx[li] : (uint32_t)li;
+      w.row = GATHER ? ridx[li] : (uint32_t)li;
       w.x2 = xn2[w.row];
     }
     w.m = f_inf();
@@ -251,7 +272,7 @@ assign_f32_kernel(const float* __restrict__ X, const float* __restrict__ C, bool
         }
       }
       // this thread holds candidates of the row (whose list has not overflowed)
-      if (mine[i] <= tau && *(volatile uint32_t*)&rs[r].cnt <= (uint32_t)F32_LIST) {
+      if (mine[i] <= tau && *(volatile uint32_t*)&rs[r].cnt <= cap && m0 + (uint64_t)r < n_log) {
         uint32_t mask = 0;
 #pragma unroll
         for (int j = 0; j < CT; ++j) mask |= (val(j) <= tau ? 1u : 0u) << j;
@@ -264,7 +285,7 @@ assign_f32_kernel(const float* __restrict__ X, const float* __restrict__ C, bool
           const uint32_t c = c0 + (uint32_t)T::col(tx, b);
           if (c < k) {
             const uint32_t at = atomicAdd(&rs[r].cnt, 1u);
-            if (at < (uint32_t)F32_LIST) list[r * F32_LIST + at] = make_uint2(__float_as_uint(v), c);
+            if (at < cap) list_of(r)[at] = make_uint2(c, __float_as_uint(v));
           }
         }
       }
@@ -272,23 +293,43 @@ assign_f32_kernel(const float* __restrict__ X, const float* __restrict__ C, bool
       if (tx == 0) rs[r].m = m;
     }
     __syncthreads();
-    // Half-full lists drop the entries that m has left behind (the product's
-    // barriers come before the next entries).
+    // Lists that another tile might fill drop the entries that m has left behind
+    // (the product's barriers come before the next entries).
     if (c0 + T::COLS < k) {
-      for (int r = tid; r < T::ROWS; r += F32_NT) {
-        const uint32_t cnt = rs[r].cnt;
-        if (cnt <= (uint32_t)F32_LIST / 2 || cnt > (uint32_t)F32_LIST) continue;
-        const float tau = tie_tau_at(rs[r].tr, rs[r].m, tb);
-        uint32_t kept = 0;
-        for (uint32_t q = 0; q < cnt; ++q) {
-          const uint2 en = list[r * F32_LIST + q];
-          if (__uint_as_float(en.x) <= tau) list[r * F32_LIST + kept++] = en;
+      const uint32_t high = max(cap / 2u, cap > (uint32_t)T::COLS ? cap - (uint32_t)T::COLS : 0u);
+      if (GATHER) {
+        for (int r = tid >> 5; r < T::ROWS; r += F32_NT / 32) {
+          const uint32_t cnt = rs[r].cnt;
+          if (cnt <= high || cnt > cap) continue;
+          const uint32_t kept = filter(list_of(r), cnt, tie_tau_at(rs[r].tr, rs[r].m, tb));
+          if ((tid & 31) == 0) rs[r].cnt = kept;
         }
-        rs[r].cnt = kept;
+      } else {
+        for (int r = tid; r < T::ROWS; r += F32_NT) {
+          const uint32_t cnt = rs[r].cnt;
+          if (cnt <= high || cnt > cap) continue;
+          const float tau = tie_tau_at(rs[r].tr, rs[r].m, tb);
+          uint2* const l = list_of(r);
+          uint32_t kept = 0;
+          for (uint32_t q = 0; q < cnt; ++q) {
+            const uint2 en = l[q];
+            if (__uint_as_float(en.y) <= tau) l[kept++] = en;
+          }
+          rs[r].cnt = kept;
+        }
       }
     }
   }
 
+  if (GATHER) {
+    for (int r = tid >> 5; r < T::ROWS; r += F32_NT / 32) {
+      const uint32_t cnt = rs[r].cnt;
+      if (cnt > cap) continue;
+      const uint32_t kept = filter(list_of(r), cnt, tie_tau_at(rs[r].tr, rs[r].m, tb));
+      if ((tid & 31) == 0) rs[r].cnt = kept;
+    }
+    __syncthreads();
+  }
   // One thread per row: the candidates in index order, classify, queue near ties.
   for (int r = tid; r < T::ROWS; r += F32_NT) {
     const F32Row w = rs[r];
@@ -297,12 +338,15 @@ assign_f32_kernel(const float* __restrict__ X, const float* __restrict__ C, bool
     const bool valid = li < n_log;
     const float tau = tie_tau_at(w.tr, w.m, tb);
     uint32_t got = 0, e[4] = {0xffffffffu, 0xffffffffu, 0xffffffffu, 0xffffffffu};
-    const uint32_t nl = min(w.cnt, (uint32_t)F32_LIST);
-    for (uint32_t q = 0; q < nl; ++q) {
-      const uint2 en = list[r * F32_LIST + q];
-      if (!(__uint_as_float(en.x) <= tau)) continue;
+    // (a gathered row's list is filtered already: only a short one is looked at)
+    const bool wide = GATHER && w.cnt > 4u && w.cnt <= cap;
+    const uint32_t nl = wide ? 0u : min(w.cnt, cap);
+    const uint2* const l = list_of(r);
+    for (uint32_t q = 0; q < nl && got <= 4u; ++q) {
+      const uint2 en = l[q];
+      if (!(__uint_as_float(en.y) <= tau)) continue;
       ++got;
-      uint32_t c = en.y;                                   // insert, smallest index first
+      uint32_t c = en.x;                                   // insert, smallest index first
 #pragma unroll
       for (int a = 0; a < 4; ++a) {
         const uint32_t lo = min(c, e[a]);
@@ -312,13 +356,17 @@ assign_f32_kernel(const float* __restrict__ X, const float* __restrict__ C, bool
     }
     // values that are not finite prove nothing: such rows take the full path
     const bool fin = isfinite(w.tr.T + w.m + w.tr.Em);
-    const bool full = !fin || w.cnt > (uint32_t)F32_LIST || got == 0u || got > 4u;
+    const bool full = !fin || w.cnt > cap || (!wide && (got == 0u || got > 4u));
     if (valid) {
       labels[w.row] = got ? e[0] : 0u;
       if (mindist) mindist[w.row] = w.m + w.x2;
     }
     RefineEntry en{w.row, got, {e[0], e[1], e[2], e[3]}};
-    seg_push(rq.cand, rq.ccnt, seg, valid && !full && got >= 2u, en);
+    seg_push(rq.cand, rq.ccnt, seg, valid && !full && !wide && got >= 2u, en);
+    if (GATHER) {
+      if (valid && wide) rq.wlc[w.row] = w.cnt;
+      seg_push(rq.wide, rq.wcnt, seg, valid && !full && wide, w.row);
+    }
     seg_push(rq.full, rq.fcnt, seg, valid && full, w.row);
   }
 }
@@ -343,7 +391,9 @@ void launch_f32(const float* X, const float* C, const float* cn2, const float* x
     using T = F32Tile<tx(), ct()>;
     const uint64_t rows = rq.nseg * 32;                    // whole segments of the queues
     const unsigned blocks = (unsigned)((rows + T::ROWS - 1) / T::ROWS);
-    auto kern = Dout ? assign_f32_kernel<tx(), ct(), true> : assign_f32_kernel<tx(), ct(), false>;
+    auto kern = ridx   ? assign_f32_kernel<tx(), ct(), false, true>
+                : Dout ? assign_f32_kernel<tx(), ct(), true, false>
+                       : assign_f32_kernel<tx(), ct(), false, false>;
     kern<<<blocks, F32_NT, f32_smem<T>(), s>>>(X, C, v4, cn2, xn2, n, d, k, tb, st, labels, mindist, rq, Dout, ridx,
                                                nidx);
   });
@@ -863,7 +913,7 @@ template <bool V4>
 __global__ void __launch_bounds__(256, 2)
 refine_wide_kernel(const float* __restrict__ X, const float* __restrict__ C, uint32_t d,
                    DevState* st, RefineQueues rq, uint32_t* __restrict__ labels,
-                   float* __restrict__ mindist) {
+                   float* __restrict__ mindist, bool count) {
   griddep_wait();
   if (st->done) return;
   const int lane = threadIdx.x & 31;
@@ -896,14 +946,15 @@ refine_wide_kernel(const float* __restrict__ X, const float* __restrict__ C, uin
       }
     }
   }
-  if (lane == 0 && done_rows) atomicAdd(&st->refined_total, (unsigned long long)done_rows);
+  if (count && lane == 0 && done_rows) atomicAdd(&st->refined_total, (unsigned long long)done_rows);
 }
 
 km_status refine_prepare() {
   cudaError_t err = cudaSuccess;
   for (uint32_t k : {32u, 48u, 64u, 96u, 128u})            // every shape of the FP32 distance kernel
     f32_shape(k, [&](auto tx, auto ct) {
-      for (auto kern : {assign_f32_kernel<tx(), ct(), true>, assign_f32_kernel<tx(), ct(), false>})
+      for (auto kern : {assign_f32_kernel<tx(), ct(), true, false>, assign_f32_kernel<tx(), ct(), false, false>,
+                        assign_f32_kernel<tx(), ct(), false, true>})
         if (err == cudaSuccess)
           err = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      (int)f32_smem<F32Tile<tx(), ct()>>());
@@ -925,12 +976,8 @@ km_status launch_refine(bool v4, int num_sms, const float* X, const float* C, co
     const StagedShape sh = staged_shape(num_sms, rq.nseg, d);
     KM_CUDA_TRY(launch_pdl(refine_staged_kernel<true>, sh.blocks, 32 * RS_WARPS, sh.smem, s, X, C, Ct, d, k,
                            sh.span, st, rq, labels, mindist, true));
-    if (rq.wide)
-      KM_CUDA_TRY(launch_pdl(refine_wide_kernel<true>, num_sms * 8, 256, 0, s, X, C, d, st, rq, labels, mindist));
   } else {
     launch_refine_cands(false, num_sms, X, C, d, st, rq, labels, mindist, true, s);
-    if (rq.wide)
-      KM_CUDA_TRY(launch_pdl(refine_wide_kernel<false>, num_sms * 8, 256, 0, s, X, C, d, st, rq, labels, mindist));
     KM_CUDA_TRY(launch_pdl(refine_full_kernel, num_sms * 4, 256, 0, s, X, Ct, d, k, st, rq, labels, mindist, true));
   }
   KM_CUDA_TRY(cudaGetLastError());
@@ -943,12 +990,11 @@ km_status launch_refine_gemm(bool v4, int num_sms, const float* X, const float* 
                              const RefineQueues& rq2, uint32_t* fidx, uint32_t* nfull,
                              uint32_t* labels, float* mindist, cudaStream_t s) {
   launch_refine_cands(v4, num_sms, X, C, d, st, rq, labels, mindist, true, s);
-  if (rq.wide) {
-    if (v4)
-      refine_wide_kernel<true><<<num_sms * 8, 256, 0, s>>>(X, C, d, st, rq, labels, mindist);
-    else
-      refine_wide_kernel<false><<<num_sms * 8, 256, 0, s>>>(X, C, d, st, rq, labels, mindist);
-  }
+  auto wide = [&](const RefineQueues& q, bool count) {
+    if (v4) refine_wide_kernel<true><<<num_sms * 8, 256, 0, s>>>(X, C, d, st, q, labels, mindist, count);
+    else refine_wide_kernel<false><<<num_sms * 8, 256, 0, s>>>(X, C, d, st, q, labels, mindist, count);
+  };
+  wide(rq, true);
   // rows of the full queue: FP32 distance pass over all k on those rows alone,
   // then the exact re-score of its own near ties
   KM_CUDA_TRY(cudaMemsetAsync(nfull, 0, sizeof(uint32_t), s));
@@ -956,9 +1002,11 @@ km_status launch_refine_gemm(bool v4, int num_sms, const float* X, const float* 
   // every other segment of rq2 must read as empty
   KM_CUDA_TRY(cudaMemsetAsync(rq2.ccnt, 0, sizeof(uint32_t) * rq2.nseg, s));
   KM_CUDA_TRY(cudaMemsetAsync(rq2.fcnt, 0, sizeof(uint32_t) * rq2.nseg, s));
+  KM_CUDA_TRY(cudaMemsetAsync(rq2.wcnt, 0, sizeof(uint32_t) * rq2.nseg, s));   // (rq's wide queue is done with)
   full_compact_kernel<<<num_sms * 4, 256, 0, s>>>(st, rq, fidx, nfull);
   launch_f32(X, C, cn2, xn2, n, d, k, tb32, st, labels, mindist, rq2, nullptr, fidx, nfull, s);
   launch_refine_cands(v4, num_sms, X, C, d, st, rq2, labels, mindist, false, s);
+  wide(rq2, false);
   refine_full_kernel<<<num_sms * 4, 256, 0, s>>>(X, Ct, d, k, st, rq2, labels, mindist, false);
   KM_CUDA_TRY(cudaGetLastError());
   return KM_OK;

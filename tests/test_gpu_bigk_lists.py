@@ -1,0 +1,29 @@
+"""k > 256: rows whose candidates overflow the chunked kernel's lists (more than
+256) go through the FP32 pass with its own lists.  Groups of 300 centroids at
+spreads from far above to far below the near-tie windows (single BF16, split and
+FP32) leave such rows with one, a few, up to 256 and more candidates: labels equal
+to the oracle's for every row."""
+import numpy as np
+import pytest
+
+import helpers
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("prec", ["bf16", "bf16x3"])
+@pytest.mark.parametrize("d,k,n", [(64, 700, 3000), (20, 1300, 1501), (33, 400, 777), (130, 2100, 2200)])
+def test_overflowing_candidate_lists(km, gpu, prec, d, k, n):
+    import torch
+    rng = np.random.default_rng(7 * d + k)
+    groups = max(1, k // 300)
+    base = (rng.standard_normal((groups, d)) * 4).astype(np.float32)
+    spread = np.array([1e-1, 3e-3, 1e-3, 1e-4, 1e-6, 1.0, 0.0], np.float32)
+    owner = rng.integers(0, groups, k)
+    C = (base[owner] + spread[owner % 7][:, None] * rng.standard_normal((k, d))).astype(np.float32)
+    g = rng.integers(0, groups, n)
+    X = (base[g] + rng.choice([1e-3, 1e-1, 1.0], (n, 1)) * rng.standard_normal((n, d))).astype(np.float32)
+    lab_o, _ = helpers.orc_assign(X, C)
+    lab, _, refined = km.assign(torch.from_numpy(X).to(gpu), torch.from_numpy(C).to(gpu), prec, want_mindist=True)
+    np.testing.assert_array_equal(lab.cpu().numpy().astype(np.uint32), lab_o)
+    assert refined > 0
