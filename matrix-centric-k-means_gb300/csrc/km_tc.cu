@@ -393,9 +393,9 @@ assign_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
 // shared memory and appends every centroid with v(c) <= tau(m) to its own
 // list of up to L (index, value) pairs in global memory.  tau grows with m and
 // m only falls, so after the last chunk the entries with v(c) <= tau(m_final)
-// are exactly the candidate set of all k centroids; a full list is first
-// compacted with the current tau, and a list that still overflows sends the
-// row to the full re-score.  Final classification: one candidate = proven
+// are exactly the candidate set of all k centroids; a list about to be overfilled
+// is first compacted with the current tau, by its warp together, and one that still
+// overflows sends the row to the full re-score.  Final classification: one candidate = proven
 // label, 2..4 = the short re-score queue, 5..L = the wide queue (one warp per
 // row re-scores its list), otherwise the full re-score.
 //
@@ -417,6 +417,37 @@ struct TcSmemC {
 };
 
 __host__ __device__ constexpr uint32_t tcc_state_bytes(uint32_t T) { return T * TC_M * 8u; }
+
+// Drops the entries above tau of the list of lane o's row (its lst, cnt and tau),
+// the warp together: the entries kept.  All lanes call.  (Each thread reading its own
+// list, one entry after the other, was half of the kernel's time at n = 4M d = 256
+// k = 4096: 50 -> 25 ms an iteration.)
+__device__ __forceinline__ uint32_t tcc_filter(uint2* lst, uint32_t cnt, float tau, int o) {
+  const int lane = threadIdx.x & 31;
+  uint2* const l = reinterpret_cast<uint2*>(__shfl_sync(0xffffffffu, reinterpret_cast<unsigned long long>(lst), o));
+  const uint32_t n = __shfl_sync(0xffffffffu, cnt, o);
+  const float t = __shfl_sync(0xffffffffu, tau, o);
+  uint32_t kept = 0;
+  __syncwarp();                                            // the row's own stores come first
+  for (uint32_t q0 = 0; q0 < n; q0 += 128u) {
+    uint2 en[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const uint32_t q = q0 + 32u * u + (uint32_t)lane;
+      en[u] = q < n ? l[q] : make_uint2(0u, 0u);
+    }
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const uint32_t q = q0 + 32u * u + (uint32_t)lane;
+      const bool keep = q < n && __uint_as_float(en[u].y) <= t;
+      const unsigned b = __ballot_sync(0xffffffffu, keep);
+      if (keep) l[kept + (uint32_t)__popc(b & ((1u << lane) - 1u))] = en[u];   // at or before q: read already
+      kept += (uint32_t)__popc(b);
+    }
+    __syncwarp();
+  }
+  return kept;
+}
 
 template <int MODE>
 __global__ void __launch_bounds__(TCC_THREADS, 1)
@@ -659,19 +690,19 @@ assign_tc_chunked_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
               const uint32_t col0 = j * NC + pr * 64u + (uint32_t)h * 32u;     // global centroid index
               uint32_t mk = collect ? mm[h] : 0u;
               mk &= (col0 >= k) ? 0u : (k - col0 >= 32u ? 0xffffffffu : ((1u << (k - col0)) - 1u));
+              // lists that these entries would overfill: drop the entries of earlier
+              // chunks that the current tau excludes (the warp together, a row at a time)
+              unsigned tight = __ballot_sync(0xffffffffu, cnt != TCC_OVF && cnt + (uint32_t)__popc(mk) > rq.L);
+              while (tight) {
+                const int o = __ffs(tight) - 1;
+                tight &= tight - 1u;
+                const uint32_t kept = tcc_filter(lst, cnt, tau, o);
+                if (lane == o) cnt = kept;
+              }
+              if (cnt != TCC_OVF && cnt + (uint32_t)__popc(mk) > rq.L) cnt = TCC_OVF;
               while (mk != 0u && cnt != TCC_OVF) {
                 const uint32_t bit = (uint32_t)(__ffs(mk) - 1);
                 mk &= mk - 1u;
-                if (cnt == rq.L) {
-                  // full: drop entries of earlier chunks that the current tau excludes
-                  uint32_t kept = 0;
-                  for (uint32_t e = 0; e < cnt; ++e) {
-                    const uint2 en = lst[e];
-                    if (__uint_as_float(en.y) <= tau) { if (kept != e) lst[kept] = en; ++kept; }
-                  }
-                  cnt = kept;
-                  if (cnt == rq.L) { cnt = TCC_OVF; break; }
-                }
                 // the candidate's accumulator by selection (static register indices)
                 uint32_t a = 0u;
 #pragma unroll
@@ -680,6 +711,7 @@ assign_tc_chunked_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
                 lst[cnt] = make_uint2(col0 + bit, __float_as_uint(vv));
                 ++cnt;
               }
+              __syncwarp();
             }
             if (Dout && valid) {
 #pragma unroll
@@ -698,9 +730,18 @@ assign_tc_chunked_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
           } else {
             // Final filter with tau(m): keep {c : v(c) <= tau}, compacted in
             // list order; note the first four for the short queue.
+            // Long lists by the warp together, short ones by their own thread.
+            unsigned longs = __ballot_sync(0xffffffffu, cnt != TCC_OVF && cnt > 8u);
+            while (longs) {
+              const int o = __ffs(longs) - 1;
+              longs &= longs - 1u;
+              const uint32_t left = tcc_filter(lst, cnt, tau, o);
+              if (lane == o) cnt = left;
+            }
             uint32_t kept = 0, c0 = 0, c1 = 0, c2 = 0, c3 = 0;
             if (cnt != TCC_OVF) {
-              for (uint32_t e = 0; e < cnt; ++e) {
+              const uint32_t look = cnt > 8u ? 4u : cnt;      // a long list is filtered already
+              for (uint32_t e = 0; e < look; ++e) {
                 const uint2 en = lst[e];
                 if (__uint_as_float(en.y) <= tau) {
                   if (kept != e) lst[kept] = en;
@@ -709,6 +750,7 @@ assign_tc_chunked_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
                   ++kept;
                 }
               }
+              if (cnt > 8u) kept = cnt;
             }
             // NaN leaves kept == 0: full re-score, as does an overflowed list.
             const uint32_t cf = (cnt == TCC_OVF) ? TCC_OVF : kept;
