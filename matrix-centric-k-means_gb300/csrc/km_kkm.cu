@@ -16,6 +16,7 @@
 //      (kmeans.cu:1054-1061; it leaves out K_ii), stop on |score - last| < tol
 //      from iteration 2 when checking (kmeans.cu:1064-1073).
 #include "km_lloyd.cuh"
+#include "km_simt.cuh"
 
 #include <cudaTypedefs.h>
 #include <cmath>
@@ -33,25 +34,8 @@ struct KFn {
   int degree;
 };
 
-__device__ __forceinline__ float kfn_apply(const KFn& f, float dot, float ni, float nj) {
-  switch (f.kind) {
-    case KM_KERNEL_LINEAR: return dot;
-    case KM_KERNEL_POLY: {
-      const float b = fmaf(f.gamma, dot, f.coef);
-      float r = 1.0f;
-      for (int e = 0; e < f.degree; ++e) r *= b;
-      return r;
-    }
-    case KM_KERNEL_SIGMOID: return tanhf(fmaf(f.gamma, dot, f.coef));
-    default: {
-      const float d2 = fmaxf(ni + nj - 2.0f * dot, 0.0f);
-      return expf(-d2 * f.inv2s2);
-    }
-  }
-}
-
-// The same functions with the kind fixed at compile time (one small body per
-// kernel-matrix instantiation; the tensor-core epilogue unrolls it per column).
+// The kernel functions, the kind fixed at compile time (one small body per
+// kernel-matrix instantiation; the epilogues unroll it per column).
 template <int KIND>
 __device__ __forceinline__ float kfn_apply_k(const KFn& f, float dot, float ni, float nj) {
   if constexpr (KIND == KM_KERNEL_LINEAR) {
@@ -98,60 +82,105 @@ __device__ __forceinline__ void kstore(void* K, uint64_t idx, float v) {
 }
 
 // ---------------------------------------------------------------------------
-// (a) SIMT FP32 kernel-matrix GEMM: 128 x 128 tiles, 256 threads, 8 x 8
-// micro-tiles, K chunks of 16 through shared memory.  Builds rows
-// [row0, row_end) of K into K (row stride n, first row = row0); with `stop`
-// set it does nothing once the fit has stopped (panels rebuilt per iteration).
+// (a) SIMT FP32 kernel matrix, 64 x 128 tiles (km_simt.cuh has the product).
+// Builds rows [row0, row_end) of K into K (row stride n, first row = row0); with
+// `stop` set it does nothing once the fit has stopped (panels rebuilt per
+// iteration).  Symmetry: a build of all rows computes only the blocks of 128 x 128
+// on and above the diagonal (two tiles each, column block by column block) and
+// stores the ones above it twice, the second time transposed (a product and a
+// transposed one multiply and add the same numbers in the same order, so both
+// halves are what a full build gives); a panel computes its own rows.
+// Bound by the FP32 pipes and the product's shared-memory reads, then by writing K:
+// n = 20,000 d = 64 2182 -> 807 us (16 x 16 threads with one buffered stage, scalar
+// loads and every tile computed before).
 // ---------------------------------------------------------------------------
+using KmTile = SimtTile<128, 8, 16, 8, 16>;
+
 template <bool OUT_BF16>
-__global__ void __launch_bounds__(256)
-kmat_f32_kernel(const float* __restrict__ X, const float* __restrict__ xn2, uint64_t n, uint32_t d,
-                uint64_t row0, uint64_t row_end, KFn f, void* __restrict__ K, float* __restrict__ diag,
-                const DevState* stop) {
+__device__ __forceinline__ void kstore4(void* K, uint64_t idx, const float (&v)[4], bool vec, uint64_t col, uint64_t n) {
+  if (vec) {                       // n % 4 == 0 and K aligned: four columns start 16 (8) byte aligned
+    if (col >= n) return;
+    if (OUT_BF16) {
+      const __nv_bfloat162 a = __floats2bfloat162_rn(v[0], v[1]), b = __floats2bfloat162_rn(v[2], v[3]);
+      uint2 u;
+      u.x = *reinterpret_cast<const uint32_t*>(&a);
+      u.y = *reinterpret_cast<const uint32_t*>(&b);
+      *reinterpret_cast<uint2*>(reinterpret_cast<__nv_bfloat16*>(K) + idx) = u;
+    } else {
+      *reinterpret_cast<float4*>(reinterpret_cast<float*>(K) + idx) = make_float4(v[0], v[1], v[2], v[3]);
+    }
+  } else {
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+      if (col + q < n) kstore<OUT_BF16>(K, idx + q, v[q]);
+  }
+}
+
+template <bool OUT_BF16, int KIND>
+__global__ void __launch_bounds__(128, 3)
+kmat_f32_kernel(const float* __restrict__ X, bool v4, const float* __restrict__ xn2, uint64_t n, uint32_t d,
+                uint64_t row0, uint64_t row_end, int symmetric, KFn f, void* __restrict__ K, bool vec,
+                float* __restrict__ diag, const DevState* stop) {
+  using T = KmTile;
   if (stop && stop->done) return;
-  __shared__ __align__(16) float As[16][128 + 4];
-  __shared__ __align__(16) float Bs[16][128 + 4];
-  const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
-  const uint64_t m0 = row0 + (uint64_t)blockIdx.y * 128, c0 = (uint64_t)blockIdx.x * 128;
-  float acc[8][8];
+  extern __shared__ __align__(16) float km_smem[];
+  uint64_t m0, c0;
+  bool mirror = false;
+  if (symmetric) {
+    const uint64_t p = blockIdx.x >> 1;                    // pair (bi <= bj), column block bj by column block
+    uint64_t bj = (uint64_t)((sqrt(8.0 * (double)p + 1.0) - 1.0) * 0.5);
+    while (bj * (bj + 1) / 2 > p) --bj;
+    while ((bj + 1) * (bj + 2) / 2 <= p) ++bj;
+    const uint64_t bi = p - bj * (bj + 1) / 2;
+    m0 = bi * 128 + (blockIdx.x & 1u) * 64;
+    c0 = bj * 128;
+    mirror = bi < bj;
+  } else {
+    const uint64_t nb = (n + 127) / 128;
+    m0 = row0 + blockIdx.x / nb * 64;
+    c0 = blockIdx.x % nb * 128;
+  }
+  if (m0 >= row_end) return;
+  float2 acc[4][8];
+  simt_product<T>(
+      km_smem, d, v4, [&](int r) { return m0 + (uint64_t)r < row_end ? X + (m0 + (uint64_t)r) * d : (const float*)nullptr; },
+      [&](int c) { return c0 + (uint64_t)c < n ? X + (c0 + (uint64_t)c) * d : (const float*)nullptr; }, acc);
+  const int tx = threadIdx.x % T::TX, ty = threadIdx.x / T::TX;
+  const uint64_t r0 = m0 + (uint64_t)ty * 8;
+  float nj[8];
 #pragma unroll
-  for (int i = 0; i < 8; ++i)
-#pragma unroll
-    for (int j = 0; j < 8; ++j) acc[i][j] = 0.0f;
-  for (uint32_t kc = 0; kc < d; kc += 16) {
-#pragma unroll
-    for (int e = 0; e < 8; ++e) {
-      const int idx = e * 256 + tid;
-      const int r = idx >> 4, kk = idx & 15;
-      const uint32_t col = kc + kk;
-      As[kk][r] = (m0 + r < row_end && col < d) ? X[(m0 + r) * d + col] : 0.0f;
-      Bs[kk][r] = (c0 + r < n && col < d) ? X[(c0 + r) * d + col] : 0.0f;
-    }
-    __syncthreads();
-#pragma unroll
-    for (int kk = 0; kk < 16; ++kk) {
-      float a[8], b[8];
-#pragma unroll
-      for (int i = 0; i < 8; ++i) { a[i] = As[kk][ty * 8 + i]; b[i] = Bs[kk][tx * 8 + i]; }
-#pragma unroll
-      for (int i = 0; i < 8; ++i)
-#pragma unroll
-        for (int j = 0; j < 8; ++j) acc[i][j] = fmaf(a[i], b[j], acc[i][j]);
-    }
-    __syncthreads();
+  for (int j = 0; j < 8; ++j) {
+    const uint64_t c = c0 + (uint64_t)T::col(tx, j);
+    nj[j] = (KIND == KM_KERNEL_GAUSSIAN && c < n) ? xn2[c] : 0.0f;
   }
 #pragma unroll
   for (int i = 0; i < 8; ++i) {
-    const uint64_t row = m0 + ty * 8 + i;
-    if (row >= row_end) continue;
-    const float ni = xn2[row];
+    const uint64_t row = r0 + i;
+    if (row >= row_end) break;
+    const float ni = KIND == KM_KERNEL_GAUSSIAN ? xn2[row] : 0.0f;
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+      const uint64_t col = c0 + (uint64_t)T::col(tx, 4 * q);
+      float v[4];
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        float& a = (i & 1) ? acc[i / 2][4 * q + e].y : acc[i / 2][4 * q + e].x;
+        a = v[e] = kfn_apply_k<KIND>(f, a, ni, nj[4 * q + e]);
+        if (diag && col + e == row) diag[row] = v[e];
+      }
+      kstore4<OUT_BF16>(K, (row - row0) * n + col, v, vec, col, n);
+    }
+  }
+  if (mirror) {
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
-      const uint64_t col = c0 + tx * 8 + j;
+      const uint64_t col = c0 + (uint64_t)T::col(tx, j);
       if (col >= n) continue;
-      const float v = kfn_apply(f, acc[i][j], ni, xn2[col]);
-      kstore<OUT_BF16>(K, (row - row0) * n + col, v);
-      if (diag && row == col) diag[row] = v;
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {                        // four rows of this column
+        const float v[4] = {acc[2 * h][j].x, acc[2 * h][j].y, acc[2 * h + 1][j].x, acc[2 * h + 1][j].y};
+        kstore4<OUT_BF16>(K, col * n + r0 + 4 * h, v, vec, r0 + 4 * h, n);
+      }
     }
   }
 }
@@ -978,11 +1007,22 @@ km_status build_kernel_matrix(LloydEngine& e, const float* X, uint64_t n, uint32
   if (row0 >= row_end || row_end > n) return KM_ERR_ARG;
   const uint64_t rows = row_end - row0;
   if (precision == KM_PREC_FP32) {
-    if ((rows + 127) / 128 > 65535) return KM_ERR_UNSUPPORTED;
-    dim3 grid((unsigned)((n + 127) / 128), (unsigned)((rows + 127) / 128));
+    const bool symmetric = rows == n;
+    const uint64_t nb = (n + 127) / 128, tiles = symmetric ? nb * (nb + 1) : nb * ((rows + 63) / 64);
+    if (tiles > 0x7fffffffull) return KM_ERR_UNSUPPORTED;
     const DevState* stop = skip_done ? e.st : nullptr;
-    if (out_bf16) kmat_f32_kernel<true><<<grid, 256, 0, s>>>(X, e.xn2, n, d, row0, row_end, f, K, diag, stop);
-    else kmat_f32_kernel<false><<<grid, 256, 0, s>>>(X, e.xn2, n, d, row0, row_end, f, K, diag, stop);
+    const bool v4 = d % 4 == 0 && reinterpret_cast<uintptr_t>(X) % 16 == 0;
+    const bool vec = n % 4 == 0 && reinterpret_cast<uintptr_t>(K) % 16 == 0;
+    auto launch = [&](auto kern) {
+      kern<<<(unsigned)tiles, 128, KmTile::SMEM, s>>>(X, v4, e.xn2, n, d, row0, row_end, symmetric ? 1 : 0, f, K, vec, diag,
+                                                    stop);
+    };
+    switch (f.kind) {
+      case KM_KERNEL_LINEAR: out_bf16 ? launch(kmat_f32_kernel<true, KM_KERNEL_LINEAR>) : launch(kmat_f32_kernel<false, KM_KERNEL_LINEAR>); break;
+      case KM_KERNEL_POLY: out_bf16 ? launch(kmat_f32_kernel<true, KM_KERNEL_POLY>) : launch(kmat_f32_kernel<false, KM_KERNEL_POLY>); break;
+      case KM_KERNEL_SIGMOID: out_bf16 ? launch(kmat_f32_kernel<true, KM_KERNEL_SIGMOID>) : launch(kmat_f32_kernel<false, KM_KERNEL_SIGMOID>); break;
+      default: out_bf16 ? launch(kmat_f32_kernel<true, KM_KERNEL_GAUSSIAN>) : launch(kmat_f32_kernel<false, KM_KERNEL_GAUSSIAN>); break;
+    }
     KM_CUDA_TRY(cudaGetLastError());
     return KM_OK;
   }
