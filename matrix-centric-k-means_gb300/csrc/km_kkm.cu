@@ -191,9 +191,12 @@ kmat_f32_kernel(const float* __restrict__ X, bool v4, const float* __restrict__ 
 // tiles; per K-block the A tile (128 rows) and B tile (256 rows) of the BF16
 // copy of X (hi, and lo for X3) come in by TMA into a ring of stages; one
 // thread issues the MMAs into a TMEM accumulator (two buffers of 256
-// columns); eight epilogue warps (two sets, one per buffer; warp w on TMEM
-// lanes 32*(w%4)) read the accumulator 64 columns at a time, apply f and store
-// K.  Every wait is bounded (2 s) and a timeout raises KM_DEVERR_TIMEOUT after
+// columns); sixteen epilogue warps (two sets of eight, one per buffer; warp w on TMEM
+// lanes 32*(w%4) and one half of the columns) read the accumulator 32 columns at a
+// time, apply f and store K.  Bound by the stores of K (and, for long rows in the split
+// form, the MMAs); with eight warps and a range check at every store the epilogue's
+// latency was: n = 24,000 d = 200 Gaussian 966 -> 543 us, n = 65,536 d = 512 polynomial
+// 8.28 -> 5.12 ms (split-BF16x3, FP32 K).  Every wait is bounded (2 s) and a timeout raises KM_DEVERR_TIMEOUT after
 // draining this CTA's copies and MMAs.  The kernel builds rows
 // [prow0, prow_end) of K into K (row stride n, first row = prow0): all of K,
 // or one panel of it; with skip_done it does nothing once the fit has stopped.
@@ -219,7 +222,9 @@ constexpr uint64_t KWAIT_NS = 2000000000ull;
 constexpr uint64_t KM_GROUP = 16;   // row tiles per raster group of the kernel-matrix build
 
 
-constexpr uint32_t KM_STG_BYTES = 8u * 32u * 32u * 4u;   // epilogue staging tiles, one per epilogue warp
+constexpr int KM_EPI_WARPS = 16;
+constexpr int KM_THREADS = 32 * (4 + KM_EPI_WARPS);
+constexpr uint32_t KM_STG_BYTES = KM_EPI_WARPS * 32u * 16u * 4u;   // epilogue staging tiles, one per epilogue warp
 
 struct KmSmem {
   uint64_t full[8];
@@ -233,7 +238,7 @@ struct KmSmem {
 }  // namespace
 
 template <bool X3, bool OUT_BF16, int KIND>
-__global__ void __launch_bounds__(384, 1)
+__global__ void __launch_bounds__(KM_THREADS, 1)
 kmat_tc_kernel(const __grid_constant__ CUtensorMap tA, const __grid_constant__ CUtensorMap tAlo,
                const __grid_constant__ CUtensorMap tB, const __grid_constant__ CUtensorMap tBlo,
                const float* __restrict__ xn2, uint64_t n, uint64_t prow0, uint64_t prow_end, uint32_t KB,
@@ -244,12 +249,12 @@ kmat_tc_kernel(const __grid_constant__ CUtensorMap tA, const __grid_constant__ C
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
                                              ~uintptr_t(1023));
   const uint32_t stage_bytes = (KA_BYTES + KB_BYTES) * (X3 ? 2u : 1u);
-  float* stg_all = reinterpret_cast<float*>(smem + (size_t)S * stage_bytes);    // [8 warps][32][32]
+  float* stg_all = reinterpret_cast<float*>(smem + (size_t)S * stage_bytes);    // [16 warps][32][16]
   KmSmem* ts = reinterpret_cast<KmSmem*>(smem + (size_t)S * stage_bytes + KM_STG_BYTES);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (threadIdx.x == 0) {
     for (uint32_t s = 0; s < S; ++s) { mbar_init(&ts->full[s], 1); mbar_init(&ts->empty[s], 1); }
-    for (int b = 0; b < 2; ++b) { mbar_init(&ts->tfull[b], 1); mbar_init(&ts->tempty[b], 4); }
+    for (int b = 0; b < 2; ++b) { mbar_init(&ts->tfull[b], 1); mbar_init(&ts->tempty[b], 8); }
     mbar_init(&ts->tdone, 1);
     ts->abort = 0;
     mbar_fence_init();
@@ -331,9 +336,14 @@ kmat_tc_kernel(const __grid_constant__ CUtensorMap tA, const __grid_constant__ C
       }
     }
   } else if (warp >= 4) {
-    const int q = warp & 3, set = (warp - 4) >> 2;
+    // Epilogue: warp (4 + e) on TMEM lanes 32 (warp % 4) of accumulator buffer
+    // (e / 4) % 2, columns 128 (e / 8) .. + 127, 32 at a time.
+    const int q = warp & 3, set = ((warp - 4) >> 2) & 1, half = (warp - 4) >> 3;
     const uint32_t r = (uint32_t)q * 32u + (uint32_t)lane;
-    const uint32_t tbase = tmem_base + (((uint32_t)q * 32u) << 16) + (uint32_t)set * 256u;
+    const uint32_t tbase = tmem_base + (((uint32_t)q * 32u) << 16) + (uint32_t)set * 256u + (uint32_t)half * 128u;
+    float* const stg = stg_all + (size_t)(warp - 4) * 32 * 16;
+    using KT = std::conditional_t<OUT_BF16, __nv_bfloat16, float>;
+    KT* const Kt = reinterpret_cast<KT*>(K);
     uint64_t t = (uint64_t)set;
     for (uint64_t tile = blockIdx.x + (uint64_t)set * gridDim.x; tile < ntiles;
          tile += 2ull * gridDim.x, t += 2) {
@@ -341,100 +351,88 @@ kmat_tc_kernel(const __grid_constant__ CUtensorMap tA, const __grid_constant__ C
       const uint32_t njf = tlist[2 * tile + 1];
       const uint64_t nj = njf & 0x3fffffffu;
       const bool direct = (njf >> 30) & 1u, mirror = (njf >> 31) & 1u;
-      const uint64_t row = mi * KM_M + r, c0 = nj * KM_N;
+      const uint64_t row = mi * KM_M + r, row0 = mi * KM_M + (uint64_t)q * 32u;   // this lane's, the warp's first
+      const uint64_t c0 = nj * KM_N + (uint64_t)half * 128u;
       const bool row_in = row < n;
-      const float ni = row_in ? xn2[row] : 0.0f;
-      // column norms only matter for the Gaussian kernel (broadcast loads)
-      auto colnorm = [&](uint64_t c) -> float {
-        return (KIND == KM_KERNEL_GAUSSIAN && c < n) ? __ldg(xn2 + c) : 0.0f;
-      };
+      const float ni = (KIND == KM_KERNEL_GAUSSIAN && row_in) ? xn2[row] : 0.0f;
+      // whole blocks of the warp inside K (and inside the panel): stores without checks
+      const bool fast_d = direct && vec && row0 >= prow0 && row0 + 32 <= prow_end && c0 + 128 <= n;
+      const bool fast_m = mirror && row0 + 32 <= n && c0 >= prow0 && c0 + 128 <= prow_end;
+      const bool on_diag = diag && direct && mi / 2 == nj && row >= prow0 && row < prow_end;
       const bool okw = mbar_wait_bounded(&ts->tfull[set], (uint32_t)(t >> 1) & 1u, abort_flag, KWAIT_NS);
       if (!__all_sync(0xffffffffu, okw)) { if (lane == 0) fail(4); break; }
       tc_fence_after();
-      // Values of this lane's row go to the warp's staging tile (32 rows x 32
-      // columns, 16-byte chunks XOR-swizzled by row) and leave as whole
-      // 128-byte row segments: eight lanes per row, four rows per store.
-      float* stg = stg_all + (size_t)(warp - 4) * 32 * 32;
-      const uint64_t row0 = mi * KM_M + (uint64_t)q * 32u;  // first row of this warp
 #pragma unroll 1
-      for (uint32_t pr = 0; pr < KM_N / 64; ++pr) {       // not unrolled: the body is large
-        uint32_t acc[64];
-        tmem_ld_32x32b_x64(tbase + pr * 64u, acc);
+      for (uint32_t ch = 0; ch < 4; ++ch) {
+        const uint64_t cb = c0 + ch * 32u;
+        uint32_t acc[32];
+        tmem_ld_32x32b_x32(tbase + ch * 32u, acc);
         tmem_ld_wait();
-        if (pr + 1 == KM_N / 64) {
+        if (ch == 3) {
           // the accumulator's last columns are in registers: the MMAs of the
           // next tile on this buffer may start while this one is stored
           tc_fence_before();
           __syncwarp();
           if (lane == 0) mbar_arrive(&ts->tempty[set]);
         }
+        float v[32];
 #pragma unroll
-        for (int h = 0; h < 2; ++h) {
-          const uint64_t cb = c0 + pr * 64u + (uint32_t)h * 32u;
-          __syncwarp();                                  // the previous half has been read back
-#pragma unroll
-          for (int c = 0; c < 8; ++c) {
-            float4 o;
-            o.x = kfn_apply_k<KIND>(f, __uint_as_float(acc[h * 32 + 4 * c + 0]), ni, colnorm(cb + 4 * c + 0));
-            o.y = kfn_apply_k<KIND>(f, __uint_as_float(acc[h * 32 + 4 * c + 1]), ni, colnorm(cb + 4 * c + 1));
-            o.z = kfn_apply_k<KIND>(f, __uint_as_float(acc[h * 32 + 4 * c + 2]), ni, colnorm(cb + 4 * c + 2));
-            o.w = kfn_apply_k<KIND>(f, __uint_as_float(acc[h * 32 + 4 * c + 3]), ni, colnorm(cb + 4 * c + 3));
-            if (diag && direct && row >= prow0 && row < prow_end) {
-              if (cb + 4 * c + 0 == row) diag[row] = o.x;
-              if (cb + 4 * c + 1 == row) diag[row] = o.y;
-              if (cb + 4 * c + 2 == row) diag[row] = o.z;
-              if (cb + 4 * c + 3 == row) diag[row] = o.w;
-            }
-            *reinterpret_cast<float4*>(stg + lane * 32 + ((c ^ (lane & 7)) * 4)) = o;
-            if (mirror && row_in) {
-              // transposed: K[gcol][row]; the warp's lanes write one contiguous run
-              const float ov[4] = {o.x, o.y, o.z, o.w};
-#pragma unroll
-              for (int qq = 0; qq < 4; ++qq) {
-                const uint64_t gcol = cb + 4 * c + qq;
-                if (gcol >= prow0 && gcol < prow_end) {
-                  if (OUT_BF16)
-                    reinterpret_cast<__nv_bfloat16*>(K)[(gcol - prow0) * n + row] = __float2bfloat16_rn(ov[qq]);
-                  else
-                    reinterpret_cast<float*>(K)[(gcol - prow0) * n + row] = ov[qq];
-                }
-              }
+        for (int c4 = 0; c4 < 8; ++c4) {
+          float4 w = make_float4(0.f, 0.f, 0.f, 0.f);      // column norms only matter for the Gaussian kernel
+          if (KIND == KM_KERNEL_GAUSSIAN) {
+            const uint64_t c = cb + 4 * c4;
+            if (c + 3 < n) {
+              w = __ldg(reinterpret_cast<const float4*>(xn2 + c));
+            } else {
+              if (c + 0 < n) w.x = __ldg(xn2 + c);
+              if (c + 1 < n) w.y = __ldg(xn2 + c + 1);
+              if (c + 2 < n) w.z = __ldg(xn2 + c + 2);
             }
           }
-          __syncwarp();
-          if (!direct) continue;                         // the staged copy is stored only for own rows
+          v[4 * c4 + 0] = kfn_apply_k<KIND>(f, __uint_as_float(acc[4 * c4 + 0]), ni, w.x);
+          v[4 * c4 + 1] = kfn_apply_k<KIND>(f, __uint_as_float(acc[4 * c4 + 1]), ni, w.y);
+          v[4 * c4 + 2] = kfn_apply_k<KIND>(f, __uint_as_float(acc[4 * c4 + 2]), ni, w.z);
+          v[4 * c4 + 3] = kfn_apply_k<KIND>(f, __uint_as_float(acc[4 * c4 + 3]), ni, w.w);
+        }
+        if (on_diag) {
 #pragma unroll
-          for (int step = 0; step < 8; ++step) {
-            const uint32_t rr = (uint32_t)step * 4u + ((uint32_t)lane >> 3);   // row within the warp's 32
-            const uint32_t ch = (uint32_t)lane & 7u;                           // 16-byte chunk of the row
-            const float4 o = *reinterpret_cast<const float4*>(stg + rr * 32 + ((ch ^ (rr & 7u)) * 4u));
-            const uint64_t grow = row0 + rr, gcol = cb + ch * 4u;
-            if (grow < prow0 || grow >= prow_end) continue;
-            if (OUT_BF16) {
-              __nv_bfloat16* Kp = reinterpret_cast<__nv_bfloat16*>(K) + (grow - prow0) * n + gcol;
-              if (vec && gcol + 3 < n) {
-                const __nv_bfloat162 a = __floats2bfloat162_rn(o.x, o.y), b = __floats2bfloat162_rn(o.z, o.w);
-                uint2 u;
-                u.x = *reinterpret_cast<const uint32_t*>(&a);
-                u.y = *reinterpret_cast<const uint32_t*>(&b);
-                *reinterpret_cast<uint2*>(Kp) = u;
-              } else {
-                if (gcol + 0 < n) Kp[0] = __float2bfloat16_rn(o.x);
-                if (gcol + 1 < n) Kp[1] = __float2bfloat16_rn(o.y);
-                if (gcol + 2 < n) Kp[2] = __float2bfloat16_rn(o.z);
-                if (gcol + 3 < n) Kp[3] = __float2bfloat16_rn(o.w);
-              }
-            } else {
-              float* Kp = reinterpret_cast<float*>(K) + (grow - prow0) * n + gcol;
-              if (vec && gcol + 3 < n) {
-                *reinterpret_cast<float4*>(Kp) = o;
-              } else {
-                if (gcol + 0 < n) Kp[0] = o.x;
-                if (gcol + 1 < n) Kp[1] = o.y;
-                if (gcol + 2 < n) Kp[2] = o.z;
-                if (gcol + 3 < n) Kp[3] = o.w;
-              }
-            }
+          for (int c = 0; c < 32; ++c)
+            if (cb + c == row) diag[row] = v[c];
+        }
+        // transposed: K[gcol][row]; the warp's lanes write one contiguous run
+        if (fast_m) {
+          KT* p = Kt + (cb - prow0) * n + row;
+#pragma unroll
+          for (int c = 0; c < 32; ++c, p += n) kstore<OUT_BF16>(p, 0, v[c]);
+        } else if (mirror && row_in) {
+#pragma unroll
+          for (int c = 0; c < 32; ++c) {
+            const uint64_t gcol = cb + c;
+            if (gcol >= prow0 && gcol < prow_end) kstore<OUT_BF16>(Kt, (gcol - prow0) * n + row, v[c]);
+          }
+        }
+        if (!direct) continue;
+        // Own rows: 16 columns at a time through the warp's staging tile (32 rows x
+        // 16 columns, 16-byte chunks XOR-swizzled by row pair), out as row segments:
+        // four lanes a row, eight rows a store.
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          __syncwarp();                                    // the previous segment has been read back
+#pragma unroll
+          for (int c = 0; c < 4; ++c)
+            *reinterpret_cast<float4*>(stg + lane * 16 + ((c ^ ((lane >> 1) & 3)) * 4)) =
+                make_float4(v[16 * h + 4 * c], v[16 * h + 4 * c + 1], v[16 * h + 4 * c + 2], v[16 * h + 4 * c + 3]);
+          __syncwarp();
+          const uint32_t r8 = (uint32_t)lane >> 2, c4 = (uint32_t)lane & 3u;
+          const uint64_t gcol = cb + 16u * h + 4u * c4;
+#pragma unroll
+          for (int step = 0; step < 4; ++step) {
+            const uint32_t rr = 8u * step + r8;
+            const float4 o = *reinterpret_cast<const float4*>(stg + rr * 16 + ((c4 ^ ((rr >> 1) & 3u)) * 4));
+            const uint64_t grow = row0 + rr;
+            const float ov[4] = {o.x, o.y, o.z, o.w};
+            if (fast_d) kstore4<OUT_BF16>(K, (grow - prow0) * n + gcol, ov, true, gcol, n);
+            else if (grow >= prow0 && grow < prow_end) kstore4<OUT_BF16>(K, (grow - prow0) * n + gcol, ov, vec, gcol, n);
           }
         }
       }
@@ -1110,7 +1108,7 @@ km_status build_kernel_matrix(LloydEngine& e, const float* X, uint64_t n, uint32
   do {                                                                                             \
     KM_CUDA_TRY(cudaFuncSetAttribute(kmat_tc_kernel<X3_, BF_, KIND_>,                              \
                                      cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));     \
-    kmat_tc_kernel<X3_, BF_, KIND_><<<grid, 384, smem, s>>>(tA, tAlo, tB, tBlo, e.xn2, n, row0,    \
+    kmat_tc_kernel<X3_, BF_, KIND_><<<grid, KM_THREADS, smem, s>>>(tA, tAlo, tB, tBlo, e.xn2, n, row0,    \
                                                             row_end, KBn, (uint32_t)S, f, K, diag, \
                                                             vec, skip_done ? 1 : 0, e.st, tl, tiles); \
   } while (0)
