@@ -747,6 +747,7 @@ kkm_vk_kernel(const void* __restrict__ K, uint64_t n, uint32_t k, const uint32_t
   using T = std::conditional_t<KBF16, __nv_bfloat16, float>;
   using V = std::conditional_t<KBF16, uint2, float4>;
   griddep_wait();
+  griddep_launch();
   if (st->done) return;
   extern __shared__ __align__(16) uint8_t kk_smem[];
   const uint8_t* lab = GLAB ? lab8 : kk_smem;                        // n bytes
@@ -844,6 +845,8 @@ kkm_vk_kernel(const void* __restrict__ K, uint64_t n, uint32_t k, const uint32_t
 __global__ void kkm_ctilde_kernel(const float* __restrict__ E, uint32_t k, const uint32_t* __restrict__ perm,
                                   const uint32_t* __restrict__ cstart, double* __restrict__ ct,
                                   DevState* st) {
+  griddep_wait();
+  griddep_launch();
   if (st->done) return;
   const uint32_t c = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
@@ -864,6 +867,8 @@ __global__ void __launch_bounds__(256)
 kkm_dist_kernel(const float* __restrict__ E, uint64_t n, uint32_t k, const uint32_t* __restrict__ counts,
                 const double* __restrict__ ct, uint32_t* __restrict__ newlab,
                 double* __restrict__ part, DevState* st) {
+  griddep_wait();
+  griddep_launch();
   if (st->done) return;
   extern __shared__ float kd_smem[];
   float* inv = kd_smem;            // -2/|c| (0 for empty clusters)
@@ -902,6 +907,8 @@ kkm_dist_kernel(const float* __restrict__ E, uint64_t n, uint32_t k, const uint3
 // rule, label hand-over.
 __global__ void kkm_control_kernel(const double* __restrict__ part, int np, LoopConsts lc,
                                    int check, DevState* st) {
+  griddep_wait();
+  griddep_launch();
   if (st->done) return;
   if (threadIdx.x == 0 && blockIdx.x == 0) {
     double s = 0.0;
@@ -922,6 +929,8 @@ __global__ void kkm_control_kernel(const double* __restrict__ part, int np, Loop
 // they do not fit shared memory.
 __global__ void kkm_copy_labels_kernel(const uint32_t* __restrict__ src, uint32_t* __restrict__ dst,
                                        uint8_t* __restrict__ dst8, uint64_t n, DevState* st) {
+  griddep_wait();
+  griddep_launch();
   // runs after the control kernel: the labels of the final iteration are
   // copied too (the done flag is set by then), so only stop after copying.
   if (st->iter == 0) return;
@@ -1226,11 +1235,11 @@ km_status kkm_launch_vk(km_kkm* h, uint64_t r0, uint64_t r1) {
   const uint32_t k = h->p.k;
   cudaStream_t s = e.stream;
   if (h->p.k_bf16) {
-    if (h->glab) kkm_vk_kernel<true, true><<<grid, block, h->vk_smem, s>>>(h->K, n, k, h->lab, h->lab8, r0, r1, h->E, e.st);
-    else kkm_vk_kernel<true, false><<<grid, block, h->vk_smem, s>>>(h->K, n, k, h->lab, h->lab8, r0, r1, h->E, e.st);
+    if (h->glab) KM_CUDA_TRY(launch_pdl(kkm_vk_kernel<true, true>, grid, block, h->vk_smem, s, h->K, n, k, h->lab, h->lab8, r0, r1, h->E, e.st));
+    else KM_CUDA_TRY(launch_pdl(kkm_vk_kernel<true, false>, grid, block, h->vk_smem, s, h->K, n, k, h->lab, h->lab8, r0, r1, h->E, e.st));
   } else {
-    if (h->glab) kkm_vk_kernel<false, true><<<grid, block, h->vk_smem, s>>>(h->K, n, k, h->lab, h->lab8, r0, r1, h->E, e.st);
-    else kkm_vk_kernel<false, false><<<grid, block, h->vk_smem, s>>>(h->K, n, k, h->lab, h->lab8, r0, r1, h->E, e.st);
+    if (h->glab) KM_CUDA_TRY(launch_pdl(kkm_vk_kernel<false, true>, grid, block, h->vk_smem, s, h->K, n, k, h->lab, h->lab8, r0, r1, h->E, e.st));
+    else KM_CUDA_TRY(launch_pdl(kkm_vk_kernel<false, false>, grid, block, h->vk_smem, s, h->K, n, k, h->lab, h->lab8, r0, r1, h->E, e.st));
   }
   KM_CUDA_TRY(cudaGetLastError());
   return KM_OK;
@@ -1260,12 +1269,12 @@ km_status kkm_enqueue_iteration(km_kkm* h, const LoopConsts& lc) {
     KM_TRY(kkm_launch_vk(h, 0, n));
   }
   if (!h->fused) KM_TRY(e.enqueue_sort(h->lab));
-  kkm_ctilde_kernel<<<(k * 32 + 255) / 256, 256, 0, s>>>(h->E, k, e.perm, e.cstart, h->ct, e.st);
-  kkm_dist_kernel<<<h->dist_blocks, 256, 2 * k * sizeof(float), s>>>(h->E, n, k, e.counts, h->ct, h->nlab,
-                                                                      h->part, e.st);
-  kkm_control_kernel<<<1, 32, 0, s>>>(h->part, h->dist_blocks, lc, h->p.check_converged, e.st);
-  kkm_copy_labels_kernel<<<(unsigned)std::min<uint64_t>((n + 255) / 256, 4096), 256, 0, s>>>(
-      h->nlab, h->lab, h->glab ? h->lab8 : nullptr, n, e.st);
+  KM_CUDA_TRY(launch_pdl(kkm_ctilde_kernel, (k * 32 + 255) / 256, 256, 0, s, h->E, k, e.perm, e.cstart, h->ct, e.st));
+  KM_CUDA_TRY(launch_pdl(kkm_dist_kernel, h->dist_blocks, 256, 2 * k * sizeof(float), s, h->E, n, k, e.counts, h->ct,
+                         h->nlab, h->part, e.st));
+  KM_CUDA_TRY(launch_pdl(kkm_control_kernel, 1, 32, 0, s, h->part, h->dist_blocks, lc, (int)h->p.check_converged, e.st));
+  KM_CUDA_TRY(launch_pdl(kkm_copy_labels_kernel, (unsigned)std::min<uint64_t>((n + 255) / 256, 4096), 256, 0, s, h->nlab,
+                         h->lab, h->glab ? h->lab8 : (uint8_t*)nullptr, n, e.st));
   KM_CUDA_TRY(cudaGetLastError());
   return KM_OK;
 }

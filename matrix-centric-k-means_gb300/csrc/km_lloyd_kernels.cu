@@ -395,8 +395,8 @@ void launch_f32(const float* X, const float* C, const float* cn2, const float* x
     auto kern = ridx   ? assign_f32_kernel<tx(), ct(), false, true>
                 : Dout ? assign_f32_kernel<tx(), ct(), true, false>
                        : assign_f32_kernel<tx(), ct(), false, false>;
-    kern<<<blocks, F32_NT, f32_smem<T>(), s>>>(X, C, v4, cn2, xn2, n, d, k, tb, st, labels, mindist, rq, Dout, ridx,
-                                               nidx);
+    (void)launch_pdl(kern, blocks, F32_NT, f32_smem<T>(), s, X, C, v4, cn2, xn2, n, d, k, tb, st, labels, mindist, rq,
+                     Dout, ridx, nidx);
   });
 }
 }  // namespace
