@@ -840,22 +840,38 @@ kkm_vk_kernel(const void* __restrict__ K, uint64_t n, uint32_t k, const uint32_t
   }
 }
 
-// ctilde_c = (1/|c|^2) sum_{i in c} E[i, c] in FP64, one warp per cluster over
-// its rows (label-sorted permutation), fixed reduction order.
-__global__ void kkm_ctilde_kernel(const float* __restrict__ E, uint32_t k, const uint32_t* __restrict__ perm,
-                                  const uint32_t* __restrict__ cstart, double* __restrict__ ct,
-                                  DevState* st) {
+// Sum of one value per thread of a 256-thread block (result in thread 0), fixed order.
+__device__ __forceinline__ double block_sum_256(double v, double* red) {
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
+  __syncthreads();
+  return ((red[0] + red[1]) + (red[2] + red[3])) + ((red[4] + red[5]) + (red[6] + red[7]));
+}
+
+// ctilde_c = (1/|c|^2) sum_{i in c} E[i, c] in FP64, one block per cluster over its
+// rows (label-sorted permutation), fixed reduction order.  Bound by latency (gathered
+// loads, FP64 additions of about 40 ns each): four rows in flight per thread.
+// n = 20,000 k = 20 17 -> 6 us, n = 65,536 k = 64 30 -> 7 us (a warp per cluster,
+// one row after the other, before).
+__global__ void __launch_bounds__(256)
+kkm_ctilde_kernel(const float* __restrict__ E, uint32_t k, const uint32_t* __restrict__ perm,
+                  const uint32_t* __restrict__ cstart, double* __restrict__ ct, DevState* st) {
   griddep_wait();
   griddep_launch();
   if (st->done) return;
-  const uint32_t c = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int lane = threadIdx.x & 31;
-  if (c >= k) return;
+  __shared__ double red[8];
+  const uint32_t c = blockIdx.x;
   const uint32_t s0 = cstart[c], s1 = cstart[c + 1];
   double s = 0.0;
-  for (uint32_t p = s0 + lane; p < s1; p += 32) s += (double)E[(uint64_t)perm[p] * k + c];
-  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-  if (lane == 0) {
+  for (uint32_t p = s0 + threadIdx.x; p < s1; p += 4u * 256u) {
+    float v[4];
+#pragma unroll
+    for (uint32_t u = 0; u < 4; ++u)
+      v[u] = s1 - p > 256u * u ? E[(uint64_t)perm[p + 256u * u] * k + c] : 0.0f;
+    s += ((double)v[0] + (double)v[1]) + ((double)v[2] + (double)v[3]);
+  }
+  s = block_sum_256(s, red);
+  if (threadIdx.x == 0) {
     const double cnt = (double)(s1 - s0);
     ct[c] = (s1 > s0) ? s / (cnt * cnt) : 0.0;
   }
@@ -893,26 +909,24 @@ kkm_dist_kernel(const float* __restrict__ E, uint64_t n, uint32_t k, const uint3
     newlab[i] = key;
     acc += (double)val;
   }
-  __shared__ double red[256];
-  red[threadIdx.x] = acc;
-  __syncthreads();
-  for (int o = 128; o > 0; o >>= 1) {
-    if (threadIdx.x < o) red[threadIdx.x] += red[threadIdx.x + o];
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) part[blockIdx.x] = red[0];
+  __shared__ double red[8];
+  acc = block_sum_256(acc, red);
+  if (threadIdx.x == 0) part[blockIdx.x] = acc;
 }
 
-// End of iteration: score (fixed-order sum of the block partials), the stop
-// rule, label hand-over.
-__global__ void kkm_control_kernel(const double* __restrict__ part, int np, LoopConsts lc,
+// End of iteration: score (fixed-order sum of the block partials) and the stop rule.
+// One thread's chain of FP64 additions was 7 us of an iteration at n = 20,000 (79
+// partials); by 256 threads and a tree it is hidden in the launch.
+__global__ void __launch_bounds__(256) kkm_control_kernel(const double* __restrict__ part, int np, LoopConsts lc,
                                    int check, DevState* st) {
   griddep_wait();
   griddep_launch();
   if (st->done) return;
-  if (threadIdx.x == 0 && blockIdx.x == 0) {
-    double s = 0.0;
-    for (int i = 0; i < np; ++i) s += part[i];
+  __shared__ double red[8];
+  double s = 0.0;
+  for (int i = threadIdx.x; i < np; i += 256) s += part[i];
+  s = block_sum_256(s, red);
+  if (threadIdx.x == 0) {
     const uint32_t it = st->iter + 1;
     st->iter = it;
     st->score = s;
@@ -1269,10 +1283,10 @@ km_status kkm_enqueue_iteration(km_kkm* h, const LoopConsts& lc) {
     KM_TRY(kkm_launch_vk(h, 0, n));
   }
   if (!h->fused) KM_TRY(e.enqueue_sort(h->lab));
-  KM_CUDA_TRY(launch_pdl(kkm_ctilde_kernel, (k * 32 + 255) / 256, 256, 0, s, h->E, k, e.perm, e.cstart, h->ct, e.st));
+  KM_CUDA_TRY(launch_pdl(kkm_ctilde_kernel, k, 256, 0, s, h->E, k, e.perm, e.cstart, h->ct, e.st));
   KM_CUDA_TRY(launch_pdl(kkm_dist_kernel, h->dist_blocks, 256, 2 * k * sizeof(float), s, h->E, n, k, e.counts, h->ct,
                          h->nlab, h->part, e.st));
-  KM_CUDA_TRY(launch_pdl(kkm_control_kernel, 1, 32, 0, s, h->part, h->dist_blocks, lc, (int)h->p.check_converged, e.st));
+  KM_CUDA_TRY(launch_pdl(kkm_control_kernel, 1, 256, 0, s, h->part, h->dist_blocks, lc, (int)h->p.check_converged, e.st));
   KM_CUDA_TRY(launch_pdl(kkm_copy_labels_kernel, (unsigned)std::min<uint64_t>((n + 255) / 256, 4096), 256, 0, s, h->nlab,
                          h->lab, h->glab ? h->lab8 : (uint8_t*)nullptr, n, e.st));
   KM_CUDA_TRY(cudaGetLastError());
