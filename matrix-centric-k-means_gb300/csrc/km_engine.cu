@@ -307,18 +307,17 @@ km_status LloydEngine::set_points(const float* Xsrc, bool on_device, bool copy) 
       cudaStream_t sc = (c & 1) ? aux : stream;
       KM_CUDA_TRY(cudaMemcpyAsync(X_owned + r0 * d, Xsrc + r0 * d, sizeof(float) * (r1 - r0) * d,
                                   cudaMemcpyHostToDevice, sc));
-      const int blocks = (int)std::min<uint64_t>((r1 - r0 + 7) / 8, (uint64_t)num_sms * 8);
-      prep_points_kernel<<<blocks, 256, 0, sc>>>(X + r0 * d, r1 - r0, d, dp, xn2 + r0, xn2d ? xn2d + r0 : nullptr,
-                                                 Xb ? Xb + r0 * dp : nullptr, Xlo ? Xlo + r0 * dp : nullptr, st);
+      launch_prep_points(X + r0 * d, r1 - r0, d, dp, xn2 + r0, xn2d ? xn2d + r0 : nullptr, nullptr,
+                         Xb ? Xb + r0 * dp : nullptr, Xlo ? Xlo + r0 * dp : nullptr, st, num_sms, sc);
     }
     KM_CUDA_TRY(cudaEventRecord(ev_join, aux));
     KM_CUDA_TRY(cudaStreamWaitEvent(stream, ev_join, 0));
   } else {
-    if (copy || !on_device)
-      KM_CUDA_TRY(cudaMemcpyAsync(X_owned, Xsrc, bytes,
-                                  on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice, stream));
-    const int blocks = (int)std::min<uint64_t>((n + 7) / 8, (uint64_t)num_sms * 16);
-    prep_points_kernel<<<blocks, 256, 0, stream>>>(X, n, d, dp, xn2, xn2d, Xb, Xlo, st);
+    // A device-to-device copy is made by the preparation, which reads the points anyway.
+    if (!on_device)
+      KM_CUDA_TRY(cudaMemcpyAsync(X_owned, Xsrc, bytes, cudaMemcpyHostToDevice, stream));
+    launch_prep_points(on_device ? Xsrc : X, n, d, dp, xn2, xn2d, on_device && copy ? X_owned : nullptr, Xb, Xlo, st,
+                       num_sms, stream);
   }
   KM_CUDA_TRY(cudaGetLastError());
   if (xn2d) {

@@ -10,9 +10,8 @@
 namespace km {
 
 // ---- kernels (km_lloyd_kernels.cu) ----
-__global__ void prep_points_kernel(const float* X, uint64_t n, uint32_t d, uint32_t dp, float* xn2,
-                                   double* xn2d, __nv_bfloat16* Xb, __nv_bfloat16* Xlo,
-                                   DevState* st);
+void launch_prep_points(const float* X, uint64_t n, uint32_t d, uint32_t dp, float* xn2, double* xn2d, float* Xc,
+                        __nv_bfloat16* Xb, __nv_bfloat16* Xlo, DevState* st, int sms, cudaStream_t s);
 __global__ void reduce_f64_partial_kernel(const double* v, uint64_t n, double* part);
 __global__ void reduce_f64_final_kernel(const double* part, int np, double* out);
 __global__ void prep_centroids_kernel(const float* C, uint32_t k, uint32_t kp, uint32_t d,

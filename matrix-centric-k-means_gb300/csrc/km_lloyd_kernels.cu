@@ -16,6 +16,7 @@
 #include "km_simt.cuh"
 #include "km_sums.cuh"
 
+#include <algorithm>
 #include <cmath>
 #include <cfloat>
 #include <type_traits>
@@ -28,56 +29,153 @@ static __device__ __forceinline__ float f_inf() { return __int_as_float(0x7f8000
 // Preparation
 // ---------------------------------------------------------------------------
 
-// One warp per row: ||x||^2 (an FP32 pair, stored as float and as a per-row
-// double for the deterministic total), non-finite check, and the BF16 hi/lo
-// copies padded with zeros to dp columns (only when Xb != nullptr).
-__global__ void prep_points_kernel(const float* __restrict__ X, uint64_t n, uint32_t d, uint32_t dp,
-                                   float* __restrict__ xn2, double* __restrict__ xn2d,
-                                   __nv_bfloat16* __restrict__ Xb, __nv_bfloat16* __restrict__ Xlo,
-                                   DevState* st) {
+// h + l += a + al, the first addition by TwoSum (the FP64 units of this GPU are a
+// small fraction of its FP32 rate): a sum of squares split exactly by an FMA each is
+// within a few units of 2^-48 of the exact value, and float(h + l) is the correctly
+// rounded norm.
+static __device__ __forceinline__ void two_sum(float& h, float& l, float a, float al) {
+  const float t = __fadd_rn(h, a), bp = __fsub_rn(t, h);
+  const float err = __fadd_rn(__fsub_rn(h, __fsub_rn(t, bp)), __fsub_rn(a, bp));
+  h = t;
+  l = __fadd_rn(l, __fadd_rn(al, err));
+}
+
+// Per row: ||x||^2 (an FP32 pair, stored as float and as a per-row double for the
+// deterministic total), non-finite check, the row's copy (only when Xc != nullptr) and
+// its BF16 hi/lo copies padded with zeros to dp columns (only when Xb != nullptr).
+// NaN/Inf and non-BF16 coordinates are flagged once per warp (after its rows), not once
+// per row: an atomic per row on one word serialises.
+// VEC: the widest of 4, 2 and 1 columns that d divides by and X (and Xc) are aligned
+// to.  A row is taken by G lanes, VEC columns each and a step of G * VEC columns; four steps' loads (of four
+// rows, or of one row that has more columns than a step) are in flight per warp.
+// Bound by HBM: n = 1,048,576 d = 128 with the copy, Xb and Xlo 433 us (a copy, then a warp
+// a row and a column a lane) -> 277 (5.8 TB/s); n = 200,000 d = 100 with the copy 81 -> 36;
+// n = 300,007 d = 50 with Xb and Xlo 40 (84 with a column a lane).
+template <int VEC, int G, bool ONE>
+__global__ void __launch_bounds__(256, 4)
+prep_points_kernel(const float* __restrict__ X, uint64_t n, uint32_t d, uint32_t dp, float* __restrict__ xn2,
+                   double* __restrict__ xn2d, float* __restrict__ Xc, __nv_bfloat16* __restrict__ Xb,
+                   __nv_bfloat16* __restrict__ Xlo, DevState* st) {
+  constexpr int U = 4, R = 32 / G;
+  constexpr uint32_t STEP = G * VEC;
   const uint64_t warp = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int lane = threadIdx.x & 31;
   const uint64_t nw = ((uint64_t)gridDim.x * blockDim.x) >> 5;
-  // ||x||^2 as an unevaluated FP32 pair (hi + lo): each square split exactly
-  // by an FMA, each addition by TwoSum (the FP64 units of this GPU are a
-  // small fraction of its FP32 rate); the pair is within a few units of 2^-48
-  // of the exact value, and float(hi + lo) is the correctly rounded norm.
-  auto two_sum = [](float& h, float& l, float a, float al) {
-    const float t = __fadd_rn(h, a), bp = __fsub_rn(t, h);
-    const float err = __fadd_rn(__fsub_rn(h, __fsub_rn(t, bp)), __fsub_rn(a, bp));
-    h = t;
-    l = __fadd_rn(l, __fadd_rn(al, err));
-  };
-  // NaN/Inf and non-BF16 coordinates are flagged once per warp (after its
-  // rows), not once per row: an atomic per row on one word serialises.
-  bool bad = false, inexact = false;
-  for (uint64_t r = warp; r < n; r += nw) {
-    const float* x = X + r * d;
-    float sh = 0.0f, sl = 0.0f;
-    for (uint32_t j = lane; j < dp; j += 32) {
-      float v = (j < d) ? x[j] : 0.0f;
-      if (!isfinite(v)) bad = true;
-      if ((__float_as_uint(v) & 0xffffu) != 0u) inexact = true;    // not a BF16 value
-      const float p = __fmul_rn(v, v);
-      two_sum(sh, sl, p, fmaf(v, v, -p));
-      if (Xb) {
-        __nv_bfloat16 hi = __float2bfloat16_rn(v);
-        Xb[r * dp + j] = hi;
-        if (Xlo) Xlo[r * dp + j] = __float2bfloat16_rn(v - __bfloat162float(hi));
+  const int lane = threadIdx.x & 31;
+  const uint32_t col0 = (uint32_t)(lane % G) * VEC;
+  const uint32_t cols = Xb ? dp : d;
+  constexpr int NR = ONE ? U : 1;              // rows per lane and round; ONE: a row is one step
+  constexpr uint64_t rows = R * NR;
+  uint32_t top = 0, low = 0;                   // largest |x| as bits; bits below BF16's
+  for (uint64_t base = warp * rows; base < n; base += nw * rows) {
+    const uint64_t row0 = base + lane / G;
+    float sh[NR], sl[NR];
+#pragma unroll
+    for (int u = 0; u < NR; ++u) sh[u] = sl[u] = 0.0f;
+    for (uint32_t j0 = 0; j0 < cols; j0 += ONE ? STEP : STEP * U) {
+      float v[U][VEC];
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const uint64_t r = ONE ? row0 + (uint64_t)u * R : row0;
+        const uint32_t j = j0 + col0 + (ONE ? 0u : u * STEP);
+        const bool in = r < n && j < d;
+        if constexpr (VEC == 4) {
+          const float4 t = in ? *reinterpret_cast<const float4*>(X + r * d + j) : make_float4(0.f, 0.f, 0.f, 0.f);
+          v[u][0] = t.x; v[u][1] = t.y; v[u][2] = t.z; v[u][3] = t.w;
+        } else if constexpr (VEC == 2) {
+          const float2 t = in ? *reinterpret_cast<const float2*>(X + r * d + j) : make_float2(0.f, 0.f);
+          v[u][0] = t.x; v[u][1] = t.y;
+        } else {
+          v[u][0] = in ? X[r * d + j] : 0.0f;
+        }
+      }
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const uint64_t r = ONE ? row0 + (uint64_t)u * R : row0;
+        const uint32_t j = j0 + col0 + (ONE ? 0u : u * STEP);
+        alignas(8) __nv_bfloat16 hi[VEC], lo[VEC];
+#pragma unroll
+        for (int e = 0; e < VEC; ++e) {
+          const float x = v[u][e];
+          top = max(top, __float_as_uint(x) & 0x7fffffffu);
+          low |= __float_as_uint(x);
+          const float p = __fmul_rn(x, x);
+          two_sum(sh[ONE ? u : 0], sl[ONE ? u : 0], p, fmaf(x, x, -p));
+          hi[e] = __float2bfloat16_rn(x);
+          if (Xlo) lo[e] = __float2bfloat16_rn(x - __bfloat162float(hi[e]));
+        }
+        if (Xc && r < n && j < d) {
+          if constexpr (VEC == 4) *reinterpret_cast<float4*>(Xc + r * d + j) = make_float4(v[u][0], v[u][1], v[u][2], v[u][3]);
+          else if constexpr (VEC == 2) *reinterpret_cast<float2*>(Xc + r * d + j) = make_float2(v[u][0], v[u][1]);
+          else Xc[r * d + j] = v[u][0];
+        }
+        if (Xb && r < n && j < dp) {            // dp is a multiple of 64
+          if constexpr (VEC == 4) {
+            *reinterpret_cast<uint2*>(Xb + r * dp + j) = *reinterpret_cast<const uint2*>(hi);
+            if (Xlo) *reinterpret_cast<uint2*>(Xlo + r * dp + j) = *reinterpret_cast<const uint2*>(lo);
+          } else if constexpr (VEC == 2) {
+            *reinterpret_cast<uint32_t*>(Xb + r * dp + j) = *reinterpret_cast<const uint32_t*>(hi);
+            if (Xlo) *reinterpret_cast<uint32_t*>(Xlo + r * dp + j) = *reinterpret_cast<const uint32_t*>(lo);
+          } else {
+            Xb[r * dp + j] = hi[0];
+            if (Xlo) Xlo[r * dp + j] = lo[0];
+          }
+        }
       }
     }
-    for (int o = 16; o > 0; o >>= 1) {
-      const float oh = __shfl_xor_sync(0xffffffffu, sh, o), ol = __shfl_xor_sync(0xffffffffu, sl, o);
-      two_sum(sh, sl, oh, ol);
+    // Over the G lanes: while a lane holds several rows' sums, each exchange leaves it
+    // half of them (6 additions for four rows of a warp instead of 20).
+    int o = G / 2, u = 0;                      // u: the row that this lane ends with
+    auto add_from = [&](float& h, float& l, float oh, float ol, int off) {
+      oh = __shfl_xor_sync(0xffffffffu, oh, off);
+      ol = __shfl_xor_sync(0xffffffffu, ol, off);
+      two_sum(h, l, oh, ol);
+    };
+    if constexpr (NR == 4) {
+      const bool up = lane & o, up2 = lane & (o >> 1);
+#pragma unroll
+      for (int i = 0; i < 2; ++i) {            // keeps rows i (lower lanes) or i + 2 (upper)
+        const float gh = up ? sh[i] : sh[i + 2], gl = up ? sl[i] : sl[i + 2];
+        if (up) { sh[i] = sh[i + 2]; sl[i] = sl[i + 2]; }
+        add_from(sh[i], sl[i], gh, gl, o);
+      }
+      const float gh = up2 ? sh[0] : sh[1], gl = up2 ? sl[0] : sl[1];
+      if (up2) { sh[0] = sh[1]; sl[0] = sl[1]; }
+      add_from(sh[0], sl[0], gh, gl, o >> 1);
+      u = (up ? 2 : 0) + (up2 ? 1 : 0);
+      o >>= 2;
     }
-    const double s = (double)sh + (double)sl;
-    if (lane == 0) {
+    const int holders = o;                     // lanes l % (2 * holders) == 0 write a row each
+#pragma unroll
+    for (; o > 0; o >>= 1) add_from(sh[0], sl[0], sh[0], sl[0], o);
+    const uint64_t r = row0 + (uint64_t)u * R;
+    if (lane % max(2 * holders, 1) == 0 && r < n) {
+      const double s = (double)sh[0] + (double)sl[0];
       xn2[r] = (float)s;
       if (xn2d) xn2d[r] = s;
     }
   }
+  const bool bad = top >= 0x7f800000u, inexact = (low & 0xffffu) != 0u;
   if (__any_sync(0xffffffffu, bad) && lane == 0) atomicOr(&st->err, KM_DEVERR_NONFINITE);
   if (__any_sync(0xffffffffu, inexact) && lane == 0) atomicOr(&st->x_not_bf16, 1u);
+}
+
+// The narrowest group of lanes that takes a row in one step, at most a warp (a warp a row
+// leaves 28 of 32 lanes idle at d = 16).  sms: one wave of four blocks on each.
+void launch_prep_points(const float* X, uint64_t n, uint32_t d, uint32_t dp, float* xn2, double* xn2d, float* Xc,
+                        __nv_bfloat16* Xb, __nv_bfloat16* Xlo, DevState* st, int sms, cudaStream_t s) {
+  const uint32_t cols = Xb ? dp : d;
+  const uintptr_t at = reinterpret_cast<uintptr_t>(X) | reinterpret_cast<uintptr_t>(Xc);
+  const int vec = d % 4 == 0 && at % 16 == 0 ? 4 : d % 2 == 0 && at % 8 == 0 ? 2 : 1;
+  auto go = [&](auto kernel, uint64_t rows) {            // rows: per warp and round
+    const int blocks = (int)std::min<uint64_t>((n + 8 * rows - 1) / (8 * rows), (uint64_t)sms * 4);
+    kernel<<<blocks, 256, 0, s>>>(X, n, d, dp, xn2, xn2d, Xc, Xb, Xlo, st);
+  };
+  if (vec == 1) cols <= 8 ? go(prep_points_kernel<1, 8, true>, 16) : go(prep_points_kernel<1, 32, false>, 1);
+  else if (vec == 2) cols <= 64 ? go(prep_points_kernel<2, 32, true>, 4) : go(prep_points_kernel<2, 32, false>, 1);
+  else if (cols <= 16) go(prep_points_kernel<4, 4, true>, 32);
+  else if (cols <= 64) go(prep_points_kernel<4, 16, true>, 8);
+  else if (cols <= 128) go(prep_points_kernel<4, 32, true>, 4);
+  else go(prep_points_kernel<4, 32, false>, 1);
 }
 
 // Deterministic FP64 sum: fixed-shape tree per block, block partials summed in
