@@ -315,7 +315,7 @@ km_status km_lloyd_fit(km_lloyd* h, const float* C0, uint32_t* labels_out, float
     res->converged_iter = s.converged_iter ? s.converged_iter : h->p.maxiter;
     res->objective = s.objective;
     res->score = s.score;
-    res->max_shift = s.max_shift;
+    res->max_shift = std::sqrt(s.max_move2);
     res->refined_rows = s.refined_total;
     res->full_rescore_rows = s.full_total;
     res->fit_ms = ms;

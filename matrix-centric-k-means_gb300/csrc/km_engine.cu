@@ -271,7 +271,7 @@ km_status LloydEngine::init(uint64_t n_, uint32_t d_, uint32_t k_, int precision
     KM_TRY(take(&Cn, (size_t)k * d));
     KM_TRY(take(&dsq, (size_t)k * d));
     KM_TRY(take(&objpart, (size_t)k * d));
-    KM_TRY(take(&shift_c, k));
+    KM_TRY(take(&move2_c, k));
     KM_TRY(take(&obj_c, k));
   }
   KM_TRY(take(&seghist, (size_t)k * nseg));
@@ -433,8 +433,9 @@ km_status LloydEngine::enqueue_assign(float* Dout) {
 }
 
 km_status LloydEngine::enqueue_finalize(const LoopConsts& lc) {
-  KM_CUDA_TRY(launch_pdl(finalize_kernel, (k * 32 + 255) / 256, 256, 0, stream, Cn, C, dsq, objpart, counts,
-                         lc.empty, d, dp, k, lc.tol, cn2, Cb, Clo, Ct, shift_c, obj_c, st, lc));
+  const unsigned threads = k <= 512 ? 64 : 256;      // (see the kernel)
+  KM_CUDA_TRY(launch_pdl(finalize_kernel, (k * 32 + threads - 1) / threads, threads, 0, stream, Cn, C, dsq, objpart, counts,
+                         lc.empty, d, dp, k, lc.tol, cn2, Cb, Clo, Ct, move2_c, obj_c, st, lc));
   KM_CUDA_TRY(cudaGetLastError());
   return KM_OK;
 }

@@ -75,7 +75,7 @@ struct DevState {
   double objective;         // FP64 objective of the last assignment
   double last_score;
   double score;
-  double max_shift;
+  double max_move2;        // largest squared centroid move
   double sum_x2;            // FP64 sum_i ||x_i||^2
 };
 

@@ -48,7 +48,7 @@ __global__ void finalize_kernel(const float* Cn, float* C, const float* dsq, con
                                 const uint32_t* counts, int32_t empty_excl,
                                 uint32_t d, uint32_t dp, uint32_t k, float tol, float* cn2,
                                 __nv_bfloat16* Cb, __nv_bfloat16* Clo, float* Ct,
-                                double* shift_c, double* obj_c, DevState* st, LoopConsts lc);
+                                double* move2_c, double* obj_c, DevState* st, LoopConsts lc);
 
 // ---- tensor-core distance stage (km_tc.cu) ----
 struct TcPlan {
@@ -124,7 +124,7 @@ struct LloydEngine {
   float* cn2 = nullptr;
   float* dsq = nullptr;
   double* objpart = nullptr;
-  double* shift_c = nullptr;
+  double* move2_c = nullptr;
   double* obj_c = nullptr;
   __nv_bfloat16* Cb = nullptr;
   __nv_bfloat16* Clo = nullptr;

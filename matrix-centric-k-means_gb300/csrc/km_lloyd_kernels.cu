@@ -1503,7 +1503,10 @@ km_status launch_update_sums(const float* X, const uint32_t* perm, const uint32_
 // cluster, new ||c||^2 and BF16 copies; then C <- Cn.  The block that finishes
 // last (a ticket in DevState) then ends the iteration: deterministic
 // reductions over the clusters, the stop decision, counters for the next
-// iteration.
+// iteration.  Bound by latency and by the FP64 units (two lanes a cycle and SM, so eight
+// warps' 40 operations each were 3 us): two warps a block up to 512 clusters (beyond,
+// the last block's sums would take longer), maxima of squares with one root at the end.
+// d = 64 k = 10 8.4 -> 5.8 us, d = 100 k = 64 11.1 -> 7.8, d = 128 k = 256 9.1 -> 8.1.
 __global__ void __launch_bounds__(256)
 finalize_kernel(const float* __restrict__ Cn, float* __restrict__ C,
                 const float* __restrict__ dsq, const double* __restrict__ objpart,
@@ -1511,13 +1514,13 @@ finalize_kernel(const float* __restrict__ Cn, float* __restrict__ C,
                 uint32_t d, uint32_t dp, uint32_t k, float tol,
                 float* __restrict__ cn2, __nv_bfloat16* __restrict__ Cb,
                 __nv_bfloat16* __restrict__ Clo, float* __restrict__ Ct,
-                double* __restrict__ shift_c, double* __restrict__ obj_c,
+                double* __restrict__ move2_c, double* __restrict__ obj_c,
                 DevState* st, LoopConsts lc) {
   griddep_wait();
   if (st->done) return;
-  __shared__ double s_obj[256];
-  __shared__ double s_sh[256];
-  __shared__ float s_cm[256];
+  __shared__ double s_obj[8];
+  __shared__ double s_mv[8];
+  __shared__ float s_cm[8];
   __shared__ int is_last;
   const uint32_t c = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
@@ -1564,6 +1567,7 @@ finalize_kernel(const float* __restrict__ Cn, float* __restrict__ C,
 #pragma unroll
       for (int q = 0; q < 4; ++q) {
         const uint32_t jq = j0 + 32u * q;
+        if (jq >= d) break;
 #pragma unroll
         for (int l = 0; l < 32; ++l) {
           const float tq = __shfl_sync(0xffffffffu, dq[q], l);
@@ -1579,7 +1583,7 @@ finalize_kernel(const float* __restrict__ Cn, float* __restrict__ C,
     if (lane == 0) {
       if (sqrtf(s) > tol) st->moved = 1u;
       cn2[c] = excl ? f_inf() : (float)nrm;
-      shift_c[c] = sqrt(mv);
+      move2_c[c] = mv;
       obj_c[c] = ob;
     }
   }
@@ -1592,33 +1596,34 @@ finalize_kernel(const float* __restrict__ Cn, float* __restrict__ C,
   __threadfence();
   // other blocks' results: read past L1 (this SM may hold stale lines)
   volatile DevState* vs = st;
-  double ob = 0.0, sh = 0.0;
-  float cm = 0.0f;
-  const uint32_t per = (k + blockDim.x - 1) / blockDim.x;
-  const uint32_t b = threadIdx.x * per, e = min(k, b + per);
-  for (uint32_t cc = b; cc < e; ++cc) {
+  double ob = 0.0, mv2 = 0.0;
+  float cm = 0.0f;                               // largest squared norm
+  for (uint32_t cc = threadIdx.x; cc < k; cc += blockDim.x) {
     ob += __ldcg(obj_c + cc);
-    sh = fmax(sh, __ldcg(shift_c + cc));
+    mv2 = fmax(mv2, __ldcg(move2_c + cc));
     const float v = __ldcg(cn2 + cc);
-    if (v < f_inf()) cm = fmaxf(cm, sqrtf(v));   // excluded (empty) clusters hold +inf
+    if (v < f_inf()) cm = fmaxf(cm, v);          // excluded (empty) clusters hold +inf
   }
-  s_obj[threadIdx.x] = ob; s_sh[threadIdx.x] = sh; s_cm[threadIdx.x] = cm;
+  for (int o = 16; o > 0; o >>= 1) {
+    ob += __shfl_xor_sync(0xffffffffu, ob, o);
+    mv2 = fmax(mv2, __shfl_xor_sync(0xffffffffu, mv2, o));
+    cm = fmaxf(cm, __shfl_xor_sync(0xffffffffu, cm, o));
+  }
+  if (lane == 0) { s_obj[threadIdx.x >> 5] = ob; s_mv[threadIdx.x >> 5] = mv2; s_cm[threadIdx.x >> 5] = cm; }
   __syncthreads();
-  for (int o = blockDim.x / 2; o > 0; o >>= 1) {
-    if (threadIdx.x < o) {
-      s_obj[threadIdx.x] += s_obj[threadIdx.x + o];
-      s_sh[threadIdx.x] = fmax(s_sh[threadIdx.x], s_sh[threadIdx.x + o]);
-      s_cm[threadIdx.x] = fmaxf(s_cm[threadIdx.x], s_cm[threadIdx.x + o]);
-    }
-    __syncthreads();
-  }
   if (threadIdx.x == 0) {
     const uint32_t it = vs->iter + 1;
     vs->iter = it;
-    vs->objective = s_obj[0];
-    vs->max_shift = s_sh[0];
-    vs->cmax = s_cm[0] * 1.000001f;
-    const double score = s_obj[0] - vs->sum_x2;
+    ob = s_obj[0]; mv2 = s_mv[0]; cm = s_cm[0];
+    for (uint32_t w = 1; w < (blockDim.x >> 5); ++w) {
+      ob += s_obj[w];
+      mv2 = fmax(mv2, s_mv[w]);
+      cm = fmaxf(cm, s_cm[w]);
+    }
+    vs->objective = ob;
+    vs->max_move2 = mv2;
+    vs->cmax = sqrtf(cm) * 1.000001f;
+    const double score = ob - vs->sum_x2;
     vs->score = score;
     bool stop = false;
     if (lc.conv == KM_CONV_SHIFT) {
