@@ -102,14 +102,14 @@ km_status LloydEngine::take_bytes(void** p, size_t bytes) {
 }
 
 // Relative error coefficients of the fast distance path (see TieBound).
-TieBound make_tie_bound(int precision, uint32_t d, bool a_exact) {
+TieBound make_tie_bound(int precision, uint32_t d, bool a_exact, uint32_t terms) {
   const double u = std::ldexp(1.0, -24);
   const double ub = std::ldexp(1.0, -8);
   const double uacc = std::ldexp(1.0, -22);  // tensor-core FP32 accumulation, 4 ulp per add
   auto gamma = [](double m, double uu) { return m * uu / (1.0 - m * uu); };
   double eps;
   if (precision == KM_PREC_FP32) {
-    eps = gamma((double)d, u);
+    eps = gamma((double)(terms ? terms : d), u);
   } else if (precision == KM_PREC_BF16) {
     // |x^ c^ - x c| <= (2ub + ub^2) |x||c| per term (ub only when x^ = x),
     // plus FP32 accumulation of d products
@@ -232,7 +232,7 @@ km_status LloydEngine::init(uint64_t n_, uint32_t d_, uint32_t k_, int precision
       KM_TRY(take(&nfull, 1));
       // the FP32 pass's queues; its wide queue and lists take over the first ones'
       rq2 = RefineQueues{q2, q2full, q2cnt, q2fcnt, rows / 32, qwide, qwcnt, wl, wlc, L};
-      tb32 = make_tie_bound(KM_PREC_FP32, d, false);
+      tb32 = make_tie_bound(KM_PREC_FP32, d, false, f32_gather_terms(d));
     }
     KM_TRY(refine_prepare());
   }

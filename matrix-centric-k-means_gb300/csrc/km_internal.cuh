@@ -155,8 +155,9 @@ struct TieBound {
 };
 
 // a_exact: every point coordinate is exactly a BF16 value, so only the
-// centroid operand carries a rounding error.
-TieBound make_tie_bound(int precision, uint32_t d, bool a_exact);
+// centroid operand carries a rounding error.  terms (FP32): operations in the longest
+// chain of a product, 0 for d.
+TieBound make_tie_bound(int precision, uint32_t d, bool a_exact, uint32_t terms = 0);
 
 // Refinement queue entry: a row whose reference argmin is proven to be one of
 // `cnt` (2..4) candidate centroids.  Rows with more candidates go to the

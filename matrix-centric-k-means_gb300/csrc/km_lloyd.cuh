@@ -27,6 +27,8 @@ km_status launch_refine(bool v4, int num_sms, const float* X, const float* C, co
 // Chunked-kernel refinement: candidate and wide queues as launch_refine; rows
 // of the full queue go through the FP32 distance kernel on those rows alone
 // (gathered by index into fidx) and then the exact re-score of its near ties.
+// Operations in the longest chain of a product of launch_refine_gemm's FP32 pass.
+uint32_t f32_gather_terms(uint32_t d);
 km_status launch_refine_gemm(bool v4, int num_sms, const float* X, const float* C, const float* Ct,
                              const float* cn2, const float* xn2, uint64_t n, uint32_t d, uint32_t k,
                              TieBound tb32, DevState* st, const RefineQueues& rq,

@@ -260,6 +260,7 @@ __global__ void prep_centroids_kernel(const float* __restrict__ C, uint32_t k, u
 // left eight warps an SM, 44 % of the issue slots used and 21 T).
 // ---------------------------------------------------------------------------
 constexpr int F32_NT = 128, F32_RT = 8, F32_LIST = 8;
+constexpr int F32_GATHER_RUN = 64;       // (GATHER) coordinates summed on their own
 template <int TX, int CT>
 using F32Tile = SimtTile<F32_NT, F32_RT, TX, CT, TX == 16 && CT == 8 ? 16 : 8>;
 // Shared memory after the product's stages: per row m, tau's row terms, the
@@ -270,17 +271,21 @@ struct F32Row {
   uint32_t cnt;
   uint32_t row;                 // row of X
 };
-template <class T>
+template <class T, bool GATHER>
 constexpr size_t f32_smem() {
-  return T::SMEM + T::ROWS * (sizeof(F32Row) + F32_LIST * sizeof(uint2)) + T::COLS * sizeof(float);
+  return T::SMEM + (GATHER ? T::TOT_BYTES : 0) + T::ROWS * (sizeof(F32Row) + F32_LIST * sizeof(uint2)) +
+         T::COLS * sizeof(float);
 }
 
 // GATHER: logical row li of the tiles is row ridx[li] of X, for li < *nidx; queue
 // segments are taken over the logical rows.  These rows have many near ties (the
 // chunked tensor-core kernel found more than its lists hold), so their lists are the
 // global ones (rq.wl, L entries a row), filtered by a warp a row, and rows with
-// 5..L candidates go to the wide queue instead of the full re-score: n = 4M d = 256
-// k = 4096 (BF16 points, Zipf sizes) 57 -> 24 ms of full re-score an iteration.
+// 5..L candidates go to the wide queue instead of the full re-score.  Their products are
+// summed in runs of F32_GATHER_RUN coordinates, which makes the near-tie bound (tb)
+// narrower by as much as the chains are shorter: n = 4M d = 256 k = 4096 (BF16 points,
+// Zipf sizes), an iteration: full re-score 57 (lists of 8) -> 24 (lists of 256) -> none
+// (runs of 64; runs of 32 took this pass 22.9 ms for 21.7, and no row less to the queues).
 template <int TX, int CT, bool DOUT, bool GATHER>
 __global__ void __launch_bounds__(F32_NT, CT == 8 ? 3 : 4)
 assign_f32_kernel(const float* __restrict__ X, const float* __restrict__ C, bool v4,
@@ -298,7 +303,7 @@ assign_f32_kernel(const float* __restrict__ X, const float* __restrict__ C, bool
   // all have to be written; a gather's start at zero.)
   if (GATHER && m0 >= n_log) return;
   extern __shared__ __align__(16) float f32_smem_raw[];
-  uint2* const list = reinterpret_cast<uint2*>(f32_smem_raw + T::SMEM / sizeof(float));   // [ROWS][F32_LIST]
+  uint2* const list = reinterpret_cast<uint2*>(f32_smem_raw + (T::SMEM + (GATHER ? T::TOT_BYTES : 0)) / sizeof(float));   // [ROWS][F32_LIST]
   F32Row* const rs = reinterpret_cast<F32Row*>(list + T::ROWS * F32_LIST);
   float* const cns = reinterpret_cast<float*>(rs + T::ROWS);
   const int tid = threadIdx.x, tx = tid % TX, ty = tid / TX;
@@ -335,10 +340,11 @@ assign_f32_kernel(const float* __restrict__ X, const float* __restrict__ C, bool
   for (uint32_t c0 = 0; c0 < k; c0 += T::COLS) {
     for (int c = tid; c < T::COLS; c += F32_NT) cns[c] = c0 + (uint32_t)c < k ? cn2[c0 + c] : f_inf();
     float2 acc[F32_RT / 2][CT];
-    simt_product<T>(
+    simt_product<T, GATHER ? F32_GATHER_RUN : 0>(
         f32_smem_raw, d, v4,
         [&](int r) { return m0 + (uint64_t)r < n_log ? X + (uint64_t)rs[r].row * d : (const float*)nullptr; },
-        [&](int c) { return c0 + (uint32_t)c < k ? C + (uint64_t)(c0 + c) * d : (const float*)nullptr; }, acc);
+        [&](int c) { return c0 + (uint32_t)c < k ? C + (uint64_t)(c0 + c) * d : (const float*)nullptr; }, acc,
+        reinterpret_cast<float4*>(f32_smem_raw + T::SMEM / sizeof(float)));
     // v = ||c||^2 - 2 x.c in place; columns at or past k hold +inf (or NaN)
     float cn[CT];
 #pragma unroll
@@ -493,7 +499,7 @@ void launch_f32(const float* X, const float* C, const float* cn2, const float* x
     auto kern = ridx   ? assign_f32_kernel<tx(), ct(), false, true>
                 : Dout ? assign_f32_kernel<tx(), ct(), true, false>
                        : assign_f32_kernel<tx(), ct(), false, false>;
-    (void)launch_pdl(kern, blocks, F32_NT, f32_smem<T>(), s, X, C, v4, cn2, xn2, n, d, k, tb, st, labels, mindist, rq,
+    (void)launch_pdl(kern, blocks, F32_NT, ridx ? f32_smem<T, true>() : f32_smem<T, false>(), s, X, C, v4, cn2, xn2, n, d, k, tb, st, labels, mindist, rq,
                      Dout, ridx, nidx);
   });
 }
@@ -1056,7 +1062,7 @@ km_status refine_prepare() {
                         assign_f32_kernel<tx(), ct(), false, true>})
         if (err == cudaSuccess)
           err = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)f32_smem<F32Tile<tx(), ct()>>());
+                                     (int)f32_smem<F32Tile<tx(), ct()>, true>());
     });
   KM_CUDA_TRY(err);
   KM_CUDA_TRY(cudaFuncSetAttribute(refine_staged_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -1081,6 +1087,10 @@ km_status launch_refine(bool v4, int num_sms, const float* X, const float* C, co
   }
   KM_CUDA_TRY(cudaGetLastError());
   return KM_OK;
+}
+
+uint32_t f32_gather_terms(uint32_t d) {
+  return std::min<uint32_t>(d, F32_GATHER_RUN) + (d + F32_GATHER_RUN - 1) / F32_GATHER_RUN;
 }
 
 km_status launch_refine_gemm(bool v4, int num_sms, const float* X, const float* C, const float* Ct,

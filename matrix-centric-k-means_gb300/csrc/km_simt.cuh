@@ -25,6 +25,7 @@ struct SimtTile {
   static constexpr int LDA = ROWS + 4;
   static constexpr int A_FLOATS = KC * LDA, B_FLOATS = KC * COLS, FLOATS = A_FLOATS + B_FLOATS;
   static constexpr size_t SMEM = 2 * sizeof(float) * (size_t)FLOATS;   // two stages
+  static constexpr size_t TOT_BYTES = sizeof(float) * (size_t)NT * RT * CT;
   static constexpr int NA = (ROWS * KC + 4 * NT - 1) / (4 * NT);       // float4 loads per thread and stage
   static constexpr int NB = (COLS * KC + 4 * NT - 1) / (4 * NT);
   // Column of this thread's j-th accumulator (ascending in j).
@@ -53,9 +54,14 @@ __device__ __forceinline__ float4 simt_load4(const float* row, uint32_t col, uin
 
 // The product over all d coordinates.  rowp(r) / colp(c): the tile's row r / column
 // c as a pointer to d floats, or null past the end.  Ends with a block barrier.
-template <class T, class RowP, class ColP>
+// RUN > 0: every RUN coordinates start a sum of their own, added in order, so that an
+// accumulator's rounding errors are those of a chain of RUN + d / RUN operations
+// (simt_chain) instead of d.  The sums so far are kept in shared memory (tot,
+// T::TOT_BYTES), which a run of 64 visits for an eighth of the product's own reads.
+template <class T, int RUN = 0, class RowP, class ColP>
 __device__ __forceinline__ void simt_product(float* smem, uint32_t d, bool v4, RowP rowp, ColP colp,
-                                             float2 (&acc)[T::RT / 2][T::CT]) {
+                                             float2 (&acc)[T::RT / 2][T::CT], float4* tot = nullptr) {
+  static_assert(RUN % T::KC == 0 && T::CT % 2 == 0, "whole stages; pairs of accumulators");
   const int tid = threadIdx.x, tx = tid % T::TX, ty = tid / T::TX;
   constexpr int QR = T::KC / 4;                            // float4 per row and stage
   const uint32_t nk = (d + T::KC - 1) / T::KC;
@@ -156,6 +162,28 @@ __device__ __forceinline__ void simt_product(float* smem, uint32_t d, bool v4, R
       multiply(1);
     }
     if (kt + 1 < nk) sstore((kt + 1) & 1u);
+    if constexpr (RUN > 0) {                               // (a thread's own slots: no barrier)
+      const bool end = kt + 1 == nk;
+      if (end ? nk > RUN / T::KC : (kt + 1) % (RUN / T::KC) == 0) {
+        const bool first = kt < RUN / T::KC;
+#pragma unroll
+        for (int i = 0; i < T::RT / 2; ++i)
+#pragma unroll
+          for (int j = 0; j < T::CT; j += 2) {
+            float4* const t = tot + (i * (T::CT / 2) + j / 2) * T::NT + tid;
+            float4 v = first ? make_float4(0.0f, 0.0f, 0.0f, 0.0f) : *t;
+            v.x = __fadd_rn(v.x, acc[i][j].x); v.y = __fadd_rn(v.y, acc[i][j].y);
+            v.z = __fadd_rn(v.z, acc[i][j + 1].x); v.w = __fadd_rn(v.w, acc[i][j + 1].y);
+            if (end) {
+              acc[i][j] = make_float2(v.x, v.y);
+              acc[i][j + 1] = make_float2(v.z, v.w);
+            } else {
+              *t = v;
+              acc[i][j] = acc[i][j + 1] = make_float2(0.0f, 0.0f);
+            }
+          }
+      }
+    }
     __syncthreads();
   }
 }

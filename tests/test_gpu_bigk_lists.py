@@ -27,3 +27,20 @@ def test_overflowing_candidate_lists(km, gpu, prec, d, k, n):
     lab, _, refined = km.assign(torch.from_numpy(X).to(gpu), torch.from_numpy(C).to(gpu), prec, want_mindist=True)
     np.testing.assert_array_equal(lab.cpu().numpy().astype(np.uint32), lab_o)
     assert refined > 0
+
+
+@pytest.mark.parametrize("d", [15, 16, 63, 64, 65, 79, 80, 127, 128, 129, 192, 256])
+def test_runs_of_the_fp32_pass(km, gpu, d):
+    """The FP32 pass sums its products in runs of 64 coordinates and narrows its near-tie
+    window accordingly: centroids closer to one another than the window for the whole
+    chain, at the edges of the runs."""
+    import torch
+    rng = np.random.default_rng(d)
+    k, n = 600, 1000
+    base = (rng.standard_normal(d) * 6).astype(np.float32)
+    C = (base + 1e-3 * rng.standard_normal((k, d))).astype(np.float32)
+    X = (base + rng.choice([1e-4, 1e-3, 1e-2], (n, 1)) * rng.standard_normal((n, d))).astype(np.float32)
+    lab_o, md_o = helpers.orc_assign(X, C)
+    lab, _, refined = km.assign(torch.from_numpy(X).to(gpu), torch.from_numpy(C).to(gpu), "bf16x3", want_mindist=True)
+    np.testing.assert_array_equal(lab.cpu().numpy().astype(np.uint32), lab_o)
+    assert refined > 0
