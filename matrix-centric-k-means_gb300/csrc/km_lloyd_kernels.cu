@@ -585,49 +585,6 @@ refine_cands_kernel(const float* __restrict__ X, const float* __restrict__ C, ui
     atomicAdd(&st->refined_total, (unsigned long long)block_rows);
 }
 
-// Reference CPU distance with 16-byte loads (d % 4 == 0 and 16-byte aligned
-// rows): the operation order of cpu_dist, the loads arranged for memory-level
-// parallelism (below).
-__device__ __forceinline__ float4 ldg_nc_v4(const float4* p) {
-  float4 v;
-  asm volatile("ld.global.nc.v4.f32 {%0, %1, %2, %3}, [%4];"
-               : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p));
-  return v;
-}
-__device__ __forceinline__ float cpu_dist_v4(const float* __restrict__ x, const float* __restrict__ c,
-                                                 uint32_t d) {
-  const float4* x4 = reinterpret_cast<const float4*>(x);
-  const float4* c4 = reinterpret_cast<const float4*>(c);
-  const uint32_t d4 = d / 4;
-  float s = 0.0f;
-  auto step = [&](const float4 a, const float4 b) {
-    float t = __fsub_rn(a.x, b.x); s = __fadd_rn(s, __fmul_rn(t, t));
-    t = __fsub_rn(a.y, b.y); s = __fadd_rn(s, __fmul_rn(t, t));
-    t = __fsub_rn(a.z, b.z); s = __fadd_rn(s, __fmul_rn(t, t));
-    t = __fsub_rn(a.w, b.w); s = __fadd_rn(s, __fmul_rn(t, t));
-  };
-  // Groups of four 128-byte lines of each row: the first 16 bytes of all eight
-  // lines are loaded together (eight misses in flight), so the rest of each
-  // line is already in L1 when the ordered chain reaches it.
-  uint32_t q = 0;
-  for (; q + 32 <= d4; q += 32) {
-    float4 a[4], b[4];
-#pragma unroll
-    for (int i = 0; i < 4; ++i) { a[i] = ldg_nc_v4(x4 + q + 8 * i); b[i] = ldg_nc_v4(c4 + q + 8 * i); }
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      step(a[i], b[i]);
-      float4 ra[7], rb[7];
-#pragma unroll
-      for (int r = 0; r < 7; ++r) { ra[r] = __ldg(x4 + q + 8 * i + 1 + r); rb[r] = __ldg(c4 + q + 8 * i + 1 + r); }
-#pragma unroll
-      for (int r = 0; r < 7; ++r) step(ra[r], rb[r]);
-    }
-  }
-  for (; q < d4; ++q) step(x4[q], c4[q]);
-  return s;
-}
-
 // Exact re-score of a group of up to FULL_ROWS rows (row ids rows[0..nr))
 // against all k centroids by one warp: lanes over centroids (eight chains per
 // lane and row), centroids read from the transposed copy Ct (d x k) so that
@@ -1011,10 +968,10 @@ __global__ void full_compact_kernel(DevState* st, RefineQueues rq, uint32_t* __r
   }
 }
 
-// Exact re-score of rows with 5..L candidates (chunked distance kernel): one
-// warp per row, lanes stride over the row's candidates, the reference's CPU
-// distance; smallest distance wins, lowest index on ties.
-template <bool V4>
+// Exact re-score of rows with 5..L candidates (chunked distance kernel), for rows that are
+// not 16-byte aligned or d % 4 != 0 (refine_wide_staged_kernel below is the vector path):
+// one warp per row, lanes stride over the row's candidates, the reference's CPU distance;
+// smallest distance wins, lowest index on ties.
 __global__ void __launch_bounds__(256, 2)
 refine_wide_kernel(const float* __restrict__ X, const float* __restrict__ C, uint32_t d,
                    DevState* st, RefineQueues rq, uint32_t* __restrict__ labels,
@@ -1036,8 +993,7 @@ refine_wide_kernel(const float* __restrict__ X, const float* __restrict__ C, uin
       const float* x = X + (uint64_t)row * d;
       for (uint32_t e = (uint32_t)lane; e < nc; e += 32u) {
         const uint32_t c = rq.wl[(uint64_t)row * rq.L + e].x;
-        const float* cc = C + (uint64_t)c * d;
-        const float v = V4 ? cpu_dist_v4(x, cc, d) : cpu_dist(x, cc, d);
+        const float v = cpu_dist(x, C + (uint64_t)c * d, d);
         if (v < bv || (v == bv && c < bi)) { bv = v; bi = c; }
       }
       for (int o = 16; o > 0; o >>= 1) {
@@ -1046,6 +1002,140 @@ refine_wide_kernel(const float* __restrict__ X, const float* __restrict__ C, uin
         if (ov < bv || (ov == bv && oi < bi)) { bv = ov; bi = oi; }
       }
       if (lane == 0) {
+        labels[row] = (bi == 0xffffffffu) ? 0u : bi;
+        if (mindist) mindist[row] = bv;
+      }
+    }
+  }
+  if (count && lane == 0 && done_rows) atomicAdd(&st->refined_total, (unsigned long long)done_rows);
+}
+
+// The same with the operands staged in shared memory by bulk copies, as in
+// refine_staged_kernel (d % 4 == 0, 16-byte aligned rows).  A warp takes a segment's
+// rows (one per lane) and walks their (row, candidate) pairs in passes of up to 32, one
+// pair per lane, of up to RW_ENTRIES rows: a lane's distance joins its row's over the
+// pass by a segmented scan, and the row's lane keeps the best over the passes (a row's
+// candidates can span several).  A lane that reads its candidate's row from global memory
+// itself touches 32 lines per instruction, whose L1 wavefronts set the time; now bound by
+// the copies' bytes out of L2.  n = 4M d = 256 k = 4096 (BF16 points, Zipf sizes): 22.5 ->
+// 10.9 ms an iteration, both queues.
+constexpr int RW_ENTRIES = RS_ROWS - 32;      // point rows of a pass, staged before the candidates'
+__global__ void __launch_bounds__(32 * RS_WARPS, RS_BLOCKS_PER_SM)
+refine_wide_staged_kernel(const float* __restrict__ X, const float* __restrict__ C, uint32_t d, DevState* st,
+                          RefineQueues rq, uint32_t* __restrict__ labels, float* __restrict__ mindist, bool count) {
+  griddep_wait();
+  if (st->done) return;
+  extern __shared__ __align__(16) float rs_smem[];
+  __shared__ __align__(8) uint64_t rw_bar[RS_WARPS];
+  __shared__ int rw_no_abort[RS_WARPS];
+  const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
+  const uint32_t ch = min(d, RS_CH), ld = rs_ld(ch);
+  float* const stg = rs_smem + (size_t)wib * RS_ROWS * ld;
+  uint64_t* const bar = &rw_bar[wib];   // this warp's copies
+  if (lane == 0) {
+    mbar_init(bar, 1);
+    rw_no_abort[wib] = 0;
+    mbar_fence_init();
+  }
+  __syncwarp();
+  uint32_t ph = 0;
+  const uint64_t warp = (uint64_t)blockIdx.x * RS_WARPS + wib, nw = (uint64_t)gridDim.x * RS_WARPS;
+  uint32_t done_rows = 0;
+  auto better = [](float v, uint32_t i, float bv, uint32_t bi) { return v < bv || (v == bv && i < bi); };
+  for (uint64_t g0 = warp; g0 < rq.nseg; g0 += nw * 32) {
+    const uint64_t sgl = g0 + (uint64_t)lane * nw;
+    const uint32_t cl = sgl < rq.nseg ? rq.wcnt[sgl] : 0u;
+    uint32_t nz = __ballot_sync(0xffffffffu, cl != 0u);
+    while (nz) {
+      const int sl = __ffs(nz) - 1;
+      nz &= nz - 1u;
+      const uint64_t seg = g0 + (uint64_t)sl * nw;
+      const uint32_t cnt = __shfl_sync(0xffffffffu, cl, sl);
+      done_rows += cnt;
+      // lane e: row e of the segment, its candidates [incl - nc, incl) of the pairs
+      const bool mine = (uint32_t)lane < cnt;
+      const uint32_t row = mine ? rq.wide[seg * 32 + lane] : 0u;
+      const uint32_t nc = mine ? min(rq.wlc[row], rq.L) : 0u;
+      uint32_t incl = nc;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += y;
+      }
+      const uint32_t total = __shfl_sync(0xffffffffu, incl, 31);
+      float bv = f_inf();
+      uint32_t bi = 0xffffffffu;
+      for (uint32_t p0 = 0; p0 < total;) {
+        const uint32_t p = p0 + (uint32_t)lane;
+        uint32_t e = 0;                          // the pair's row: the lanes whose incl is <= p
+#pragma unroll
+        for (int step = 16; step > 0; step >>= 1) {
+          const uint32_t pv = __shfl_sync(0xffffffffu, incl, (int)(e + (uint32_t)step - 1u));
+          if (pv <= p) e += (uint32_t)step;
+        }
+        const uint32_t first = __shfl_sync(0xffffffffu, e, 0);
+        const uint32_t np = (uint32_t)__popc(__ballot_sync(0xffffffffu, p < total && e - first < (uint32_t)RW_ENTRIES));
+        const uint32_t ne = __shfl_sync(0xffffffffu, e, (int)np - 1) - first + 1u;
+        const bool has = (uint32_t)lane < np;
+        const uint32_t row_e = __shfl_sync(0xffffffffu, row, (int)e);
+        const uint32_t excl_e = __shfl_sync(0xffffffffu, incl - nc, (int)e);
+        const uint32_t cand = has ? rq.wl[(uint64_t)row_e * rq.L + (p - excl_e)].x : 0u;
+        const uint32_t xrow = __shfl_sync(0xffffffffu, row, (int)((first + (uint32_t)lane) & 31u));
+        const float* xp = X + (uint64_t)xrow * d;            // lane < ne
+        const float* cp = C + (uint64_t)cand * d;            // lane < np
+        const float4* xs = reinterpret_cast<const float4*>(stg + (has ? e - first : 0u) * ld);
+        const float4* cs = reinterpret_cast<const float4*>(stg + (RW_ENTRIES + lane) * ld);
+        float s = 0.0f;
+        auto step4 = [&](const float4 a, const float4 b) {
+          float t = __fsub_rn(a.x, b.x); s = __fadd_rn(s, __fmul_rn(t, t));
+          t = __fsub_rn(a.y, b.y); s = __fadd_rn(s, __fmul_rn(t, t));
+          t = __fsub_rn(a.z, b.z); s = __fadd_rn(s, __fmul_rn(t, t));
+          t = __fsub_rn(a.w, b.w); s = __fadd_rn(s, __fmul_rn(t, t));
+        };
+        for (uint32_t j0 = 0; j0 < d; j0 += ch) {
+          const uint32_t cols = min(ch, d - j0), bytes = cols * 4u;
+          // every lane's reads of the rows before were ordered by the barrier below
+          if (lane == 0) mbar_arrive_expect_tx(bar, (np + ne) * bytes);
+          __syncwarp();
+          if ((uint32_t)lane < ne) bulk_copy_g2s(stg + lane * ld, xp + j0, bytes, bar);
+          if (has) bulk_copy_g2s(stg + (RW_ENTRIES + lane) * ld, cp + j0, bytes, bar);
+          const bool okw = mbar_wait_bounded(bar, ph, &rw_no_abort[wib], RS_WAIT_NS);
+          ph ^= 1u;
+          if (!__all_sync(0xffffffffu, okw)) {
+            // copies that never landed: flag, give the ones in flight a bounded
+            // second wait, and end this warp (no block barrier follows)
+            if (lane == 0) atomicOr(&st->err, KM_DEVERR_TIMEOUT);
+            mbar_wait_bounded(bar, ph ^ 1u, &rw_no_abort[wib], RS_WAIT_NS);
+            return;
+          }
+          if (has) {
+            if (cols == RS_CH) {
+#pragma unroll 8
+              for (uint32_t q = 0; q < RS_CH / 4u; ++q) step4(xs[q], cs[q]);
+            } else {
+              for (uint32_t q = 0; q < cols / 4u; ++q) step4(xs[q], cs[q]);
+            }
+          }
+          __syncwarp();   // the rows are restaged only after every lane's chain
+        }
+        // smallest distance per row over the pass, in the row's last lane; a distance
+        // that is not a number is never chosen
+        uint32_t i = has && s == s ? cand : 0xffffffffu;
+        float v = has && s == s ? s : f_inf();
+        const uint32_t key = has ? e : 64u + (uint32_t)lane;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+          const float ov = __shfl_up_sync(0xffffffffu, v, o);
+          const uint32_t oi = __shfl_up_sync(0xffffffffu, i, o), ok = __shfl_up_sync(0xffffffffu, key, o);
+          if (lane >= o && ok == key && better(ov, oi, v, i)) { v = ov; i = oi; }
+        }
+        const uint32_t last = min(incl, p0 + np) - 1u - p0;
+        const float rv = __shfl_sync(0xffffffffu, v, (int)(last & 31u));
+        const uint32_t ri = __shfl_sync(0xffffffffu, i, (int)(last & 31u));
+        if (mine && incl > p0 && incl - nc < p0 + np && better(rv, ri, bv, bi)) { bv = rv; bi = ri; }
+        p0 += np;
+      }
+      if (mine) {
         labels[row] = (bi == 0xffffffffu) ? 0u : bi;
         if (mindist) mindist[row] = bv;
       }
@@ -1068,6 +1158,8 @@ km_status refine_prepare() {
   KM_CUDA_TRY(cudaFuncSetAttribute(refine_staged_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                    (int)RS_SMEM_MAX));
   KM_CUDA_TRY(cudaFuncSetAttribute(refine_staged_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                   (int)RS_SMEM_MAX));
+  KM_CUDA_TRY(cudaFuncSetAttribute(refine_wide_staged_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                    (int)RS_SMEM_MAX));
   return KM_OK;
 }
@@ -1100,8 +1192,11 @@ km_status launch_refine_gemm(bool v4, int num_sms, const float* X, const float* 
                              uint32_t* labels, float* mindist, cudaStream_t s) {
   launch_refine_cands(v4, num_sms, X, C, d, st, rq, labels, mindist, true, s);
   auto wide = [&](const RefineQueues& q, bool count) {
-    if (v4) refine_wide_kernel<true><<<num_sms * 8, 256, 0, s>>>(X, C, d, st, q, labels, mindist, count);
-    else refine_wide_kernel<false><<<num_sms * 8, 256, 0, s>>>(X, C, d, st, q, labels, mindist, count);
+    if (v4)
+      refine_wide_staged_kernel<<<num_sms * RS_BLOCKS_PER_SM, 32 * RS_WARPS,
+                                  (size_t)RS_WARPS * RS_ROWS * rs_ld(std::min(d, RS_CH)) * sizeof(float), s>>>(
+          X, C, d, st, q, labels, mindist, count);
+    else refine_wide_kernel<<<num_sms * 8, 256, 0, s>>>(X, C, d, st, q, labels, mindist, count);
   };
   wide(rq, true);
   // rows of the full queue: FP32 distance pass over all k on those rows alone,

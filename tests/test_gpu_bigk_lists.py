@@ -44,3 +44,24 @@ def test_runs_of_the_fp32_pass(km, gpu, d):
     lab, _, refined = km.assign(torch.from_numpy(X).to(gpu), torch.from_numpy(C).to(gpu), "bf16x3", want_mindist=True)
     np.testing.assert_array_equal(lab.cpu().numpy().astype(np.uint32), lab_o)
     assert refined > 0
+
+
+@pytest.mark.parametrize("d", [4, 5, 12, 64, 124, 128, 132, 200, 256])
+@pytest.mark.parametrize("sizes", [(5,) * 60, (5, 6, 7, 8, 31, 32, 33, 63, 64, 65, 100, 255, 256), (16, 256, 5, 250, 9)])
+def test_wide_rows(km, gpu, d, sizes):
+    """Rows with 5..256 candidates, of groups of equal and of nearly equal centroids, many
+    and few in a segment, over the passes of 32 pairs and of 8 rows."""
+    import torch
+    rng = np.random.default_rng(d + len(sizes))
+    base = (rng.standard_normal((len(sizes), d)) * 5).astype(np.float32)
+    C = np.repeat(base, sizes, axis=0)
+    C = np.where(rng.random((len(C), 1)) < 0.5, C, C + 1e-5 * rng.standard_normal(C.shape)).astype(np.float32)
+    C = C[rng.permutation(len(C))]
+    n = 1500
+    g = rng.integers(0, len(sizes), n)
+    X = (base[g] + 1e-2 * rng.standard_normal((n, d))).astype(np.float32)
+    X[::3] = rng.standard_normal((len(X[::3]), d)) * 5                # rows of other queues between
+    lab_o, md_o = helpers.orc_assign(X, C)
+    lab, md, refined = km.assign(torch.from_numpy(X).to(gpu), torch.from_numpy(C).to(gpu), "bf16x3", want_mindist=True)
+    np.testing.assert_array_equal(lab.cpu().numpy().astype(np.uint32), lab_o)
+    assert refined > 0
