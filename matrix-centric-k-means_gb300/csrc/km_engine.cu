@@ -266,6 +266,7 @@ km_status LloydEngine::init(uint64_t n_, uint32_t d_, uint32_t k_, int precision
     KM_CUDA_TRY(cudaFuncSetAttribute(seg_hist_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, DYN_SMEM_MAX));
     KM_CUDA_TRY(cudaFuncSetAttribute(seg_scatter_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, DYN_SMEM_MAX));
   }
+  one_block_sort = n <= ONE_BLOCK_ROWS && k <= 256;
   KM_TRY(update_sums_prepare());
   if (use == EngineUse::FIT) {
     KM_TRY(take(&Cn, (size_t)k * d));
@@ -441,6 +442,12 @@ km_status LloydEngine::enqueue_finalize(const LoopConsts& lc) {
 }
 
 km_status LloydEngine::enqueue_sort(const uint32_t* lab) {
+  if (one_block_sort) {
+    KM_CUDA_TRY(launch_pdl(one_block_sort_kernel, 1, 1024, 32 * k * sizeof(uint32_t), stream, lab, (uint32_t)n, k, counts,
+                           cstart, order, perm, st));
+    KM_CUDA_TRY(cudaGetLastError());
+    return KM_OK;
+  }
   const unsigned hb = (nseg + sort_wpb - 1) / sort_wpb;
   // programmatic dependent launches: each kernel waits for its predecessor
   // (griddepcontrol.wait) before reading, but is scheduled while it drains

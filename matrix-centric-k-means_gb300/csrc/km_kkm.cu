@@ -1345,6 +1345,7 @@ km_status km_kkm_create(const km_kkm_params* p, km_kkm** out) {
   km_status s = h->eng.init(p->n, p->d, p->k, p->precision, p->device, p->stream, EngineUse::FIT);
   auto fail = [&](km_status st) { km_kkm_destroy(h); return st; };
   if (s != KM_OK) return fail(s);
+  h->eng.one_block_sort = false;               // kkm_kernels_per_iter counts the kernels of the general sort
   if (cudaMalloc(&h->diag, sizeof(float) * p->n) != cudaSuccess ||
       cudaMalloc(&h->E, sizeof(float) * p->n * p->k) != cudaSuccess ||
       cudaMalloc(&h->ct, sizeof(double) * p->k) != cudaSuccess ||

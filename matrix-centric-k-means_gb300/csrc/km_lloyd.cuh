@@ -43,6 +43,9 @@ __global__ void seg_scan_kernel(uint32_t* seghist, uint32_t k, uint32_t nseg, ui
 // order (nullable, k <= 1024): clusters by descending count, ties by index.
 __global__ void cluster_scan_kernel(const uint32_t* counts, uint32_t k, uint32_t* cstart,
                                     DevState* st, uint32_t* order);
+constexpr uint32_t ONE_BLOCK_ROWS = 4096;
+__global__ void one_block_sort_kernel(const uint32_t* labels, uint32_t n, uint32_t k, uint32_t* counts,
+                                      uint32_t* cstart, uint32_t* order, uint32_t* perm, DevState* st);
 __global__ void seg_scatter_kernel(const uint32_t* labels, uint64_t n, uint32_t k, uint32_t seg,
                                    uint32_t nseg, const uint32_t* seghist, const uint32_t* cstart,
                                    uint32_t* perm, DevState* st);
@@ -149,6 +152,7 @@ struct LloydEngine {
   DevState h_one{};           // the mirror of one call
   uint32_t seg = 1024, nseg = 0;
   int sort_wpb = 8;
+  bool one_block_sort = false;    // few rows and clusters: the sort in one launch
   size_t sort_smem = 0;
   RefineQueues rq2{};           // chunked kernel: queues of the FP32 pass over full rows
   RefineEntry* q2 = nullptr;

@@ -1,4 +1,4 @@
-"""Label sort at the edges of its segments (128 to 1024 rows, 1024 segments) and of the
+"""Label sort at the edges of the one-block form (4096 rows, 256 clusters), of its segments (128 to 1024 rows, 1024 segments) and of the
 scan's thread counts: permutation, counts and offsets equal the stable sort's, labels that
 leave clusters empty or fill one included."""
 import numpy as np
@@ -8,7 +8,8 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("n,k", [(1, 1), (2, 2), (127, 5), (128, 5), (129, 128), (1000, 129), (4096, 256), (4097, 257),
-                                 (5000, 1024), (5000, 1025), (20000, 3), (131072, 40), (131073, 40), (140000, 129),
+                                 (5000, 1024), (5000, 1025), (31, 31), (32, 4), (1023, 17), (1024, 33), (1025, 64),
+                                 (4095, 100), (4097, 256), (20000, 3), (131072, 40), (131073, 40), (140000, 129),
                                  (262144, 255), (262145, 7), (300001, 513), (524289, 64), (1049000, 11)])
 @pytest.mark.parametrize("kind", ["uniform", "skewed", "sorted"])
 def test_sort_equals_stable_argsort(km, gpu, n, k, kind):
