@@ -687,14 +687,17 @@ __global__ void kkm_permute_points_kernel(const __nv_bfloat16* __restrict__ Xb,
 // matrix with row0 = 0, or one panel).  Both label sources give the same sums in the
 // same order.
 //
-// Bound by HBM (K is read once).  Four columns are taken together: their bins are
-// read at once and a column whose label one of the others of the four shares takes
-// that one's sum instead, so that the round trip through shared memory is paid once
-// for four columns.  The next batch of loads is in flight while one is summed, and
-// the next row's first while a row's bins are reduced; for that the bins pass through
-// registers into a layout that both sides reach without bank conflicts (a lane
-// walking its cluster's bins in place meets 31 others on the same bank).
-// n = 65,536 k = 64 (17.2 GB): 3.22 -> 2.61 ms = 6.6 TB/s; n = 20,000 k = 20 347 -> 285 us.
+// Bound by HBM (K is read once) in FP32, by the bins' round trips through shared memory
+// in BF16.  The next batch of loads is in flight while one is summed, and the next
+// row's first while a row's bins are reduced; for that the bins pass through registers
+// into a layout that both sides reach without bank conflicts (a lane walking its
+// cluster's bins in place meets 31 others on the same bank).  Rows of n % 4 != 0 come a
+// column a lane, four columns' bins together: one whose label another of the four shares
+// takes that one's sum, so that the round trip is paid once for four (with four columns a
+// lane and load the selects cost more than they save: 2.59 -> 2.49 ms without).
+// An iteration at n = 65,536 k = 64 3.31 -> 2.49 ms (FP32 K, 7 TB/s) and 2.42 -> 2.05 (BF16
+// K), n = 20,000 k = 20 414 -> 286 and 320 -> 243 us, n = 40,001 k = 10 2.30 -> 1.67 ms and
+// 2.52 -> 1.56.
 // ---------------------------------------------------------------------------
 namespace {
 __device__ __forceinline__ float4 ld_stream4(const float* p, bool ok) {
@@ -796,7 +799,7 @@ kkm_vk_kernel(const void* __restrict__ K, uint64_t n, uint32_t k, const uint32_t
   // With n % 4 == 0 every row starts 16-byte (FP32) / 8-byte (BF16) aligned: lane l
   // takes columns 4l..4l+3 of each 128-column stride.  Otherwise one column per lane.
   if ((n & 3) == 0) {
-    constexpr int U = KBF16 ? 12 : 8;                      // loads per lane and batch
+    constexpr int U = KBF16 ? 14 : 8;                      // loads per lane and batch
     constexpr uint64_t S = 128ull * U;                     // columns per batch
     const uint64_t j1 = (uint64_t)lane * 4;
     auto load = [&](V (&v)[U], uint64_t row, uint64_t j) {
@@ -809,8 +812,14 @@ kkm_vk_kernel(const void* __restrict__ K, uint64_t n, uint32_t k, const uint32_t
 #pragma unroll
       for (int u = 0; u < U; ++u) l4[u] = j + 128ull * u < n ? lab4(j + 128ull * u) : 0u;
 #pragma unroll
-      for (int u = 0; u < U; ++u)
-        if (j + 128ull * u < n) bins_add4(B + lane, l4[u], as_float4(v[u]));
+      for (int u = 0; u < U; ++u) {
+        if (j + 128ull * u >= n) break;
+        const float4 x = as_float4(v[u]);
+        B[(l4[u] & 255u) * 32 + lane] += x.x;
+        B[((l4[u] >> 8) & 255u) * 32 + lane] += x.y;
+        B[((l4[u] >> 16) & 255u) * 32 + lane] += x.z;
+        B[(l4[u] >> 24) * 32 + lane] += x.w;
+      }
     };
     V va[U], vb[U];
     load(va, first, j1);
