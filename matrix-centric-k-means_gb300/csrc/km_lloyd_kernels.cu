@@ -366,8 +366,15 @@ assign_f32_kernel(const float* __restrict__ X, const float* __restrict__ C, bool
       float m = mine[i];
 #pragma unroll
       for (int o = 1; o < TX; o <<= 1) m = fminf(m, __shfl_xor_sync(0xffffffffu, m, o));
-      m = fminf(m, rs[r].m);
+      const float before = rs[r].m;
+      m = fminf(m, before);
       const float tau = tie_tau_at(rs[r].tr, m, tb);
+      // every entry so far is at least the minimum before: past tau the list starts
+      // again, overflowed or not (many equal centroids that were the nearest so far)
+      if (c0 != 0u) {
+        if (tx == 0 && before > tau) rs[r].cnt = 0u;
+        __syncwarp();
+      }
       auto val = [&](int j) { return (i & 1) ? acc[i / 2][j].y : acc[i / 2][j].x; };
       if (DOUT && m0 + (uint64_t)r < n_log) {
 #pragma unroll

@@ -28,3 +28,21 @@ def test_f32_labels_at_tile_edges(km, gpu, n, k):
     # fast-path distances: FP32 products of d terms and the cancellation against ||x||^2 + ||c||^2
     scale = (X.astype(np.float64) ** 2).sum(1) + (C.astype(np.float64) ** 2).sum(1).max()
     assert np.all(np.abs(md.cpu().numpy() - md_o) <= 4 * (d + 4) * 2.0 ** -24 * scale)
+
+
+@pytest.mark.parametrize("k", [129, 200, 256, 300])
+def test_f32_lists_start_again_past_equal_centroids(km, gpu, k):
+    """Equal centroids (the zeros of emptied clusters) before a row's own one: they are the
+    nearest so far and fill the row's list, and are left behind without a re-score."""
+    import torch
+    rng = np.random.default_rng(k)
+    d, n = 40, 3000
+    C = (rng.standard_normal((k, d)) * 20).astype(np.float32)
+    C[:30] = 0.0
+    own = rng.integers(k // 2, k, n)
+    X = (C[own] + 0.1 * rng.standard_normal((n, d))).astype(np.float32)
+    lab_o, _ = helpers.orc_assign(X, C)
+    np.testing.assert_array_equal(lab_o, own)
+    lab, _, refined = km.assign(torch.from_numpy(X).to(gpu), torch.from_numpy(C).to(gpu), "fp32", want_mindist=True)
+    np.testing.assert_array_equal(lab.cpu().numpy().astype(np.uint32), lab_o)
+    assert refined == 0
