@@ -248,17 +248,25 @@ __device__ __forceinline__ void pp_tree(const float* xs, int LD, const float* cs
   }
 }
 
-// h + l <- h + l + a + al, an unevaluated FP32 pair (TwoSum): FP64 additions are
-// slow on this GPU.
-__device__ __forceinline__ void pp_pair_add(float& h, float& l, float a, float al) {
-  const float t = __fadd_rn(h, a), bp = __fsub_rn(t, h);
-  const float err = __fadd_rn(__fsub_rn(h, __fsub_rn(t, bp)), __fsub_rn(a, bp));
-  h = t;
-  l = __fadd_rn(l, __fadd_rn(al, err));
+// a + b = s + e without a rounding (TwoSum); s is returned.
+__device__ __forceinline__ float pp_two_sum(float a, float b, float& e) {
+  const float s = __fadd_rn(a, b), bp = __fsub_rn(s, a);
+  e = __fadd_rn(__fsub_rn(a, __fsub_rn(s, bp)), __fsub_rn(b, bp));
+  return s;
 }
 
-// D[j][i] = ||x_i - x_cand_j||^2 and the block's costs sum_i min(d2_i, D[j][i]) (FP32
-// pairs, stored as FP64), d <= PP_TILE_MAX_D: a thread per row for all candidates, the rows staged
+// h + l + m <- h + l + m + a, an unevaluated sum of three FP32 parts: FP64
+// additions are slow on this GPU, and a sum of two parts (48 bits) would hold
+// less than FP64's 53.  Only the additions into m, 2^-48 of the sum, round.
+__device__ __forceinline__ void pp_sum_add(float& h, float& l, float& m, float a) {
+  float e, f;
+  h = pp_two_sum(h, a, e);
+  l = pp_two_sum(l, e, f);
+  m = __fadd_rn(m, f);
+}
+
+// D[j][i] = ||x_i - x_cand_j||^2 and the block's costs sum_i min(d2_i, D[j][i]) (three
+// FP32 parts, rounded once to FP64), d <= PP_TILE_MAX_D: a thread per row for all candidates, the rows staged
 // transposed in shared memory.  Bound by the FP32 pipes (two operations an element
 // and candidate, 31 a row and candidate for the tree) and by reading X.  A warp per
 // row instead spends most of its instructions exchanging partial sums: n = 262,144
@@ -324,12 +332,18 @@ pp_cost_kernel(const float* __restrict__ X, uint64_t n, uint32_t d, bool v4, con
   __syncthreads();
   // a warp per candidate: each lane every 32nd row, then the lanes
   for (uint32_t c = (uint32_t)warp; c < s; c += rows / 32u) {
-    float h = 0.0f, l = 0.0f;
-    for (uint32_t t = (uint32_t)lane; t < rows; t += 32u) pp_pair_add(h, l, mins[c * rows + t], 0.0f);
+    float h = 0.0f, l = 0.0f, m = 0.0f;
+    for (uint32_t t = (uint32_t)lane; t < rows; t += 32u) pp_sum_add(h, l, m, mins[c * rows + t]);
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1)
-      pp_pair_add(h, l, __shfl_xor_sync(0xffffffffu, h, o), __shfl_xor_sync(0xffffffffu, l, o));
-    double t = (double)h + (double)l;
+    for (int o = 16; o > 0; o >>= 1) {
+      const float ho = __shfl_xor_sync(0xffffffffu, h, o), lo = __shfl_xor_sync(0xffffffffu, l, o);
+      const float mo = __shfl_xor_sync(0xffffffffu, m, o);
+      pp_sum_add(h, l, m, ho);
+      float e;
+      l = pp_two_sum(l, lo, e);
+      m = __fadd_rn(m, __fadd_rn(mo, e));
+    }
+    double t = (double)h + ((double)l + (double)m);
     if (__any_sync(0xffffffffu, !isfinite(h))) {     // past the FP32 range: the sum in FP64
       t = 0.0;
       for (uint32_t q = (uint32_t)lane; q < rows; q += 32u) t += (double)mins[c * rows + q];
