@@ -1608,7 +1608,8 @@ update_sums_bulk_kernel(const float* __restrict__ X, const uint32_t* __restrict_
   } else if (objpart) {
     // The objective: lane l on columns 4 (l % 8) .. + 3 of every fourth row
     // (rows l / 8, + 4, ...), 16 bytes a load.  Per batch a lane sums its 32
-    // rows in FP32, across batches as an unevaluated FP32 pair (TwoSum).
+    // rows in FP32, two runs of 16 (the length of a run sets the error of the
+    // whole sum), and the runs as an unevaluated FP32 pair (TwoSum).
     const uint32_t c4 = ((uint32_t)lane & 7u) * 4u, r0 = (uint32_t)lane >> 3;
     const uint64_t p = (uint64_t)c * d + j0 + c4;
     float cold[4];
@@ -1629,8 +1630,8 @@ update_sums_bulk_kernel(const float* __restrict__ X, const uint32_t* __restrict_
       if (!__all_sync(0xffffffffu, ok)) { if (lane == 0) fail(); return; }
       const uint32_t m = min((uint32_t)BLK_ROWS, s1 - (s0 + b * BLK_ROWS));
       const float4* src = reinterpret_cast<const float4*>(ring + ((size_t)s * BLK_ROWS + r0) * BLK_COLS + c4);
-      float2 ea = make_float2(0.0f, 0.0f), eb = ea;
-      auto add = [&](const float4 v) {
+      float2 ea = make_float2(0.0f, 0.0f), eb = ea, fa = ea, fb = ea;
+      auto add = [&](const float4 v, float2& ea, float2& eb) {
         const float2 ta = __fadd2_rn(make_float2(v.x, v.y), ma), tb = __fadd2_rn(make_float2(v.z, v.w), mb);
         ea = __ffma2_rn(ta, ta, ea);
         eb = __ffma2_rn(tb, tb, eb);
@@ -1642,13 +1643,18 @@ update_sums_bulk_kernel(const float* __restrict__ X, const uint32_t* __restrict_
 #pragma unroll
           for (int u = 0; u < 8; ++u) v[u] = src[(u0 + u) * BLK_COLS];
 #pragma unroll
-          for (int u = 0; u < 8; ++u) add(v[u]);
+          for (int u = 0; u < 8; ++u) add(v[u], u & 1 ? fa : ea, u & 1 ? fb : eb);
         }
       } else {
-        for (uint32_t u = 0; r0 + 4u * u < m; ++u) add(src[u * BLK_COLS]);
+        for (uint32_t u = 0; r0 + 4u * u < m; u += 2u) {
+          add(src[u * BLK_COLS], ea, eb);
+          if (r0 + 4u * u + 4u < m) add(src[(u + 1u) * BLK_COLS], fa, fb);
+        }
       }
       two_sum(ha, la, ea);
       two_sum(hb, lb, eb);
+      two_sum(ha, la, fa);
+      two_sum(hb, lb, fb);
       __syncwarp();
       if (lane == 0) mbar_arrive(&empty[s]);
     }
