@@ -46,3 +46,22 @@ def test_f32_lists_start_again_past_equal_centroids(km, gpu, k):
     lab, _, refined = km.assign(torch.from_numpy(X).to(gpu), torch.from_numpy(C).to(gpu), "fp32", want_mindist=True)
     np.testing.assert_array_equal(lab.cpu().numpy().astype(np.uint32), lab_o)
     assert refined == 0
+
+
+@pytest.mark.parametrize("k", [64, 130, 256, 300])
+def test_f32_two_nearest_within_rounding(km, gpu, k):
+    """Rows whose two nearest centroids differ by less than the fast product's rounding, in
+    one tile and across tiles: the reference's label, not the fast value's."""
+    import torch
+    rng = np.random.default_rng(7 * k)
+    d, n = 128, 6000
+    C = rng.uniform(-10, 10, (k, d)).astype(np.float32)
+    a = rng.integers(0, k, n)
+    b = (a + rng.integers(1, k, n)) % k
+    mid = (C[a].astype(np.float64) + C[b]) / 2
+    w = (C[a] - C[b]).astype(np.float64)
+    off = rng.uniform(-1, 1, (n, 1)) * 10.0 ** rng.uniform(-9, -6, (n, 1))
+    X = (mid + off * w).astype(np.float32)
+    lab_o, _ = helpers.orc_assign(X, C)
+    lab, _, _ = km.assign(torch.from_numpy(X).to(gpu), torch.from_numpy(C).to(gpu), "fp32", want_mindist=True)
+    np.testing.assert_array_equal(lab.cpu().numpy().astype(np.uint32), lab_o)
