@@ -270,7 +270,7 @@ __device__ __forceinline__ void pp_sum_add(float& h, float& l, float& m, float a
 // transposed in shared memory.  Bound by the FP32 pipes (two operations an element
 // and candidate, 31 a row and candidate for the tree) and by reading X.  A warp per
 // row instead spends most of its instructions exchanging partial sums: n = 262,144
-// d = 32, 7 candidates 336 us, now 22 us (46 us with FP64 cost sums in every warp).
+// d = 32, 7 candidates 336 us, now 23 us (46 us with FP64 cost sums in every warp).
 template <int S>
 __global__ void __launch_bounds__(256)
 pp_cost_kernel(const float* __restrict__ X, uint64_t n, uint32_t d, bool v4, const int32_t* cand, uint32_t s,
