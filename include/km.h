@@ -109,7 +109,8 @@ typedef struct km_lloyd_params {
   int32_t precision;   /* km_precision */
   int32_t conv;        /* km_conv */
   int32_t device;      /* CUDA device ordinal */
-  void* stream;        /* cudaStream_t, or NULL */
+  void* stream;        /* cudaStream_t, or NULL: a stream of the handle's own, ordered
+                        * after the default stream's work where device memory is passed */
   int32_t empty;       /* km_empty */
 } km_lloyd_params;
 
@@ -187,7 +188,9 @@ km_status km_lloyd_profile(km_lloyd* h, uint64_t iters, double* stage_ms);
 
 void km_lloyd_destroy(km_lloyd* h);
 
-/* ---- Kernel groups on device pointers (stream-ordered, no host sync) ---- */
+/* ---- Kernel groups on device pointers ----
+ * Each call runs on `stream` and has finished when it returns.  NULL: a stream of the
+ * call's own, ordered after the work queued on the default stream. */
 
 /* (a)+(b) Distance stage fused with argmin, plus exact near-tie refinement:
  * labels[i] = argmin_c sum_j (x_ij - c_cj)^2 evaluated as the reference CPU

@@ -137,9 +137,29 @@ LloydEngine::~LloydEngine() {
   }
   if (h_st && h_st != &h_one) cudaFreeHost(h_st);
   if (aux) cudaStreamDestroy(aux);
+  if (ev_default) cudaEventDestroy(ev_default);
   if (ev_fork) cudaEventDestroy(ev_fork);
   if (ev_join) cudaEventDestroy(ev_join);
   if (own_stream && stream) cudaStreamDestroy(stream);
+}
+
+// A caller without a stream makes and uses its device memory on the default stream, which
+// a non-blocking stream does not wait for by itself: its points may still be on their way,
+// and memory handed out for the outputs may still be in use.  The default stream in turn
+// follows every blocking stream, so their work is waited for too.
+km_status LloydEngine::follow_default_stream() {
+  if (!own_stream) return KM_OK;
+  // While a blocking stream is captured, nothing may be queued on the default stream,
+  // by the caller either.
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(cudaStreamLegacy, &cap) != cudaSuccess) {
+    (void)cudaGetLastError();
+    return KM_OK;
+  }
+  if (!ev_default) KM_CUDA_TRY(cudaEventCreateWithFlags(&ev_default, cudaEventDisableTiming));
+  KM_CUDA_TRY(cudaEventRecord(ev_default, cudaStreamLegacy));
+  KM_CUDA_TRY(cudaStreamWaitEvent(stream, ev_default, 0));
+  return KM_OK;
 }
 
 km_status LloydEngine::init(uint64_t n_, uint32_t d_, uint32_t k_, int precision_, int device_,
@@ -163,6 +183,7 @@ km_status LloydEngine::init(uint64_t n_, uint32_t d_, uint32_t k_, int precision
   } else {
     KM_CUDA_TRY(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking));
     own_stream = true;
+    if (use != EngineUse::FIT) KM_TRY(follow_default_stream());   // (a handle's device inputs come later)
   }
   dp = round_up(d, 64);
   kp = round_up(std::max<uint32_t>(k, 16), 16);
@@ -285,6 +306,7 @@ km_status LloydEngine::init(uint64_t n_, uint32_t d_, uint32_t k_, int precision
 
 km_status LloydEngine::set_points(const float* Xsrc, bool on_device, bool copy) {
   KM_CUDA_TRY(cudaSetDevice(device));
+  if (on_device && use == EngineUse::FIT) KM_TRY(follow_default_stream());
   const size_t bytes = sizeof(float) * n * d;
   // A large host source is copied in row chunks alternating between the
   // handle's stream and a second one (two copy engines), and each chunk's
@@ -364,6 +386,7 @@ __global__ void bf16_decode_kernel(const uint16_t* __restrict__ src, uint64_t co
 
 km_status LloydEngine::set_points_bf16(const uint16_t* Xsrc, bool on_device) {
   KM_CUDA_TRY(cudaSetDevice(device));
+  if (on_device) KM_TRY(follow_default_stream());
   if (!X_owned) KM_TRY(take(&X_owned, (size_t)n * d));
   const uint64_t count = n * (uint64_t)d;
   const uint16_t* src = Xsrc;

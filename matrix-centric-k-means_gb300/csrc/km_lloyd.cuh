@@ -111,6 +111,7 @@ struct LloydEngine {
   int device = 0;
   cudaStream_t stream = nullptr;
   bool own_stream = false;
+  cudaEvent_t ev_default = nullptr;   // follow_default_stream
   cudaStream_t aux = nullptr;           // second stream of the chunked host-to-device copy
   cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
   int num_sms = 0;
@@ -182,6 +183,9 @@ struct LloydEngine {
     return KM_OK;
   }
   km_status take_bytes(void** p, size_t bytes);
+  // Orders a stream of the engine's own after the work queued so far on the default
+  // stream, before device memory of a caller who passed no stream is read or written.
+  km_status follow_default_stream();
   km_status set_points(const float* Xsrc, bool on_device, bool copy);
   // Points stored as BF16 (raw bit patterns, n*d): decoded once to the FP32
   // copy, which is then exactly representable in BF16 (Xb = the input).
