@@ -79,6 +79,15 @@ void scratch_trim(int device) {
   }
 }
 
+void scratch_settle(int device, cudaStream_t s) {
+  cudaMemPool_t pool = device_pool(device);
+  uint64_t held = 0;
+  if (pool && cudaMemPoolGetAttribute(pool, cudaMemPoolAttrReservedMemCurrent, &held) == cudaSuccess &&
+      held > SCRATCH_KEEP && cudaStreamSynchronize(s) == cudaSuccess)
+    cudaMemPoolTrimTo(pool, SCRATCH_KEEP);
+  (void)cudaGetLastError();
+}
+
 km_status LloydEngine::take_bytes(void** p, size_t bytes) {
   *p = nullptr;
   if (use != EngineUse::FIT) {
@@ -135,6 +144,7 @@ LloydEngine::~LloydEngine() {
     if (use != EngineUse::FIT) scratch_free(p, device, stream);
     else cudaFree(p);
   }
+  if (use != EngineUse::FIT && !owned.empty()) scratch_settle(device, stream);
   if (h_st && h_st != &h_one) cudaFreeHost(h_st);
   if (aux) cudaStreamDestroy(aux);
   if (ev_default) cudaEventDestroy(ev_default);

@@ -40,8 +40,9 @@ constexpr int DYN_SMEM_MAX = 227 * 1024;
 // Device scratch of one call (stateless entry points, seeding), stream-ordered:
 // a pool of the library's own per device, so that a call neither maps memory nor
 // synchronises the device to give it back.  At most SCRATCH_KEEP bytes stay with
-// the pool between calls, and all of it goes back when an allocation fails for
-// want of memory.  Safe with several threads and streams (the CUDA pool orders
+// the pool when a call returns (scratch_settle; in a fit the synchronisations that
+// follow its seeding release the rest), and all of it goes back when an allocation
+// fails for want of memory.  Safe with several threads and streams (the CUDA pool orders
 // reuse between streams).  Without pool support it falls back to cudaMalloc.
 // Measured, a call: assignment of 65,536 points (d = 64, k = 128) 863 -> 181 us, centroid
 // update of 500,000 (d = 30, k = 100) 1130 -> 179 us (17 to 23 cudaMalloc / cudaFree pairs
@@ -52,6 +53,10 @@ km_status scratch_alloc(void** p, size_t bytes, int device, cudaStream_t s);
 void scratch_free(void* p, int device, cudaStream_t s);
 // Gives the pool's unused memory back (before a retry of a failed allocation).
 void scratch_trim(int device);
+// At the end of a call, its buffers freed on s: memory past SCRATCH_KEEP goes back now.  (By
+// itself the pool gives it back at the next synchronisation after the frees, which may be
+// long in coming: the call's own came before them.)
+void scratch_settle(int device, cudaStream_t s);
 
 // ---------------------------------------------------------------------------
 // Device-resident loop state of one fit.  Every per-iteration kernel reads
