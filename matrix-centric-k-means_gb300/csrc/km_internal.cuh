@@ -51,7 +51,8 @@ constexpr int DYN_SMEM_MAX = 227 * 1024;
 constexpr uint64_t SCRATCH_KEEP = 256ull << 20;
 km_status scratch_alloc(void** p, size_t bytes, int device, cudaStream_t s);
 void scratch_free(void* p, int device, cudaStream_t s);
-// Gives the pool's unused memory back (before a retry of a failed allocation).
+// Gives the pool's unused memory back (before a retry of a failed allocation, and before
+// free memory is counted; cudaMalloc takes it by itself when the device is full).
 void scratch_trim(int device);
 // At the end of a call, its buffers freed on s: memory past SCRATCH_KEEP goes back now.  (By
 // itself the pool gives it back at the next synchronisation after the frees, which may be

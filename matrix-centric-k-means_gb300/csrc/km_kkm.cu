@@ -1374,6 +1374,7 @@ km_status km_kkm_create(const km_kkm_params* p, km_kkm** out) {
     if (!tensor) return fail(KM_ERR_UNSUPPORTED);
     fused = true;
   } else if (p->panel_rows == KM_KKM_PANEL_AUTO) {
+    scratch_trim(h->eng.device);               // what the scratch pool keeps is free for K too
     size_t fr = 0, tot = 0;
     if (cudaMemGetInfo(&fr, &tot) != cudaSuccess) { (void)cudaGetLastError(); return fail(KM_ERR_CUDA); }
     if ((double)nn * bpe > 0.9 * (double)fr) {

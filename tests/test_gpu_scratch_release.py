@@ -1,5 +1,6 @@
 """Scratch memory of the stateless calls: what a call took beyond 256 MiB is back when it
-returns, without anybody's synchronising."""
+returns, without anybody's synchronising, and the rest counts as free where a handle
+chooses its mode by the free memory."""
 import ctypes
 
 import pytest
@@ -46,3 +47,21 @@ def _check_release(km, gpu, call):
     free0 = _free(km)
     big()
     assert free0 - _free(km) <= KEEP + SLACK
+
+
+def _fill_pool(km, gpu):
+    """Leaves between 150 and 256 MiB of scratch with the library."""
+    import torch
+    X = torch.randn(700000, 64, device=gpu)        # two operand copies of 90 MB
+    C = torch.randn(8, 64, device=gpu)
+    km.assign(X, C, "bf16x3")
+    torch.cuda.synchronize()
+    return _free(km)
+
+
+def test_automatic_panel_choice_counts_kept_memory_as_free(km, gpu):
+    free0 = _fill_pool(km, gpu)
+    m = km.KernelKMeans(256, 4, 3, panel_rows="auto", precision="fp32")
+    free1 = _free(km)
+    m.close()
+    assert free1 - free0 >= (150 << 20) - SLACK
