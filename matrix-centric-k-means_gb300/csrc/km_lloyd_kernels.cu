@@ -1609,20 +1609,30 @@ update_sums_bulk_kernel(const float* __restrict__ X, const uint32_t* __restrict_
     // The objective: lane l on columns 4 (l % 8) .. + 3 of every fourth row
     // (rows l / 8, + 4, ...), 16 bytes a load.  Per batch a lane sums its 32
     // rows in FP32, two runs of 16 (the length of a run sets the error of the
-    // whole sum), and the runs as an unevaluated FP32 pair (TwoSum).
+    // whole sum), and the runs as an unevaluated sum of FP32 parts (TwoSum; FP64
+    // additions are slow on this GPU).  Two parts hold 48 bits; rows that are not
+    // 16-byte aligned take three, whose sum holds no less than an FP64 one (n =
+    // 300,007 d = 50 k = 37, 10 iterations: 1555 -> 1581 us for the third).
     const uint32_t c4 = ((uint32_t)lane & 7u) * 4u, r0 = (uint32_t)lane >> 3;
     const uint64_t p = (uint64_t)c * d + j0 + c4;
     float cold[4];
 #pragma unroll
     for (int q = 0; q < 4; ++q) cold[q] = (C && c4 + q < w) ? C[p + q] : 0.0f;
     const float2 ma = make_float2(-cold[0], -cold[1]), mb = make_float2(-cold[2], -cold[3]);
-    float2 ha = make_float2(0.0f, 0.0f), la = ha, hb = ha, lb = ha;   // pairs hi + lo of columns 0,1 and 2,3
+    // parts h + l (+ g) of columns 0,1 (a) and 2,3 (b)
+    float2 ha = make_float2(0.0f, 0.0f), la = ha, ga = ha, hb = ha, lb = ha, gb = ha;
     auto neg = [](float2 v) { return make_float2(-v.x, -v.y); };
-    // TwoSum: h + g = s + err exactly; err accumulates into l
-    auto two_sum = [&](float2& h, float2& l, float2 g) {
-      const float2 s_ = __fadd2_rn(h, g), bb = __fadd2_rn(s_, neg(h));
-      l = __fadd2_rn(l, __fadd2_rn(__fadd2_rn(h, neg(__fadd2_rn(s_, neg(bb)))), __fadd2_rn(g, neg(bb))));
+    // TwoSum: h <- the rounded h + v; returns the rounding error
+    auto two_sum = [&](float2& h, float2 v) {
+      const float2 s_ = __fadd2_rn(h, v), bb = __fadd2_rn(s_, neg(h));
+      const float2 err = __fadd2_rn(__fadd2_rn(h, neg(__fadd2_rn(s_, neg(bb)))), __fadd2_rn(v, neg(bb)));
       h = s_;
+      return err;
+    };
+    auto sum_add = [&](float2& h, float2& l, float2& g, float2 v) {
+      const float2 e = two_sum(h, v);
+      if constexpr (VEC == 4) l = __fadd2_rn(l, e);
+      else g = __fadd2_rn(g, two_sum(l, e));
     };
     for (uint32_t b = 0; b < nb; ++b) {
       const uint32_t s = b % BLK_STAGES, ph = (b / BLK_STAGES) & 1u;
@@ -1651,15 +1661,15 @@ update_sums_bulk_kernel(const float* __restrict__ X, const uint32_t* __restrict_
           if (r0 + 4u * u + 4u < m) add(src[(u + 1u) * BLK_COLS], fa, fb);
         }
       }
-      two_sum(ha, la, ea);
-      two_sum(hb, lb, eb);
-      two_sum(ha, la, fa);
-      two_sum(hb, lb, fb);
+      sum_add(ha, la, ga, ea);
+      sum_add(hb, lb, gb, eb);
+      sum_add(ha, la, ga, fa);
+      sum_add(hb, lb, gb, fb);
       __syncwarp();
       if (lane == 0) mbar_arrive(&empty[s]);
     }
-    double o[4] = {(double)ha.x + (double)la.x, (double)ha.y + (double)la.y, (double)hb.x + (double)lb.x,
-                   (double)hb.y + (double)lb.y};
+    double o[4] = {(double)ha.x + ((double)la.x + (double)ga.x), (double)ha.y + ((double)la.y + (double)ga.y),
+                   (double)hb.x + ((double)lb.x + (double)gb.x), (double)hb.y + ((double)lb.y + (double)gb.y)};
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
       o[q] += __shfl_xor_sync(0xffffffffu, o[q], 8);
