@@ -325,7 +325,9 @@ typedef struct km_batch_params {
 typedef struct km_batch_result {
   uint64_t converged_iter;  /* as the reference's run(): converged iteration or maxiter */
   uint64_t iterations;
-  double objective;         /* FP64 sum of the final assignment's distances */
+  double objective;         /* FP64 sum of the final assignment's (float) distances: blocks of 32 rows, each by a
+                             * tree (r with r ^ 16, ^ 8, .. ^ 1), then every 32nd block in turn, then these by
+                             * the tree; the same for every tile variant */
 } km_batch_result;
 
 typedef struct km_batch km_batch;

@@ -37,7 +37,7 @@ struct BatchInst {
   uint64_t xoff;      // floats: first coordinate of the problem's points
   uint64_t loff;      // uint32: first label (and sorted row) of this instance
   uint64_t coff;      // floats: first centroid value of this instance (k*d)
-  uint64_t toff;      // doubles: first tile objective of this instance
+  uint64_t toff;      // doubles: first objective of 32 rows of this instance
   uint32_t n, d, k;
   uint32_t prob, restart;
 };
@@ -129,8 +129,7 @@ extern __shared__ __align__(16) float batch_smem[];
 template <int RT, int TX, int CT>
 __device__ __forceinline__ void batch_tile(const float* __restrict__ Xp, const float* __restrict__ C, uint32_t n,
                                            uint32_t d, uint32_t k, bool v4, uint32_t m0, uint32_t* __restrict__ lab,
-                                           double* __restrict__ objtile, float2 nz) {
-  __shared__ double s_obj[BA_NT / 32];
+                                           double* __restrict__ objblk, float2 nz) {
   float* const smem = batch_smem;
   using T = BatchTile<RT, TX, CT>;
   const int tid = threadIdx.x, tx = tid % TX, ty = tid / TX;
@@ -272,22 +271,26 @@ __device__ __forceinline__ void batch_tile(const float* __restrict__ Xp, const f
     if (h) { row0 += up ? h : 0; live = h; }
   }
   constexpr int LEFT = RT > TX ? RT / TX : 1;              // rows a thread ends with
-  double obj = 0.0;
+  // The objective by blocks of 32 rows, each by one tree over its rows, so that it does
+  // not depend on the tile's height.  (The stages are free: the product ends with a barrier.)
+  float* const dist = smem;
 #pragma unroll
   for (int i = 0; i < LEFT; ++i) {
     const uint32_t row = m0 + (uint32_t)(row0 + i);
-    if ((tx < RT || RT > TX) && row < n) {                 // TX > RT: the lanes above hold copies
-      lab[row] = bi[i];
-      obj += (double)bv[i];
+    if (tx < RT || RT > TX) {                              // TX > RT: the lanes above hold copies
+      dist[row0 + i] = row < n ? bv[i] : 0.0f;
+      if (row < n) lab[row] = bi[i];
     }
   }
-  for (int o = 16; o > 0; o >>= 1) obj += __shfl_xor_sync(0xffffffffu, obj, o);
-  if ((tid & 31) == 0) s_obj[tid >> 5] = obj;
   __syncthreads();
-  if (tid == 0) {
-    double t = 0.0;
-    for (int w = 0; w < BA_NT / 32; ++w) t += s_obj[w];
-    *objtile = t;
+#pragma unroll
+  for (int b = 0; b < T::ROWS / 32; b += BA_NT / 32) {
+    const int blk = b + (tid >> 5);
+    if (blk >= T::ROWS / 32 || m0 + 32u * (uint32_t)blk >= n) break;
+    double o = (double)dist[32 * blk + (tid & 31)];
+#pragma unroll
+    for (int x = 16; x > 0; x >>= 1) o += __shfl_xor_sync(0xffffffffu, o, x);
+    if ((tid & 31) == 0) objblk[blk] = o;
   }
 }
 
@@ -309,7 +312,7 @@ template <int RT, int GROUP>
 __global__ void __launch_bounds__(BA_NT, RT == 8 ? 3 : 4)
 batch_assign_kernel(const float* __restrict__ X, const BatchInst* __restrict__ insts, BatchCtl* ctl,
                     const uint32_t* __restrict__ act, const uint32_t* __restrict__ tile0,
-                    const float* __restrict__ Call, uint32_t* __restrict__ labels, double* __restrict__ objtile,
+                    const float* __restrict__ Call, uint32_t* __restrict__ labels, double* __restrict__ objblk,
                     float neg0) {
   griddep_wait();
   __shared__ uint32_t s_tile;
@@ -323,12 +326,12 @@ batch_assign_kernel(const float* __restrict__ X, const BatchInst* __restrict__ i
     if (t >= end) break;
     const uint32_t a = batch_owner(tile0, nact, t);
     const BatchInst I = insts[act[a]];
-    const uint32_t ti = t - tile0[a], m0 = ti * batch_tile_rows(I.k, RT);
+    const uint32_t m0 = (t - tile0[a]) * batch_tile_rows(I.k, RT);
     const float* Xp = X + I.xoff;
     const float* C = Call + I.coff;
     const bool v4 = (I.d % 4u) == 0u && (I.xoff % 4u) == 0u;
     uint32_t* lab = labels + I.loff;
-    double* ob = objtile + I.toff + ti;
+    double* ob = objblk + I.toff + m0 / 32u;
 #define KM_BATCH_TILE(TX_, CT_) batch_tile<RT, TX_, CT_>(Xp, C, I.n, I.d, I.k, v4, m0, lab, ob, make_float2(neg0, neg0))
     if constexpr (GROUP == 0) {
       if (batch_cols(I.k) == 96u) KM_BATCH_TILE(16, 6); else KM_BATCH_TILE(16, 8);
@@ -605,7 +608,7 @@ batch_begin_kernel(const BatchInst* __restrict__ insts, BatchCtl* ctl, uint32_t*
 __global__ void __launch_bounds__(256)
 batch_stop_kernel(const BatchInst* __restrict__ insts, BatchCtl* ctl, uint32_t* act, uint32_t* tile0, uint32_t* done,
                   float* __restrict__ Call, const float* __restrict__ Cn_all,
-                  const double* __restrict__ objtile, float tol, uint64_t maxiter, uint32_t rt,
+                  const double* __restrict__ objblk, float tol, uint64_t maxiter, uint32_t rt,
                   BatchOut* __restrict__ out) {
   griddep_wait();
   __shared__ int s_moved;
@@ -646,9 +649,15 @@ batch_stop_kernel(const BatchInst* __restrict__ insts, BatchCtl* ctl, uint32_t* 
     for (uint32_t q = tid; q < k * d; q += 256u) C[q] = Cn[q];
     if (stop || iter >= maxiter) {
       if (warp == 0) {
-        const uint32_t nt = batch_tiles(I.n, I.k, rt);
+        const uint32_t nt = (I.n + 31u) / 32u;             // blocks of rows (see batch_tile)
         double o = 0.0;
-        for (uint32_t t = (uint32_t)lane; t < nt; t += 32u) o += objtile[I.toff + t];
+        for (uint32_t t = (uint32_t)lane; t < nt; t += 32u * 8u) {
+          double v[8];
+#pragma unroll
+          for (uint32_t u = 0; u < 8; ++u) v[u] = nt - t > 32u * u ? objblk[I.toff + t + 32u * u] : 0.0;
+#pragma unroll
+          for (uint32_t u = 0; u < 8; ++u) o += v[u];
+        }
         for (int w = 16; w > 0; w >>= 1) o += __shfl_xor_sync(0xffffffffu, o, w);
         if (lane == 0) {
           out[id].converged_iter = stop ? iter : maxiter;
@@ -719,7 +728,7 @@ struct km_batch {
   uint32_t* labels = nullptr;
   uint32_t* perm = nullptr;
   BatchTask* tasks = nullptr;           // long, then short: task_total each
-  double* objtile = nullptr;
+  double* objblk = nullptr;
   BatchInst* dinst = nullptr;
   BatchOut* dout = nullptr;
   BatchCtl* ctl = nullptr;
@@ -731,7 +740,7 @@ struct km_batch {
   ~km_batch() {
     if (device >= 0) cudaSetDevice(device);
     for (void* q : {(void*)X, (void*)C0, (void*)C, (void*)Cn, (void*)labels, (void*)perm, (void*)tasks,
-                    (void*)objtile, (void*)dinst, (void*)dout, (void*)ctl, (void*)lists})
+                    (void*)objblk, (void*)dinst, (void*)dout, (void*)ctl, (void*)lists})
       if (q) cudaFree(q);
     if (h_ctl) cudaFreeHost(h_ctl);
     if (own_stream && stream) cudaStreamDestroy(stream);
@@ -758,7 +767,7 @@ km_status enqueue_batch_iteration(km_batch* h, int ctas, const BatchInst* dinst,
   auto assign = [&](auto kern, int group) -> km_status {
     if (!(h->groups & (1u << group))) return KM_OK;
     KM_CUDA_TRY(launch_pdl(kern, h->num_sms * ctas, BA_NT, batch_assign_smem<RT>(), h->stream, h->X, dinst, h->ctl, act,
-                           tile0, h->C, h->labels, h->objtile, -0.0f));
+                           tile0, h->C, h->labels, h->objblk, -0.0f));
     return KM_OK;
   };
   KM_TRY(assign(batch_assign_kernel<RT, 0>, 0));
@@ -769,7 +778,7 @@ km_status enqueue_batch_iteration(km_batch* h, int ctas, const BatchInst* dinst,
   KM_CUDA_TRY(launch_pdl(batch_update_kernel, h->num_sms * 2, 32 * BU_WARPS, BLK_SMEM, h->stream, h->ctl, longs,
                          shorts));
   KM_CUDA_TRY(launch_pdl(batch_stop_kernel, per_inst, 256, 0, h->stream, dinst, h->ctl, act, tile0, done, h->C, h->Cn,
-                         h->objtile, h->p.tol, maxiter, (uint32_t)RT, h->dout));
+                         h->objblk, h->p.tol, maxiter, (uint32_t)RT, h->dout));
   return KM_OK;
 }
 
@@ -864,7 +873,7 @@ km_status km_batch_create(const km_batch_params* p, const km_batch_problem* prob
     loff += I.n;
     coff += ((uint64_t)I.k * I.d + 3) / 4 * 4;              // 16-byte aligned centroids
     tasks += (uint64_t)I.k * ((I.d + 31) / 32);
-    toff += batch_tiles(I.n, I.k, 4);                       // the smallest tiles of the variants
+    toff += (I.n + 31) / 32;
   }
   h->lab_total = loff;
   h->c_total = coff;
@@ -884,7 +893,7 @@ km_status km_batch_create(const km_batch_params* p, const km_batch_problem* prob
   if (s == KM_OK) s = balloc(&h->labels, h->lab_total);
   if (s == KM_OK) s = balloc(&h->perm, h->lab_total);
   if (s == KM_OK) s = balloc(&h->tasks, 2 * h->task_total);
-  if (s == KM_OK) s = balloc(&h->objtile, h->t_total);
+  if (s == KM_OK) s = balloc(&h->objblk, h->t_total);
   if (s == KM_OK) s = balloc(&h->dinst, inst.size());
   if (s == KM_OK) s = balloc(&h->dout, inst.size());
   if (s == KM_OK) s = balloc(&h->ctl, 1);
