@@ -6,7 +6,8 @@
 // same few launches, whose work items are cut from the instances so that one
 // large instance spreads over the whole GPU (one CTA per instance instead left
 // the GPU waiting for the largest ones: 64 problems x 4 restarts, n 1024..65536,
-// 767 ms, now 88 ms):
+// 776 ms, now 82 ms; batches of small instances only keep that form,
+// batch_small_kernel):
 //   assign   a tile of rows against all centroids of its instance; distances by
 //            the CPU formula sum_j fl((x_j - c_j)^2) in column order (exact, no
 //            bound or refinement needed), strict '<' over centroids in ascending
@@ -29,6 +30,7 @@
 #include <cmath>
 #include <cstring>
 #include <random>
+#include <type_traits>
 #include <vector>
 
 namespace km {
@@ -679,6 +681,275 @@ batch_stop_kernel(const BatchInst* __restrict__ insts, BatchCtl* ctl, uint32_t* 
   if (tid == 0) ctl->iter = iter;
 }
 
+// ---------------------------------------------------------------------------
+// Small instances: a CTA takes one instance at a time and runs all of its iterations,
+// so that a fit is one launch.  The steps are those above, with the same roundings:
+// the centroids live in shared memory (transposed),
+// a warp assigns a contiguous run of rows, one row a lane, counts them by label and
+// scatters them; a thread adds one (cluster, column) in row order.  Bound by latency:
+// five barriers an iteration and the chains of the ordered sums.  (batch_is_small has
+// the line to the tiles, and both sides' times.)
+// ---------------------------------------------------------------------------
+constexpr int SM_NT = 256, SM_WARPS = SM_NT / 32;
+// Centroids side by side in a lane's registers (a row is read once for them all), and the
+// centroids' padding.
+__host__ __device__ constexpr uint32_t small_cg(uint32_t k) { return k <= 8u ? 8u : k <= 16u ? 16u : 32u; }
+__host__ __device__ constexpr uint32_t small_kpad(uint32_t k) { return (k + small_cg(k) - 1u) / small_cg(k) * small_cg(k); }
+
+// The nearest centroids of R rows at once (Cs: d x kpad in shared memory).
+template <int CG, int R>
+__device__ __forceinline__ void small_nearest(const float* const (&x)[R], bool v4, const float* Cs, uint32_t d,
+                                              uint32_t k, uint32_t kpad, uint32_t (&bi)[R]) {
+  float best[R];
+#pragma unroll
+  for (int r = 0; r < R; ++r) { best[r] = f_inf_b(); bi[r] = 0u; }
+  for (uint32_t c0 = 0; c0 < k; c0 += CG) {
+    float acc[R][CG];
+#pragma unroll
+    for (int r = 0; r < R; ++r)
+#pragma unroll
+      for (int c = 0; c < CG; ++c) acc[r][c] = 0.0f;
+    auto add = [&](const float (&xj)[R], uint32_t j) {
+#pragma unroll
+      for (int q = 0; q < CG / 4; ++q) {
+        const float4 v = *reinterpret_cast<const float4*>(Cs + j * kpad + c0 + 4 * q);
+        const float cc[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+        for (int r = 0; r < R; ++r)
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            const float t = __fsub_rn(xj[r], cc[e]);
+            acc[r][4 * q + e] = __fadd_rn(acc[r][4 * q + e], __fmul_rn(t, t));
+          }
+      }
+    };
+    if (v4) {                                              // 16-byte loads: d % 4 == 0, rows aligned
+      for (uint32_t j = 0; j < d; j += 4u) {
+        float4 v[R];
+#pragma unroll
+        for (int r = 0; r < R; ++r) v[r] = __ldg(reinterpret_cast<const float4*>(x[r] + j));
+        float xj[R];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+#pragma unroll
+          for (int r = 0; r < R; ++r) xj[r] = e == 0 ? v[r].x : e == 1 ? v[r].y : e == 2 ? v[r].z : v[r].w;
+          add(xj, j + (uint32_t)e);
+        }
+      }
+    } else {
+#pragma unroll 2
+      for (uint32_t j = 0; j < d; ++j) {
+        float xj[R];
+#pragma unroll
+        for (int r = 0; r < R; ++r) xj[r] = __ldg(x[r] + j);
+        add(xj, j);
+      }
+    }
+#pragma unroll
+    for (int c = 0; c < CG; ++c)
+#pragma unroll
+      for (int r = 0; r < R; ++r)
+        if (c0 + c < k && acc[r][c] < best[r]) { best[r] = acc[r][c]; bi[r] = c0 + c; }
+  }
+}
+
+constexpr uint32_t BATCH_SMALL_SMEM = 64u * 1024u;   // two copies of the centroids at most
+constexpr uint32_t SMALL_WARP_SUMS = 3u * SM_WARPS;
+
+__global__ void __launch_bounds__(SM_NT)
+batch_small_kernel(const float* __restrict__ X, const BatchInst* __restrict__ insts, uint32_t ninst, BatchCtl* ctl,
+                   const float* __restrict__ C0, float* __restrict__ Call, uint32_t* labels, uint32_t* perm_all,
+                   double* objblk, float tol, uint64_t maxiter, BatchOut* __restrict__ out) {
+  __shared__ uint32_t pos[SM_WARPS][256];
+  __shared__ uint32_t cstart[257], part[SM_WARPS];
+  __shared__ uint32_t s_inst;
+  __shared__ int s_moved;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  for (;;) {
+    __syncthreads();                                       // the instance before is done with the shared arrays
+    if (tid == 0) s_inst = atomicAdd(&ctl->next_short, 1u);
+    __syncthreads();
+    const uint32_t id = s_inst;
+    if (id >= ninst) break;
+    const BatchInst I = insts[id];
+    const uint32_t n = I.n, d = I.d, k = I.k, kpad = small_kpad(k);
+    const float* Xp = X + I.xoff;
+    const bool v4 = d % 4u == 0u && I.xoff % 4u == 0u;
+    uint32_t* const lab = labels + I.loff;
+    uint32_t* const perm = perm_all + I.loff;
+    float *Cs = batch_smem, *Cn = batch_smem + d * kpad;
+    for (uint32_t q = tid; q < d * kpad; q += SM_NT) {
+      const uint32_t j = q / kpad, c = q % kpad;
+      Cs[q] = c < k ? C0[I.coff + (uint64_t)c * d + j] : 0.0f;
+    }
+    const uint32_t per = ((n + SM_WARPS - 1) / SM_WARPS + 31u) & ~31u;
+    const uint32_t r0 = min(n, (uint32_t)warp * per), r1 = min(n, r0 + per);
+    uint64_t iter = 0;
+    bool stop = false;
+    while (!stop && iter < maxiter) {
+      ++iter;
+      for (uint32_t c = lane; c < 256u; c += 32u) pos[warp][c] = 0u;
+      __syncthreads();                                     // centroids in place; s_moved has been read
+      if (tid == 0) s_moved = 0;
+      // assign and count, two rows a lane (one where a warp has no more)
+      auto assign = [&](uint32_t g, auto rows) {
+        constexpr int R = rows();
+        const float* x[R];
+        uint32_t bi[R];
+#pragma unroll
+        for (int r = 0; r < R; ++r) x[r] = Xp + (uint64_t)min(g + 32u * r + (uint32_t)lane, n - 1u) * d;
+        if (k <= 8u) small_nearest<8, R>(x, v4, Cs, d, k, kpad, bi);
+        else if (k <= 16u) small_nearest<16, R>(x, v4, Cs, d, k, kpad, bi);
+        else small_nearest<32, R>(x, v4, Cs, d, k, kpad, bi);
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+          const uint32_t row = g + 32u * r + (uint32_t)lane;
+          const unsigned m = __match_any_sync(0xffffffffu, row < r1 ? bi[r] : 0xffffffffu);
+          if (row < r1) {
+            lab[row] = bi[r];
+            if ((m & ((1u << lane) - 1u)) == 0u) pos[warp][bi[r]] += (uint32_t)__popc(m);
+          }
+          __syncwarp();
+        }
+      };
+      for (uint32_t g = r0; g < r1; g += 64u) {
+        if (r1 - g > 32u) assign(g, std::integral_constant<int, 2>{});
+        else assign(g, std::integral_constant<int, 1>{});
+      }
+      __syncthreads();
+      // thread c: cluster c's rows over the warps, scanned over the clusters (k <= 256)
+      uint32_t cnt = 0;
+#pragma unroll
+      for (int w = 0; w < SM_WARPS; ++w) cnt += pos[w][tid];
+      uint32_t inc = cnt;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(0xffffffffu, inc, o);
+        if (lane >= o) inc += y;
+      }
+      if (lane == 31) part[warp] = inc;
+      __syncthreads();
+      uint32_t base = inc - cnt;
+      for (int w = 0; w < warp; ++w) base += part[w];
+      cstart[tid] = base;
+      if (tid == 255) cstart[256] = base + cnt;
+#pragma unroll
+      for (int w = 0; w < SM_WARPS; ++w) {
+        const uint32_t v = pos[w][tid];
+        pos[w][tid] = base;
+        base += v;
+      }
+      __syncthreads();
+      // stable scatter (a lane's own labels, 4 loads in flight)
+      for (uint32_t g0 = r0; g0 < r1; g0 += 128u) {
+        uint32_t lv[4];
+#pragma unroll
+        for (uint32_t q = 0; q < 4u; ++q) {
+          const uint32_t row = g0 + 32u * q + (uint32_t)lane;
+          lv[q] = row < r1 ? lab[row] : 0xffffffffu;
+        }
+#pragma unroll
+        for (uint32_t q = 0; q < 4u; ++q) {
+          if (g0 + 32u * q >= r1) break;
+          const uint32_t row = g0 + 32u * q + (uint32_t)lane, l = lv[q];
+          const unsigned m = __match_any_sync(0xffffffffu, l);
+          const uint32_t rank = (uint32_t)__popc(m & ((1u << lane) - 1u));
+          const uint32_t at = row < r1 ? pos[warp][l] : 0u;
+          __syncwarp();
+          if (row < r1) {
+            perm[at + rank] = row;
+            if (rank == 0u) pos[warp][l] = at + (uint32_t)__popc(m);
+          }
+          __syncwarp();
+        }
+      }
+      __syncthreads();
+      // ordered sums: few of them by a warp each, which loads 32 rows at once and adds
+      // them by shuffles, else a thread each
+      auto put = [&](uint32_t c, uint32_t j, float sum) {
+        const uint32_t count = cstart[c + 1] - cstart[c];
+        Cn[j * kpad + c] = __fmul_rn(sum, (float)(1.0 / (double)(count > 1u ? count : 1u)));
+      };
+      if (k * d <= SMALL_WARP_SUMS && d <= 8u) {
+        for (uint32_t q = (uint32_t)warp; q < k * d; q += SM_WARPS) {
+          const uint32_t c = q / d, j = q % d, p1 = cstart[c + 1];
+          float s = 0.0f, v = 0.0f;
+          uint32_t p = cstart[c] + (uint32_t)lane;
+          if (p < p1) v = __ldg(Xp + (uint64_t)perm[p] * d + j);
+          for (uint32_t p0 = cstart[c]; p0 < p1; p0 += 32u) {
+            p += 32u;
+            const float w = p < p1 ? __ldg(Xp + (uint64_t)perm[p] * d + j) : 0.0f;
+#pragma unroll
+            for (int l = 0; l < 32; ++l) s = __fadd_rn(s, __shfl_sync(0xffffffffu, v, l));   // past the end: + 0
+            v = w;
+          }
+          if (lane == 0) put(c, j, s);
+        }
+      } else {
+        for (uint32_t q = tid; q < k * d; q += SM_NT) {
+          const uint32_t c = q / d, j = q % d, p1 = cstart[c + 1];
+          const float* xj = Xp + j;
+          float s = 0.0f;
+          uint32_t p = cstart[c];
+          for (; p + 8u <= p1; p += 8u) {
+            float v[8];
+#pragma unroll
+            for (uint32_t u = 0; u < 8u; ++u) v[u] = __ldg(xj + (uint64_t)perm[p + u] * d);
+#pragma unroll
+            for (uint32_t u = 0; u < 8u; ++u) s = __fadd_rn(s, v[u]);
+          }
+          for (; p < p1; ++p) s = __fadd_rn(s, __ldg(xj + (uint64_t)perm[p] * d));
+          put(c, j, s);
+        }
+      }
+      __syncthreads();
+      if (iter > 1) {
+        for (uint32_t c = tid; c < k; c += SM_NT) {
+          float s = 0.0f;                                  // column order
+          for (uint32_t j = 0; j < d; ++j) {
+            const float t = __fsub_rn(Cn[j * kpad + c], Cs[j * kpad + c]);
+            s = __fadd_rn(s, __fmul_rn(t, t));
+          }
+          if (sqrtf(s) > tol) s_moved = 1;
+        }
+        __syncthreads();
+        stop = s_moved == 0;
+      }
+      if (stop || iter >= maxiter) {
+        // the objective of this assignment, in the order of batch_tile and the stop kernel
+        for (uint32_t g = r0; g < r1; g += 32u) {
+          const uint32_t row = g + (uint32_t)lane;
+          float s = 0.0f;
+          if (row < r1) {
+            const float* x = Xp + (uint64_t)row * d;
+            const uint32_t c = lab[row];
+            for (uint32_t j = 0; j < d; ++j) {
+              const float t = __fsub_rn(__ldg(x + j), Cs[j * kpad + c]);
+              s = __fadd_rn(s, __fmul_rn(t, t));
+            }
+          }
+          double o = (double)s;
+#pragma unroll
+          for (int x = 16; x > 0; x >>= 1) o += __shfl_xor_sync(0xffffffffu, o, x);
+          if (lane == 0) objblk[I.toff + g / 32u] = o;
+        }
+        for (uint32_t q = tid; q < k * d; q += SM_NT) Call[I.coff + q] = Cn[(q % d) * kpad + q / d];
+        __syncthreads();
+        if (warp == 0) {
+          double o = 0.0;
+          for (uint32_t t = (uint32_t)lane; t < (n + 31u) / 32u; t += 32u) o += objblk[I.toff + t];
+#pragma unroll
+          for (int x = 16; x > 0; x >>= 1) o += __shfl_xor_sync(0xffffffffu, o, x);
+          if (lane == 0) out[id] = BatchOut{stop ? iter : maxiter, iter, o};
+        }
+      }
+      float* const t = Cs;
+      Cs = Cn;
+      Cn = t;
+    }
+  }
+}
+
 // Reference sample picks (kmeans.cpp:22-29, :49-84) on the host copy of X.
 bool host_sample_picks(const float* X, uint64_t n, uint32_t d, uint32_t k, int seed, int32_t* picks) {
   std::seed_seq ss{seed};
@@ -696,6 +967,34 @@ bool host_sample_picks(const float* X, uint64_t n, uint32_t d, uint32_t k, int s
       found = eq;
     }
     if (!found) picks[have++] = p;
+  }
+  return true;
+}
+
+// Whether a CTA an instance wins (every instance has to pass).  An iteration in tiles costs
+// four to six launches, 20 to 30 us, whatever it does; a CTA alone has an SM at most.
+// Few instances, 20 iterations, CTA / tiles: n 2000 d 8 k 32 0.30 / 0.44 ms, n 4000 d 8 k 32
+// 0.55 / 0.56, n 4000 d 1 k 128 0.91 / 0.57, n 30000 d 1 k 2 1.2 / 0.9, n 1000 d 128 k 8
+// 0.78 / 0.61.  With instances enough for every SM (the largest no more than an SM's share
+// of all rows) the CTAs fill the GPU, and what the tiles win by is reading the points
+// fewer times: 152 of n 16000 d 2 k 32 2.5 / 4.1, d 6 k 32 3.8 / 4.8, d 4 k 3 4.1 / 2.0, n
+// 4000 d 32 k 8 1.9 / 1.6.  Rows of up to three columns leave most of a tile empty, which
+// many centroids make felt: 600 of n 65536 d 3 k 32 44 / 82, 152 of d 2 k 3 17 / 10.
+bool batch_is_small(const std::vector<BatchInst>& inst, int num_sms, size_t* smem) {
+  uint64_t rows = 0, top = 0;
+  for (const BatchInst& I : inst) {
+    rows += I.n;
+    top = std::max<uint64_t>(top, I.n);
+  }
+  const bool many = rows >= top * (uint64_t)num_sms;
+  *smem = 0;
+  for (const BatchInst& I : inst) {
+    const uint64_t nd = (uint64_t)I.n * I.d, work = nd * I.k;
+    const bool in = many ? (nd <= (1u << 16) && work <= (1u << 23)) ||
+                               (I.k >= 32u && (I.d <= 3u || (I.d <= 8u && nd <= (1u << 17))))
+                         : nd <= (1u << 15) && work <= 640000u && (uint64_t)I.n * I.k <= (1u << 18) && I.n <= (1u << 13);
+    *smem = std::max(*smem, 2 * sizeof(float) * I.d * small_kpad(I.k));
+    if (!in || *smem > BATCH_SMALL_SMEM) return false;
   }
   return true;
 }
@@ -720,6 +1019,9 @@ struct km_batch {
   cudaStream_t stream = nullptr;
   bool own_stream = false;
   uint32_t groups = 0;                  // groups of assign shapes in use (bit mask)
+  bool small = false;                   // every instance is one CTA's work (batch_small_kernel)
+  size_t small_smem = 0;
+  int small_ctas = 1;                   // of them an SM
   uint64_t x_floats = 0, lab_total = 0, c_total = 0, task_total = 0, t_total = 0;
   float* X = nullptr;
   float* C0 = nullptr;
@@ -782,34 +1084,51 @@ km_status enqueue_batch_iteration(km_batch* h, int ctas, const BatchInst* dinst,
   return KM_OK;
 }
 
-// All iterations of instances [0, ninst) of dinst.
-km_status run_batch(km_batch* h, int v, const BatchInst* dinst, uint32_t ninst, uint64_t maxiter,
-                    float* ms_out) {
+// All iterations of instances [0, ninst) of dinst, a CTA an instance.
+km_status enqueue_batch_small(km_batch* h, const BatchInst* dinst, uint32_t ninst, uint64_t maxiter) {
+  KM_CUDA_TRY(cudaMemsetAsync(h->ctl, 0, sizeof(BatchCtl), h->stream));
+  const unsigned ctas = (unsigned)std::min<uint64_t>(ninst, (uint64_t)h->num_sms * h->small_ctas);
+  batch_small_kernel<<<ctas, SM_NT, h->small_smem, h->stream>>>(h->X, dinst, ninst, h->ctl, h->C0, h->C, h->labels,
+                                                                h->perm, h->objblk, h->p.tol, maxiter, h->dout);
+  KM_CUDA_TRY(cudaGetLastError());
+  return KM_OK;
+}
+
+// The same by tile variant v, all instances an iteration at a time.
+km_status enqueue_batch_tiles(km_batch* h, int v, const BatchInst* dinst, uint32_t ninst, uint64_t maxiter) {
   const BatchVariant& V = kVariants[v];
   const size_t total = h->inst.size();
+  KM_CUDA_TRY(cudaMemcpyAsync(h->C, h->C0, sizeof(float) * h->c_total, cudaMemcpyDeviceToDevice, h->stream));
+  batch_begin_kernel<<<1, 1024, 0, h->stream>>>(dinst, h->ctl, h->lists, h->lists + total, h->lists + 2 * total,
+                                                ninst, (uint32_t)V.rt);
+  KM_CUDA_TRY(cudaGetLastError());
+  // A few iterations are queued between looks at the device's count of
+  // running instances (launches past the end find none and return).
+  uint64_t done = 0, step = 2;
+  while (done < maxiter) {
+    const uint64_t target = std::min<uint64_t>(maxiter, done + step);
+    for (; done < target; ++done)
+      KM_TRY(V.rt == 8 ? enqueue_batch_iteration<8>(h, V.ctas, dinst, ninst, maxiter)
+                       : enqueue_batch_iteration<4>(h, V.ctas, dinst, ninst, maxiter));
+    if (done >= maxiter) break;
+    KM_CUDA_TRY(cudaMemcpyAsync(h->h_ctl, h->ctl, sizeof(BatchCtl), cudaMemcpyDeviceToHost, h->stream));
+    KM_CUDA_TRY(cudaStreamSynchronize(h->stream));
+    if (h->h_ctl->nact == 0u || h->h_ctl->err) break;
+    step = 4;
+  }
+  return KM_OK;
+}
+
+// Runs instances [0, ninst) of dinst to their ends (v: tile variant; SMALL: a CTA an instance).
+constexpr int SMALL = -1;
+km_status run_batch(km_batch* h, int v, const BatchInst* dinst, uint32_t ninst, uint64_t maxiter,
+                    float* ms_out) {
   cudaEvent_t e0, e1;
   KM_CUDA_TRY(cudaEventCreate(&e0));
   if (cudaEventCreate(&e1) != cudaSuccess) { cudaEventDestroy(e0); return KM_ERR_CUDA; }
   auto body = [&]() -> km_status {
     KM_CUDA_TRY(cudaEventRecord(e0, h->stream));
-    KM_CUDA_TRY(cudaMemcpyAsync(h->C, h->C0, sizeof(float) * h->c_total, cudaMemcpyDeviceToDevice, h->stream));
-    batch_begin_kernel<<<1, 1024, 0, h->stream>>>(dinst, h->ctl, h->lists, h->lists + total, h->lists + 2 * total,
-                                                  ninst, (uint32_t)V.rt);
-    KM_CUDA_TRY(cudaGetLastError());
-    // A few iterations are queued between looks at the device's count of
-    // running instances (launches past the end find none and return).
-    uint64_t done = 0, step = 2;
-    while (done < maxiter) {
-      const uint64_t target = std::min<uint64_t>(maxiter, done + step);
-      for (; done < target; ++done)
-        KM_TRY(V.rt == 8 ? enqueue_batch_iteration<8>(h, V.ctas, dinst, ninst, maxiter)
-                         : enqueue_batch_iteration<4>(h, V.ctas, dinst, ninst, maxiter));
-      if (done >= maxiter) break;
-      KM_CUDA_TRY(cudaMemcpyAsync(h->h_ctl, h->ctl, sizeof(BatchCtl), cudaMemcpyDeviceToHost, h->stream));
-      KM_CUDA_TRY(cudaStreamSynchronize(h->stream));
-      if (h->h_ctl->nact == 0u || h->h_ctl->err) break;
-      step = 4;
-    }
+    KM_TRY(v == SMALL ? enqueue_batch_small(h, dinst, ninst, maxiter) : enqueue_batch_tiles(h, v, dinst, ninst, maxiter));
     KM_CUDA_TRY(cudaEventRecord(e1, h->stream));
     KM_CUDA_TRY(cudaMemcpyAsync(h->h_ctl, h->ctl, sizeof(BatchCtl), cudaMemcpyDeviceToHost, h->stream));
     KM_CUDA_TRY(cudaStreamSynchronize(h->stream));
@@ -883,6 +1202,7 @@ km_status km_batch_create(const km_batch_params* p, const km_batch_problem* prob
   km_status s = KM_OK;
   if (cudaSetDevice(h->device) != cudaSuccess) { (void)cudaGetLastError(); delete h; return KM_ERR_CUDA; }
   cudaDeviceGetAttribute(&h->num_sms, cudaDevAttrMultiProcessorCount, h->device);
+  h->small = batch_is_small(inst, h->num_sms, &h->small_smem);
   if (p->stream) h->stream = static_cast<cudaStream_t>(p->stream);
   else if (cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking) == cudaSuccess) h->own_stream = true;
   else { (void)cudaGetLastError(); delete h; return KM_ERR_CUDA; }
@@ -910,7 +1230,11 @@ km_status km_batch_create(const km_batch_params* p, const km_batch_problem* prob
     for (auto kern : {batch_assign_kernel<4, 0>, batch_assign_kernel<4, 1>, batch_assign_kernel<4, 2>})
       if (e == cudaSuccess)
         e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)batch_assign_smem<4>());
-    if (e != cudaSuccess) s = KM_ERR_CUDA;
+    if (e == cudaSuccess)
+      e = cudaFuncSetAttribute(batch_small_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)BATCH_SMALL_SMEM);
+    if (e == cudaSuccess && h->small)
+      e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&h->small_ctas, batch_small_kernel, SM_NT, h->small_smem);
+    if (e != cudaSuccess || h->small_ctas < 1) s = KM_ERR_CUDA;
   }
   if (s != KM_OK) { (void)cudaGetLastError(); delete h; return s; }
   *out = h;
@@ -980,7 +1304,7 @@ km_status km_batch_fit(km_batch* h, km_batch_result* results, uint32_t* best_lab
   if (!h->ready) return KM_ERR_STATE;
   KM_CUDA_TRY(cudaSetDevice(h->device));
   float ms = 0.f;
-  KM_TRY(run_batch(h, h->variant, h->dinst, (uint32_t)h->inst.size(), h->p.maxiter, &ms));
+  KM_TRY(run_batch(h, h->small ? SMALL : h->variant, h->dinst, (uint32_t)h->inst.size(), h->p.maxiter, &ms));
   if (fit_ms) *fit_ms = ms;
   std::vector<BatchOut> out(h->inst.size());
   KM_CUDA_TRY(cudaMemcpy(out.data(), h->dout, sizeof(BatchOut) * out.size(), cudaMemcpyDeviceToHost));
