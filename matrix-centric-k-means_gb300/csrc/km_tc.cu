@@ -419,9 +419,10 @@ struct TcSmemC {
 __host__ __device__ constexpr uint32_t tcc_state_bytes(uint32_t T) { return T * TC_M * 8u; }
 
 // Drops the entries above tau of the list of lane o's row (its lst, cnt and tau),
-// the warp together: the entries kept.  All lanes call.  (Each thread reading its own
-// list, one entry after the other, was half of the kernel's time at n = 4M d = 256
-// k = 4096: 50 -> 25 ms an iteration.)
+// the warp together: the entries kept.  All lanes call.  For the few lists that are about
+// to be overfilled: at n = 4M d = 256 k = 4096, where most are, each thread reading its
+// own list, one entry after the other, was half of the kernel's time (50 -> 25 ms an
+// iteration).
 __device__ __forceinline__ uint32_t tcc_filter(uint2* lst, uint32_t cnt, float tau, int o) {
   const int lane = threadIdx.x & 31;
   uint2* const l = reinterpret_cast<uint2*>(__shfl_sync(0xffffffffu, reinterpret_cast<unsigned long long>(lst), o));
@@ -685,31 +686,39 @@ assign_tc_chunked_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
                 mm[h] |= (vb.y <= tau ? 1u : 0u) << (4 * j4 + 3);
               }
             }
+            const uint32_t col0 = j * NC + pr * 64u;       // global centroid index
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
-              const uint32_t col0 = j * NC + pr * 64u + (uint32_t)h * 32u;     // global centroid index
-              uint32_t mk = collect ? mm[h] : 0u;
-              mk &= (col0 >= k) ? 0u : (k - col0 >= 32u ? 0xffffffffu : ((1u << (k - col0)) - 1u));
-              // lists that these entries would overfill: drop the entries of earlier
-              // chunks that the current tau excludes (the warp together, a row at a time)
-              unsigned tight = __ballot_sync(0xffffffffu, cnt != TCC_OVF && cnt + (uint32_t)__popc(mk) > rq.L);
+              const uint32_t ch = col0 + (uint32_t)h * 32u;
+              mm[h] &= !collect || ch >= k ? 0u : (k - ch >= 32u ? 0xffffffffu : ((1u << (k - ch)) - 1u));
+            }
+            // One vote for the pair's 64 columns (most pairs add to no list of the warp): lists
+            // that they would overfill first drop the entries that the current tau excludes (the
+            // warp together, a row at a time); what does not fit even so overflows.
+            const uint32_t more = (uint32_t)(__popc(mm[0]) + __popc(mm[1]));
+            if (__any_sync(0xffffffffu, more != 0u)) {
+              unsigned tight = __ballot_sync(0xffffffffu, cnt != TCC_OVF && cnt + more > rq.L);
               while (tight) {
                 const int o = __ffs(tight) - 1;
                 tight &= tight - 1u;
                 const uint32_t kept = tcc_filter(lst, cnt, tau, o);
                 if (lane == o) cnt = kept;
               }
-              if (cnt != TCC_OVF && cnt + (uint32_t)__popc(mk) > rq.L) cnt = TCC_OVF;
-              while (mk != 0u && cnt != TCC_OVF) {
-                const uint32_t bit = (uint32_t)(__ffs(mk) - 1);
-                mk &= mk - 1u;
-                // the candidate's accumulator by selection (static register indices)
-                uint32_t a = 0u;
+              if (cnt != TCC_OVF && cnt + more > rq.L) cnt = TCC_OVF;
 #pragma unroll
-                for (int jj = 0; jj < 32; ++jj) a = ((uint32_t)jj == bit) ? acc[h * 32 + jj] : a;
-                const float vv = fmaf(-2.0f, __uint_as_float(a), __ldg(cnj + pr * 64u + h * 32u + bit));
-                lst[cnt] = make_uint2(col0 + bit, __float_as_uint(vv));
-                ++cnt;
+              for (int h = 0; h < 2; ++h) {
+                uint32_t mk = mm[h];
+                while (mk != 0u && cnt != TCC_OVF) {
+                  const uint32_t bit = (uint32_t)(__ffs(mk) - 1);
+                  mk &= mk - 1u;
+                  // the candidate's accumulator by selection (static register indices)
+                  uint32_t a = 0u;
+#pragma unroll
+                  for (int jj = 0; jj < 32; ++jj) a = ((uint32_t)jj == bit) ? acc[h * 32 + jj] : a;
+                  const float vv = fmaf(-2.0f, __uint_as_float(a), __ldg(cnj + pr * 64u + h * 32u + bit));
+                  lst[cnt] = make_uint2(col0 + h * 32u + bit, __float_as_uint(vv));
+                  ++cnt;
+                }
               }
               __syncwarp();
             }
@@ -730,27 +739,28 @@ assign_tc_chunked_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
           } else {
             // Final filter with tau(m): keep {c : v(c) <= tau}, compacted in
             // list order; note the first four for the short queue.
-            // Long lists by the warp together, short ones by their own thread.
-            unsigned longs = __ballot_sync(0xffffffffu, cnt != TCC_OVF && cnt > 8u);
-            while (longs) {
-              const int o = __ffs(longs) - 1;
-              longs &= longs - 1u;
-              const uint32_t left = tcc_filter(lst, cnt, tau, o);
-              if (lane == o) cnt = left;
-            }
+            // Each thread its own, eight entries in flight: 32 lists at once, whatever their
+            // lengths.  n = 312,500 d = 256 k = 500 (blobs, split form), distance stage: 291
+            // us one entry at a time, 357 by the warp together a row at a time, 283 so.
             uint32_t kept = 0, c0 = 0, c1 = 0, c2 = 0, c3 = 0;
             if (cnt != TCC_OVF) {
-              const uint32_t look = cnt > 8u ? 4u : cnt;      // a long list is filtered already
-              for (uint32_t e = 0; e < look; ++e) {
-                const uint2 en = lst[e];
-                if (__uint_as_float(en.y) <= tau) {
-                  if (kept != e) lst[kept] = en;
-                  c0 = (kept == 0) ? en.x : c0; c1 = (kept == 1) ? en.x : c1;
-                  c2 = (kept == 2) ? en.x : c2; c3 = (kept == 3) ? en.x : c3;
-                  ++kept;
+              for (uint32_t e0 = 0; e0 < cnt; e0 += 8u) {
+                uint4 v[4];                                // two entries each (lists are 256-byte aligned)
+#pragma unroll
+                for (uint32_t u = 0; u < 4u; ++u)
+                  v[u] = e0 + 2u * u < cnt ? *reinterpret_cast<const uint4*>(lst + e0 + 2u * u) : make_uint4(0u, 0u, 0u, 0u);
+#pragma unroll
+                for (uint32_t u = 0; u < 8u; ++u) {
+                  const uint4 w = v[u / 2u];
+                  const uint2 en = u & 1u ? make_uint2(w.z, w.w) : make_uint2(w.x, w.y);
+                  if (e0 + u < cnt && __uint_as_float(en.y) <= tau) {
+                    if (kept != e0 + u) lst[kept] = en;    // (before e0: read already)
+                    c0 = (kept == 0) ? en.x : c0; c1 = (kept == 1) ? en.x : c1;
+                    c2 = (kept == 2) ? en.x : c2; c3 = (kept == 3) ? en.x : c3;
+                    ++kept;
+                  }
                 }
               }
-              if (cnt > 8u) kept = cnt;
             }
             // NaN leaves kept == 0: full re-score, as does an overflowed list.
             const uint32_t cf = (cnt == TCC_OVF) ? TCC_OVF : kept;
