@@ -80,14 +80,14 @@ km_status sample_init(LloydEngine& e, int seed) {
   int32_t* d_idx = nullptr;
   float* d_rows = nullptr;
   const uint32_t cap = std::max<uint32_t>(64, 2 * e.k + 16);
-  void *q_idx = nullptr, *q_rows = nullptr;
+  Scratch q_idx, q_rows;
   KM_TRY(scratch_alloc(&q_idx, sizeof(int32_t) * cap, e.device, e.stream));
   if (km_status s = scratch_alloc(&q_rows, sizeof(float) * (size_t)cap * e.d, e.device, e.stream)) {
     scratch_free(q_idx, e.device, e.stream);
     return s;
   }
-  d_idx = static_cast<int32_t*>(q_idx);
-  d_rows = static_cast<float*>(q_rows);
+  d_idx = static_cast<int32_t*>(q_idx.p);
+  d_rows = static_cast<float*>(q_rows.p);
   std::vector<int32_t> cand;
   std::vector<float> rows;
   km_status rc = KM_OK;
@@ -119,8 +119,8 @@ km_status sample_init(LloydEngine& e, int seed) {
         cudaStreamSynchronize(e.stream) != cudaSuccess)
       rc = KM_ERR_CUDA;
   }
-  scratch_free(d_idx, e.device, e.stream);
-  scratch_free(d_rows, e.device, e.stream);
+  scratch_free(q_idx, e.device, e.stream);
+  scratch_free(q_rows, e.device, e.stream);
   return rc;
 }
 

@@ -51,25 +51,34 @@ void set_last_error(cudaError_t e, const char* what, const char* file, int line)
 
 const char* last_error_text() { return g_last_error.c_str(); }
 
-km_status scratch_alloc(void** p, size_t bytes, int device, cudaStream_t s) {
-  *p = nullptr;
+km_status scratch_alloc(Scratch* b, size_t bytes, int device, cudaStream_t s) {
+  *b = Scratch{};
   cudaMemPool_t pool = device_pool(device);
+  uint64_t lent = 0;
+  if (pool && (cudaMemPoolGetAttribute(pool, cudaMemPoolAttrUsedMemCurrent, &lent) != cudaSuccess ||
+               lent + bytes > SCRATCH_KEEP)) {
+    (void)cudaGetLastError();
+    pool = nullptr;
+  }
   for (int attempt = 0; attempt < 2; ++attempt) {
-    const cudaError_t e = pool ? cudaMallocFromPoolAsync(p, bytes, pool, s) : cudaMalloc(p, bytes);
-    if (e == cudaSuccess) return KM_OK;
+    const cudaError_t e = pool ? cudaMallocFromPoolAsync(&b->p, bytes, pool, s) : cudaMalloc(&b->p, bytes);
+    if (e == cudaSuccess) {
+      b->pooled = pool != nullptr;
+      return KM_OK;
+    }
     set_last_error(e, "scratch allocation", __FILE__, __LINE__);
     (void)cudaGetLastError();
-    *p = nullptr;
+    b->p = nullptr;
     if (e != cudaErrorMemoryAllocation) return KM_ERR_CUDA;
     scratch_trim(device);
   }
   return KM_ERR_ALLOC;
 }
 
-void scratch_free(void* p, int device, cudaStream_t s) {
-  if (!p) return;
-  if (device_pool(device)) cudaFreeAsync(p, s);
-  else cudaFree(p);
+void scratch_free(const Scratch& b, int, cudaStream_t s) {
+  if (!b.p) return;
+  if (b.pooled) cudaFreeAsync(b.p, s);
+  else cudaFree(b.p);                        // (waits for the work that uses it)
 }
 
 void scratch_trim(int device) {
@@ -90,23 +99,24 @@ void scratch_settle(int device, cudaStream_t s) {
 
 km_status LloydEngine::take_bytes(void** p, size_t bytes) {
   *p = nullptr;
+  Scratch b;
   if (use != EngineUse::FIT) {
-    KM_TRY(scratch_alloc(p, bytes, device, stream));
+    KM_TRY(scratch_alloc(&b, bytes, device, stream));
   } else {
-    cudaError_t e = cudaMalloc(p, bytes);
+    cudaError_t e = cudaMalloc(&b.p, bytes);
     if (e == cudaErrorMemoryAllocation) {
       (void)cudaGetLastError();
       scratch_trim(device);
-      e = cudaMalloc(p, bytes);
+      e = cudaMalloc(&b.p, bytes);
     }
     if (e != cudaSuccess) {
       set_last_error(e, "cudaMalloc", __FILE__, __LINE__);
       (void)cudaGetLastError();
-      *p = nullptr;
       return KM_ERR_ALLOC;
     }
   }
-  owned.push_back(*p);
+  owned.push_back(b);
+  *p = b.p;
   return KM_OK;
 }
 
@@ -140,10 +150,7 @@ TieBound make_tie_bound(int precision, uint32_t d, bool a_exact, uint32_t terms)
 
 LloydEngine::~LloydEngine() {
   if (device >= 0) cudaSetDevice(device);
-  for (void* p : owned) {
-    if (use != EngineUse::FIT) scratch_free(p, device, stream);
-    else cudaFree(p);
-  }
+  for (const Scratch& b : owned) scratch_free(b, device, stream);
   if (use != EngineUse::FIT && !owned.empty()) scratch_settle(device, stream);
   if (h_st && h_st != &h_one) cudaFreeHost(h_st);
   if (aux) cudaStreamDestroy(aux);
@@ -401,11 +408,11 @@ km_status LloydEngine::set_points_bf16(const uint16_t* Xsrc, bool on_device) {
   const uint64_t count = n * (uint64_t)d;
   const uint16_t* src = Xsrc;
   uint16_t* tmp = nullptr;
+  Scratch staging;
   if (!on_device) {
     // host BF16 bits go to a staging buffer (half the bytes of the FP32 copy)
-    void* q = nullptr;
-    KM_TRY(scratch_alloc(&q, sizeof(uint16_t) * count, device, stream));
-    tmp = static_cast<uint16_t*>(q);
+    KM_TRY(scratch_alloc(&staging, sizeof(uint16_t) * count, device, stream));
+    tmp = static_cast<uint16_t*>(staging.p);
     KM_CUDA_TRY(cudaMemcpyAsync(tmp, Xsrc, sizeof(uint16_t) * count, cudaMemcpyHostToDevice, stream));
     src = tmp;
   }
@@ -414,7 +421,7 @@ km_status LloydEngine::set_points_bf16(const uint16_t* Xsrc, bool on_device) {
   cudaError_t le = cudaGetLastError();
   if (tmp) {
     cudaError_t se = cudaStreamSynchronize(stream);
-    scratch_free(tmp, device, stream);
+    scratch_free(staging, device, stream);
     KM_CUDA_TRY(le);
     KM_CUDA_TRY(se);
   }

@@ -465,13 +465,13 @@ namespace {
 template <typename T>
 struct DevBuf {
   LloydEngine& e;
+  Scratch b;
   T* p = nullptr;
   explicit DevBuf(LloydEngine& eng) : e(eng) {}
-  ~DevBuf() { scratch_free(p, e.device, e.stream); }
+  ~DevBuf() { scratch_free(b, e.device, e.stream); }
   km_status alloc(size_t count) {
-    void* q = nullptr;
-    KM_TRY(scratch_alloc(&q, sizeof(T) * count, e.device, e.stream));
-    p = static_cast<T*>(q);
+    KM_TRY(scratch_alloc(&b, sizeof(T) * count, e.device, e.stream));
+    p = static_cast<T*>(b.p);
     return KM_OK;
   }
 };

@@ -39,18 +39,26 @@ constexpr int DYN_SMEM_MAX = 227 * 1024;
 // ---------------------------------------------------------------------------
 // Device scratch of one call (stateless entry points, seeding), stream-ordered:
 // a pool of the library's own per device, so that a call neither maps memory nor
-// synchronises the device to give it back.  At most SCRATCH_KEEP bytes stay with
-// the pool when a call returns (scratch_settle; in a fit the synchronisations that
-// follow its seeding release the rest), and all of it goes back when an allocation
-// fails for want of memory.  Safe with several threads and streams (the CUDA pool orders
-// reuse between streams).  Without pool support it falls back to cudaMalloc.
+// synchronises the device to give it back.  The pool lends SCRATCH_KEEP bytes at most and
+// keeps no more when a call returns (scratch_settle; in a fit the synchronisations
+// that follow its seeding do it); what goes beyond comes from cudaMalloc, which maps and
+// unmaps large buffers faster than a pool that has to give them back: 512 MB 524 us a
+// pair by the pool, 436 by cudaMalloc, 2 GB 3737 and 1597, 256 MB kept 4 and 253.  All of
+// the pool goes back when an allocation fails for want of memory.  Safe with several
+// threads and streams (the CUDA pool orders reuse between streams).  Without pool
+// support everything comes from cudaMalloc.
 // Measured, a call: assignment of 65,536 points (d = 64, k = 128) 863 -> 181 us, centroid
-// update of 500,000 (d = 30, k = 100) 1130 -> 179 us (17 to 23 cudaMalloc / cudaFree pairs
-// and a pinned buffer took the difference).
+// update of 500,000 (d = 30, k = 100) 1245 -> 179 us (17 to 23 cudaMalloc / cudaFree pairs
+// and a pinned buffer took the difference); of 1M points against 500 centroids, with 2 GB of
+// candidate lists, 3.99 -> 2.85 ms (5.15 with all of it from the pool).
 // ---------------------------------------------------------------------------
 constexpr uint64_t SCRATCH_KEEP = 256ull << 20;
-km_status scratch_alloc(void** p, size_t bytes, int device, cudaStream_t s);
-void scratch_free(void* p, int device, cudaStream_t s);
+struct Scratch {
+  void* p = nullptr;
+  bool pooled = false;
+};
+km_status scratch_alloc(Scratch* b, size_t bytes, int device, cudaStream_t s);
+void scratch_free(const Scratch& b, int device, cudaStream_t s);
 // Gives the pool's unused memory back (before a retry of a failed allocation, and before
 // free memory is counted; cudaMalloc takes it by itself when the device is full).
 void scratch_trim(int device);

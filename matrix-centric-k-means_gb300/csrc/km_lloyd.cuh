@@ -107,7 +107,7 @@ enum class EngineUse { FIT, ASSIGN, UPDATE, KMAT };
 
 struct LloydEngine {
   EngineUse use = EngineUse::FIT;
-  std::vector<void*> owned;   // every device buffer below
+  std::vector<Scratch> owned;   // every device buffer below
   int device = 0;
   cudaStream_t stream = nullptr;
   bool own_stream = false;
