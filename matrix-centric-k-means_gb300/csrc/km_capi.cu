@@ -129,7 +129,7 @@ km_status sample_init(LloydEngine& e, int seed) {
 km_status round_robin_init(LloydEngine& e) {
   round_robin_labels_kernel<<<(unsigned)((e.n + 255) / 256), 256, 0, e.stream>>>(e.labels, e.n, e.k);
   KM_TRY(e.enqueue_sort(e.labels));
-  return launch_update_sums(e.X, e.perm, e.cstart, e.d, e.k, nullptr, e.C, nullptr, nullptr, e.st,
+  return launch_update_sums(e.X, e.perm, e.cstart, e.n, e.d, e.k, nullptr, e.C, nullptr, nullptr, e.st,
                             e.stream);
 }
 
@@ -459,8 +459,8 @@ km_status km_update(const float* X_dev, const uint32_t* labels_dev, uint64_t n, 
   e.X = X_dev;
   KM_TRY(e.enqueue_sort(labels_dev));
   KM_TRY(e.check_device_error());   // labels >= k are rejected before the sums run
-  KM_TRY(launch_update_sums(X_dev, e.perm, e.cstart, d, k, nullptr, C_dev, nullptr, nullptr, e.st,
-                            e.stream, k <= 1024u ? e.order : nullptr));
+  KM_TRY(launch_update_sums(X_dev, e.perm, e.cstart, n, d, k, nullptr, C_dev, nullptr, nullptr, e.st,
+                            e.stream, e.order));
   if (counts_dev) KM_CUDA_TRY(cudaMemcpyAsync(counts_dev, e.counts, sizeof(uint32_t) * k, cudaMemcpyDeviceToDevice, e.stream));
   if (perm_dev) KM_CUDA_TRY(cudaMemcpyAsync(perm_dev, e.perm, sizeof(uint32_t) * n, cudaMemcpyDeviceToDevice, e.stream));
   if (offsets_dev) KM_CUDA_TRY(cudaMemcpyAsync(offsets_dev, e.cstart, sizeof(uint32_t) * (k + 1), cudaMemcpyDeviceToDevice, e.stream));

@@ -495,7 +495,7 @@ km_status LloydEngine::enqueue_sort(const uint32_t* lab) {
   // per-cluster segment scans; the last block also scans the cluster counts
   const unsigned st_threads = k <= 256 ? 128 : 512;
   KM_CUDA_TRY(launch_pdl(seg_scan_kernel, (k * 32 + st_threads - 1) / st_threads, st_threads, 0, stream, seghist, k, nseg, counts, st,
-                         cstart, k <= 1024u ? order : (uint32_t*)nullptr));
+                         cstart, order));
   KM_CUDA_TRY(launch_pdl(seg_scatter_kernel, hb, sort_wpb * 32, sort_smem, stream, lab, n, k, seg, nseg, seghist,
                          cstart, perm, st));
   KM_CUDA_TRY(cudaGetLastError());
@@ -504,8 +504,7 @@ km_status LloydEngine::enqueue_sort(const uint32_t* lab) {
 
 km_status LloydEngine::enqueue_update_step(float tol) {
   (void)tol;
-  return launch_update_sums(X, perm, cstart, d, k, C, Cn, dsq, objpart, st, stream,
-                            k <= 1024u ? order : nullptr);
+  return launch_update_sums(X, perm, cstart, n, d, k, C, Cn, dsq, objpart, st, stream, order);
 }
 
 km_status LloydEngine::enqueue_iteration(const LoopConsts& lc) {

@@ -1263,9 +1263,14 @@ __global__ void seg_hist_kernel(const uint32_t* __restrict__ labels, uint64_t n,
   }
 }
 
+// Clusters of fewer rows are summed by a warp alone where most are small
+// (launch_update_sums).
+constexpr uint32_t SUMS_WARP_ROWS = 256;
+
 // Exclusive scan of the k counts -> cstart[0..k] (CSR row pointers of V) by one
-// block (any size up to 1024 threads); order (nullable, k <= 1024): clusters by
-// descending count, ties by index.  Counts are read from L2 (other blocks may
+// block (any size up to 1024 threads); order (nullable): clusters by descending count,
+// ties by index, for k <= 1024; above, those of at least SUMS_WARP_ROWS rows first, each
+// part by index.  Counts are read from L2 (other blocks may
 // have written them in the same launch); null: scnt holds them, followed by zeros up to a
 // multiple of 4 (k <= 1024).  sstart (nullable): cstart in shared memory as well.
 __device__ void cluster_scan_block(const uint32_t* counts, uint32_t k, uint32_t* __restrict__ cstart,
@@ -1325,6 +1330,31 @@ __device__ void cluster_scan_block(const uint32_t* counts, uint32_t k, uint32_t*
   }
   if (e == k && b < e) cstart[k] = acc;
   if (k == 0 && threadIdx.x == 0) cstart[0] = 0;
+  if (order && !cached) {
+    uint32_t large = 0;
+    for (uint32_t i = b; i < e; ++i) large += count(i) >= SUMS_WARP_ROWS ? 1u : 0u;
+    __syncthreads();                                 // part has been read
+    if (threadIdx.x < 32u) part[threadIdx.x] = 0u;
+    __syncthreads();
+    uint32_t y = large;                              // inclusive over the warp
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t z = __shfl_up_sync(0xffffffffu, y, o);
+      if (lane >= o) y += z;
+    }
+    if (lane == 31) part[wid] = y;
+    __syncthreads();
+    uint32_t before = 0, all = 0;
+    for (uint32_t w = 0; w < 32u; ++w) {
+      if ((int)w < wid) before += part[w];
+      all += part[w];
+    }
+    before += y - large;                             // large clusters before b
+    for (uint32_t i = b; i < e; ++i) {
+      if (count(i) >= SUMS_WARP_ROWS) order[before++] = i;
+      else order[all + i - before] = i;
+    }
+  }
 }
 
 // One warp per cluster: exclusive scan over its segments, total -> counts.
@@ -1555,7 +1585,7 @@ update_sums_bulk_kernel(const float* __restrict__ X, const uint32_t* __restrict_
                         const uint32_t* __restrict__ cstart, uint32_t d, uint32_t k,
                         const float* __restrict__ C, float* __restrict__ Cn,
                         float* __restrict__ dsq, double* __restrict__ objpart, DevState* st,
-                        const uint32_t* __restrict__ order) {
+                        const uint32_t* __restrict__ order, uint32_t min_rows) {
   constexpr int PROD = blk_producers(VEC);
   griddep_wait();
   if (st && st->done) return;
@@ -1569,6 +1599,7 @@ update_sums_bulk_kernel(const float* __restrict__ X, const uint32_t* __restrict_
   const uint32_t j0 = (blockIdx.x % nblk) * BLK_COLS;
   const uint32_t w = min((uint32_t)BLK_COLS, d - j0);   // columns of this block
   const uint32_t s0 = cstart[c], s1 = cstart[c + 1];
+  if (s1 - s0 < min_rows) return;                       // update_sums_warp_kernel's
   const uint32_t nb = (s1 - s0 + BLK_ROWS - 1) / BLK_ROWS;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (threadIdx.x == 0) {
@@ -1679,6 +1710,95 @@ update_sums_bulk_kernel(const float* __restrict__ X, const uint32_t* __restrict_
   }
 }
 
+// The same for clusters of fewer than max_rows rows: a warp per (cluster, 32 columns), which
+// copies its rows 32 at a time into SW_STAGES buffers of its own and adds them, lane =
+// column.  Rows past the cluster's end zero-fill (adding +0); the objective in FP32 runs of
+// 16 rows, added in FP64.  Bound by latency (four loads one after the other before the
+// first addition), so by the warps an SM holds: sixteen, where the ring holds two
+// clusters whatever their sizes (launch_update_sums has both sides' times; with the rows in
+// registers, a batch ahead, this took two to five times as long).
+constexpr int SW_WARPS = 4, SW_STAGES = 3;
+constexpr size_t SW_SMEM = sizeof(float) * SW_WARPS * SW_STAGES * 32 * 32;
+template <int VEC>
+__global__ void __launch_bounds__(32 * SW_WARPS)
+update_sums_warp_kernel(const float* __restrict__ X, const uint32_t* __restrict__ perm,
+                        const uint32_t* __restrict__ cstart, uint32_t d, uint32_t k, const float* __restrict__ C,
+                        float* __restrict__ Cn, float* __restrict__ dsq, double* __restrict__ objpart, DevState* st,
+                        uint32_t max_rows) {
+  griddep_wait();
+  if (st && st->done) return;
+  extern __shared__ __align__(128) float ring[];        // [SW_WARPS][SW_STAGES][32 rows][32 columns]
+  const uint32_t nblk = (d + BLK_COLS - 1) / BLK_COLS;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const uint64_t task = (uint64_t)blockIdx.x * SW_WARPS + warp;
+  if (task >= (uint64_t)k * nblk) return;
+  const uint32_t c = (uint32_t)(task / nblk), j0 = (uint32_t)(task % nblk) * BLK_COLS;
+  const uint32_t s0 = cstart[c], cnt = cstart[c + 1] - s0;
+  if (cnt >= max_rows) return;
+  const bool in = j0 + (uint32_t)lane < d;
+  const uint64_t p = (uint64_t)c * d + j0 + (uint32_t)lane;
+  const float cold = in && C ? C[p] : 0.0f;
+  float* const buf = ring + (size_t)warp * SW_STAGES * 32 * 32;
+  constexpr uint32_t LPR = 32 / VEC, RPI = VEC;          // lanes per row, rows per copy instruction
+  const uint32_t sub = (uint32_t)lane / LPR, cv = ((uint32_t)lane % LPR) * VEC;
+  const bool has_cols = j0 + cv < d;
+  const float* const x = X + j0 + cv;
+  const uint32_t nb = (cnt + 31u) / 32u;
+  auto index = [&](uint32_t b) { return 32u * b + (uint32_t)lane < cnt ? perm[s0 + 32u * b + lane] : 0u; };
+  auto issue = [&](uint32_t b, uint32_t idx) {           // (a group of copies every time, empty past the end)
+    if (b < nb) {
+      float* dst = buf + (b % SW_STAGES) * 32 * 32 + sub * 32 + cv;
+#pragma unroll
+      for (uint32_t i = 0; i < 32u / RPI; ++i) {
+        const uint32_t u = i * RPI + sub, r = __shfl_sync(0xffffffffu, idx, (int)u);
+        const bool ok = 32u * b + u < cnt && has_cols;
+        cp_async_cols<VEC>(dst + i * RPI * 32, ok ? x + (uint64_t)r * d : X, ok);
+      }
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  float sum = 0.0f;
+  double obj = 0.0;
+  uint32_t idx = index(0), ahead = index(1);
+  issue(0, idx);
+  idx = index(2);
+  issue(1, ahead);
+  for (uint32_t b = 0; b < nb; ++b) {
+    ahead = index(b + 3u);
+    issue(b + 2u, idx);
+    idx = ahead;
+    asm volatile("cp.async.wait_group %0;" ::"n"(SW_STAGES - 1) : "memory");
+    __syncwarp();
+    const float* src = buf + (b % SW_STAGES) * 32 * 32 + lane;
+    const uint32_t m = min(32u, cnt - 32u * b);
+    float v[32];
+#pragma unroll
+    for (uint32_t u = 0; u < 32u; ++u) v[u] = src[u * 32];
+#pragma unroll
+    for (uint32_t u = 0; u < 32u; ++u) sum = __fadd_rn(sum, v[u]);
+    if (objpart) {
+      float e[2] = {0.0f, 0.0f};
+#pragma unroll
+      for (uint32_t u = 0; u < 32u; ++u) {
+        const float t = u < m ? __fsub_rn(v[u], cold) : 0.0f;
+        e[u >> 4] = fmaf(t, t, e[u >> 4]);
+      }
+      obj += (double)e[0];
+      obj += (double)e[1];
+    }
+    __syncwarp();                                        // the stage is filled again in the next step
+  }
+  asm volatile("cp.async.wait_all;" ::: "memory");
+  if (!in) return;
+  const float cn = __fmul_rn(sum, __double2float_rn(1.0 / (double)(cnt > 1u ? cnt : 1u)));
+  Cn[p] = cn;
+  if (dsq) {
+    const float t = __fsub_rn(cn, cold);
+    dsq[p] = __fmul_rn(t, t);
+  }
+  if (objpart) objpart[p] = obj;
+}
+
 // Opt-in shared memory for the ring; called before any capture.
 km_status update_sums_prepare() {
   for (auto kern : {update_sums_bulk_kernel<4>, update_sums_bulk_kernel<2>, update_sums_bulk_kernel<1>})
@@ -1687,16 +1807,32 @@ km_status update_sums_prepare() {
 }
 
 // Rows are copied in the widest pieces whose alignment every row start has
-// (row stride d floats from X): 16 bytes, else 8, else 4.
-km_status launch_update_sums(const float* X, const uint32_t* perm, const uint32_t* cstart, uint32_t d,
+// (row stride d floats from X): 16 bytes, else 8, else 4.  Many clusters of few rows go to
+// a warp each, and the ring takes those above: at most n / SUMS_WARP_ROWS of them, which
+// order lists first.  The ring takes two clusters' column blocks an SM at a time, of 2 us and
+// more each, so it loses as soon as there are more than three rounds of them.  Ring / a warp
+// each: 16-byte rows, n = 160,000 d = 256 k = 20,000 1191 / 191 us, n = 63,500 d = 16 k = 500
+// 12 / 17, n = 400,000 d = 64 k = 2000 (200 a cluster) 60 / 65; 4-byte rows, n = 4M d = 7
+// k = 20,000 441 / 166, n = 200,000 d = 7 k = 1000 30 / 21, n = 3000 d = 7 k = 100 12 / 10.
+km_status launch_update_sums(const float* X, const uint32_t* perm, const uint32_t* cstart, uint64_t n, uint32_t d,
                              uint32_t k, const float* C, float* Cn, float* dsq, double* objpart,
                              DevState* st, cudaStream_t s, const uint32_t* order) {
   const uintptr_t xa = reinterpret_cast<uintptr_t>(X);
   const int vec = (d % 4 == 0 && xa % 16 == 0) ? 4 : (d % 2 == 0 && xa % 8 == 0) ? 2 : 1;
   auto kern = vec == 4 ? update_sums_bulk_kernel<4> : vec == 2 ? update_sums_bulk_kernel<2> : update_sums_bulk_kernel<1>;
-  const uint64_t ctas = (uint64_t)k * ((d + BLK_COLS - 1) / BLK_COLS);
-  KM_CUDA_TRY(launch_pdl(kern, (unsigned)ctas, blk_threads(vec), BLK_SMEM, s, X, perm, cstart, d, k, C, Cn, dsq,
-                         objpart, st, order));
+  const uint32_t nblk = (d + BLK_COLS - 1) / BLK_COLS;
+  const bool many = (uint64_t)k * nblk >= 1000u;
+  const bool few = order && (vec == 4 ? many && n < (uint64_t)k * 128u : n < (uint64_t)k * (many ? 1024u : 128u));
+  const uint32_t limit = !few ? 0u : vec == 4 ? SUMS_WARP_ROWS : 4u * SUMS_WARP_ROWS;
+  if (few) {
+    auto small = vec == 4 ? update_sums_warp_kernel<4> : vec == 2 ? update_sums_warp_kernel<2> : update_sums_warp_kernel<1>;
+    KM_CUDA_TRY(launch_pdl(small, (unsigned)(((uint64_t)k * nblk + SW_WARPS - 1) / SW_WARPS), 32 * SW_WARPS, SW_SMEM, s, X,
+                           perm, cstart, d, k, C, Cn, dsq, objpart, st, limit));
+  }
+  const uint64_t ctas = (few ? std::min<uint64_t>(k, n / SUMS_WARP_ROWS) : (uint64_t)k) * nblk;
+  if (ctas)
+    KM_CUDA_TRY(launch_pdl(kern, (unsigned)ctas, blk_threads(vec), BLK_SMEM, s, X, perm, cstart, d, k, C, Cn, dsq, objpart,
+                           st, order, limit));
   KM_CUDA_TRY(cudaGetLastError());
   return KM_OK;
 }

@@ -117,7 +117,7 @@ extern "C" km_status km_update_noalloc(const float* X_dev, const uint32_t* label
   // A label >= k only sets an error bit: the sort skips such rows, so every
   // permutation slot the sums read was written by this call and the sums stay
   // in bounds.  The status is read once, after all the work.
-  KM_TRY(launch_update_sums(X_dev, perm, cstart, d, k, nullptr, C_dev, nullptr, nullptr, st, s));
+  KM_TRY(launch_update_sums(X_dev, perm, cstart, n, d, k, nullptr, C_dev, nullptr, nullptr, st, s));
   if (counts_dev)
     KM_CUDA_TRY(cudaMemcpyAsync(counts_dev, counts, sizeof(uint32_t) * k, cudaMemcpyDeviceToDevice, s));
   // The one host synchronisation of the call: the error bits of the sort
