@@ -250,14 +250,18 @@ __global__ void prep_centroids_kernel(const float* __restrict__ C, uint32_t k, u
 // the row's running minimum m, and every centroid with v(c) <= tau(m) (tie_tau)
 // goes to the row's list of up to F32_LIST (index, value) pairs in shared memory,
 // which drops the entries above the current tau between tiles.  tau only falls with
-// m, so the entries with v(c) <= tau(m_final) are the whole candidate set: one is the proven argmin, 2..4 go to the short re-score queue,
-// more (or a full list, or values that are not finite) to the full re-score.
+// m, so the entries with v(c) <= tau(m_final) are the whole candidate set: one is the
+// proven argmin, 2..4 go to the short re-score queue, more (or a full list, or values that
+// are not finite) to the full re-score.
 //
 // Bound by the FP32 pipes.  The tile is as wide as k asks (32, 48, 64, 96 or 128
 // centroids), so that k = 64 pays for 64.  Measured, distance kernel: n = 200,000
 // d = 100 k = 64 161 -> 75 us, k = 20 159 -> 55 us, k = 90 162 -> 109 us; n = 1M d =
 // 128 k = 256 1571 -> 1568 us = 22 T FMA/s (16 columns a thread instead, or 16 rows,
-// left eight warps an SM, 44 % of the issue slots used and 21 T).
+// left eight warps an SM, 44 % of the issue slots used and 21 T).  With few coordinates what
+// follows a tile's product counts as much: one lane works out a row's minimum and tau
+// for all (every lane on its own: n = 2M d = 16 k = 1000 2905 us, now 2410; n = 625,000 d =
+// 64 k = 1000 2173 and 2023).
 // ---------------------------------------------------------------------------
 constexpr int F32_NT = 128, F32_RT = 8, F32_LIST = 8;
 constexpr int F32_GATHER_RUN = 64;       // (GATHER) coordinates summed on their own
@@ -266,7 +270,7 @@ using F32Tile = SimtTile<F32_NT, F32_RT, TX, CT, TX == 16 && CT == 8 ? 16 : 8>;
 // Shared memory after the product's stages: per row m, tau's row terms, the
 // squared norm, the list and its length; per column the centroid's squared norm.
 struct F32Row {
-  float m, x2;
+  float m, tau, x2;
   TauRow tr;
   uint32_t cnt;
   uint32_t row;                 // row of X
@@ -360,21 +364,40 @@ assign_f32_kernel(const float* __restrict__ X, const float* __restrict__ C, bool
         mine[2 * i + 1] = fminf(mine[2 * i + 1], acc[i][j].y);
       }
     }
+    // The rows' minima over their TX lanes: each exchange leaves a lane half of the rows it
+    // goes on with, so that a lane ends with one row (lanes of 8 and above with a copy),
+    // whose tau it works out for all.
+    {
+      float red[F32_RT];
+      int own = 0;
+#pragma unroll
+      for (int i = 0; i < F32_RT; ++i) red[i] = mine[i];
+#pragma unroll
+      for (int o = 1, live = F32_RT; o < TX; o <<= 1) {
+        const bool up = (tx & o) != 0;
+        const int h = live / 2;
+#pragma unroll
+        for (int i = 0; i < (h ? h : 1); ++i) {
+          const float give = h ? (up ? red[i] : red[i + h]) : red[i], hold = h && up ? red[i + h] : red[i];
+          red[i] = fminf(hold, __shfl_xor_sync(0xffffffffu, give, o));
+        }
+        if (h) { own += up ? h : 0; live = h; }
+      }
+      if (tx < F32_RT) {
+        F32Row& w = rs[ty * F32_RT + own];
+        const float before = w.m, m = fminf(red[0], before), tau = tie_tau_at(w.tr, m, tb);
+        // every entry so far is at least the minimum before: past tau the list starts
+        // again, overflowed or not (many equal centroids that were the nearest so far)
+        if (before > tau) w.cnt = 0u;
+        w.m = m;
+        w.tau = tau;
+      }
+    }
+    __syncwarp();
 #pragma unroll
     for (int i = 0; i < F32_RT; ++i) {
       const int r = ty * F32_RT + i;
-      float m = mine[i];
-#pragma unroll
-      for (int o = 1; o < TX; o <<= 1) m = fminf(m, __shfl_xor_sync(0xffffffffu, m, o));
-      const float before = rs[r].m;
-      m = fminf(m, before);
-      const float tau = tie_tau_at(rs[r].tr, m, tb);
-      // every entry so far is at least the minimum before: past tau the list starts
-      // again, overflowed or not (many equal centroids that were the nearest so far)
-      if (c0 != 0u) {
-        if (tx == 0 && before > tau) rs[r].cnt = 0u;
-        __syncwarp();
-      }
+      const float tau = rs[r].tau;
       auto val = [&](int j) { return (i & 1) ? acc[i / 2][j].y : acc[i / 2][j].x; };
       if (DOUT && m0 + (uint64_t)r < n_log) {
 #pragma unroll
@@ -401,8 +424,6 @@ assign_f32_kernel(const float* __restrict__ X, const float* __restrict__ C, bool
           }
         }
       }
-      __syncwarp();                                        // the row's threads have read its m
-      if (tx == 0) rs[r].m = m;
     }
     __syncthreads();
     // Lists that another tile might fill drop the entries that m has left behind
