@@ -40,8 +40,7 @@ __global__ void seg_hist_kernel(const uint32_t* labels, uint64_t n, uint32_t k, 
 // work (at most 512 threads per block).
 __global__ void seg_scan_kernel(uint32_t* seghist, uint32_t k, uint32_t nseg, uint32_t* counts,
                                 DevState* st, uint32_t* cstart, uint32_t* order);
-// order (nullable): clusters by descending count, ties by index (k > 1024: only the large
-// ones first).
+// order (nullable): the clusters of at least SUMS_WARP_ROWS rows first.
 __global__ void cluster_scan_kernel(const uint32_t* counts, uint32_t k, uint32_t* cstart,
                                     DevState* st, uint32_t* order);
 constexpr uint32_t ONE_BLOCK_ROWS = 4096;
@@ -89,7 +88,7 @@ km_status update_sums_prepare();
 // Shared-memory limits of the staged re-score and FP32 distance kernels (once
 // per process and device, before their first launch).
 km_status refine_prepare();
-// order (nullable): the clusters' processing order (cluster_scan_kernel's).
+// order (nullable): the clusters' processing order (cluster_scan_block).
 km_status launch_update_sums(const float* X, const uint32_t* perm, const uint32_t* cstart, uint64_t n, uint32_t d,
                              uint32_t k, const float* C, float* Cn, float* dsq, double* objpart,
                              DevState* st, cudaStream_t s, const uint32_t* order = nullptr);

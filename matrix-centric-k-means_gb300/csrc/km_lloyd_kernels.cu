@@ -1290,19 +1290,19 @@ constexpr uint32_t SUMS_WARP_ROWS = 256;
 
 // Exclusive scan of the k counts -> cstart[0..k] (CSR row pointers of V) by one
 // block (any size up to 1024 threads); order (nullable): clusters by descending count,
-// ties by index, for k <= 1024; above, those of at least SUMS_WARP_ROWS rows first, each
-// part by index.  Counts are read from L2 (other blocks may
+// ties by index, if ranked and k <= 1024 (k^2 comparisons); else those of at least
+// SUMS_WARP_ROWS rows first, each part by index.  Counts are read from L2 (other blocks may
 // have written them in the same launch); null: scnt holds them, followed by zeros up to a
 // multiple of 4 (k <= 1024).  sstart (nullable): cstart in shared memory as well.
 __device__ void cluster_scan_block(const uint32_t* counts, uint32_t k, uint32_t* __restrict__ cstart,
                                    uint32_t* __restrict__ order, uint32_t* part, uint32_t* scnt,
-                                   uint32_t* sstart = nullptr) {
+                                   uint32_t* sstart = nullptr, bool ranked = true) {
   const bool cached = k <= 1024u;
   if (cached && counts) {
     for (uint32_t c = threadIdx.x; c < ((k + 3u) & ~3u); c += blockDim.x) scnt[c] = c < k ? __ldcg(counts + c) : 0u;
     __syncthreads();
   }
-  if (order && cached) {
+  if (order && cached && ranked) {
     // largest cluster first, so that the longest ordered sums start first
     for (uint32_t c = threadIdx.x; c < k; c += blockDim.x) {
       const uint32_t v = scnt[c];
@@ -1351,7 +1351,7 @@ __device__ void cluster_scan_block(const uint32_t* counts, uint32_t k, uint32_t*
   }
   if (e == k && b < e) cstart[k] = acc;
   if (k == 0 && threadIdx.x == 0) cstart[0] = 0;
-  if (order && !cached) {
+  if (order && !(cached && ranked)) {
     uint32_t large = 0;
     for (uint32_t i = b; i < e; ++i) large += count(i) >= SUMS_WARP_ROWS ? 1u : 0u;
     __syncthreads();                                 // part has been read
@@ -1436,7 +1436,8 @@ __global__ void __launch_bounds__(512) seg_scan_kernel(uint32_t* __restrict__ se
   if (threadIdx.x == 0) reinterpret_cast<volatile DevState*>(st)->scan_ticket = 0u;
 }
 
-// Single block: cluster_scan_block as a kernel of its own.
+// Single block: cluster_scan_block as a kernel of its own, its order not ranked (for k =
+// 1000 the ranks alone take one block 25 us).
 __global__ void cluster_scan_kernel(const uint32_t* __restrict__ counts, uint32_t k,
                                     uint32_t* __restrict__ cstart, DevState* st,
                                     uint32_t* __restrict__ order) {
@@ -1444,7 +1445,7 @@ __global__ void cluster_scan_kernel(const uint32_t* __restrict__ counts, uint32_
   if (st->done) return;
   __shared__ uint32_t part[32];
   __shared__ __align__(16) uint32_t scnt[1024];
-  cluster_scan_block(counts, k, cstart, order, part, scnt);
+  cluster_scan_block(counts, k, cstart, order, part, scnt, nullptr, false);
 }
 
 // One warp per segment: stable scatter of row ids into perm.

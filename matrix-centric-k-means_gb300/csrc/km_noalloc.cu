@@ -40,7 +40,8 @@ constexpr size_t NA_OFF_STATE = 0;
 constexpr size_t NA_OFF_COUNTS = align256(NA_OFF_STATE + sizeof(DevState));
 constexpr size_t NA_OFF_CSTART = align256(NA_OFF_COUNTS + sizeof(uint32_t) * NA_MAX_K);
 constexpr size_t NA_OFF_SEGHIST = align256(NA_OFF_CSTART + sizeof(uint32_t) * (NA_MAX_K + 1));
-constexpr size_t NA_OFF_PERM = align256(NA_OFF_SEGHIST + sizeof(uint32_t) * NA_MAX_SEGHIST);
+constexpr size_t NA_OFF_ORDER = align256(NA_OFF_SEGHIST + sizeof(uint32_t) * NA_MAX_SEGHIST);
+constexpr size_t NA_OFF_PERM = align256(NA_OFF_ORDER + sizeof(uint32_t) * NA_MAX_K);
 constexpr size_t NA_BYTES = align256(NA_OFF_PERM + sizeof(uint32_t) * NA_MAX_N);
 static_assert(NA_BYTES <= KM_NOALLOC_SCRATCH_BYTES, "scratch layout exceeds the stated size");
 
@@ -94,6 +95,8 @@ extern "C" km_status km_update_noalloc(const float* X_dev, const uint32_t* label
   uint32_t* cstart = reinterpret_cast<uint32_t*>(base + NA_OFF_CSTART);
   uint32_t* seghist = reinterpret_cast<uint32_t*>(base + NA_OFF_SEGHIST);
   uint32_t* perm = reinterpret_cast<uint32_t*>(base + NA_OFF_PERM);
+  // The clusters by size, for the sums of many small ones (without it the ring takes all).
+  uint32_t* order = n < 1024ull * k ? reinterpret_cast<uint32_t*>(base + NA_OFF_ORDER) : nullptr;
 
   // Segments of `seg` rows with k x nseg <= NA_MAX_SEGHIST (as the engine does).
   uint32_t seg = 1024;
@@ -111,13 +114,13 @@ extern "C" km_status km_update_noalloc(const float* X_dev, const uint32_t* label
   const unsigned hb = (nseg + wpb - 1) / wpb;
   seg_hist_kernel<<<hb, wpb * 32, smem, s>>>(labels_dev, n, k, seg, nseg, seghist, st);
   seg_scan_kernel<<<(k * 32 + 255) / 256, 256, 0, s>>>(seghist, k, nseg, counts, st, nullptr, nullptr);
-  cluster_scan_kernel<<<1, 1024, 0, s>>>(counts, k, cstart, st, nullptr);
+  cluster_scan_kernel<<<1, 1024, 0, s>>>(counts, k, cstart, st, order);
   seg_scatter_kernel<<<hb, wpb * 32, smem, s>>>(labels_dev, n, k, seg, nseg, seghist, cstart, perm, st);
   KM_CUDA_TRY(cudaGetLastError());
   // A label >= k only sets an error bit: the sort skips such rows, so every
   // permutation slot the sums read was written by this call and the sums stay
   // in bounds.  The status is read once, after all the work.
-  KM_TRY(launch_update_sums(X_dev, perm, cstart, n, d, k, nullptr, C_dev, nullptr, nullptr, st, s));
+  KM_TRY(launch_update_sums(X_dev, perm, cstart, n, d, k, nullptr, C_dev, nullptr, nullptr, st, s, order));
   if (counts_dev)
     KM_CUDA_TRY(cudaMemcpyAsync(counts_dev, counts, sizeof(uint32_t) * k, cudaMemcpyDeviceToDevice, s));
   // The one host synchronisation of the call: the error bits of the sort

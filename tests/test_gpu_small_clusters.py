@@ -50,3 +50,19 @@ def test_fit_with_small_clusters(km, gpu, k, d):
     _, _, before, _ = helpers.orc_lloyd(X, k, 0.0, 0, 1, C0=base)
     want = ((X.astype(np.float64) - before.astype(np.float64)[got]) ** 2).sum()
     assert abs(r.objective - want) <= 18 * 2.0 ** -24 * want
+
+
+@pytest.mark.parametrize("d", [3, 32, 50])
+@pytest.mark.parametrize("k", [700, 1024])
+def test_noalloc_update_with_small_and_large_clusters(km, gpu, k, d):
+    import torch
+    rng = np.random.default_rng(k - d)
+    lab = _labels(k, rng)
+    X = rng.standard_normal((len(lab), d)).astype(np.float32)
+    Xd, ld = torch.from_numpy(X).to(gpu), torch.from_numpy(lab.astype(np.int32)).to(gpu)
+    C, cnt = torch.empty((k, d), device=gpu), torch.empty(k, dtype=torch.int32, device=gpu)
+    km.check(km.lib().km_update_noalloc(Xd.data_ptr(), ld.data_ptr(), len(lab), d, k, C.data_ptr(), cnt.data_ptr(),
+                                        torch.cuda.current_stream().cuda_stream), "km_update_noalloc")
+    cen_o, _ = helpers.orc_update(X, lab, k)
+    np.testing.assert_array_equal(C.cpu().numpy().view(np.uint32), cen_o.view(np.uint32))
+    np.testing.assert_array_equal(cnt.cpu().numpy().astype(np.uint32), np.bincount(lab, minlength=k))
