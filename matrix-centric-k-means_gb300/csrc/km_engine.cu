@@ -321,6 +321,17 @@ km_status LloydEngine::init(uint64_t n_, uint32_t d_, uint32_t k_, int precision
   return KM_OK;
 }
 
+namespace {
+// Whether p is memory of this device itself.  A copy takes other GPUs' and managed memory
+// as well; a kernel that reads in its place would need access to the other GPU.
+bool on_this_device(const void* p, int device) {
+  cudaPointerAttributes a;
+  const bool ok = cudaPointerGetAttributes(&a, p) == cudaSuccess && a.type == cudaMemoryTypeDevice && a.device == device;
+  (void)cudaGetLastError();
+  return ok;
+}
+}  // namespace
+
 km_status LloydEngine::set_points(const float* Xsrc, bool on_device, bool copy) {
   KM_CUDA_TRY(cudaSetDevice(device));
   if (on_device && use == EngineUse::FIT) KM_TRY(follow_default_stream());
@@ -360,11 +371,13 @@ km_status LloydEngine::set_points(const float* Xsrc, bool on_device, bool copy) 
     KM_CUDA_TRY(cudaEventRecord(ev_join, aux));
     KM_CUDA_TRY(cudaStreamWaitEvent(stream, ev_join, 0));
   } else {
-    // A device-to-device copy is made by the preparation, which reads the points anyway.
+    // A copy within the device is made by the preparation, which reads the points anyway.
+    const bool fused = on_device && copy && on_this_device(Xsrc, device);
     if (!on_device)
       KM_CUDA_TRY(cudaMemcpyAsync(X_owned, Xsrc, bytes, cudaMemcpyHostToDevice, stream));
-    launch_prep_points(on_device ? Xsrc : X, n, d, dp, xn2, xn2d, on_device && copy ? X_owned : nullptr, Xb, Xlo, st,
-                       num_sms, stream);
+    else if (copy && !fused)
+      KM_CUDA_TRY(cudaMemcpyAsync(X_owned, Xsrc, bytes, cudaMemcpyDeviceToDevice, stream));
+    launch_prep_points(fused ? Xsrc : X, n, d, dp, xn2, xn2d, fused ? X_owned : nullptr, Xb, Xlo, st, num_sms, stream);
   }
   KM_CUDA_TRY(cudaGetLastError());
   if (xn2d) {
