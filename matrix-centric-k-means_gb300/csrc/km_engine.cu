@@ -3,6 +3,7 @@
 #include "km_lloyd.cuh"
 
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <cstring>
 #include <mutex>
@@ -17,6 +18,7 @@ constexpr int MAX_DEVICES = 64;
 std::mutex g_pool_mu;
 cudaMemPool_t g_pool[MAX_DEVICES] = {};
 bool g_pool_tried[MAX_DEVICES] = {};
+std::atomic<uint64_t> g_lent[MAX_DEVICES] = {};   // bytes lent by the device's pool
 
 // The device's pool (null: none), made on the first use.
 cudaMemPool_t device_pool(int device) {
@@ -54,31 +56,37 @@ const char* last_error_text() { return g_last_error.c_str(); }
 km_status scratch_alloc(Scratch* b, size_t bytes, int device, cudaStream_t s) {
   *b = Scratch{};
   cudaMemPool_t pool = device_pool(device);
-  uint64_t lent = 0;
-  if (pool && (cudaMemPoolGetAttribute(pool, cudaMemPoolAttrUsedMemCurrent, &lent) != cudaSuccess ||
-               lent + bytes > SCRATCH_KEEP)) {
-    (void)cudaGetLastError();
+  if (pool && g_lent[device].fetch_add(bytes) + bytes > SCRATCH_KEEP) {
+    g_lent[device] -= bytes;
     pool = nullptr;
   }
   for (int attempt = 0; attempt < 2; ++attempt) {
     const cudaError_t e = pool ? cudaMallocFromPoolAsync(&b->p, bytes, pool, s) : cudaMalloc(&b->p, bytes);
     if (e == cudaSuccess) {
-      b->pooled = pool != nullptr;
+      b->lent = pool ? bytes : 0;
       return KM_OK;
     }
     set_last_error(e, "scratch allocation", __FILE__, __LINE__);
     (void)cudaGetLastError();
     b->p = nullptr;
-    if (e != cudaErrorMemoryAllocation) return KM_ERR_CUDA;
+    if (e != cudaErrorMemoryAllocation) {
+      if (pool) g_lent[device] -= bytes;
+      return KM_ERR_CUDA;
+    }
     scratch_trim(device);
   }
+  if (pool) g_lent[device] -= bytes;
   return KM_ERR_ALLOC;
 }
 
-void scratch_free(const Scratch& b, int, cudaStream_t s) {
+void scratch_free(const Scratch& b, int device, cudaStream_t s) {
   if (!b.p) return;
-  if (b.pooled) cudaFreeAsync(b.p, s);
-  else cudaFree(b.p);                        // (waits for the work that uses it)
+  if (b.lent) {
+    cudaFreeAsync(b.p, s);
+    g_lent[device] -= b.lent;
+  } else {
+    cudaFree(b.p);                           // (waits for the work that uses it)
+  }
 }
 
 void scratch_trim(int device) {

@@ -55,7 +55,7 @@ constexpr int DYN_SMEM_MAX = 227 * 1024;
 constexpr uint64_t SCRATCH_KEEP = 256ull << 20;
 struct Scratch {
   void* p = nullptr;
-  bool pooled = false;
+  size_t lent = 0;              // bytes, by the pool; 0: cudaMalloc's
 };
 km_status scratch_alloc(Scratch* b, size_t bytes, int device, cudaStream_t s);
 void scratch_free(const Scratch& b, int device, cudaStream_t s);

@@ -85,8 +85,8 @@ km_status launch_assign_tc(const TcPlan& pl, int mode, const CUtensorMap& tmA,
                            float* Dout, cudaStream_t s);
 
 km_status update_sums_prepare();
-// Shared-memory limits of the staged re-score and FP32 distance kernels (once
-// per process and device, before their first launch).
+// Shared-memory limits of the staged re-score and FP32 distance kernels (set by every
+// engine's init; the same values each time, so safe beside launches).
 km_status refine_prepare();
 // order (nullable): the clusters' processing order (cluster_scan_block).
 km_status launch_update_sums(const float* X, const uint32_t* perm, const uint32_t* cstart, uint64_t n, uint32_t d,

@@ -1,5 +1,5 @@
 // Lloyd k-means kernels for sm_103a: point/centroid preparation, the SIMT FP32
-// distance stage with fused top-3 argmin, exact near-tie refinement, the
+// distance stage with fused candidate lists, exact near-tie refinement, the
 // stable label sort (one-hot V as a label-sorted permutation), the exact
 // centroid update V.X, and the per-iteration finalize kernel (whose last block
 // takes the loop decision).
