@@ -93,3 +93,27 @@ def test_outputs_in_memory_that_the_default_stream_still_uses(km, gpu):
     assert lab.data_ptr() == at
     torch.cuda.synchronize()
     np.testing.assert_array_equal(lab.cpu().numpy(), want)
+
+
+def test_inputs_written_on_a_blocking_stream(km, gpu):
+    """The default stream follows every blocking stream, so a call without a stream does."""
+    import ctypes
+    import torch
+    lib = [line.split()[-1] for line in open("/proc/self/maps") if "libcudart" in line]
+    if not lib:
+        pytest.skip("no shared CUDA runtime in this process")
+    rt, raw = ctypes.CDLL(lib[0]), ctypes.c_void_p()
+    assert rt.cudaStreamCreate(ctypes.byref(raw)) == 0
+    old, new = _data(gpu, 5), _data(gpu, 6)
+    want = _host(CALLS["assign"](km, *new))
+    bufs = [t.clone() for t in old]
+    torch.cuda.synchronize()
+    with torch.cuda.stream(torch.cuda.ExternalStream(raw.value)):
+        _busy()
+        for b, t in zip(bufs, new):
+            b.copy_(t)
+    got = _host(CALLS["assign"](km, *bufs))
+    torch.cuda.synchronize()
+    rt.cudaStreamDestroy(raw)
+    for a, b in zip(want, got):
+        np.testing.assert_array_equal(b, a)
