@@ -6,7 +6,7 @@
 // same few launches, whose work items are cut from the instances so that one
 // large instance spreads over the whole GPU (one CTA per instance instead left
 // the GPU waiting for the largest ones: 64 problems x 4 restarts, n 1024..65536,
-// 776 ms, now 82 ms; batches of small instances only keep that form,
+// 776 ms, now 83 ms; batches of small instances only keep that form,
 // batch_small_kernel):
 //   assign   a tile of rows against all centroids of its instance; distances by
 //            the CPU formula sum_j fl((x_j - c_j)^2) in column order (exact, no
@@ -67,6 +67,7 @@ struct BatchCtl {
   uint32_t nlong, nshort;     // update tasks of at least BATCH_RING_ROWS rows / of fewer
   uint32_t tile_end[3], next_tile[3];   // assign tiles by group of shapes (batch_group)
   uint32_t next_short, ticket;
+  uint32_t epoch;             // of the last iteration whose first assign kernel has waited
   uint32_t err;               // KM_DEVERR_*
 };
 
@@ -128,6 +129,20 @@ constexpr size_t batch_assign_smem() {
 // adjacent), the centroids negated and duplicated (x + (-c) rounds as x - c), both
 // a stage ahead in registers.
 extern __shared__ __align__(16) float batch_smem[];
+
+// Loads of what an earlier kernel wrote and an acquire has made visible: by the ordinary
+// path, which the acquire orders, not the read-only one.
+__device__ __forceinline__ float ld_plain(const float* p) {
+  float v;
+  asm("ld.global.f32 %0, [%1];" : "=f"(v) : "l"(p));
+  return v;
+}
+__device__ __forceinline__ float4 ld_plain(const float4* p) {
+  float4 v;
+  asm("ld.global.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p));
+  return v;
+}
+
 template <int RT, int TX, int CT>
 __device__ __forceinline__ void batch_tile(const float* __restrict__ Xp, const float* __restrict__ C, uint32_t n,
                                            uint32_t d, uint32_t k, bool v4, uint32_t m0, uint32_t* __restrict__ lab,
@@ -148,32 +163,34 @@ __device__ __forceinline__ void batch_tile(const float* __restrict__ Xp, const f
       for (int j = 0; j < CT; ++j) acc[i][j] = make_float2(0.0f, 0.0f);
     float4 ra[T::NA], rb[T::NB];
     // Four coordinates of a row (of X, or of C): zeros past n / k and past d.
-    auto load4 = [&](const float* base, uint32_t row, uint32_t rows, uint32_t col) {
+    auto load4 = [&](const float* base, uint32_t row, uint32_t rows, uint32_t col, auto ld) {
       float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
       if (row < rows) {
         const float* p = base + (uint64_t)row * d + col;
         if (v4) {
-          if (col < d) v = __ldg(reinterpret_cast<const float4*>(p));
+          if (col < d) v = ld(reinterpret_cast<const float4*>(p));
         } else {
-          if (col + 0 < d) v.x = __ldg(p);
-          if (col + 1 < d) v.y = __ldg(p + 1);
-          if (col + 2 < d) v.z = __ldg(p + 2);
-          if (col + 3 < d) v.w = __ldg(p + 3);
+          if (col + 0 < d) v.x = ld(p);
+          if (col + 1 < d) v.y = ld(p + 1);
+          if (col + 2 < d) v.z = ld(p + 2);
+          if (col + 3 < d) v.w = ld(p + 3);
         }
       }
       return v;
     };
+    auto ld_x = [](const auto* p) { return __ldg(p); };
+    auto ld_c = [](const auto* p) { return ld_plain(p); };
     constexpr int QR = T::KC / 4;                          // float4 per row and stage
     auto gload = [&](uint32_t kc) {
 #pragma unroll
       for (int e = 0; e < T::NA; ++e) {
         const uint32_t idx = (uint32_t)(e * BA_NT + tid);
-        ra[e] = load4(Xp, m0 + idx / QR, n, kc + 4u * (idx % QR));
+        ra[e] = load4(Xp, m0 + idx / QR, n, kc + 4u * (idx % QR), ld_x);
       }
 #pragma unroll
       for (int e = 0; e < T::NB; ++e) {
         const uint32_t idx = (uint32_t)(e * BA_NT + tid);
-        if (idx < (uint32_t)(T::COLS * QR)) rb[e] = load4(C, c0 + idx / QR, k, kc + 4u * (idx % QR));
+        if (idx < (uint32_t)(T::COLS * QR)) rb[e] = load4(C, c0 + idx / QR, k, kc + 4u * (idx % QR), ld_c);
       }
     };
     auto sstore = [&](int buf) {
@@ -301,23 +318,37 @@ __device__ __forceinline__ uint32_t batch_owner(const uint32_t* __restrict__ fir
   uint32_t lo = 0, hi = nact;
   while (hi - lo > 1u) {
     const uint32_t mid = (lo + hi) / 2u;
-    if (__ldg(first + mid) <= t) lo = mid; else hi = mid;
+    if (__ldcg(first + mid) <= t) lo = mid; else hi = mid;
   }
   return lo;
 }
 
-// The tiles of one group.  Every group's kernel waits for its predecessor before it
-// reads what the iteration before wrote: only a wait of its own makes that visible to
-// it.  (Groups made resident early cost more than their launches: 64 problems x 4
-// restarts, n 1024..65536, 83.9 ms against 81.6.)
+// The tiles of one group.  The groups' kernels follow one another in the stream and may
+// overlap.  The first waits for the iteration before and then says so (epoch, a release);
+// a later one whose acquire sees that may read what that iteration wrote, and one that
+// does not waits for its predecessor.  Each later one waits for its predecessor before it
+// ends, so that the next kernel's wait covers all of them.  What the iteration before
+// wrote is read by ordinary loads after the acquire, the centroids and tile0 too.
+// Against groups one after the other, each with a wait of its own: 21 problems, n 512 to
+// 19,142, 3.0 / 3.8 ms, 28 x 3 restarts, n 512 to 12,104, 4.2 / 4.9; 64 x 4, n 1024 to
+// 65,536, 82.9 / 79.7.
 template <int RT, int GROUP>
 __global__ void __launch_bounds__(BA_NT, RT == 8 ? 3 : 4)
 batch_assign_kernel(const float* __restrict__ X, const BatchInst* __restrict__ insts, BatchCtl* ctl,
                     const uint32_t* __restrict__ act, const uint32_t* __restrict__ tile0,
                     const float* __restrict__ Call, uint32_t* __restrict__ labels, double* __restrict__ objblk,
-                    float neg0) {
-  griddep_wait();
+                    uint32_t epoch, int first, float neg0) {
   __shared__ uint32_t s_tile;
+  if (first) {
+    griddep_wait();
+    if (blockIdx.x == 0 && threadIdx.x == 0)
+      asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(&ctl->epoch), "r"(epoch) : "memory");
+  } else {
+    if (threadIdx.x == 0) asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(s_tile) : "l"(&ctl->epoch) : "memory");
+    __syncthreads();
+    if (s_tile != epoch) griddep_wait();
+  }
+  griddep_launch();
   const uint32_t nact = ctl->nact, begin = GROUP ? ctl->tile_end[GROUP ? GROUP - 1 : 0] : 0u,
                  end = ctl->tile_end[GROUP];
   for (;;) {
@@ -348,6 +379,7 @@ batch_assign_kernel(const float* __restrict__ X, const BatchInst* __restrict__ i
     }
 #undef KM_BATCH_TILE
   }
+  if (!first) griddep_wait();
 }
 
 // Stable counting sort of an instance's rows by label: each warp counts and then
@@ -604,7 +636,7 @@ batch_begin_kernel(const BatchInst* __restrict__ insts, BatchCtl* ctl, uint32_t*
   __shared__ uint32_t sh[67];
   for (uint32_t i = threadIdx.x; i < ninst; i += blockDim.x) done[i] = 0u;
   batch_list(insts, ctl, act, tile0, nullptr, ninst, rt, sh);
-  if (threadIdx.x == 0) { ctl->iter = 0; ctl->err = 0u; }
+  if (threadIdx.x == 0) { ctl->iter = 0; ctl->err = 0u; ctl->epoch = 0u; }
 }
 
 __global__ void __launch_bounds__(256)
@@ -1062,14 +1094,17 @@ km_status balloc(T** p, size_t count) {
 
 // The launches of one iteration of the running instances.
 template <int RT>
-km_status enqueue_batch_iteration(km_batch* h, int ctas, const BatchInst* dinst, uint32_t ninst, uint64_t maxiter) {
+km_status enqueue_batch_iteration(km_batch* h, int ctas, const BatchInst* dinst, uint32_t ninst, uint64_t maxiter,
+                                  uint32_t epoch) {
   uint32_t *act = h->lists, *tile0 = act + h->inst.size(), *done = tile0 + h->inst.size();
   BatchTask *longs = h->tasks, *shorts = h->tasks + h->task_total;
   const unsigned per_inst = (unsigned)std::min<uint32_t>(ninst, (uint32_t)h->num_sms * 2u);
+  int first = 1;
   auto assign = [&](auto kern, int group) -> km_status {
     if (!(h->groups & (1u << group))) return KM_OK;
     KM_CUDA_TRY(launch_pdl(kern, h->num_sms * ctas, BA_NT, batch_assign_smem<RT>(), h->stream, h->X, dinst, h->ctl, act,
-                           tile0, h->C, h->labels, h->objblk, -0.0f));
+                           tile0, h->C, h->labels, h->objblk, epoch, first, -0.0f));
+    first = 0;
     return KM_OK;
   };
   KM_TRY(assign(batch_assign_kernel<RT, 0>, 0));
@@ -1108,8 +1143,8 @@ km_status enqueue_batch_tiles(km_batch* h, int v, const BatchInst* dinst, uint32
   while (done < maxiter) {
     const uint64_t target = std::min<uint64_t>(maxiter, done + step);
     for (; done < target; ++done)
-      KM_TRY(V.rt == 8 ? enqueue_batch_iteration<8>(h, V.ctas, dinst, ninst, maxiter)
-                       : enqueue_batch_iteration<4>(h, V.ctas, dinst, ninst, maxiter));
+      KM_TRY(V.rt == 8 ? enqueue_batch_iteration<8>(h, V.ctas, dinst, ninst, maxiter, (uint32_t)done + 1u)
+                       : enqueue_batch_iteration<4>(h, V.ctas, dinst, ninst, maxiter, (uint32_t)done + 1u));
     if (done >= maxiter) break;
     KM_CUDA_TRY(cudaMemcpyAsync(h->h_ctl, h->ctl, sizeof(BatchCtl), cudaMemcpyDeviceToHost, h->stream));
     KM_CUDA_TRY(cudaStreamSynchronize(h->stream));

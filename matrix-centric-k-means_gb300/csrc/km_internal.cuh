@@ -106,9 +106,10 @@ enum : uint32_t {
 // completed and its writes are visible).  A kernel that waits before it lets the next
 // one start runs after all of its predecessors, and so does the next one.  In a kernel
 // launched without the attribute both are no-ops.  griddep_launch() is used by the
-// kernel k-means iteration (n = 20,000: 393 -> 381 us); in the Lloyd iteration, seeding
-// and the batched loop the waiting blocks cost as much as the launches they hide, or
-// more (n = 1M: 345 -> 356 us).
+// kernel k-means iteration (n = 20,000: 393 -> 381 us) and between the batched
+// assignment's groups (which say themselves how they come to see earlier writes without
+// the wait); in the Lloyd iteration, seeding and the rest of the batched loop the waiting
+// blocks cost as much as the launches they hide, or more (n = 1M: 345 -> 356 us).
 __device__ __forceinline__ void griddep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
 // Lets the next kernel of the stream (launched with launch_pdl) start as this
