@@ -1832,10 +1832,12 @@ km_status update_sums_prepare() {
 // (row stride d floats from X): 16 bytes, else 8, else 4.  Many clusters of few rows go to
 // a warp each, and the ring takes those above: at most n / SUMS_WARP_ROWS of them, which
 // order lists first.  The ring takes two clusters' column blocks an SM at a time, of 2 us and
-// more each, so it loses as soon as there are more than three rounds of them.  Ring / a warp
-// each: 16-byte rows, n = 160,000 d = 256 k = 20,000 1191 / 191 us, n = 63,500 d = 16 k = 500
+// more each, so it loses as soon as there are more than three waves of them; narrower
+// copies cost it more, so that it loses earlier there.  Ring / a warp each: 16-byte rows, n = 160,000 d = 256 k = 20,000 1191 / 191 us, n = 63,500 d = 16 k = 500
 // 12 / 17, n = 400,000 d = 64 k = 2000 (200 a cluster) 60 / 65; 4-byte rows, n = 4M d = 7
-// k = 20,000 441 / 166, n = 200,000 d = 7 k = 1000 30 / 21, n = 3000 d = 7 k = 100 12 / 10.
+// k = 20,000 441 / 166, n = 200,000 d = 7 k = 1000 30 / 21, n = 15,000 d = 7 k = 500 16.8 / 10.0, n = 38,100 d = 50
+// k = 300 14.6 / 18.2, n = 3000 d = 7 k = 100 12 / 10, n = 6000 d = 50 k = 100 10.1 / 12.2; 8-byte ones, n = 200,000
+// d = 50 k = 500 26.9 / 35.5, n = 200,000 d = 50 k = 4000 94 / 30.
 km_status launch_update_sums(const float* X, const uint32_t* perm, const uint32_t* cstart, uint64_t n, uint32_t d,
                              uint32_t k, const float* C, float* Cn, float* dsq, double* objpart,
                              DevState* st, cudaStream_t s, const uint32_t* order) {
@@ -1843,8 +1845,11 @@ km_status launch_update_sums(const float* X, const uint32_t* perm, const uint32_
   const int vec = (d % 4 == 0 && xa % 16 == 0) ? 4 : (d % 2 == 0 && xa % 8 == 0) ? 2 : 1;
   auto kern = vec == 4 ? update_sums_bulk_kernel<4> : vec == 2 ? update_sums_bulk_kernel<2> : update_sums_bulk_kernel<1>;
   const uint32_t nblk = (d + BLK_COLS - 1) / BLK_COLS;
-  const bool many = (uint64_t)k * nblk >= 1000u;
-  const bool few = order && (vec == 4 ? many && n < (uint64_t)k * 128u : n < (uint64_t)k * (many ? 1024u : 128u));
+  const uint64_t blocks = (uint64_t)k * nblk;
+  const uint64_t rows = vec == 4 ? (blocks >= 1000u ? 128u : 0u)
+                        : blocks >= (vec == 2 ? 2000u : 1000u) ? 1024u
+                        : blocks >= 1000u ? 128u : blocks >= 256u ? 64u : 32u;
+  const bool few = order && n < k * rows;
   const uint32_t limit = !few ? 0u : vec == 4 ? SUMS_WARP_ROWS : 4u * SUMS_WARP_ROWS;
   if (few) {
     auto small = vec == 4 ? update_sums_warp_kernel<4> : vec == 2 ? update_sums_warp_kernel<2> : update_sums_warp_kernel<1>;

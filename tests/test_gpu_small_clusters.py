@@ -66,3 +66,17 @@ def test_noalloc_update_with_small_and_large_clusters(km, gpu, k, d):
     cen_o, _ = helpers.orc_update(X, lab, k)
     np.testing.assert_array_equal(C.cpu().numpy().view(np.uint32), cen_o.view(np.uint32))
     np.testing.assert_array_equal(cnt.cpu().numpy().astype(np.uint32), np.bincount(lab, minlength=k))
+
+
+@pytest.mark.parametrize("d", [1, 3, 6, 33, 50])
+@pytest.mark.parametrize("k,rows", [(5, 31), (60, 20), (127, 31), (127, 33), (256, 63), (256, 65), (500, 60)])
+def test_update_of_few_small_clusters(km, gpu, k, rows, d):
+    import torch
+    rng = np.random.default_rng(k * rows + d)
+    n = k * rows
+    lab = rng.integers(0, k, n).astype(np.uint32)
+    X = rng.standard_normal((n, d)).astype(np.float32)
+    cen_o, _ = helpers.orc_update(X, lab, k)
+    C, cnt, _, _ = km.update(torch.from_numpy(X).to(gpu), torch.from_numpy(lab.astype(np.int32)).to(gpu), k)
+    np.testing.assert_array_equal(C.cpu().numpy().view(np.uint32), cen_o.view(np.uint32))
+    np.testing.assert_array_equal(cnt.cpu().numpy().astype(np.uint32), np.bincount(lab, minlength=k))
